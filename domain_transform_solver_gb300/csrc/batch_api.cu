@@ -732,17 +732,15 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
   if (!st) st = dalloc(&b->d_soff, (size_t)n);
   if (!st) st = dalloc(&b->d_uptr, (size_t)3 * n);
   if (!st) {
-    e = cudaMemcpy(b->d_inst, b->inst.data(), n * sizeof(Inst), cudaMemcpyHostToDevice);
+    e = upload_table(b->d_inst, b->inst.data(), n * sizeof(Inst));
     if (e == cudaSuccess)
-      e = cudaMemcpy(b->d_soff, b->soff.data(), n * sizeof(long long), cudaMemcpyHostToDevice);
+      e = upload_table(b->d_soff, b->soff.data(), n * sizeof(long long));
     if (e == cudaSuccess)
-      e = cudaMemcpy(b->d_tb, tb.data(), tb.size() * sizeof(Tile), cudaMemcpyHostToDevice);
+      e = upload_table(b->d_tb, tb.data(), tb.size() * sizeof(Tile));
     if (e == cudaSuccess)
-      e = cudaMemcpy(b->d_ti_big, ti.data(), ti.size() * sizeof(Tile),
-                     cudaMemcpyHostToDevice);
+      e = upload_table(b->d_ti_big, ti.data(), ti.size() * sizeof(Tile));
     if (e == cudaSuccess)
-      e = cudaMemcpy(b->d_ti_small, ts.data(), ts.size() * sizeof(Tile),
-                     cudaMemcpyHostToDevice);
+      e = upload_table(b->d_ti_small, ts.data(), ts.size() * sizeof(Tile));
     if (e != cudaSuccess) st = cuda_fail(e, "batch tables");
   }
   select_tiles(b, b->small);

@@ -1524,8 +1524,7 @@ DTSGB_API int dtsgb_soft_create(int n, const int* widths, const int* heights,
   int st = dalloc(&s->d_inst, (size_t)n);
   if (!st) st = dalloc(&s->d_emin, 1);
   if (!st) st = dalloc(&s->d_stat, 2);
-  if (!st && cudaMemcpy(s->d_inst, s->inst.data(), n * sizeof(SInst),
-                        cudaMemcpyHostToDevice) != cudaSuccess)
+  if (!st && upload_table(s->d_inst, s->inst.data(), n * sizeof(SInst)) != cudaSuccess)
     st = fail(DTSGB_ERR_CUDA, "instance table upload");
   if (!st && cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess)
     st = fail(DTSGB_ERR_CUDA, "stream creation");

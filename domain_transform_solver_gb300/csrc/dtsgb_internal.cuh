@@ -146,6 +146,14 @@ int dalloc(T** p, size_t count) {
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemset");
   return 0;
 }
+// Host table -> device, complete on return: cudaMemcpy from pageable memory
+// may return while the transfer still runs on the legacy default stream,
+// which the handles' non-blocking streams do not wait for, and a kernel on
+// one of them would then read the table (a tensor map, say) half written.
+inline cudaError_t upload_table(void* dst, const void* src, size_t bytes) {
+  cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(0) : e;
+}
 template <typename T>
 void dfree(T*& p) {
   if (p) cudaFree((void*)p);

@@ -80,8 +80,7 @@ const CUtensorMap* TmaCache::upload(const std::vector<CUtensorMap>& maps,
     (void)cudaGetLastError();
     return nullptr;
   }
-  if (cudaMemcpy(d, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice) !=
-      cudaSuccess) {
+  if (upload_table(d, maps.data(), sizeof(CUtensorMap) * maps.size()) != cudaSuccess) {
     (void)cudaGetLastError();
     cudaFree(d);
     return nullptr;
