@@ -8,14 +8,14 @@
 // reference's buffers (see hfbs_internal.cuh / the oracle): index -1 reads 0
 // (zero boundary mode), index g reads the pad value of that buffer.
 //
-// The splat is atomic-free and deterministic: one thread per spatial cell
-// walks the cell's pixels in row-major order and bins them into per-thread
-// luma histograms held in shared memory.
+// The splat is atomic-free and deterministic: the threads of a spatial cell
+// bin its pixels into per-thread luma histograms held in shared memory.
 #include <algorithm>
 #include <vector>
 
 #include "../../include/dtsgb.h"
 #include "dtsgb_internal.cuh"
+#include "fixed_point.cuh"
 #include "hfbs_internal.cuh"
 #include "tma.cuh"
 
@@ -118,6 +118,164 @@ __global__ void __launch_bounds__(64)
       count[gi] = hist[(3 * z + 2) * T + threadIdx.x];
     }
     ovf[I.plane_off + cell] = I.ovf_stored ? ovf_cnt : 0.f;
+  }
+}
+
+// a12 for large cells: a CTA per cell, bit for bit k_splat's sums.  Those
+// are sums in row-major order of the cell's runs (neighbours in one luma
+// bin), each run summed in order first, so the work a thread of k_splat
+// does alone splits into parallel parts that keep every addition: the
+// pixels of a chunk are loaded together into shared memory, run starts are
+// found and compacted by a block scan, runs are summed by a thread each, and
+// a thread per luma bin adds the runs of its bin in order.  The run that a
+// chunk ends in stays open into the next one.  From kSplatCellPx pixels a
+// cell on: one thread a cell took 850 us for the 374 cells of 64 x 64
+// pixels of a 1376x1088 image (latency of one batch of loads after the
+// other, 6 CTAs); at 8 x 8 pixels the thread per cell is the faster one.
+constexpr int kSplatCellPx = 256;
+constexpr int kSplatChunk = 1024, kSplatCellT = 256, kSplatPer = kSplatChunk / kSplatCellT;
+
+template <typename TS>
+__global__ void __launch_bounds__(kSplatCellT)
+    k_splat_cell(const HInst* __restrict__ insts, const uchar4* __restrict__ guide,
+                 const TS* __restrict__ tgt, const TS* __restrict__ cnf,
+                 float* __restrict__ count, float* __restrict__ csum, float* __restrict__ b,
+                 float* __restrict__ ovf, HParams p) {
+  constexpr int T = kSplatCellT, NW = T / 32;
+  __shared__ int lbin[256];                      // luma bin of each 8-bit luma value
+  __shared__ short sbin[kSplatChunk];            // the chunk's pixels: bin, c, c*t
+  __shared__ float sc[kSplatChunk], sct[kSplatChunk];
+  __shared__ short rs[kSplatChunk], rb[kSplatChunk];  // its runs: start, bin, sums
+  __shared__ float rct[kSplatChunk], rc[kSplatChunk], rn[kSplatChunk];
+  __shared__ int wsum[NW];
+  __shared__ int o_bin;                          // the open run (-1: none)
+  __shared__ float o_ct, o_c, o_n;
+  const HInst I = insts[blockIdx.y];
+  const int cell = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (cell >= I.gx * I.gy) return;
+  const int gl = I.gl;
+  if (tid < 256) lbin[tid] = (int)floorf((float)tid * 1.0f / p.sigma_l);
+  if (tid == 0) o_bin = -1;
+  const int bx = cell % I.gx, by = cell / I.gx;
+  const int xs = cell_start(bx, p.sigma_x, I.w), xe = cell_start(bx + 1, p.sigma_x, I.w);
+  const int ys = cell_start(by, p.sigma_y, I.h), ye = cell_start(by + 1, p.sigma_y, I.h);
+  const int nx = xe - xs, total = nx * (ye - ys);
+  float h_ct = 0.f, h_c = 0.f, h_n = 0.f;  // bin tid's sums
+  __syncthreads();
+  for (int base = 0; base < total; base += kSplatChunk) {
+    const int n = min(kSplatChunk, total - base);
+    unsigned char lum[kSplatPer];
+    float cv[kSplatPer], tv[kSplatPer];
+#pragma unroll
+    for (int j = 0; j < kSplatPer; ++j) {
+      const int i = min(tid + j * T, n - 1) + base;
+      const int y = i / nx, x = i - y * nx;
+      const long long g = I.pix_off + (long long)(ys + y) * I.pitch + xs + x;
+      lum[j] = guide[g].x;
+      cv[j] = load_f(cnf + g);
+      tv[j] = load_f(tgt + g);
+    }
+#pragma unroll
+    for (int j = 0; j < kSplatPer; ++j) {
+      const int i = tid + j * T;
+      if (i < n) {
+        sbin[i] = (short)lbin[lum[j]];
+        sc[i] = cv[j];
+        sct[i] = __fmul_rn(cv[j], tv[j]);
+      }
+    }
+    __syncthreads();
+    // run starts among this thread's kSplatPer neighbours, compacted in order
+    const int open = o_bin, i0 = tid * kSplatPer;
+    int prev = i0 == 0 ? open : (i0 <= n ? sbin[i0 - 1] : 0), starts = 0, k = 0;
+#pragma unroll
+    for (int j = 0; j < kSplatPer; ++j) {
+      if (i0 + j < n) {
+        const int c = sbin[i0 + j];
+        if (c != prev) starts |= 1 << j;
+        prev = c;
+      }
+    }
+    const int mine = __popc(starts);
+    const int incl = (int)warp_incl_scan((unsigned)mine, lane);
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    int R = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      if (w < warp) k += wsum[w];
+      R += wsum[w];
+    }
+    k += incl - mine;
+#pragma unroll
+    for (int j = 0; j < kSplatPer; ++j)
+      if (starts >> j & 1) rs[k++] = (short)(i0 + j);
+    __syncthreads();
+    // a thread per run; the last thread extends the open run to the first start
+    for (int r = tid; r < R; r += T) {
+      const int a = rs[r], e = r + 1 < R ? rs[r + 1] : n;
+      float u = sct[a], v = sc[a], m = 1.f;
+      for (int i = a + 1; i < e; ++i) {
+        u += sct[i];
+        v += sc[i];
+        m += 1.f;
+      }
+      rb[r] = sbin[a];
+      rct[r] = u;
+      rc[r] = v;
+      rn[r] = m;
+    }
+    if (tid == T - 1 && open >= 0) {
+      const int e = R > 0 ? rs[0] : n;
+      float u = o_ct, v = o_c, m = o_n;
+      for (int i = 0; i < e; ++i) {
+        u += sct[i];
+        v += sc[i];
+        m += 1.f;
+      }
+      o_ct = u;
+      o_c = v;
+      o_n = m;
+    }
+    __syncthreads();
+    // a thread per bin (bin gl: the overflow count) adds its closed runs
+    if (R > 0) {
+      if (tid <= gl) {
+        if (open == tid) {
+          h_ct += o_ct;
+          h_c += o_c;
+          h_n += o_n;
+        }
+#pragma unroll 4
+        for (int r = 0; r + 1 < R; ++r)
+          if (rb[r] == tid) {
+            h_ct += rct[r];
+            h_c += rc[r];
+            h_n += rn[r];
+          }
+      }
+      __syncthreads();
+      if (tid == 0) {
+        o_bin = rb[R - 1];
+        o_ct = rct[R - 1];
+        o_c = rc[R - 1];
+        o_n = rn[R - 1];
+      }
+    }
+    __syncthreads();
+  }
+  if (tid <= gl && o_bin == tid) {
+    h_ct += o_ct;
+    h_c += o_c;
+    h_n += o_n;
+  }
+  if (tid < gl) {
+    const long long gi = gidx(I, bx, by, tid);
+    b[gi] = h_ct;
+    csum[gi] = h_c;
+    count[gi] = h_n;
+  } else if (tid == gl) {
+    ovf[I.plane_off + cell] = I.ovf_stored ? h_n : 0.f;
   }
 }
 
@@ -1109,8 +1267,20 @@ int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s) {
   const dim3 gp((unsigned)std::min<long long>((max_h + 7) / 8, 4096), ni);
   const dim3 gc((B.max_cells + 63) / 64, ni);
   const size_t splat_smem = sizeof(float) * 3 * (size_t)B.max_gl * 64;
+  // a CTA per cell for large ones (k_splat_cell holds a bin per thread)
+  const bool by_cell = (double)p.sigma_x * (double)p.sigma_y >= kSplatCellPx &&
+                       B.max_gl < kSplatCellT;
+  const dim3 gcell((unsigned)B.max_cells, ni);
   prof_begin(s, DTSGB_K_HFBS_SPLAT);
-  if (B.st == Storage::F32) {
+  if (by_cell && B.st == Storage::F32) {
+    k_splat_cell<float><<<gcell, kSplatCellT, 0, s>>>(
+        B.d_inst, B.guide, (const float*)B.target, (const float*)B.conf, B.count, B.csum, B.b,
+        B.ovf, p);
+  } else if (by_cell) {
+    k_splat_cell<__nv_bfloat16><<<gcell, kSplatCellT, 0, s>>>(
+        B.d_inst, B.guide, (const __nv_bfloat16*)B.target, (const __nv_bfloat16*)B.conf,
+        B.count, B.csum, B.b, B.ovf, p);
+  } else if (B.st == Storage::F32) {
     if (splat_smem + sizeof(int) * 256 > 48 * 1024)  // plus the static luma table
       DTSGB_CUDA(cudaFuncSetAttribute(k_splat<float>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
