@@ -881,16 +881,18 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
                                       p->num_iterations, b->v[0], b->v[1], &res,
                                       b->stream);
     }
-    int st = launch_init_var(Li, b->st, b->target, b->v[0], b->stream);
-    if (st || !iterate) return st;
+    if (!iterate) return launch_init_var(Li, b->st, b->target, b->v[0], b->stream);
+    const float* cur = nullptr;
+    int st = first_iterate(Li, b->st, b->target, b->v[0], &cur, b->stream);
+    if (st) return st;
     st = bounds();
     if (st) return st;
     const IterMode mode = p->loss == DTSGB_L2 ? IterMode::L2 : IterMode::CHARB;
     int a = 0;
     for (int it = 0; it < p->num_iterations; ++it) {
-      st = launch_dts_iter(Li, b->st, mode, b->v[a], b->v[1 - a], b->target,
+      st = launch_dts_iter(Li, b->st, mode, cur, b->v[1 - a], b->target,
                            b->conf, b->bounds, p->lambda, p->step_size, overwrite,
-                           halo, halo, b->stream);
+                           it + 1 < p->num_iterations, halo, halo, b->stream);
       if (st) return st;
       a = 1 - a;
     }
@@ -967,6 +969,9 @@ static int batch_backward(dtsgb_batch_t b, const float* const* grad_out,
   DtsGrad G = grad_view(b, n_iter);
   if (up == cudaMemcpyHostToDevice) {
     if (int st = host_upload_plane(b, grad_out, G.g[0], 0)) return st;
+      if (b->st == Storage::F32)  // the first iteration reads the target
+        (void)b->tma.get(b->inst.data(), b->n, (const float*)b->target, bw, bh, b->stream);
+    }
   } else {
     if (int st = user_plane_copy(b, const_cast<float* const*>(grad_out), G.g[0], true, 0))
       return st;
@@ -1020,6 +1025,7 @@ DTSGB_API int dtsgb_batch_dts_backward_device(dtsgb_batch_t b,
                                               const float* const* grad_out,
                                               float* const* grad_target,
                                               float* const* grad_confidence) {
+      cur = b->v[a];
   return batch_backward(b, grad_out, grad_target, grad_confidence,
                         cudaMemcpyDeviceToDevice, cudaMemcpyDeviceToDevice);
 }

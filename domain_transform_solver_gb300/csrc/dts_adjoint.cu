@@ -432,17 +432,21 @@ int dts_forward_checkpointed(const DtsLaunch& L, Storage st, IterMode mode,
                              const uint32_t* bounds, float lambda, float step, int halo,
                              int num_iterations, float* v0, float* v1, int* result_idx,
                              cudaStream_t s) {
-  int st_ = launch_init_var(L, st, target, v0, s);
-  if (st_) return st_;
+  if (num_iterations <= 0) {
+    *result_idx = 0;
+    return launch_init_var(L, st, target, v0, s);
+  }
   float* buf[2] = {v0, v1};
-  const float* cur = v0;
+  const float* cur = nullptr;
+  int st_ = first_iterate(L, st, target, v0, &cur, s);
+  if (st_) return st_;
   int ci = 0;
   for (int it = 0; it < num_iterations; ++it) {
     const int next = it + 1;
     const int di = forward_dst(ci, next, num_iterations, G.seg);
     float* dst = di < 0 ? G.cp[next / G.seg - 1] : buf[di];
     st_ = launch_dts_iter(L, st, mode, cur, dst, target, conf, bounds, lambda, step, -1.f,
-                          halo, halo, s);
+                          0, halo, halo, s);
     if (st_) return st_;
     cur = dst;
     ci = di;
@@ -474,14 +478,15 @@ int dts_backward(const DtsLaunch& L, const Inst* d_inst, int n_inst, long long p
     const int len = std::min(G.seg, num_iterations - start);
     // X-step inputs v_start .. v_start+len-1 of this segment: the first is
     // t (segment 0) or a checkpoint, the others are recomputed into segbuf
-    const float* x0 = j == 0 ? G.segbuf[0] : G.cp[j - 1];
-    if (j == 0) {
-      int st_ = launch_init_var(L, st, target, G.segbuf[0], s);
-      if (st_) return st_;
+    const float* x0 = nullptr;
+    if (j > 0) {
+      x0 = G.cp[j - 1];
+    } else if (int st_ = first_iterate(L, st, target, G.segbuf[0], &x0, s)) {
+      return st_;
     }
     for (int k = 1; k < len; ++k) {
       int st_ = launch_dts_iter(L, st, mode, k == 1 ? x0 : G.segbuf[k - 1], G.segbuf[k],
-                                target, conf, bounds, lambda, step, -1.f, halo, halo, s);
+                                target, conf, bounds, lambda, step, -1.f, 0, halo, halo, s);
       if (st_) return st_;
     }
     for (int k = len - 1; k >= 0; --k) {

@@ -210,7 +210,13 @@ __global__ void __launch_bounds__(kThreads)
 //   Y: v' = v - s*lambda*(v - B_y)
 // (src/domain_transform_solver.cuh:12-116).  With overwrite in (0,1), the
 // target replaces v where c > overwrite before each half-step
-// (src/domain_transform_solver.cu:126-130, 160-164).
+// (src/domain_transform_solver.cu:126-130, 160-164).  Before Y that is the X
+// result of this kernel; before X it is the previous iteration's output, so
+// an iteration that feeds another one (`feeds`) stores the target there
+// itself: the X phase already holds it as that pixel's X result and marks
+// the pixel by Y bounds of 0 (a window always holds its own pixel).  The
+// first iterate is the target everywhere.  A separate pass over v before
+// every iteration read c and v again: 107 of 240 us an iteration at 8 Mpx.
 // ---------------------------------------------------------------------------
 
 // X half-step update of one pixel (src/domain_transform_solver.cuh:37-86);
@@ -253,19 +259,6 @@ __device__ __forceinline__ float photometric(const StereoArgs& sa, long long row
     gr = edge_weight(b, xi > 0 ? sa.right[row + xi - 1] : make_uchar4(0, 0, 0, 0),
                      sa.ratio);
   return sa.lam_p * 2.f * sad * (__fmaf_rn(gr, gr, -1.f) * sa.alpha);
-}
-
-// v = t where c > overwrite, in place (DomainTransformSolver::Optimize's
-// overwrite before the X half-step, src/domain_transform_solver.cu:126-130).
-template <typename TS>
-__global__ void k_overwrite(const Inst* __restrict__ insts, float* __restrict__ v,
-                            const TS* __restrict__ tgt, const TS* __restrict__ cnf,
-                            float overwrite) {
-  const Inst in = insts[blockIdx.y];
-  const long long n = (long long)in.pitch * in.h;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    if (load_f(cnf + in.off + i) > overwrite) v[in.off + i] = load_f(tgt + in.off + i);
 }
 
 // ---------------------------------------------------------------------------
@@ -364,13 +357,14 @@ __device__ __forceinline__ unsigned u4_get(const uint4& v, int k) {
   return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w;
 }
 
-template <typename TS, int MODE, int TW, int TH, int NT, bool STEREO = false>
+template <typename TS, int MODE, int TW, int TH, int NT, bool STEREO, bool OVER>
 __global__ void __launch_bounds__(NT, 1024 / NT)
     k_dts_iter_vec(const Inst* __restrict__ insts, const Tile* __restrict__ tiles,
                    const float* __restrict__ vin, float* __restrict__ vout,
                    const TS* __restrict__ tgt, const TS* __restrict__ cnf,
                    const uint32_t* __restrict__ bnd, float lambda, float step,
-                   float overwrite, int hx, int hy, StereoArgs sa, VecIterSmem<TW, TH, NT> L,
+                   float overwrite, int feeds, int hx, int hy, StereoArgs sa,
+                   VecIterSmem<TW, TH, NT> L,
                    const CUtensorMap* __restrict__ tmaps) {
   constexpr int QW = TW / 4, TQ = TW + 4, RPP = NT / QW, NW = NT / 32;
   static_assert(TW % 32 == 0 && NT % TW == 0 && NW >= QW, "tile shape");
@@ -398,8 +392,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
   const int nrt = 2 * max(hx, hy) + 2;
   for (int i = tid; i < nrt; i += NT) rtx[i].x = i ? __frcp_rn((float)i) : 0.f;
   if (tid < 2) smax[tid] = 0u;
-  const bool over = overwrite > 0.f && overwrite < 1.f;  // v itself is already
-                                                          // overwritten
+  // OVER: overwrite lies in (0, 1); v itself is already overwritten, and hold
+  // keeps the target in the output too.  (A run-time test instead cost the
+  // solves without overwrite 2%.)
+  const bool hold = OVER && feeds;
   const int xs = t.x0 - HA;   // image x of staged column 0
   const int gy0 = t.y0 - hy;  // image y of row 0
   // TMA staging: the box is SWS x SR (its row stride in shared memory is
@@ -457,9 +453,12 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
     const int jmax = min(TH, H - t.y0);
     for (int j = r3; j < jmax; j += RPP) {
       float* dst = vout_i + (t.y0 + j) * P + x3;
+      const int p = (t.y0 + j) * P + x3;
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        if (x3 + k < W) dst[k] = __int_as_float(0x7fc00000);
+        if (x3 + k < W)
+          dst[k] = hold && load_f(cnf_i + p + k) > overwrite ? load_f(tgt_i + p + k)
+                                                             : __int_as_float(0x7fc00000);
     }
   };
   // ---- 1. stage the iterate, four columns per item, four items in flight -------
@@ -572,10 +571,12 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
     auto compute = [&](int r, const Quad& Q) {
       const unsigned* e0 = XP + r * SWS + HA + 4 * cq;  // e0[k]: prefix at x3 + k
       float o[4];
+      unsigned by[4];  // Y bounds; 0: the pixel holds the target
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         o[k] = 0.f;
         const uint32_t b = u4_get(Q.b, k);
+        by[k] = b >> 16;
         if (b) {  // inside the image (a window always holds its own pixel)
           const int dl = min((int)(b & 0xff), hx + 1);
           const int du = min((int)((b >> 8) & 0xff), hx);
@@ -587,14 +588,17 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
           if (STEREO)
             extra = photometric(sa, in.off + (long long)(gy0 + r) * P, x3 + k, W, vv);
           o[k] = x_update<MODE, STEREO>(vv, B, tv, cv, rn, lambda, step, extra);
-          if (over && cv > overwrite) o[k] = tv;
+          if (OVER && cv > overwrite) {
+            o[k] = tv;
+            if (hold) by[k] = 0u;
+          }
         }
         mloc = max(mloc, mag_bits(o[k]));
       }
       *reinterpret_cast<float4*>(sx + r * TQ + 4 * cq) = make_float4(o[0], o[1], o[2], o[3]);
       // the Y bytes (b >> 16) of the four pixels as four u16
       *reinterpret_cast<uint2*>(sby + r * TW + 4 * cq) =
-          make_uint2((Q.b.x >> 16) | (Q.b.y & 0xffff0000u), (Q.b.z >> 16) | (Q.b.w & 0xffff0000u));
+          make_uint2(by[0] | by[1] << 16, by[2] | by[3] << 16);
     };
     int r = r3;
     while (r < SR) {
@@ -665,7 +669,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
       const int dl = min((int)(b & 0xff), hy + 1), du = min((int)(b >> 8), hy);
       const float Bv = fx_window(c0[du * TQ + k], c0[-dl * TQ + k], rsy[dl + du]);
       const float v = f4_get(v4, k);
-      o[k] = __fmaf_rn(-slam, v - Bv, v);
+      o[k] = hold && b == 0u ? v : __fmaf_rn(-slam, v - Bv, v);
     }
     float* dst = vout_i + (t.y0 + j) * P + x3;
     if (x3 + 4 <= W) {
@@ -714,7 +718,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
                       const float* __restrict__ vin, float* __restrict__ vout,
                       const TS* __restrict__ tgt, const TS* __restrict__ cnf,
                       const uint32_t* __restrict__ bnd, float lambda, float step,
-                      float overwrite, int hx, int hy, StereoArgs sa) {
+                      float overwrite, int feeds, int hx, int hy, StereoArgs sa) {
   static_assert(TW % 32 == 0 && NT % TW == 0, "tile width: whole warps");
   constexpr int NW = NT / 32, NSEG = NT / TW, TWp = TW + 1;
   extern __shared__ __align__(128) unsigned char smraw[];
@@ -735,7 +739,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
   for (int i = tid; i < nrt; i += NT) rtab[i] = i ? __frcp_rn((float)i) : 0.f;
   if (tid == 0) *smax = 0u;
   __syncthreads();
-  const bool over = overwrite > 0.f && overwrite < 1.f;
+  const bool over = overwrite > 0.f && overwrite < 1.f;  // v is overwritten already
+  const bool hold = over && feeds;
   const int gx0 = t.x0 - hx - 1;  // image x of X prefix entry 0 (a zero entry)
   const int gy0 = t.y0 - hy;      // image y of sx row 0
   const int lgx = ceil_log2(2 * hx + 1), lgy = ceil_log2(2 * hy + 1);
@@ -749,9 +754,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
   auto load_v = [&](bool yok, long long row, int cc) -> float {  // prefix entry cc
     const int x = gx0 + cc;
     if (cc < 1 || cc >= SWX || !yok || (unsigned)x >= (unsigned)W) return 0.f;
-    float v = __ldg(vin + row + x);
-    if (over && load_f(cnf + row + x) > overwrite) v = load_f(tgt + row + x);
-    return v;
+    return __ldg(vin + row + x);
   };
   auto fetch = [&](int r, RowIn& R) {
     const int y = gy0 + r;
@@ -818,8 +821,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
       if (yok && x < W) {
         const uint32_t b = cur.b[k];
         const float tv = cur.tv[k], cv = cur.cv[k];
-        float v = cur.vc[k];
-        if (over && cv > overwrite) v = tv;
+        const float v = cur.vc[k];
         const int dl = min((int)(b & 0xff), hx + 1);
         const int du = min((int)((b >> 8) & 0xff), hx);
         const float rn = rtab[dl + du];
@@ -828,9 +830,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
         float extra = 0.f;
         if (STEREO) extra = photometric(sa, row, x, W, v);
         o = x_update<MODE, STEREO>(v, B, tv, cv, rn, lambda, step, extra);
-        if (over && cv > overwrite) o = tv;
+        const bool fixed = over && cv > overwrite;
+        if (fixed) o = tv;
         if (row_bad) o = __int_as_float(0x7fc00000);
-        if (r >= hy && r < hy + TH) sby[(r - hy) * TW + c] = (uint16_t)(b >> 16);
+        if (r >= hy && r < hy + TH)
+          sby[(r - hy) * TW + c] = hold && fixed ? (uint16_t)0 : (uint16_t)(b >> 16);
       }
       sx[r * TWp + c] = o;
       mloc = max(mloc, mag_bits(o));
@@ -846,8 +850,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
     // (every pixel of it can reach that value), never finite garbage
     const int x = t.x0 + tid % TW;
     for (int j = tid / TW; j < TH; j += NT / TW)
-      if (t.y0 + j < H && x < W)
-        vout[in.off + (long long)(t.y0 + j) * P + x] = __int_as_float(0x7fc00000);
+      if (t.y0 + j < H && x < W) {
+        const long long p = in.off + (long long)(t.y0 + j) * P + x;
+        vout[p] = hold && load_f(cnf + p) > overwrite ? load_f(tgt + p)
+                                                      : __int_as_float(0x7fc00000);
+      }
     return;
   }
   // ---- Y half-step ----------------------------------------------------------
@@ -878,7 +885,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
     const float B = fx_window(Py[(k + du) * TW + c], Py[(k - dl) * TW + c],
                               rtab[dl + du] * isFy);
     const float v = sx[(j + hy) * TWp + c];
-    vout[in.off + (long long)y * P + x] = __fmaf_rn(-slam, v - B, v);
+    vout[in.off + (long long)y * P + x] = hold && b == 0u ? v : __fmaf_rn(-slam, v - B, v);
   }
 }
 
@@ -978,17 +985,22 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// Storage plane -> float plane (and its square): four elements per thread and
+// 16-byte accesses (rows are pitched to 32 elements, so an instance is a
+// whole number of aligned groups).
 template <typename TS>
-__global__ void k_to_float(const Inst* __restrict__ insts, int n_inst,
-                           const TS* __restrict__ src, float* __restrict__ dst,
-                           float* __restrict__ dst_sq) {
+__global__ void k_to_float(const Inst* __restrict__ insts, const TS* __restrict__ src,
+                           float* __restrict__ dst, float* __restrict__ dst_sq) {
   const Inst in = insts[blockIdx.y];
   const long long n = (long long)in.pitch * in.h;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const float v = load_f(src + in.off + i);
-    dst[in.off + i] = v;
-    if (dst_sq) dst_sq[in.off + i] = v * v;
+  for (long long i = 4 * (blockIdx.x * (long long)blockDim.x + threadIdx.x); i < n;
+       i += 4 * (long long)gridDim.x * blockDim.x) {
+    Raw4<TS> v;
+    v.load(src + in.off + i);
+    *reinterpret_cast<float4*>(dst + in.off + i) = make_float4(v[0], v[1], v[2], v[3]);
+    if (dst_sq)
+      *reinterpret_cast<float4*>(dst_sq + in.off + i) =
+          make_float4(v[0] * v[0], v[1] * v[1], v[2] * v[2], v[3] * v[3]);
   }
 }
 
@@ -1141,7 +1153,7 @@ template <typename TS, int MODE, int TW, int TH, bool STEREO>
 static int launch_iter_shape(const DtsLaunch& L, const float* vin, float* vout,
                              const void* target, const void* conf,
                              const uint32_t* bounds, float lambda, float step,
-                             float overwrite, int hx, int hy, cudaStream_t s,
+                             float overwrite, int feeds, int hx, int hy, cudaStream_t s,
                              const StereoArgs& sa) {
   constexpr int NT = TW >= 64 ? 512 : 256;
   const VecIterSmem<TW, TH, NT> lay(hx, hy);
@@ -1149,23 +1161,20 @@ static int launch_iter_shape(const DtsLaunch& L, const float* vin, float* vout,
   const size_t smem_rows = PrefixIterSmem<TW, TH, NT>::bytes(hx, hy);
   if (smem > kMaxSmem && smem_rows > kMaxSmem)
     return fail(DTSGB_ERR_UNSUPPORTED, "sigma_z too large");
-  if (overwrite > 0.f && overwrite < 1.f) {
-    // the input iterate is overwritten in place, as the reference does
-    k_overwrite<TS><<<dim3(64, L.n_inst), kThreads, 0, s>>>(
-        L.d_inst, const_cast<float*>(vin), (const TS*)target, (const TS*)conf, overwrite);
-    DTSGB_CUDA(cudaGetLastError());
-  }
   if (smem > kMaxSmem) {  // halo too large for the tile-staged kernel
     int st = set_smem(k_dts_iter_rows<TS, MODE, TW, TH, NT, STEREO>, smem_rows);
     if (st) return st;
     ProfScope ps(s, DTSGB_K_DTS_ITER);
     k_dts_iter_rows<TS, MODE, TW, TH, NT, STEREO><<<L.n_tiles, NT, smem_rows, s>>>(
         L.d_inst, L.d_tiles, vin, vout, (const TS*)target, (const TS*)conf,
-        bounds, lambda, step, overwrite, hx, hy, sa);
+        bounds, lambda, step, overwrite, feeds, hx, hy, sa);
     DTSGB_CUDA(cudaGetLastError());
     return DTSGB_OK;
   }
-  int st = set_smem(k_dts_iter_vec<TS, MODE, TW, TH, NT, STEREO>, smem);
+  const bool over = overwrite > 0.f && overwrite < 1.f;
+  auto kern = over ? k_dts_iter_vec<TS, MODE, TW, TH, NT, STEREO, true>
+                   : k_dts_iter_vec<TS, MODE, TW, TH, NT, STEREO, false>;
+  int st = set_smem(kern, smem);
   if (st) return st;
   // TMA staging of the iterate box (SWS x SR, both within the 256-element
   // box limit) from the owner's tensor-map cache, when it has one
@@ -1173,10 +1182,9 @@ static int launch_iter_shape(const DtsLaunch& L, const float* vin, float* vout,
   if (L.tma && L.h_inst && lay.sws <= 256 && lay.sr <= 256)
     tm = L.tma->get(L.h_inst, L.n_inst, vin, lay.sws, lay.sr, s);
   ProfScope ps(s, DTSGB_K_DTS_ITER);
-  DTSGB_CUDA(launch_dependent(k_dts_iter_vec<TS, MODE, TW, TH, NT, STEREO>, dim3(L.n_tiles),
-                              dim3(NT), smem, s, L.d_inst, L.d_tiles, vin, vout,
+  DTSGB_CUDA(launch_dependent(kern, dim3(L.n_tiles), dim3(NT), smem, s, L.d_inst, L.d_tiles, vin, vout,
                               (const TS*)target, (const TS*)conf, bounds, lambda, step,
-                              overwrite, hx, hy, sa, lay, tm));
+                              overwrite, feeds, hx, hy, sa, lay, tm));
   return DTSGB_OK;
 }
 
@@ -1184,66 +1192,73 @@ template <typename TS, int MODE, bool STEREO>
 static int launch_iter_t(const DtsLaunch& L, const float* vin, float* vout,
                          const void* target, const void* conf,
                          const uint32_t* bounds, float lambda, float step,
-                         float overwrite, int hx, int hy, cudaStream_t s,
+                         float overwrite, int feeds, int hx, int hy, cudaStream_t s,
                          const StereoArgs& sa) {
   if (L.small)
     return launch_iter_shape<TS, MODE, kIterSmallTW, kIterSmallTH, STEREO>(
-        L, vin, vout, target, conf, bounds, lambda, step, overwrite, hx, hy, s, sa);
+        L, vin, vout, target, conf, bounds, lambda, step, overwrite, feeds, hx, hy, s, sa);
   if (L.d_tiles_small &&
       (size_t)VecIterSmem<kIterTW, kIterTH, 512>(hx, hy).total > kMaxSmem &&
       PrefixIterSmem<kIterTW, kIterTH, 512>::bytes(hx, hy) > kMaxSmem)
     return launch_iter_shape<TS, MODE, kIterSmallTW, kIterSmallTH, STEREO>(
-        L.as_small(), vin, vout, target, conf, bounds, lambda, step, overwrite, hx, hy,
+        L.as_small(), vin, vout, target, conf, bounds, lambda, step, overwrite, feeds, hx, hy,
         s, sa);
   return launch_iter_shape<TS, MODE, kIterTW, kIterTH, STEREO>(
-      L, vin, vout, target, conf, bounds, lambda, step, overwrite, hx, hy, s, sa);
+      L, vin, vout, target, conf, bounds, lambda, step, overwrite, feeds, hx, hy, s, sa);
 }
 
 template <typename TS, bool STEREO>
 static int launch_iter_mode(const DtsLaunch& L, IterMode mode, const float* vin,
                             float* vout, const void* target, const void* conf,
                             const uint32_t* bounds, float lambda, float step,
-                            float overwrite, int hx, int hy, cudaStream_t s,
+                            float overwrite, int feeds, int hx, int hy, cudaStream_t s,
                             const StereoArgs& sa) {
   if (mode == IterMode::L2)
     return launch_iter_t<TS, 0, STEREO>(L, vin, vout, target, conf, bounds, lambda,
-                                        step, overwrite, hx, hy, s, sa);
+                                        step, overwrite, feeds, hx, hy, s, sa);
   return launch_iter_t<TS, 1, STEREO>(L, vin, vout, target, conf, bounds, lambda,
-                                      step, overwrite, hx, hy, s, sa);
+                                      step, overwrite, feeds, hx, hy, s, sa);
 }
 
 int launch_dts_iter(const DtsLaunch& L, Storage st, IterMode mode,
                     const float* vin, float* vout, const void* target,
                     const void* conf, const uint32_t* bounds, float lambda,
-                    float step, float overwrite, int hx, int hy,
+                    float step, float overwrite, int feeds, int hx, int hy,
                     cudaStream_t s, const StereoArgs* stereo) {
   const StereoArgs none{nullptr, nullptr, 0.f, 0.f, 0.f, -1.f};
   if (st == Storage::F32) {
     if (stereo)
       return launch_iter_mode<float, true>(L, mode, vin, vout, target, conf, bounds,
-                                           lambda, step, overwrite, hx, hy, s, *stereo);
+                                           lambda, step, overwrite, feeds, hx, hy, s, *stereo);
     return launch_iter_mode<float, false>(L, mode, vin, vout, target, conf, bounds,
-                                          lambda, step, overwrite, hx, hy, s, none);
+                                          lambda, step, overwrite, feeds, hx, hy, s, none);
   }
   if (stereo)
     return launch_iter_mode<__nv_bfloat16, true>(L, mode, vin, vout, target, conf,
-                                                 bounds, lambda, step, overwrite, hx,
+                                                 bounds, lambda, step, overwrite, feeds, hx,
                                                  hy, s, *stereo);
   return launch_iter_mode<__nv_bfloat16, false>(L, mode, vin, vout, target, conf,
-                                                bounds, lambda, step, overwrite, hx,
+                                                bounds, lambda, step, overwrite, feeds, hx,
                                                 hy, s, none);
 }
 
 int launch_target_to_float(const DtsLaunch& L, Storage st, const void* src,
                            float* dst, float* dst_sq, cudaStream_t s) {
-  dim3 grid(64, L.n_inst);
+  // enough blocks for the largest instance (64 left most SMs idle on one image)
+  long long most = 1 << 20;
+  if (L.h_inst) {
+    most = 1;
+    for (int i = 0; i < L.n_inst; ++i)
+      most = std::max(most, (long long)L.h_inst[i].pitch * L.h_inst[i].h);
+  }
+  const int cap = std::max(64, 152 * 16 / L.n_inst);
+  const dim3 grid(std::min(grid_for((most + 3) / 4), cap), L.n_inst);
   ProfScope ps(s, DTSGB_K_DTS_OTHER);
   if (st == Storage::F32)
-    k_to_float<float><<<grid, kThreads, 0, s>>>(L.d_inst, L.n_inst,
-                                                 (const float*)src, dst, dst_sq);
+    k_to_float<float><<<grid, kThreads, 0, s>>>(L.d_inst, (const float*)src, dst, dst_sq);
   else
     k_to_float<__nv_bfloat16><<<grid, kThreads, 0, s>>>(
-        L.d_inst, L.n_inst, (const __nv_bfloat16*)src, dst, dst_sq);
+        L.d_inst, (const __nv_bfloat16*)src, dst, dst_sq);
   DTSGB_CUDA(cudaGetLastError());
   return DTSGB_OK;
 }
@@ -1251,6 +1266,12 @@ int launch_target_to_float(const DtsLaunch& L, Storage st, const void* src,
 int launch_init_var(const DtsLaunch& L, Storage st, const void* target,
                     float* v, cudaStream_t s) {
   return launch_target_to_float(L, st, target, v, nullptr, s);
+}
+
+int first_iterate(const DtsLaunch& L, Storage st, const void* target, float* v,
+                  const float** first, cudaStream_t s) {
+  *first = st == Storage::F32 ? static_cast<const float*>(target) : v;
+  return st == Storage::F32 ? DTSGB_OK : launch_init_var(L, st, target, v, s);
 }
 
 int launch_storage_from_float(const Inst*, int, Storage st, const float* src,

@@ -434,12 +434,21 @@ DTSGB_API int dtsgb_dts_optimize(dtsgb_dts_t h, const dtsgb_optimize_params* p,
     return fail(DTSGB_ERR_UNSUPPORTED, "sigma_z must be in (0, 254)");
   if (!std::isfinite(p->lambda) || !std::isfinite(p->step_size))
     return fail(DTSGB_ERR_INVALID_ARGUMENT, "lambda / step_size not finite");
-  int st = launch_init_var(h->launch_i(), h->st, h->target, h->v[0], h->stream);
-  if (st) return st;
-  h->var_idx = 0;
   // RobustLoss::L1 has no kernel in the reference's switches, so the
   // iterate stays the target (src/domain_transform_solver.cu:133-153).
-  if (p->loss == DTSGB_L1 || p->num_iterations == 0) return DTSGB_OK;
+  if (p->loss == DTSGB_L1 || p->num_iterations == 0) {
+    h->var_idx = 0;
+    return launch_init_var(h->launch_i(), h->st, h->target, h->v[0], h->stream);
+  }
+  if ((h->flags & DTSGB_FLAG_STEREO) && !h->solver_fp_valid) {
+    h->var_idx = 0;
+    if (int e = launch_init_var(h->launch_i(), h->st, h->target, h->v[0], h->stream)) return e;
+    return fail(DTSGB_ERR_INVALID_ARGUMENT,
+                "stereo Optimize needs ComputeColorSpaceDifferential first");
+  }
+  const float* cur = nullptr;
+  int st = first_iterate(h->launch_i(), h->st, h->target, h->v[0], &cur, h->stream);
+  if (st) return st;
   st = dts_bounds(h, p->sigma_z, p->sigma_z, true);
   if (st) return st;
   const int halo = (int)std::floor(p->sigma_z);
@@ -450,9 +459,6 @@ DTSGB_API int dtsgb_dts_optimize(dtsgb_dts_t h, const dtsgb_optimize_params* p,
   StereoArgs sa{};
   const StereoArgs* sp = nullptr;
   if (h->flags & DTSGB_FLAG_STEREO) {
-    if (!h->solver_fp_valid)
-      return fail(DTSGB_ERR_INVALID_ARGUMENT,
-                  "stereo Optimize needs ComputeColorSpaceDifferential first");
     const float sxr = h->solver_sr / h->solver_sx;
     sa = StereoArgs{h->guide, h->right, h->center_offset, p->photo_consis_lambda,
                     sxr * sxr, h->right_ratio};
@@ -460,11 +466,12 @@ DTSGB_API int dtsgb_dts_optimize(dtsgb_dts_t h, const dtsgb_optimize_params* p,
   }
   int a = 0, b = 1;
   for (int it = 0; it < p->num_iterations; ++it) {
-    st = launch_dts_iter(h->launch_i(), h->st, mode, h->v[a], h->v[b],
+    st = launch_dts_iter(h->launch_i(), h->st, mode, cur, h->v[b],
                          h->target, h->conf, h->bounds, p->lambda, p->step_size,
-                         overwrite, halo, halo, h->stream, sp);
+                         overwrite, it + 1 < p->num_iterations, halo, halo, h->stream, sp);
     if (st) return st;
     std::swap(a, b);
+    cur = h->v[a];
   }
   h->var_idx = a;
   return DTSGB_OK;

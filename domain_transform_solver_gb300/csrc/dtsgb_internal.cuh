@@ -245,14 +245,22 @@ struct StereoArgs {
   float offset, lam_p, alpha, ratio;
 };
 
+// One iteration from vin to vout.  feeds: another iteration reads vout, so
+// with overwrite in (0, 1) it holds the target where conf > overwrite (the
+// iterate handed in does so already: the first one is the target).
 int launch_dts_iter(const DtsLaunch& L, Storage st, IterMode mode,
                     const float* vin, float* vout, const void* target,
                     const void* conf, const uint32_t* bounds, float lambda,
-                    float step, float overwrite, int halo_x, int halo_y,
+                    float step, float overwrite, int feeds, int halo_x, int halo_y,
                     cudaStream_t s, const StereoArgs* stereo = nullptr);
 // v = target (as float), optionally overwritten nowhere: the initial iterate.
 int launch_init_var(const DtsLaunch& L, Storage st, const void* target,
                     float* v, cudaStream_t s);
+// The plane the first iteration reads: a float target is that plane itself
+// (iterations never write their input), another storage type is converted
+// into v.
+int first_iterate(const DtsLaunch& L, Storage st, const void* target, float* v,
+                  const float** first, cudaStream_t s);
 
 // Box pass of the domain-transform filter over nch channels sharing bounds.
 // When conf_out is non-null (confidence epilogue), nch must be 2 and the
