@@ -289,39 +289,184 @@ int upload_plane(dtsgb_batch_t b, int i, const float* src, void* dst,
   return DTSGB_OK;
 }
 
+// ---- dense images <-> pitched planes -------------------------------------------
+// Bound by HBM (12 B/px read, 8 or 12 written by an upload).  A block of 8
+// warps takes kCopyRows rows x `cols` pixels of one instance, a warp per row:
+// 512 columns (four rounds of loads a warp) for images that fill the SMs
+// that way, else one round's 128, or 32 where single pixels are copied (a
+// small image is latency: 333x250 loses 2 us a solve with four).  Four adjacent
+// pixels per thread and 16-byte accesses where the dense rows allow them
+// (the width a multiple of 4 and every pointer 16-byte aligned; the planes'
+// rows always are), else four single pixels whose loads are issued before
+// their stores.  With one pixel per thread and a block per row or five:
+// 84 us at 3264x2448 and 310 us for 64 ragged images of 47 Mpx in all, now
+// 36 and 217.
+constexpr int kCopyRows = 8, kCopyColsBig = 512, kCopyColsSmall = 128, kCopyColsSingle = 32;
+
+struct CopyTile {
+  int y, x0, x1;  // the warp's row and its pixels [x0, x1); y < 0: none
+};
+
+__device__ __forceinline__ CopyTile copy_tile(const Inst& I, int cols) {
+  const int nc = (I.w + cols - 1) / cols;
+  const int rb = (int)blockIdx.x / nc, cb = (int)blockIdx.x - rb * nc;
+  const int y = rb * kCopyRows + (int)(threadIdx.x >> 5);
+  return CopyTile{y < I.h ? y : -1, cb * cols, min((cb + 1) * cols, I.w)};
+}
+
+__device__ __forceinline__ bool aligned16(const void* p) {
+  return (reinterpret_cast<unsigned long long>(p) & 15ull) == 0;
+}
+
+__device__ __forceinline__ void store4(float* d, float4 v) {
+  *reinterpret_cast<float4*>(d) = v;
+}
+__device__ __forceinline__ void store4(__nv_bfloat16* d, float4 v) {
+  __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  uint2 u;
+  u.x = *reinterpret_cast<unsigned*>(&a);
+  u.y = *reinterpret_cast<unsigned*>(&b);
+  *reinterpret_cast<uint2*>(d) = u;
+}
+
+// One instance's dense images (g null: the guide stays; c null: ones) into
+// its pitched planes at `off`.
+template <typename TS>
+__device__ __forceinline__ void ingest_tile(const Inst& I, const uchar4* g, const float* t,
+                                            const float* c, uchar4* __restrict__ guide,
+                                            TS* __restrict__ target, TS* __restrict__ conf,
+                                            int cs, int cols) {
+  const CopyTile T = copy_tile(I, cols);
+  if (T.y < 0) return;
+  const int lane = threadIdx.x & 31;
+  const long long srow = (long long)T.y * I.w, drow = I.off + (long long)T.y * I.pitch;
+  if ((I.w & 3) == 0 && aligned16(g) && aligned16(t) && aligned16(c)) {
+#pragma unroll
+    for (int u = 0; u < kCopyColsBig / 128; ++u) {
+      const int x = T.x0 + 4 * lane + 128 * u;
+      if (x >= T.x1) break;
+      const float4 tv = __ldg(reinterpret_cast<const float4*>(t + srow + x));
+      const float4 cv = c ? __ldg(reinterpret_cast<const float4*>(c + srow + x))
+                          : make_float4(1.f, 1.f, 1.f, 1.f);
+      if (g) {
+        uint4 q = __ldg(reinterpret_cast<const uint4*>(g + srow + x));
+        if (cs != DTSGB_RGB) {
+          unsigned* w = &q.x;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uchar4 r = convert_pixel(*reinterpret_cast<const uchar4*>(w + k), cs);
+            w[k] = *reinterpret_cast<const unsigned*>(&r);
+          }
+        }
+        *reinterpret_cast<uint4*>(guide + drow + x) = q;
+      }
+      store4(target + drow + x, tv);
+      store4(conf + drow + x, cv);
+    }
+    return;
+  }
+  constexpr int U = 4;  // pixels whose loads are issued before any store
+  for (int xb = T.x0 + lane; xb < T.x1; xb += 32 * U) {
+    unsigned q[U];
+    float tv[U], cv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int x = min(xb + 32 * u, I.w - 1);  // past the row: a copy, not stored
+      tv[u] = __ldg(t + srow + x);
+      cv[u] = c ? __ldg(c + srow + x) : 1.f;
+      q[u] = g ? __ldg(reinterpret_cast<const unsigned*>(g + srow + x)) : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int x = xb + 32 * u;
+      if (x >= T.x1) break;
+      if (g) {
+        const uchar4 p = *reinterpret_cast<const uchar4*>(q + u);
+        guide[drow + x] = cs == DTSGB_RGB ? p : convert_pixel(p, cs);
+      }
+      target[drow + x] = store_cast<TS>(tv[u]);
+      conf[drow + x] = store_cast<TS>(cv[u]);
+    }
+  }
+}
+
+// One instance's dense float image <-> its rows of a pitched plane.
+template <bool TO_ARENA>
+__device__ __forceinline__ void copy_tile_f32(const Inst& I, float* dense, float* arena,
+                                              int cols) {
+  const CopyTile T = copy_tile(I, cols);
+  if (T.y < 0) return;
+  const int lane = threadIdx.x & 31;
+  float* d = dense + (long long)T.y * I.w;
+  float* a = arena + I.off + (long long)T.y * I.pitch;
+  const float* from = TO_ARENA ? d : a;
+  float* to = TO_ARENA ? a : d;
+  if ((I.w & 3) == 0 && aligned16(dense)) {
+#pragma unroll
+    for (int u = 0; u < kCopyColsBig / 128; ++u) {
+      const int x = T.x0 + 4 * lane + 128 * u;
+      if (x >= T.x1) break;
+      *reinterpret_cast<float4*>(to + x) = *reinterpret_cast<const float4*>(from + x);
+    }
+    return;
+  }
+  constexpr int U = 4;
+  for (int xb = T.x0 + lane; xb < T.x1; xb += 32 * U) {
+    float v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = from[min(xb + 32 * u, I.w - 1)];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (xb + 32 * u < T.x1) to[xb + 32 * u] = v[u];
+  }
+}
+
 // Dense staged images -> pitched planes: the guide (color-converted; not
 // written when guide is null), target and confidence in the storage type.
 template <typename TS>
-__global__ void k_ingest(const Inst* __restrict__ insts, const long long* __restrict__ soff,
-                         const uchar4* __restrict__ s_rgba, const float* __restrict__ s_t,
-                         const float* __restrict__ s_c, uchar4* __restrict__ guide,
-                         TS* __restrict__ target, TS* __restrict__ conf, int cs) {
+__global__ void __launch_bounds__(256)
+    k_ingest(const Inst* __restrict__ insts, const long long* __restrict__ soff,
+             const uchar4* __restrict__ s_rgba, const float* __restrict__ s_t,
+             const float* __restrict__ s_c, uchar4* __restrict__ guide,
+             TS* __restrict__ target, TS* __restrict__ conf, int cs, int cols) {
   const Inst I = insts[blockIdx.y];
   const long long so = soff[blockIdx.y];
-  for (int y = blockIdx.x; y < I.h; y += gridDim.x) {
-    const long long srow = so + (long long)y * I.w, drow = I.off + (long long)y * I.pitch;
-    for (int x = threadIdx.x; x < I.w; x += blockDim.x) {
-      if (guide) {
-        const uchar4 p = s_rgba[srow + x];
-        guide[drow + x] = cs == DTSGB_RGB ? p : convert_pixel(p, cs);
-      }
-      target[drow + x] = store_cast<TS>(s_t[srow + x]);
-      conf[drow + x] = store_cast<TS>(s_c[srow + x]);
-    }
-  }
+  ingest_tile<TS>(I, guide ? s_rgba + so : nullptr, s_t + so, s_c + so, guide, target, conf, cs,
+                  cols);
 }
 
 // Dense staged plane -> pitched plane (gradient uploads).  Downloads stay
 // row-by-row DMA copies: those need no SM, so in a pipeline they do not wait
 // behind another chunk's solve.
-__global__ void k_unstage(const Inst* __restrict__ insts, const long long* __restrict__ soff,
-                          const float* __restrict__ src, float* __restrict__ dst) {
-  const Inst I = insts[blockIdx.y];
-  const long long so = soff[blockIdx.y];
-  for (int y = blockIdx.x; y < I.h; y += gridDim.x) {
-    const long long drow = so + (long long)y * I.w, prow = I.off + (long long)y * I.pitch;
-    for (int x = threadIdx.x; x < I.w; x += blockDim.x) dst[prow + x] = src[drow + x];
+__global__ void __launch_bounds__(256)
+    k_unstage(const Inst* __restrict__ insts, const long long* __restrict__ soff, float* src,
+              float* dst, int cols) {
+  copy_tile_f32<true>(insts[blockIdx.y], src + soff[blockIdx.y], dst, cols);
+}
+
+// Blocks of the copy kernels (every instance's row blocks times its column
+// blocks on x, the instances on y) and their columns: the small ones where
+// the big ones would leave the SMs fewer than four blocks each.
+dim3 copy_grid(dtsgb_batch_t b, int* cols) {
+  auto blocks = [&](int c, long long* most) {
+    long long sum = 0;
+    *most = 1;
+    for (const Inst& I : b->inst) {
+      const long long k =
+          (long long)((I.h + kCopyRows - 1) / kCopyRows) * ((I.w + c - 1) / c);
+      *most = std::max(*most, k);
+      sum += k;
+    }
+    return sum;
+  };
+  long long most = 1;
+  *cols = kCopyColsBig;
+  if (blocks(kCopyColsBig, &most) < 4 * 152) {
+    bool single = false;
+    for (const Inst& I : b->inst) single = single || (I.w & 3) != 0;
+    blocks(*cols = single ? kCopyColsSingle : kCopyColsSmall, &most);
   }
+  return dim3((unsigned)most, (unsigned)b->n);
 }
 
 int ensure_stage(dtsgb_batch_t b) {
@@ -344,8 +489,9 @@ int host_upload_plane(dtsgb_batch_t b, const float* const* src, float* dst, int 
     DTSGB_CUDA(cudaMemcpyAsync(d + b->soff[i], src[i], (size_t)I.w * I.h * 4,
                                cudaMemcpyHostToDevice, b->stream));
   }
-  const dim3 grid((unsigned)std::min(b->max_h, 512), (unsigned)b->n);
-  k_unstage<<<grid, 256, 0, b->stream>>>(b->d_inst, b->d_soff, d, dst);
+  int cols = 0;
+  const dim3 grid = copy_grid(b, &cols);
+  k_unstage<<<grid, 256, 0, b->stream>>>(b->d_inst, b->d_soff, d, dst, cols);
   DTSGB_CUDA(cudaGetLastError());
   return DTSGB_OK;
 }
@@ -353,21 +499,11 @@ int host_upload_plane(dtsgb_batch_t b, const float* const* src, float* dst, int 
 // Caller device images (dense W x H, one pointer each; null: skipped) <->
 // pitched arena plane: one kernel instead of a row-by-row copy per image.
 template <bool TO_ARENA>
-__global__ void k_user_copy(const Inst* __restrict__ insts, float* const* __restrict__ user,
-                            float* __restrict__ arena) {
-  const Inst I = insts[blockIdx.y];
+__global__ void __launch_bounds__(256)
+    k_user_copy(const Inst* __restrict__ insts, float* const* __restrict__ user, float* arena,
+                int cols) {
   float* u = user[blockIdx.y];
-  if (!u) return;
-  for (int y = blockIdx.x; y < I.h; y += gridDim.x) {
-    float* urow = u + (long long)y * I.w;
-    float* arow = arena + I.off + (long long)y * I.pitch;
-    for (int x = threadIdx.x; x < I.w; x += blockDim.x) {
-      if (TO_ARENA)
-        arow[x] = urow[x];
-      else
-        urow[x] = arow[x];
-    }
-  }
+  if (u) copy_tile_f32<TO_ARENA>(insts[blockIdx.y], u, arena, cols);
 }
 
 // Copies between n caller device images and an arena plane (slot 0..2 of the
@@ -391,11 +527,12 @@ int user_plane_copy(dtsgb_batch_t b, float* const* user, float* arena, bool to_a
                     int slot) {
   float** d = b->d_uptr + (size_t)slot * b->n;
   if (int st = upload_slot(b, slot, reinterpret_cast<const void* const*>(user))) return st;
-  const dim3 grid((unsigned)std::min(b->max_h, 512), (unsigned)b->n);
+  int cols = 0;
+  const dim3 grid = copy_grid(b, &cols);
   if (to_arena)
-    k_user_copy<true><<<grid, 256, 0, b->stream>>>(b->d_inst, d, arena);
+    k_user_copy<true><<<grid, 256, 0, b->stream>>>(b->d_inst, d, arena, cols);
   else
-    k_user_copy<false><<<grid, 256, 0, b->stream>>>(b->d_inst, d, arena);
+    k_user_copy<false><<<grid, 256, 0, b->stream>>>(b->d_inst, d, arena, cols);
   DTSGB_CUDA(cudaGetLastError());
   return DTSGB_OK;
 }
@@ -404,25 +541,13 @@ int user_plane_copy(dtsgb_batch_t b, float* const* user, float* arena, bool to_a
 // (color-converted; not written when rgba is null), target and confidence in
 // the storage type; a null confidence image stands for ones.
 template <typename TS>
-__global__ void k_ingest_ptr(const Inst* __restrict__ insts, uchar4* const* __restrict__ rgba,
-                             float* const* __restrict__ tgt, float* const* __restrict__ cnf,
-                             uchar4* __restrict__ guide, TS* __restrict__ target,
-                             TS* __restrict__ conf, int cs) {
-  const Inst I = insts[blockIdx.y];
-  const uchar4* g = rgba ? rgba[blockIdx.y] : nullptr;
-  const float* t = tgt[blockIdx.y];
-  const float* c = cnf ? cnf[blockIdx.y] : nullptr;
-  for (int y = blockIdx.x; y < I.h; y += gridDim.x) {
-    const long long srow = (long long)y * I.w, drow = I.off + (long long)y * I.pitch;
-    for (int x = threadIdx.x; x < I.w; x += blockDim.x) {
-      if (g) {
-        const uchar4 p = g[srow + x];
-        guide[drow + x] = cs == DTSGB_RGB ? p : convert_pixel(p, cs);
-      }
-      target[drow + x] = store_cast<TS>(t[srow + x]);
-      conf[drow + x] = store_cast<TS>(c ? c[srow + x] : 1.f);
-    }
-  }
+__global__ void __launch_bounds__(256)
+    k_ingest_ptr(const Inst* __restrict__ insts, uchar4* const* __restrict__ rgba,
+                 float* const* __restrict__ tgt, float* const* __restrict__ cnf,
+                 uchar4* __restrict__ guide, TS* __restrict__ target, TS* __restrict__ conf,
+                 int cs, int cols) {
+  ingest_tile<TS>(insts[blockIdx.y], rgba ? rgba[blockIdx.y] : nullptr, tgt[blockIdx.y],
+                  cnf ? cnf[blockIdx.y] : nullptr, guide, target, conf, cs, cols);
 }
 
 int device_ingest(dtsgb_batch_t b, int cs, const void* const* rgba,
@@ -439,17 +564,18 @@ int device_ingest(dtsgb_batch_t b, int cs, const void* const* rgba,
   if (st) return st;
   // the pointer copies come from pageable host memory: the calls return
   // once the arrays are copied out, so cf may go out of scope
-  const dim3 grid((unsigned)std::min(b->max_h, 512), (unsigned)b->n);
+  int cols = 0;
+  const dim3 grid = copy_grid(b, &cols);
   uchar4* const* rp = rgba ? reinterpret_cast<uchar4* const*>(slots) : nullptr;
   uchar4* g = rgba ? b->guide : nullptr;
   if (b->st == Storage::F32)
     k_ingest_ptr<float><<<grid, 256, 0, b->stream>>>(b->d_inst, rp, slots + n, slots + 2 * n,
                                                      g, (float*)b->target, (float*)b->conf,
-                                                     cs);
+                                                     cs, cols);
   else
     k_ingest_ptr<__nv_bfloat16><<<grid, 256, 0, b->stream>>>(
         b->d_inst, rp, slots + n, slots + 2 * n, g, (__nv_bfloat16*)b->target,
-        (__nv_bfloat16*)b->conf, cs);
+        (__nv_bfloat16*)b->conf, cs, cols);
   DTSGB_CUDA(cudaGetLastError());
   if (rgba) ++b->guide_gen;
   b->dts_res = -1;
@@ -485,15 +611,16 @@ int host_ingest(dtsgb_batch_t b, int cs, const void* const* rgba,
       if (st) return st;
     }
   }
-  const dim3 grid((unsigned)std::min(b->max_h, 512), (unsigned)b->n);
+  int cols = 0;
+  const dim3 grid = copy_grid(b, &cols);
   uchar4* g = rgba ? b->guide : nullptr;
   if (b->st == Storage::F32)
     k_ingest<float><<<grid, 256, 0, b->stream>>>(b->d_inst, b->d_soff, s_rgba, s_t, s_c, g,
-                                                 (float*)b->target, (float*)b->conf, cs);
+                                                 (float*)b->target, (float*)b->conf, cs, cols);
   else
     k_ingest<__nv_bfloat16><<<grid, 256, 0, b->stream>>>(
         b->d_inst, b->d_soff, s_rgba, s_t, s_c, g, (__nv_bfloat16*)b->target,
-        (__nv_bfloat16*)b->conf, cs);
+        (__nv_bfloat16*)b->conf, cs, cols);
   DTSGB_CUDA(cudaGetLastError());
   if (rgba) ++b->guide_gen;
   b->dts_res = -1;
@@ -838,8 +965,11 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
   {
     int bw = 0, bh = 0;
     dts_iter_tma_box(Li, halo, halo, &bw, &bh);
-    if (bw > 0)
+    if (bw > 0) {
       for (float* v : b->v) (void)b->tma.get(b->inst.data(), b->n, v, bw, bh, b->stream);
+      if (b->st == Storage::F32)  // the first iteration reads the target
+        (void)b->tma.get(b->inst.data(), b->n, (const float*)b->target, bw, bh, b->stream);
+    }
   }
   const bool over = overwrite > 0.f && overwrite < 1.f;
   const int n_kept = iterate ? p->num_iterations : 0;
@@ -895,6 +1025,7 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
                            it + 1 < p->num_iterations, halo, halo, b->stream);
       if (st) return st;
       a = 1 - a;
+      cur = b->v[a];
     }
     return DTSGB_OK;
   };
@@ -969,9 +1100,6 @@ static int batch_backward(dtsgb_batch_t b, const float* const* grad_out,
   DtsGrad G = grad_view(b, n_iter);
   if (up == cudaMemcpyHostToDevice) {
     if (int st = host_upload_plane(b, grad_out, G.g[0], 0)) return st;
-      if (b->st == Storage::F32)  // the first iteration reads the target
-        (void)b->tma.get(b->inst.data(), b->n, (const float*)b->target, bw, bh, b->stream);
-    }
   } else {
     if (int st = user_plane_copy(b, const_cast<float* const*>(grad_out), G.g[0], true, 0))
       return st;
@@ -1025,7 +1153,6 @@ DTSGB_API int dtsgb_batch_dts_backward_device(dtsgb_batch_t b,
                                               const float* const* grad_out,
                                               float* const* grad_target,
                                               float* const* grad_confidence) {
-      cur = b->v[a];
   return batch_backward(b, grad_out, grad_target, grad_confidence,
                         cudaMemcpyDeviceToDevice, cudaMemcpyDeviceToDevice);
 }
