@@ -1,0 +1,116 @@
+"""The paths that a launch picks by size, type or alignment, each at the sizes
+where it can go wrong."""
+import numpy as np
+import pytest
+
+import parity as P
+
+pytestmark = pytest.mark.gpu
+
+
+# ---- splat: a CTA per cell from 256 pixels a cell on ---------------------------
+@pytest.mark.parametrize("w,h,sx,sy,sl,guide", [
+    (97, 53, 16.0, 16.0, 16.0, "noise"),      # 256-pixel cells, runs of one pixel
+    (255, 130, 51.0, 5.0, 16.0, "noise"),     # 255 pixels: a thread per cell
+    (200, 170, 32.0, 32.0, 5.0, "noise"),     # one chunk exactly; luma bin 51 overflows
+    (200, 170, 33.0, 31.5, 4.0, "steps"),     # ragged cells
+    (150, 140, 128.0, 100.0, 16.0, "flat"),   # one run through every chunk
+    (300, 41, 300.0, 41.0, 1.0, "noise"),     # one cell, 255 luma bins (and an overflow bin)
+])
+@pytest.mark.parametrize("bf16", [0, 1])
+def test_splat_sums_of_large_cells(gpu_ready, w, h, sx, sy, sl, guide, bf16):
+    """Counts are exact; a sum of n float products is within n * 2^-23 of
+    their absolute sum (n - 1 additions and one product, each 2^-24)."""
+    D = gpu_ready
+    rng = np.random.default_rng(w + h)
+    y, x = np.mgrid[0:h, 0:w]
+    luma = {"noise": rng.integers(0, 256, (h, w)), "flat": np.full((h, w), 200),
+            "steps": (x // 7 + y // 3) * 11 % 256}[guide].astype(np.uint8)
+    rgba = np.repeat(luma[..., None], 4, axis=2)
+    t = rng.normal(0, 10, (h, w)).astype(np.float32)
+    c = rng.random((h, w)).astype(np.float32)
+    b = D.Batch([(w, h)], flags=D.FLAG_BF16_STORAGE if bf16 else 0)
+    b.upload(D.COLOR_SPACE.RGB, [rgba], [t], [c])
+    b.solve_hfbs(D.HFBSGridParams(sigma_x=sx, sigma_y=sy, sigma_l=sl, bistoch_iter_max=1,
+                                  optim_iter_max=1))
+    if bf16:
+        t, c = P.bf16_round(t), P.bf16_round(c)
+    f = np.float32
+    dims = (int(np.ceil(f(w) / f(sx))), int(np.ceil(f(h) / f(sy))), int(np.ceil(255.0 / sl)))
+    bx = np.floor(x.astype(f) / f(sx)).astype(int)
+    by = np.floor(y.astype(f) / f(sy)).astype(int)
+    bl = np.floor(luma.astype(f) / f(sl)).astype(int)
+    at = ((bl * dims[1] + by) * dims[0] + bx).ravel()
+
+    def bins(v):
+        full = np.bincount(at, weights=v.astype(np.float64).ravel(),
+                           minlength=(dims[2] + 1) * dims[1] * dims[0])
+        return full[:dims[2] * dims[1] * dims[0]].reshape(dims[2], dims[1], dims[0])
+    n = bins(np.ones((h, w)))
+    assert np.array_equal(b.debug_grid(0, 1, dims), n.astype(f))
+    ct = c.astype(np.float64) * t
+    for which, v in ((2, c.astype(np.float64)), (3, ct)):
+        err = np.abs(b.debug_grid(0, which, dims) - bins(v))
+        assert (err <= n * 2.0 ** -23 * bins(np.abs(v))).all(), which
+
+
+# ---- overwrite: held by the iteration itself ----------------------------------
+@pytest.mark.parametrize("w,h,sz", [(70, 45, 8.0), (33, 140, 30.0), (400, 300, 71.0),
+                                    (900, 700, 12.0)])
+@pytest.mark.parametrize("loss,flags", [(1, 0), (2, 0), (1, 1)])
+def test_overwritten_pixels_hold_the_target(gpu_ready, oracle_mod, w, h, sz, loss, flags):
+    """Against the FP64 oracle on the GPU's windows, within the parity bar;
+    one iteration alone leaves its last Y half-step on them."""
+    from domain_transform_solver_gb300 import workloads as W
+    from test_gpu_dts import _run_dts
+    D, O = gpu_ready, oracle_mod
+    inst = W.depth_sr_instance(90 + w, w, h, n_poly=9, sample_frac=0.2)
+    inst.target[:] += (inst.confidence == 0) * np.float32(2.0)
+    t, c = inst.target, inst.confidence
+    if flags:
+        t, c = P.bf16_round(t), P.bf16_round(c)
+    for n in (1, 4):
+        opt = dict(W.CFG0_OPT, num_iterations=n, loss=loss, sigma_z=sz)
+        v, s = _run_dts(D, inst, 1, W.CFG0_FILTER, opt, 0.85, flags)
+        szf = float(np.float32(sz))
+        win = {(a, szf): s.DebugBounds(a, szf) for a in (0, 1)}
+        ref, _ = O.dts_solve(inst.rgba, t, c, 1, W.CFG0_FILTER, opt, 0.85, overrides=win)
+        assert np.abs(v - ref).max() <= P.TOL_REL * P.target_range(t), n
+
+
+# ---- device copies: vectors or single pixels -----------------------------------
+@pytest.mark.parametrize("sizes", [[(64, 40)], [(65, 40)], [(1, 1), (3, 9), (512, 8)],
+                                   [(2048, 1700), (513, 9)]])
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("flags", [0, 1])
+def test_device_copies_of_any_alignment(gpu_ready, sizes, shift, flags):
+    """Images at 16-byte boundaries and one element past them, of widths that
+    are and are not multiples of four: what comes back after no iterations is
+    the target, bit for bit."""
+    torch = pytest.importorskip("torch")
+    D = gpu_ready
+    rng = np.random.default_rng(7)
+    dev = torch.device("cuda:0")
+    ts = [rng.normal(0, 5, (h, w)).astype(np.float32) for w, h in sizes]
+    rg = [rng.integers(0, 256, (h, w, 4)).astype(np.uint8) for w, h in sizes]
+
+    def put(a):
+        flat = torch.from_numpy(np.ascontiguousarray(a).view(np.float32).reshape(-1))
+        buf = torch.zeros(flat.numel() + 4, device=dev)
+        buf[shift:shift + flat.numel()] = flat
+        return buf
+    tb, gb = [put(t) for t in ts], [put(g) for g in rg]
+    ob = [torch.full((w * h + 4,), -1.0, device=dev) for w, h in sizes]
+    torch.cuda.synchronize()
+    b = D.Batch(sizes, flags=flags)
+    b.upload_device(D.COLOR_SPACE.YCbCr, [x.data_ptr() + 4 * shift for x in gb],
+                    [x.data_ptr() + 4 * shift for x in tb], None)
+    b.solve_dts(D.DomainFilterParams(8.0, 8.0, 0.1), D.DomainOptimizeParams(num_iterations=0))
+    b.download_device(0, [x.data_ptr() + 4 * shift for x in ob])
+    host = b.download(0)
+    for t, o, hv in zip(ts, ob, host):
+        want = P.bf16_round(t) if flags else t
+        assert np.array_equal(hv, want)
+        got = o.cpu().numpy()
+        assert np.array_equal(got[shift:shift + t.size].reshape(t.shape), want)
+        assert (got[:shift] == -1).all() and (got[shift + t.size:] == -1).all()
