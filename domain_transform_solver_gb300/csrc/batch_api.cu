@@ -1254,7 +1254,7 @@ DTSGB_API int dtsgb_batch_solve_hfbs(dtsgb_batch_t b, const dtsgb_hfbs_params* p
     if ((st = hfbs_prepare_grad(b, p->optim_iter_max, goff))) return st;
     B.grad = &b->hgs;
   }
-  hfbs_prepare_tma(B, b->stream);  // before any capture of the solve
+  hfbs_prepare_tma(B, hp, b->stream);  // before any capture of the solve
   std::vector<char> key;
   key_append(key, hp);
   key_append(key, b->hfbs_group_voxels);
@@ -1375,7 +1375,7 @@ DTSGB_API int dtsgb_batch_set_tuning(dtsgb_batch_t b, int knob, long long value)
     return DTSGB_OK;
   }
   if (knob == DTSGB_TUNE_HFBS_SOLVE_STEPS) {
-    if (value != 1 && value != kHfbsTBSteps)
+    if (value != 1 && value != kHfbsMarchSteps)
       return fail(DTSGB_ERR_INVALID_ARGUMENT, "HFBS steps per launch must be 1 or 4");
     if (value != b->hfbs_solve_steps) b->hgrad_ready = false;  // kept iterates' arithmetic
     b->hfbs_solve_steps = (int)value;
@@ -1458,8 +1458,8 @@ DTSGB_API int dtsgb_batch_autotune(dtsgb_batch_t b, const dtsgb_filter_params* f
   if (hp && !st) {
     auto hfbs = [&]() { return dtsgb_batch_solve_hfbs(b, hp); };
     float best = 3.4e38f;
-    long long best_s = kHfbsTBSteps, best_g = 0;
-    for (long long steps : {(long long)kHfbsTBSteps, 1LL}) {
+    long long best_s = kHfbsMarchSteps, best_g = 0;
+    for (long long steps : {(long long)kHfbsMarchSteps, 1LL}) {
       if ((st = dtsgb_batch_set_tuning(b, DTSGB_TUNE_HFBS_SOLVE_STEPS, steps))) break;
       for (long long g : {0LL, 1000000LL, 2000000LL, 4000000LL, 8000000LL}) {
         if ((st = dtsgb_batch_set_tuning(b, DTSGB_TUNE_HFBS_GROUP_VOXELS, g))) break;

@@ -1086,6 +1086,7 @@ DTSGB_API int dtsgb_hfbs_optimize(dtsgb_hfbs_t h) {
   }
   HParams hp{p.sigma_x, p.sigma_y, p.sigma_l, p.lambda, p.alpha, p.beta,
              p.bistoch_iter_max, p.optim_iter_max, p.neg_exp_beta};
+  hfbs_prepare_tma(B, hp, h->stream);
   dtsgb_hfbs_s::NormKey nk{};  // zero padding, so that memcmp compares fields
   nk.guide_gen = h->guide_gen;
   nk.inst = I;

@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kGatherThreads)
 // neighbours comes from the previous launch).  step: the adjoint of step k
 // with its forward iterate z_k, into gh, gb, ginv and gg_out, gw_out.  The
 // neighbour sum and q are formed as in the forward step (kRounded: the
-// temporally blocked kernel's rounded z * n products), so the Huber mask is
+// march's rounded z * n products), so the Huber mask is
 // the forward's.
 template <bool kRounded>
 __global__ void k_hb_step_adj(const HInst* __restrict__ insts, const float* __restrict__ zk,
@@ -312,7 +312,7 @@ int hfbs_enqueue_backward(const HfbsBatch& B, const HParams& p, const float* gou
   const dim3 gcol((unsigned)((B.max_cells + kGatherCols - 1) / kGatherCols), ni);
   k_hb_slice_gather<<<gcol, kGatherThreads, hsmem, s>>>(B.d_inst, B.guide, sp, B.count, G.gz,
                                                         p);
-  const bool tb = hfbs_uses_tb(B);
+  const bool tb = hfbs_uses_march(B);
   // (gg, gw) ping-pong: a launch reads the pair the previous one wrote
   float* pg[2] = {G.gg, G.gg2};
   float* pw[2] = {G.gw, G.gw2};
@@ -347,10 +347,11 @@ int hfbs_enqueue_backward(const HfbsBatch& B, const HParams& p, const float* gou
         hin = G.hrec;
       }
       for (int k = start; k + 1 < end;) {
-        const int steps = tb ? std::min(kHfbsTBSteps, end - 1 - k) : 1;
+        const int steps = tb ? std::min(kHfbsMarchSteps, end - 1 - k) : 1;
         float* hout = tb ? hbuf[hb] : G.hrec;
-        hfbs_launch_steps(B, p, norm, zk(k), zk(k + steps), hin, hout, steps,
-                          tb ? zk(k + 1) : nullptr, tb ? steps : 0, s);
+        if (int st = hfbs_launch_steps(B, p, norm, zk(k), zk(k + steps), hin, hout, steps,
+                                       tb ? zk(k + 1) : nullptr, tb ? steps : 0, s))
+          return st;
         hin = hout;
         hb ^= 1;
         k += steps;

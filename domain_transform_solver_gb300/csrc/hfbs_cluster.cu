@@ -1,0 +1,318 @@
+// The iterative HFBS stages on grids small enough to stay on chip: all
+// heavy-ball steps (src/hfbs.cu:201-239), or all bistochastization iterations
+// (src/hfbs.cu:126-155), of an instance in one launch of one thread-block
+// cluster.
+//
+// Each CTA of the cluster owns a slab of grid rows y; a thread owns items of
+// four levels of one (x, y) column and keeps their z, h, n, b and invA in
+// registers for the whole solve.  Per step the products z * n go to shared
+// memory (two buffers in turn), those of a slab's first and last row also to
+// the neighbouring CTA's halo row through distributed shared memory; one
+// cluster barrier later every neighbour is a local read.  Memory is touched
+// before the first and after the last step only.
+//
+// Bound by latency: a step is one exchange (18 shared-memory reads per four
+// voxels, about 25 instructions a voxel) and one cluster barrier.  Measured:
+// 140 steps on a 22 x 17 x 16 grid in 90 us, 64 on 80 x 60 x 16 in 105; a
+// launch per four steps, the form this replaces, took 12 to 16 us on such grids
+// whatever their size (a launch, a round of loads and four block barriers).
+//
+// Taken where every instance of the launch fits: per CTA 2048 items (8192
+// voxels; registers) and 227 KB of the two buffers, so 131072 voxels for 16
+// CTAs.  On such grids it beats the march (hfbs_march.cu) also when many run
+// side by side, since nothing is recomputed at block borders.
+//
+// Out-of-grid values, neighbour order and arithmetic are the march's
+// (hfbs_march.cu): the results are the same bit for bit.
+#include <algorithm>
+#include <vector>
+
+#include "../../include/dtsgb.h"
+#include "dtsgb_internal.cuh"
+#include "hfbs_internal.cuh"
+
+namespace dtsgb {
+namespace {
+
+constexpr int kCV = 4;  // levels of an item
+// Threads a CTA may have when each owns that many items (registers: 20 an
+// item and about 45), and items a CTA can hold.
+__host__ __device__ constexpr int max_threads(int ipt) {
+  return ipt == 1 ? 1024 : ipt == 2 ? 768 : ipt == 3 ? 576 : 512;
+}
+constexpr int kCItems = 4;
+constexpr int kMaxItems = kCItems * max_threads(kCItems);
+constexpr size_t kMaxSmem = 227 * 1024;
+
+struct ClusterArgs {
+  const float *z, *h, *n, *b, *a;  // normalisation: n the counts
+  float *zd, *hd;                  // hd null: h is not needed afterwards
+  float* rec;                      // z after step k + 1 in plane k, rec_steps of them
+  long long rec_stride;
+  int rec_steps, steps;
+  float lambda, alpha, beta;
+};
+
+enum { kHeavyBall = 0, kBistoch = 1 };
+
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned cluster_size() {
+  unsigned n;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+  return n;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;"
+               ::: "memory");
+}
+// Stores v at the address that `local` has in the shared memory of CTA `rank`.
+__device__ __forceinline__ void store_remote(const float* local, unsigned rank, float v) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(local), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(r), "f"(v) : "memory");
+}
+
+// Rows of a CTA's slab, items of a CTA and its shared memory for a cluster of
+// `c` CTAs.
+__host__ __device__ inline int slab_rows(int gy, int c) { return (gy + c - 1) / c; }
+inline long long slab_items(const HInst& H, int c) {
+  return (long long)slab_rows(H.gy, c) * H.gx * ((H.gl + kCV - 1) / kCV);
+}
+inline size_t slab_smem(const HInst& H, int c) {
+  return sizeof(float) * 2 * (size_t)((H.gl + kCV - 1) / kCV * kCV) *
+         (slab_rows(H.gy, c) + 2) * (H.gx + 2);
+}
+
+template <int MODE, bool REC, int IPT>
+__global__ void __launch_bounds__(max_threads(IPT), 1)
+    k_hfbs_cluster(const HInst* __restrict__ insts, ClusterArgs A) {
+  pdl_wait_then_release();
+  extern __shared__ __align__(16) float smc[];
+  const HInst I = insts[blockIdx.y];
+  const int gx = I.gx, gy = I.gy, gl = I.gl;
+  const int rank = (int)cluster_rank(), C = (int)cluster_size();
+  const int R = slab_rows(gy, C), nlc = (gl + kCV - 1) / kCV;
+  const int gxp = gx + 2, PS = (R + 2) * gxp, BUF = nlc * kCV * PS;
+  const int tid = threadIdx.x, T = blockDim.x;
+  for (int i = tid; i < 2 * BUF; i += T) smc[i] = 0.f;
+  __syncthreads();
+  if (MODE == kBistoch) {
+    // the covered pad faces read 1 on even iterations (the first buffer), 0 on
+    // odd ones
+    const int rows = min(R, gy - rank * R);  // may be <= 0
+    if (I.cov_x)
+      for (int i = tid; i < gl * max(rows, 0); i += T) {
+        const int l = i / rows, yy = i - l * rows;
+        smc[l * PS + (yy + 1) * gxp + gx + 1] = 1.f;
+      }
+    if (I.cov_y && rows > 0 && rank * R + rows == gy)
+      for (int i = tid; i < gl * gx; i += T) {
+        const int l = i / gx, x = i - l * gx;
+        smc[l * PS + (rows + 1) * gxp + x + 1] = 1.f;
+      }
+  }
+  const int items = R * gx * nlc, plane = I.px * gy;
+  float z[IPT][kCV], h[IPT][kCV], n[IPT][kCV], b[IPT][kCV], a[IPT][kCV];
+  int o[IPT];        // index of level 0 of the item in a buffer
+  int lc[IPT];       // its group of levels (-1: no item)
+  int edge[IPT];     // bit 0: first row of the slab, bit 1: last
+  long long g[IPT];  // element of level 0 in a grid plane
+#pragma unroll
+  for (int j = 0; j < IPT; ++j) {
+    const int i = tid + j * T;
+    lc[j] = -1;
+    o[j] = edge[j] = 0;
+    g[j] = 0;
+#pragma unroll
+    for (int v = 0; v < kCV; ++v) z[j][v] = h[j][v] = n[j][v] = b[j][v] = a[j][v] = 0.f;
+    if (i < items) {
+      const int c = i / (R * gx), q = i - c * (R * gx), yy = q / gx, x = q - yy * gx;
+      const int y = rank * R + yy;
+      if (y < gy) {
+        lc[j] = c;
+        o[j] = c * kCV * PS + (yy + 1) * gxp + x + 1;
+        edge[j] = (yy == 0 && rank > 0 ? 1 : 0) | (yy == R - 1 && rank + 1 < C ? 2 : 0);
+        g[j] = I.grid_off + (long long)c * kCV * plane + (long long)y * I.px + x;
+#pragma unroll
+        for (int v = 0; v < kCV; ++v)
+          if (c * kCV + v < gl) {
+            const long long gv = g[j] + (long long)v * plane;
+            n[j][v] = A.n[gv];
+            if (MODE == kHeavyBall) {
+              z[j][v] = A.z[gv];
+              h[j][v] = A.h[gv];
+              b[j][v] = A.b[gv];
+              a[j][v] = A.a[gv];
+            } else {
+              z[j][v] = 1.f;
+            }
+          }
+      }
+    }
+  }
+  // every CTA of the cluster runs and its buffers are zeroed
+  cluster_barrier();
+  for (int s = 0; s < A.steps; ++s) {
+    float* P = smc + (s & 1) * BUF;
+    float p[IPT][kCV];
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+#pragma unroll
+      for (int v = 0; v < kCV; ++v) {
+        p[j][v] = MODE == kHeavyBall ? __fmul_rn(z[j][v], n[j][v]) : z[j][v];
+        if (lc[j] >= 0) {
+          float* q = P + o[j] + v * PS;
+          *q = p[j][v];
+          if (edge[j] & 1) store_remote(q + R * gxp, rank - 1, p[j][v]);
+          if (edge[j] & 2) store_remote(q - R * gxp, rank + 1, p[j][v]);
+        }
+      }
+    }
+    cluster_barrier();
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+      if (lc[j] < 0) continue;
+      const float* q = P + o[j];
+      const float lo = lc[j] > 0 ? q[-PS] : 0.f;
+      const float hi = lc[j] + 1 < nlc ? q[kCV * PS] : 0.f;
+      const float pz = MODE == kBistoch && I.cov_l && !(s & 1) ? 1.f : 0.f;
+#pragma unroll
+      for (int v = 0; v < kCV; ++v) {
+        const float below = v > 0 ? p[j][v > 0 ? v - 1 : 0] : lo;
+        float above = v + 1 < kCV ? p[j][v + 1 < kCV ? v + 1 : v] : hi;
+        const float* qv = q + v * PS;
+        if (MODE == kHeavyBall) {
+          hfbs_step(qv[-1], qv[1], qv[-gxp], qv[gxp], below, above, n[j][v], b[j][v], a[j][v],
+                    A.lambda, A.alpha, A.beta, z[j][v], h[j][v]);
+        } else if (lc[j] * kCV + v < gl) {
+          if (lc[j] * kCV + v + 1 == gl) above = pz;
+          float t = qv[-1];
+          t += qv[1];
+          t += qv[-gxp];
+          t += qv[gxp];
+          t += below;
+          t += above;
+          const float blurred = 2.f * p[j][v] + t;
+          z[j][v] = __fsqrt_rn(__fdiv_rn(p[j][v] * (n[j][v] + 0.00001f), blurred + 0.00001f));
+        }
+      }
+      if (REC && s < A.rec_steps) {
+        float* r = A.rec + s * A.rec_stride + g[j];
+#pragma unroll
+        for (int v = 0; v < kCV; ++v)
+          if (lc[j] * kCV + v < gl) r[(long long)v * plane] = z[j][v];
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < IPT; ++j) {
+    if (lc[j] < 0) continue;
+#pragma unroll
+    for (int v = 0; v < kCV; ++v)
+      if (lc[j] * kCV + v < gl) {
+        const long long gv = g[j] + (long long)v * plane;
+        A.zd[gv] = z[j][v];
+        if (MODE == kHeavyBall && A.hd) A.hd[gv] = h[j][v];
+      }
+  }
+}
+
+template <int MODE, bool REC, int IPT>
+cudaError_t launch(const HfbsBatch& B, const HfbsClusterPlan& P, const ClusterArgs& A,
+                   cudaStream_t s, int* clusters) {
+  auto kern = k_hfbs_cluster<MODE, REC, IPT>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)P.smem);
+  if (e == cudaSuccess && P.size > 8)
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = P.size;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(P.size, P.count);
+  c.blockDim = dim3(P.threads);
+  c.dynamicSmemBytes = P.smem;
+  c.stream = s;
+  c.attrs = at;
+  c.numAttrs = 2;
+  if (clusters) {  // only asked whether a cluster can be resident
+    c.numAttrs = 1;
+    return cudaOccupancyMaxActiveClusters(clusters, kern, &c);
+  }
+  return cudaLaunchKernelEx(&c, kern, B.d_inst + P.first, A);
+}
+
+template <int MODE, bool REC>
+cudaError_t launch_items(const HfbsBatch& B, const HfbsClusterPlan& P, const ClusterArgs& A,
+                         cudaStream_t s, int* clusters = nullptr) {
+  switch (P.items) {
+    case 1: return launch<MODE, REC, 1>(B, P, A, s, clusters);
+    case 2: return launch<MODE, REC, 2>(B, P, A, s, clusters);
+    case 3: return launch<MODE, REC, 3>(B, P, A, s, clusters);
+  }
+  return launch<MODE, REC, kCItems>(B, P, A, s, clusters);
+}
+
+}  // namespace
+
+HfbsClusterPlan hfbs_cluster_plan(const HfbsBatch& B, int first, int count) {
+  HfbsClusterPlan P;
+  if (!hfbs_uses_march(B)) return P;
+  int min_gy = 1 << 30;
+  for (int i = 0; i < count; ++i) min_gy = std::min(min_gy, B.h_inst[first + i].gy);
+  for (int c = 16; c >= 1; c /= 2) {
+    if (c > 1 && c > min_gy) continue;
+    long long items = 0;
+    size_t smem = 0;
+    for (int i = 0; i < count; ++i) {
+      items = std::max(items, slab_items(B.h_inst[first + i], c));
+      smem = std::max(smem, slab_smem(B.h_inst[first + i], c));
+    }
+    if (items > kMaxItems || smem > kMaxSmem) break;  // smaller clusters hold less
+    P.size = c;
+    P.items = 1;
+    while (items > (long long)P.items * max_threads(P.items)) ++P.items;
+    P.threads = (int)((items + P.items - 1) / P.items + 31) / 32 * 32;
+    P.smem = smem;
+    P.first = first;
+    P.count = count;
+    // the largest cluster whose instances run side by side
+    if ((long long)c * count <= 128) break;
+  }
+  if (P.size > 0) {
+    int n = 0;
+    if (launch_items<kHeavyBall, false>(B, P, ClusterArgs{}, nullptr, &n) != cudaSuccess || n < 1) {
+      (void)cudaGetLastError();
+      P.size = 0;
+    }
+  }
+  return P;
+}
+
+int hfbs_cluster_solve(const HfbsBatch& B, const HfbsClusterPlan& P, const HParams& p,
+                       const float* norm, const float* zs, float* zd, const float* hs, float* hd,
+                       int steps, float* rec, int rec_steps, cudaStream_t s) {
+  const ClusterArgs A{zs, hs, norm, B.b, B.invA, zd, hd, rec, B.total_voxels, rec_steps, steps,
+                      p.lambda, p.alpha, p.beta};
+  if (rec_steps > 0) DTSGB_CUDA((launch_items<kHeavyBall, true>(B, P, A, s)));
+  else DTSGB_CUDA((launch_items<kHeavyBall, false>(B, P, A, s)));
+  return DTSGB_OK;
+}
+
+int hfbs_cluster_bistoch(const HfbsBatch& B, const HfbsClusterPlan& P, float* dst, int steps,
+                         cudaStream_t s) {
+  const ClusterArgs A{nullptr, nullptr, B.count, nullptr, nullptr, dst, nullptr, nullptr, 0, 0,
+                      steps, 0.f, 0.f, 0.f};
+  DTSGB_CUDA((launch_items<kBistoch, false>(B, P, A, s)));
+  return DTSGB_OK;
+}
+
+}  // namespace dtsgb

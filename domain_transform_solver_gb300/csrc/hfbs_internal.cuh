@@ -42,6 +42,24 @@ __device__ __forceinline__ int cell_start(int cell, float sigma, int n) {
   return p;
 }
 
+// One heavy-ball step of one voxel (src/hfbs.cu:201-239): the rounded products
+// z * n of its neighbours in the reference's order, n, b, invA, and z and h
+// updated in place.  Every operation is spelled out, so that all kernels that
+// step give the same bits.
+__device__ __forceinline__ void hfbs_step(float xm, float xp, float ym, float yp, float lm,
+                                          float lp, float n, float b, float a, float lambda,
+                                          float alpha, float beta, float& z, float& h) {
+  const float d = __fadd_rn(
+      __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(xm, xp), ym), yp), lm), lp);
+  const float t = __fmaf_rn(__fmul_rn(lambda, n), d, b);
+  const float grad = __fmaf_rn(-t, a, z);
+  // |grad| > 1.345 with the double threshold of the reference: the smallest
+  // float above 1.345 (double) is 1.345f
+  const float gc = fabsf(grad) >= 1.345f ? copysignf(1.f, grad) : grad;
+  h = __fmaf_rn(beta, h, gc);
+  z = __fmaf_rn(-alpha, h, z);
+}
+
 // Solver parameters shared by a batch (HFBSGridParams minus the grid dims).
 struct HParams {
   float sigma_x, sigma_y, sigma_l, lambda, alpha, beta;
@@ -109,12 +127,12 @@ struct HfbsBatch {
   // group (0: all instances together); see hfbs_enqueue_solve
   const HInst* h_inst = nullptr;
   long long group_voxels = 0;
-  // heavy-ball steps per launch: kHfbsTBSteps (the temporally blocked
-  // kernel, where every grid has at most 16 levels) or 1 (the one-step
-  // kernel for every grid)
+  // heavy-ball steps per launch: kHfbsMarchSteps (the march, where every
+  // grid has at most kHfbsMarchMaxGL levels) or 1 (the one-step kernel for
+  // every grid)
   int solve_steps = 4;
-  // tensor maps of the grid planes for the temporally blocked kernels' TMA
-  // staging (null: they stage by 4-byte copies); owned by the caller, which
+  // tensor maps of the grid planes for the marches' TMA loads (null: they
+  // load by threads); owned by the caller, which
   // clears it when the instances' grids change
   TmaCache* tma = nullptr;
   // the bistochastized normalisation in n0 / n1 (by the parity of
@@ -142,34 +160,72 @@ struct HfbsBatch {
   const HfbsGradState* grad = nullptr;
 };
 
+// ---- the marching kernels (hfbs_march.cu) -------------------------------------
+// Levels a grid may have for them, and steps per pass over the grid.
+constexpr int kHfbsMarchMaxGL = 64;
+constexpr int kHfbsMarchSteps = 4;
+// How the instances [first, first + count) are cut into blocks.
+struct HfbsMarchPlan {
+  int first = 0, count = 0, warps = 1, rows = 1, ahead = 1;
+  unsigned blocks = 1;  // per instance, at most
+};
+HfbsMarchPlan hfbs_march_plan(const HfbsBatch& B, int first, int count);
+// `steps` (1 .. kHfbsMarchSteps) heavy-ball steps of the plan's instances from
+// (zs, hs) to (zd, hd), other buffers; rec: z after each of the first
+// rec_steps steps, plane stride total_voxels.
+int hfbs_march_solve(const HfbsBatch& B, const HfbsMarchPlan& P, const HParams& p,
+                     const float* norm, const float* zs, float* zd, const float* hs, float* hd,
+                     int steps, float* rec, int rec_steps, cudaStream_t s);
+// `steps` bistochastization iterations from src to dst; it0: index of the
+// first one (its parity is the pad faces' value).
+int hfbs_march_bistoch(const HfbsBatch& B, const HfbsMarchPlan& P, const float* src, float* dst,
+                       int it0, int steps, cudaStream_t s);
+// ---- grids that stay on chip (hfbs_cluster.cu) ---------------------------------
+struct HfbsClusterPlan {
+  int size = 0;  // CTAs of an instance's cluster; 0: the instances do not fit
+  int items = 0, threads = 0, first = 0, count = 0;
+  size_t smem = 0;
+};
+// The cluster that holds each of the instances [first, first + count), or
+// size 0.
+HfbsClusterPlan hfbs_cluster_plan(const HfbsBatch& B, int first, int count);
+// Any number of heavy-ball steps in one launch, bit for bit
+// hfbs_march_solve's; hd null: h is not wanted.
+int hfbs_cluster_solve(const HfbsBatch& B, const HfbsClusterPlan& P, const HParams& p,
+                       const float* norm, const float* zs, float* zd, const float* hs, float* hd,
+                       int steps, float* rec, int rec_steps, cudaStream_t s);
+// All `steps` bistochastization iterations, from ones, into dst.
+int hfbs_cluster_bistoch(const HfbsBatch& B, const HfbsClusterPlan& P, float* dst, int steps,
+                         cudaStream_t s);
+// Builds the tensor maps of grid planes (before a capture).
+void hfbs_march_prepare(const HfbsBatch& B, const std::vector<const float*>& planes,
+                        cudaStream_t s);
+
 // Enqueue the whole HFBS::Optimize sequence (splat .. slice) on a stream.
 int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s);
-
-// Heavy-ball steps per launch of the temporally blocked kernel.
-constexpr int kHfbsTBSteps = 4;
 
 // Builds the grid tensor maps the solve of B will stage from (grid planes
 // b, invA, both z and h buffers, both normalisation buffers, the counts),
 // so that a graph capture of the solve finds them; a no-op without B.tma.
-void hfbs_prepare_tma(const HfbsBatch& B, cudaStream_t s);
+void hfbs_prepare_tma(const HfbsBatch& B, const HParams& p, cudaStream_t s);
 
-// CTAs of the temporally blocked kernels that gave up waiting for their TMA
-// staging since the library was loaded (0 on a healthy run).
+// CTAs of the marching kernels that gave up waiting for their TMA loads since
+// the library was loaded (0 on a healthy run).
 unsigned long long hfbs_wait_timeouts();
 
-// Whether the batch's heavy-ball steps run temporally blocked (every grid
-// at most 16 levels, host instance table given, solve_steps not 1).  Its neighbour sums add
-// rounded z * n products; the one-step kernel's fuse them (FMA).
-bool hfbs_uses_tb(const HfbsBatch& B);
+// Whether the batch's heavy-ball steps and normalisation march (every grid
+// at most kHfbsMarchMaxGL levels, host instance table given, solve_steps not
+// 1).  The march's neighbour sums add rounded z * n products; the one-step
+// kernel's fuse them (FMA).
+bool hfbs_uses_march(const HfbsBatch& B);
 
 // `steps` heavy-ball steps of every instance from (zs, hs) to (zd, hd): one
-// temporally blocked launch (steps <= kHfbsTBSteps), else one one-step launch
-// (steps == 1, h updated in place in hd: the caller passes hs == hd).  rec:
-// z after each of the first rec_steps steps, plane stride total_voxels
-// (temporally blocked launches only).
-void hfbs_launch_steps(const HfbsBatch& B, const HParams& p, const float* norm,
-                       const float* zs, float* zd, const float* hs, float* hd, int steps,
-                       float* rec, int rec_steps, cudaStream_t s);
+// march (steps <= kHfbsMarchSteps), else one one-step launch (steps == 1, h
+// updated in place in hd: the caller passes hs == hd).  rec: z after each of
+// the first rec_steps steps, plane stride total_voxels (marches only).
+int hfbs_launch_steps(const HfbsBatch& B, const HParams& p, const float* norm,
+                      const float* zs, float* zd, const float* hs, float* hd, int steps,
+                      float* rec, int rec_steps, cudaStream_t s);
 
 // X -> Y -> Z Laplace blur of two grids s0, s1 into x0, x1 (y0, y1 scratch).
 void hfbs_launch_blur_pair(const HfbsBatch& B, const HParams& p, const float* s0,

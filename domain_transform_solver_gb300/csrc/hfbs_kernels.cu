@@ -25,9 +25,6 @@ namespace {
 
 constexpr int kT = 256;
 
-// CTAs of this file's kernels that gave up waiting for their TMA staging.
-__device__ unsigned long long g_wait_timeouts = 0;
-
 __device__ __forceinline__ long long gidx(const HInst& I, int x, int y, int z) {
   return I.grid_off + ((long long)z * I.gy + y) * I.px + x;
 }
@@ -600,456 +597,6 @@ __global__ void k_solve(const HInst* __restrict__ insts,
   }
 }
 
-// a16, K steps per pass (temporal blocking).  A CTA loads a 24 x 24 block of
-// (x, y) columns, a 16 x 16 tile plus a K = 4 column halo, with all l levels;
-// each thread keeps the z, h and n of its column in registers (b and invA
-// in shared memory) and the z * n products of a step go through shared
-// memory to the x and y neighbours.  Step k updates the columns at least k
-// inside the block, whose neighbours the previous step updated, so after K
-// steps the tile is exact.  Outside the grid (and above level gl) z = n = 0,
-// so z * n there adds zero to a neighbour sum without bounds tests.  The
-// neighbour sum adds the six rounded products in the reference's order
-// (x-1, x+1, y-1, y+1, l-1, l+1).  HBM traffic is about a quarter of four
-// one-step passes: the halo comes from L2.  h ping-pongs between hs and hd
-// because a neighbouring CTA reads the old h of this tile's columns as its
-// halo.
-//
-// The block arrives by TMA: one cp.async.bulk.tensor load per plane of the
-// 24 x 24 x 16 box (tensor maps of the pitched grids, zeros outside the
-// grid and above level gl), issued by one thread and waited for on an
-// mbarrier; without tensor maps, by 4-byte cp.async copies (zero-filled
-// outside the grid).  z, h and n are staged in the space the z * n buffers
-// use afterwards.  Every thread reads and writes only its own column there,
-// so the reuse needs no barrier.
-constexpr int kTBT = 16, kTBK = 4, kTBL = kTBT + 2 * kTBK;
-static_assert(kTBK == kHfbsTBSteps, "steps per temporally blocked launch");
-constexpr int kTBMaxGL = 16;
-constexpr int kTBThreads = kTBL * kTBL;  // one thread per (x, y) column
-constexpr int kTBPlane = kTBMaxGL * kTBThreads;  // floats per staged array
-// b, invA, then z, h, n staged (later z * n, double-buffered), an mbarrier
-constexpr size_t kTBSmem = sizeof(float) * 5 * kTBPlane + 16;
-constexpr unsigned kTBBoxBytes = sizeof(float) * kTBPlane;  // one plane's box
-
-// Tensor-map tables (one entry per instance of the launch) of the planes a
-// temporally blocked launch stages; all null: staged by 4-byte copies.
-struct TBMaps {
-  const CUtensorMap *b, *a, *z, *h, *n;
-};
-
-// Issues the block's TMA loads (thread 0; the mbarrier initialised for one
-// arrival) of np planes into consecutive kTBPlane regions from dst, and
-// waits, bounded.  False (the same in every thread) when the wait ran out.
-__device__ __forceinline__ bool tb_tma_stage(const CUtensorMap* const* maps, int np, float* dst,
-                                             int x0, int y0, unsigned long long* bar) {
-  if (threadIdx.x == 0) {
-    mbar_init(bar, 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    mbar_arrive_expect_tx(bar, (unsigned)np * kTBBoxBytes);
-    for (int k = 0; k < np; ++k)
-      tma_load_3d(dst + (size_t)k * kTBPlane, maps[k] + blockIdx.y, x0, y0, 0, bar);
-  }
-  const bool ok = mbar_wait_bounded(bar, 0, kTmaWaitPolls);
-  if (__syncthreads_or(!ok)) {
-    if (threadIdx.x == 0) atomicAdd(&g_wait_timeouts, 1ull);
-    (void)mbar_wait_bounded(bar, 0, kTmaWaitPolls);  // copies may still land
-    return false;
-  }
-  return true;
-}
-
-// True when column (xx, yy) of a temporally blocked block is updated at step
-// k: it lies at least k columns inside the block.
-__device__ __forceinline__ bool tb_active(int xx, int yy, int k) {
-  return xx >= k && xx < kTBL - k && yy >= k && yy < kTBL - k;
-}
-
-// 4-byte global -> shared copy; copies zero bytes (the destination is
-// zero-filled) when !valid, and src must then still be a mapped address.
-__device__ __forceinline__ void cp_async_f32(float* dst, const float* src, bool valid) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src),
-               "r"(valid ? 4 : 0)
-               : "memory");
-}
-
-// a13, up to K bistochastization iterations per pass (temporal blocking as
-// in k_solve_tb): a thread per (x, y) column of a 24 x 24 block keeps its
-// column's v in registers (its counts in shared memory), and v goes through
-// shared memory to the x and y neighbours.  Columns past the grid hold what
-// the one-step kernel reads there: the covered pad faces (x = gx, y = gy,
-// and level gl when covered) the pad value of the iteration's parity (1 on
-// even iterations, 0 on odd ones), everything else 0.  The neighbour order
-// and the arithmetic are k_bistoch's, so the result is bitwise that of the
-// one-step passes.  it0: the global index of the pass's first iteration.
-// v x 2 (the first also the staged src), count, an mbarrier
-constexpr size_t kTBBistochSmem = sizeof(float) * 3 * kTBPlane + 16;
-// Small grids only: there one-step passes are launch-latency-bound (about
-// 12 us each on GB300 whatever the size) and four iterations per pass win
-// (a 640x480 colorization's two 80x60x16 grids: 0.097 against 0.246 ms).  At 11.7 M voxels
-// the one-step kernel's 0.056 ms per iteration beats this kernel's 0.063 (one
-// 576-thread CTA per SM, a division and a square root per voxel and
-// iteration), and batches of a few hundred thousand voxels solved side by
-// side on several streams (the pipeline's chunks) hide the one-step
-// latency, where this kernel's large blocks only crowd the SMs.
-constexpr long long kBistochTBMaxVoxels = 1ll << 18;
-
-__global__ void __launch_bounds__(kTBThreads, 1)
-    k_bistoch_tb(const HInst* __restrict__ insts, const float* __restrict__ src,
-                 float* __restrict__ dst, const float* __restrict__ count, int it0,
-                 int steps, const CUtensorMap* __restrict__ msrc,
-                 const CUtensorMap* __restrict__ mcnt) {
-  pdl_wait_then_release();  // launched as a dependent of the previous pass
-  extern __shared__ __align__(128) float tb_s[];
-  float* Cs = tb_s + 2 * kTBPlane;  // counts of the block's columns
-  unsigned long long* bar = reinterpret_cast<unsigned long long*>(tb_s + 3 * kTBPlane);
-  const HInst I = insts[blockIdx.y];
-  const int gx = I.gx, gy = I.gy, gl = I.gl;  // gl <= kTBMaxGL (host checks)
-  const int tiles_x = (gx + kTBT - 1) / kTBT;
-  if ((int)blockIdx.x >= tiles_x * ((gy + kTBT - 1) / kTBT)) return;
-  const int ty = blockIdx.x / tiles_x, tx = blockIdx.x - ty * tiles_x;
-  const int c = threadIdx.x, yy = c / kTBL, xx = c - yy * kTBL;
-  const int x = tx * kTBT - kTBK + xx, y = ty * kTBT - kTBK + yy;
-  const bool in = x >= 0 && x < gx && y >= 0 && y < gy;
-  const bool face = (I.cov_x && x == gx && y >= 0 && y < gy) ||
-                    (I.cov_y && y == gy && x >= 0 && x < gx);
-  const int plane = I.px * gy, col = in ? y * I.px + x : 0;
-  const long long g0 = I.grid_off + col;
-  if (msrc && mcnt && (smem_u32(tb_s) & 127u) == 0) {
-    // src into plane 0 (the first step's exchange then writes plane 1),
-    // the counts into plane 2
-    if (threadIdx.x == 0) {
-      mbar_init(bar, 1);
-      mbar_fence_init();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      mbar_arrive_expect_tx(bar, 2u * kTBBoxBytes);
-      tma_load_3d(tb_s, msrc + blockIdx.y, tx * kTBT - kTBK, ty * kTBT - kTBK, 0, bar);
-      tma_load_3d(Cs, mcnt + blockIdx.y, tx * kTBT - kTBK, ty * kTBT - kTBK, 0, bar);
-    }
-    const bool ok = mbar_wait_bounded(bar, 0, kTmaWaitPolls);
-    if (__syncthreads_or(!ok)) {
-      if (threadIdx.x == 0) atomicAdd(&g_wait_timeouts, 1ull);
-      (void)mbar_wait_bounded(bar, 0, kTmaWaitPolls);
-      return;
-    }
-  } else {
-#pragma unroll
-    for (int l = 0; l < kTBMaxGL; ++l) {
-      const bool v = in && l < gl;
-      const long long i = g0 + (v ? (long long)l * plane : 0);
-      cp_async_f32(tb_s + l * kTBThreads + c, src + i, v);
-      cp_async_f32(Cs + l * kTBThreads + c, count + i, v);
-    }
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-  }
-  float v[kTBMaxGL];
-#pragma unroll
-  for (int l = 0; l < kTBMaxGL; ++l) v[l] = tb_s[l * kTBThreads + c];
-  for (int k = 1; k <= steps; ++k) {
-    const float pad = ((it0 + k - 1) & 1) ? 0.f : 1.f;
-    const float pz = I.cov_l ? pad : 0.f;
-    float* P = tb_s + (k & 1) * kTBPlane;
-#pragma unroll
-    for (int l = 0; l < kTBMaxGL; ++l)
-      P[l * kTBThreads + c] = in ? v[l] : (face && l < gl ? pad : 0.f);
-    __syncthreads();
-    if (in && tb_active(xx, yy, k)) {
-      float below = 0.f;
-#pragma unroll
-      for (int l = 0; l < kTBMaxGL; ++l) {
-        if (l < gl) {
-          const float* q = P + l * kTBThreads + c;
-          const float vc = v[l];
-          float a = q[-1];
-          a += q[1];
-          a += q[-kTBL];
-          a += q[kTBL];
-          a += below;
-          a += l + 1 < gl ? v[l + 1] : pz;
-          const float blurred = 2.f * vc + a;
-          v[l] = __fsqrt_rn(
-              __fdiv_rn(vc * (Cs[l * kTBThreads + c] + 0.00001f), blurred + 0.00001f));
-          below = vc;
-        }
-      }
-    }
-  }
-  if (in && xx >= kTBK && xx < kTBK + kTBT && yy >= kTBK && yy < kTBK + kTBT) {
-    float* o = dst + g0;
-#pragma unroll
-    for (int l = 0; l < kTBMaxGL; ++l)
-      if (l < gl) o[l * plane] = v[l];
-  }
-}
-
-__global__ void __launch_bounds__(kTBThreads, 1)
-    k_solve_tb(const HInst* __restrict__ insts, const float* __restrict__ zs,
-               float* __restrict__ zd, const float* __restrict__ hs, float* __restrict__ hd,
-               const float* __restrict__ norm, const float* __restrict__ b,
-               const float* __restrict__ invA, float lambda, float alpha, float beta,
-               int steps, float* __restrict__ rec, long long rec_stride, int rec_steps,
-               TBMaps m) {
-  pdl_wait_then_release();  // launched as a dependent of the previous pass
-  extern __shared__ __align__(128) float tb_s[];
-  float* Bs = tb_s;
-  float* As = Bs + kTBPlane;
-  float* R = As + kTBPlane;  // z, h, n staging; then z * n [2]
-  unsigned long long* bar = reinterpret_cast<unsigned long long*>(tb_s + 5 * kTBPlane);
-  const HInst I = insts[blockIdx.y];
-  const int gx = I.gx, gy = I.gy, gl = I.gl;  // gl <= kTBMaxGL (host checks)
-  const int tiles_x = (gx + kTBT - 1) / kTBT;
-  if ((int)blockIdx.x >= tiles_x * ((gy + kTBT - 1) / kTBT)) return;
-  const int ty = blockIdx.x / tiles_x, tx = blockIdx.x - ty * tiles_x;
-  const int c = threadIdx.x, yy = c / kTBL, xx = c - yy * kTBL;
-  const int x = tx * kTBT - kTBK + xx, y = ty * kTBT - kTBK + yy;
-  const bool in = x >= 0 && x < gx && y >= 0 && y < gy;
-  const int plane = I.px * gy, col = in ? y * I.px + x : 0;
-  const long long g0 = I.grid_off + col;
-  if (m.b && (smem_u32(tb_s) & 127u) == 0) {
-    // b, invA, z, h, n: the five consecutive plane regions from Bs
-    const CUtensorMap* maps[5] = {m.b, m.a, m.z, m.h, m.n};
-    if (!tb_tma_stage(maps, 5, Bs, tx * kTBT - kTBK, ty * kTBT - kTBK, bar)) return;
-  } else {
-#pragma unroll
-    for (int l = 0; l < kTBMaxGL; ++l) {
-      const bool v = in && l < gl;
-      const long long i = g0 + (v ? (long long)l * plane : 0);
-      cp_async_f32(R + l * kTBThreads + c, zs + i, v);
-      cp_async_f32(R + kTBPlane + l * kTBThreads + c, hs + i, v);
-      cp_async_f32(R + 2 * kTBPlane + l * kTBThreads + c, norm + i, v);
-      cp_async_f32(Bs + l * kTBThreads + c, b + i, v);
-      cp_async_f32(As + l * kTBThreads + c, invA + i, v);
-    }
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-  }
-  float z[kTBMaxGL], h[kTBMaxGL], n[kTBMaxGL];
-#pragma unroll
-  for (int l = 0; l < kTBMaxGL; ++l) {
-    z[l] = R[l * kTBThreads + c];
-    h[l] = R[kTBPlane + l * kTBThreads + c];
-    n[l] = R[2 * kTBPlane + l * kTBThreads + c];
-  }
-  for (int k = 1; k <= steps; ++k) {
-    float* P = R + (k & 1) * kTBPlane;
-#pragma unroll
-    for (int l = 0; l < kTBMaxGL; ++l) P[l * kTBThreads + c] = z[l] * n[l];
-    __syncthreads();
-    if (in && tb_active(xx, yy, k)) {
-      float below = 0.f, cur = z[0] * n[0];
-#pragma unroll
-      for (int l = 0; l < kTBMaxGL; ++l) {
-        const float above = l + 1 < kTBMaxGL ? z[l + 1] * n[l + 1] : 0.f;
-        const float* q = P + l * kTBThreads + c;
-        const float d = q[-1] + q[1] + q[-kTBL] + q[kTBL] + below + above;
-        const float qb = (Bs[l * kTBThreads + c] + lambda * n[l] * d) * As[l * kTBThreads + c];
-        const float grad = z[l] - qb;
-        // |grad| > 1.345 with the double threshold of the reference: the
-        // smallest float above 1.345 (double) is 1.345f
-        const float gc = fabsf(grad) >= 1.345f ? copysignf(1.f, grad) : grad;
-        h[l] = __fmaf_rn(beta, h[l], gc);
-        z[l] = z[l] - alpha * h[l];
-        below = cur;
-        cur = above;
-      }
-    }
-    // iterates kept for the adjoint: z after step k of the tile's columns
-    if (k <= rec_steps && in && xx >= kTBK && xx < kTBK + kTBT && yy >= kTBK &&
-        yy < kTBK + kTBT) {
-      float* zr = rec + (long long)(k - 1) * rec_stride + g0;
-#pragma unroll
-      for (int l = 0; l < kTBMaxGL; ++l)
-        if (l < gl) zr[l * plane] = z[l];
-    }
-  }
-  if (in && xx >= kTBK && xx < kTBK + kTBT && yy >= kTBK && yy < kTBK + kTBT) {
-    float* zo = zd + g0;
-    float* ho = hd + g0;
-#pragma unroll
-    for (int l = 0; l < kTBMaxGL; ++l)
-      if (l < gl) {
-        zo[l * plane] = z[l];
-        ho[l * plane] = h[l];
-      }
-  }
-}
-
-// a16 as k_solve_tb (the same K-step blocks, the same arithmetic in the
-// same order: bitwise the same z and h), in a persistent form that keeps the
-// SM busy while a block is staged.  One CTA per SM walks the launch's
-// blocks L = blockIdx.x, + gridDim.x, ... (the blocks of the (tile,
-// instance) grid that lie inside their instance).  Shared memory: the z, n
-// staging area (two planes), the current block's b and invA (two planes)
-// and the z * n exchange (two planes, alternating by step).  As soon as a
-// block's z and n are in registers, the next block's are requested by TMA
-// into the staging area, so that they arrive while this block is solved;
-// the next b and invA are requested after this block's last step, and a
-// block's h (read by its own column's thread only) comes straight from
-// global memory into registers, in flight during the first exchange.  Each
-// of the two mbarriers completes once per block, so both are waited for
-// with the parity of the block's position in the CTA's walk.  A wait that
-// runs out (bounded) is counted in g_wait_timeouts (as is a shared-memory
-// base that TMA cannot write to); the CTA then waits, bounded, for its
-// copies in flight and returns.
-constexpr size_t kTBPSmem = sizeof(float) * 6 * kTBPlane + 32;
-// registers a thread: warps take registers in groups of four, so the 18
-// warps of a block count as 20 and 65536 / 640 leaves 96
-constexpr int kTBPRegs = 96;
-static_assert(kTBPRegs * 640 <= 65536, "one CTA per SM");
-
-__global__ void __maxnreg__(kTBPRegs)
-    k_solve_tbp(const HInst* __restrict__ insts, int n_inst, int tiles_max,
-                float* __restrict__ zd, const float* __restrict__ hs, float* __restrict__ hd,
-                float lambda, float alpha, float beta, int steps, TBMaps m) {
-  pdl_wait_then_release();  // launched as a dependent of the previous pass
-  extern __shared__ __align__(128) float tb_s[];
-  float* ZS = tb_s;                 // z, n of the block being staged
-  float* Bs = tb_s + 2 * kTBPlane;  // b, invA of the current block
-  float* As = Bs + kTBPlane;
-  float* PP = tb_s + 4 * kTBPlane;  // z * n of a step, two buffers
-  unsigned long long* bar = reinterpret_cast<unsigned long long*>(tb_s + 6 * kTBPlane);
-  const int c = threadIdx.x, yy = c / kTBL, xx = c - yy * kTBL;
-  const long long total = (long long)tiles_max * n_inst;
-  // block L: instance and tile
-  auto decode = [&](long long L, int& inst, int& tx, int& ty) -> bool {
-    inst = (int)(L / tiles_max);
-    const int t = (int)(L - (long long)inst * tiles_max);
-    const int gx = insts[inst].gx, gy = insts[inst].gy;
-    const int tiles_x = (gx + kTBT - 1) / kTBT;
-    ty = t / tiles_x;
-    tx = t - ty * tiles_x;
-    return t < tiles_x * ((gy + kTBT - 1) / kTBT);
-  };
-  // the first block inside its instance at or after L in this CTA's walk
-  auto next_block = [&](long long L) -> long long {
-    int i, tx, ty;
-    for (; L < total; L += gridDim.x)
-      if (decode(L, i, tx, ty)) return L;
-    return -1;
-  };
-  auto issue_zn = [&](long long L) {  // thread 0
-    int i, tx, ty;
-    decode(L, i, tx, ty);
-    const int x0 = tx * kTBT - kTBK, y0 = ty * kTBT - kTBK;
-    mbar_arrive_expect_tx(&bar[0], 2u * kTBBoxBytes);
-    tma_load_3d(ZS, m.z + i, x0, y0, 0, &bar[0]);
-    tma_load_3d(ZS + kTBPlane, m.n + i, x0, y0, 0, &bar[0]);
-  };
-  auto issue_ba = [&](long long L) {  // thread 0
-    int i, tx, ty;
-    decode(L, i, tx, ty);
-    const int x0 = tx * kTBT - kTBK, y0 = ty * kTBT - kTBK;
-    mbar_arrive_expect_tx(&bar[1], 2u * kTBBoxBytes);
-    tma_load_3d(Bs, m.b + i, x0, y0, 0, &bar[1]);
-    tma_load_3d(As, m.a + i, x0, y0, 0, &bar[1]);
-  };
-  long long L = next_block(blockIdx.x);
-  if (L < 0) return;
-  if ((smem_u32(tb_s) & 127u) != 0) {  // TMA destinations need 128-byte alignment
-    if (c == 0) atomicAdd(&g_wait_timeouts, 1ull);
-    return;
-  }
-  if (c == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-  if (c == 0) {
-    issue_zn(L);
-    issue_ba(L);
-  }
-  unsigned ph = 0;  // parity of this block's phase of both barriers
-  for (;;) {
-    int inst, tx, ty;
-    decode(L, inst, tx, ty);
-    const HInst& I = insts[inst];
-    const int gx = I.gx, gy = I.gy, gl = I.gl;
-    const int x = tx * kTBT - kTBK + xx, y = ty * kTBT - kTBK + yy;
-    const bool in = x >= 0 && x < gx && y >= 0 && y < gy;
-    const int plane = I.px * gy, col = in ? y * I.px + x : 0;
-    const long long g0 = I.grid_off + col;
-    // h straight into registers (zero outside the grid and above level gl,
-    // as the staged planes read there)
-    float h[kTBMaxGL];
-#pragma unroll
-    for (int l = 0; l < kTBMaxGL; ++l) h[l] = in && l < gl ? hs[g0 + (long long)l * plane] : 0.f;
-    // this block's z, n
-    const bool ok0 = mbar_wait_bounded(&bar[0], ph, kTmaWaitPolls);
-    if (__syncthreads_or(!ok0)) {
-      if (c == 0) atomicAdd(&g_wait_timeouts, 1ull);
-      (void)mbar_wait_bounded(&bar[0], ph, kTmaWaitPolls);  // copies may still land
-      (void)mbar_wait_bounded(&bar[1], ph, kTmaWaitPolls);
-      return;
-    }
-    float z[kTBMaxGL], n[kTBMaxGL];
-#pragma unroll
-    for (int l = 0; l < kTBMaxGL; ++l) {
-      z[l] = ZS[l * kTBThreads + c];
-      n[l] = ZS[kTBPlane + l * kTBThreads + c];
-    }
-    __syncthreads();  // the staging area is free
-    const long long Ln = next_block(L + gridDim.x);
-    if (c == 0 && Ln >= 0) {
-      fence_proxy_async_shared();
-      issue_zn(Ln);
-    }
-    // this block's b, invA
-    const bool ok1 = mbar_wait_bounded(&bar[1], ph, kTmaWaitPolls);
-    if (__syncthreads_or(!ok1)) {
-      if (c == 0) atomicAdd(&g_wait_timeouts, 1ull);
-      (void)mbar_wait_bounded(&bar[1], ph, kTmaWaitPolls);
-      if (Ln >= 0) (void)mbar_wait_bounded(&bar[0], ph ^ 1u, kTmaWaitPolls);
-      return;
-    }
-    for (int k = 1; k <= steps; ++k) {
-      float* P = PP + (k & 1) * kTBPlane;
-#pragma unroll
-      for (int l = 0; l < kTBMaxGL; ++l) P[l * kTBThreads + c] = z[l] * n[l];
-      __syncthreads();
-      if (in && tb_active(xx, yy, k)) {
-        float below = 0.f, cur = z[0] * n[0];
-#pragma unroll
-        for (int l = 0; l < kTBMaxGL; ++l) {
-          const float above = l + 1 < kTBMaxGL ? z[l + 1] * n[l + 1] : 0.f;
-          const float* q = P + l * kTBThreads + c;
-          const float d = q[-1] + q[1] + q[-kTBL] + q[kTBL] + below + above;
-          const float qb = (Bs[l * kTBThreads + c] + lambda * n[l] * d) * As[l * kTBThreads + c];
-          const float grad = z[l] - qb;
-          // |grad| > 1.345 with the double threshold of the reference: the
-          // smallest float above 1.345 (double) is 1.345f
-          const float gc = fabsf(grad) >= 1.345f ? copysignf(1.f, grad) : grad;
-          h[l] = __fmaf_rn(beta, h[l], gc);
-          z[l] = z[l] - alpha * h[l];
-          below = cur;
-          cur = above;
-        }
-      }
-    }
-    __syncthreads();  // b, invA and the exchange buffers read
-    if (c == 0 && Ln >= 0) {
-      fence_proxy_async_shared();
-      issue_ba(Ln);
-    }
-    if (in && xx >= kTBK && xx < kTBK + kTBT && yy >= kTBK && yy < kTBK + kTBT) {
-      float* zo = zd + g0;
-      float* ho = hd + g0;
-#pragma unroll
-      for (int l = 0; l < kTBMaxGL; ++l)
-        if (l < gl) {
-          zo[l * plane] = z[l];
-          ho[l * plane] = h[l];
-        }
-    }
-    if (Ln < 0) return;
-    L = Ln;
-    ph ^= 1u;
-  }
-}
-
 constexpr int kSliceXTable = 2048;
 
 // The slice's corner values, once per solve: (count * z, count) at every
@@ -1172,29 +719,6 @@ __global__ void k_slice(const HInst* __restrict__ insts,
   }
 }
 
-// The table of tensor maps of grid plane `plane` over B's instances (TMA
-// boxes of the temporally blocked kernels), or null.
-const CUtensorMap* grid_map(const HfbsBatch& B, const float* plane, cudaStream_t s) {
-  if (!B.tma || !B.h_inst || B.max_gl > kTBMaxGL) return nullptr;
-  std::vector<TmaGrid> g(B.n_inst);
-  for (int i = 0; i < B.n_inst; ++i) {
-    const HInst& H = B.h_inst[i];
-    g[i] = TmaGrid{H.grid_off, H.gx, H.gy, H.gl, H.px};
-  }
-  return B.tma->get_grid(g.data(), B.n_inst, plane, kTBL, kTBL, kTBMaxGL, s);
-}
-
-// The five tables of a temporally blocked heavy-ball launch over the
-// instances from `first`; all null when any is missing.
-TBMaps tb_maps(const HfbsBatch& B, int first, const float* zs, const float* hs,
-               const float* norm, cudaStream_t s) {
-  const float* planes[5] = {B.b, B.invA, zs, hs, norm};
-  const CUtensorMap* t[5];
-  for (int k = 0; k < 5; ++k)
-    if (!(t[k] = grid_map(B, planes[k], s))) return TBMaps{};
-  return TBMaps{t[0] + first, t[1] + first, t[2] + first, t[3] + first, t[4] + first};
-}
-
 int blocks_for(long long n) {
   long long b = (n + kT - 1) / kT;
   if (b > 152 * 8) b = 152 * 8;
@@ -1203,47 +727,31 @@ int blocks_for(long long n) {
 
 }  // namespace
 
-unsigned long long hfbs_wait_timeouts() {
-  unsigned long long v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_wait_timeouts, sizeof v) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return 0;
-  }
-  return v;
+void hfbs_prepare_tma(const HfbsBatch& B, const HParams& p, cudaStream_t s) {
+  if (!hfbs_uses_march(B)) return;
+  std::vector<const float*> planes = {B.b, B.invA, B.z0, B.z1, B.h, B.t2, B.n0, B.n1, B.count};
+  if (B.grad && B.grad->segment == 1)  // the kept iterates that start a march
+    for (int it = 0; it < p.optim_iter_max; it += kHfbsMarchSteps)
+      planes.push_back(B.grad->hist + (size_t)it * B.total_voxels);
+  hfbs_march_prepare(B, planes, s);
 }
 
-void hfbs_prepare_tma(const HfbsBatch& B, cudaStream_t s) {
-  for (const float* p : {(const float*)B.b, (const float*)B.invA, (const float*)B.z0,
-                         (const float*)B.z1, (const float*)B.h, (const float*)B.t2,
-                         (const float*)B.n0, (const float*)B.n1, (const float*)B.count})
-    (void)grid_map(B, p, s);
+bool hfbs_uses_march(const HfbsBatch& B) {
+  return B.max_gl <= kHfbsMarchMaxGL && B.h_inst && B.solve_steps != 1;
 }
 
-bool hfbs_uses_tb(const HfbsBatch& B) {
-  return B.max_gl <= kTBMaxGL && B.h_inst && B.solve_steps != 1;
-}
-
-void hfbs_launch_steps(const HfbsBatch& B, const HParams& p, const float* norm,
-                       const float* zs, float* zd, const float* hs, float* hd, int steps,
-                       float* rec, int rec_steps, cudaStream_t s) {
-  prof_begin(s, DTSGB_K_HFBS_SOLVE);
-  if (hfbs_uses_tb(B)) {
-    long long tiles = 1;
-    for (int i = 0; i < B.n_inst; ++i) {
-      const HInst& H = B.h_inst[i];
-      tiles = std::max(tiles, (long long)((H.gx + kTBT - 1) / kTBT) * ((H.gy + kTBT - 1) / kTBT));
-    }
-    cudaFuncSetAttribute(k_solve_tb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTBSmem);
-    k_solve_tb<<<dim3((unsigned)tiles, B.n_inst), kTBThreads, kTBSmem, s>>>(
-        B.d_inst, zs, zd, hs, hd, norm, B.b, B.invA, p.lambda, p.alpha, p.beta, steps, rec,
-        B.total_voxels, rec_steps, tb_maps(B, 0, zs, hs, norm, s));
-  } else {
-    // one step; h in place (hs == hd)
-    const dim3 gr((unsigned)std::min<long long>((B.max_rows + 7) / 8, 4096), B.n_inst);
-    k_solve<<<gr, kT, 0, s>>>(B.d_inst, zs, zd, hd, norm, B.b, B.invA, p.lambda, p.alpha,
-                              p.beta);
-  }
-  prof_end(s, DTSGB_K_HFBS_SOLVE);
+int hfbs_launch_steps(const HfbsBatch& B, const HParams& p, const float* norm,
+                      const float* zs, float* zd, const float* hs, float* hd, int steps,
+                      float* rec, int rec_steps, cudaStream_t s) {
+  ProfScope ps(s, DTSGB_K_HFBS_SOLVE);
+  if (hfbs_uses_march(B))
+    return hfbs_march_solve(B, hfbs_march_plan(B, 0, B.n_inst), p, norm, zs, zd, hs, hd, steps,
+                            rec, rec_steps, s);
+  // one step; h in place (hs == hd)
+  const dim3 gr((unsigned)std::min<long long>((B.max_rows + 7) / 8, 4096), B.n_inst);
+  k_solve<<<gr, kT, 0, s>>>(B.d_inst, zs, zd, hd, norm, B.b, B.invA, p.lambda, p.alpha, p.beta);
+  DTSGB_CUDA(cudaGetLastError());
+  return DTSGB_OK;
 }
 
 void hfbs_launch_blur_pair(const HfbsBatch& B, const HParams& p, const float* s0,
@@ -1344,17 +852,18 @@ int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s) {
       if (p.bistoch_iter_max % 2) std::swap(src, dst);
       continue;
     }
-    long long gvox = 0;  // the group's voxels
-    for (int i = 0; B.h_inst && i < g.count; ++i) {
-      const HInst& H = B.h_inst[g.first + i];
-      gvox += (long long)H.gx * H.gy * H.gl;
-    }
-    if (hfbs_uses_tb(B) && gvox <= kBistochTBMaxVoxels) {
-      // up to kTBK iterations per pass; one pass split in two when the number
-      // of passes and of iterations differ in parity, so that the result
-      // lands in the buffer the one-step ping-pong leaves it in
+    const HfbsClusterPlan CP = hfbs_cluster_plan(B, g.first, g.count);
+    if (CP.size > 0) {  // into the buffer the one-step ping-pong leaves it in
+      if (p.bistoch_iter_max % 2) std::swap(src, dst);
+      ProfScope ps(s, DTSGB_K_HFBS_BISTOCH);
+      if (int st = hfbs_cluster_bistoch(B, CP, src, p.bistoch_iter_max, s)) return st;
+    } else if (hfbs_uses_march(B)) {
+      // up to kHfbsMarchSteps iterations per pass; one pass split in two when
+      // the number of passes and of iterations differ in parity, so that the
+      // result lands in the buffer the one-step ping-pong leaves it in
+      constexpr int K = kHfbsMarchSteps;
       std::vector<int> plan;
-      for (int r = p.bistoch_iter_max; r > 0; r -= kTBK) plan.push_back(std::min(kTBK, r));
+      for (int r = p.bistoch_iter_max; r > 0; r -= K) plan.push_back(std::min(K, r));
       if ((int)(plan.size() % 2) != p.bistoch_iter_max % 2) {
         for (int i = (int)plan.size() - 1; i >= 0; --i)
           if (plan[i] >= 2) {
@@ -1364,24 +873,11 @@ int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s) {
             break;
           }
       }
-      long long tiles = 1;
-      for (int i = 0; i < g.count; ++i) {
-        const HInst& H = B.h_inst[g.first + i];
-        tiles = std::max(tiles, (long long)((H.gx + kTBT - 1) / kTBT) * ((H.gy + kTBT - 1) / kTBT));
-      }
-      DTSGB_CUDA(cudaFuncSetAttribute(k_bistoch_tb, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kTBBistochSmem));
+      const HfbsMarchPlan P = hfbs_march_plan(B, g.first, g.count);
       int it0 = 0;
       for (int steps : plan) {
-        const CUtensorMap* ms = grid_map(B, src, s);
-        const CUtensorMap* mc = ms ? grid_map(B, B.count, s) : nullptr;
-        if (!mc) ms = nullptr;
-        prof_begin(s, DTSGB_K_HFBS_BISTOCH);
-        DTSGB_CUDA(launch_dependent(k_bistoch_tb, dim3((unsigned)tiles, g.count),
-                                    dim3(kTBThreads), kTBBistochSmem, s, B.d_inst + g.first,
-                                    src, dst, B.count, it0, steps, ms ? ms + g.first : nullptr,
-                                    mc ? mc + g.first : nullptr));
-        prof_end(s, DTSGB_K_HFBS_BISTOCH);
+        ProfScope ps(s, DTSGB_K_HFBS_BISTOCH);
+        if (int st = hfbs_march_bistoch(B, P, src, dst, it0, steps, s)) return st;
         std::swap(src, dst);
         it0 += steps;
       }
@@ -1424,21 +920,30 @@ int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s) {
     // iterates kept for the adjoint (HfbsGradState)
     const HfbsGradState& G = *B.grad;
     const int K = p.optim_iter_max, S = G.segment;
-    const bool tb = hfbs_uses_tb(B);
+    const bool tb = hfbs_uses_march(B);
     const long long tv = B.total_voxels;
     const size_t gbytes = (size_t)tv * sizeof(float);
-    if (S == 1) {
+    const HfbsClusterPlan CP = hfbs_cluster_plan(B, 0, ni);
+    if (S == 1 && CP.size > 0 && K > 0) {
+      DTSGB_CUDA(cudaMemcpyAsync(G.hist, B.z0, gbytes, cudaMemcpyDeviceToDevice, s));
+      ProfScope ps(s, DTSGB_K_HFBS_SOLVE);
+      if (int st = hfbs_cluster_solve(B, CP, p, norm, B.z0, B.z1, B.h, nullptr, K, G.hist + tv,
+                                      K - 1, s))
+        return st;
+      zs = B.z1;
+    } else if (S == 1) {
       // z_k in hist plane k; h ping-pongs through the free blur temporary t2
       if (K > 0)
         DTSGB_CUDA(cudaMemcpyAsync(G.hist, B.z0, gbytes, cudaMemcpyDeviceToDevice, s));
       float* hs = B.h;
       float* hd = tb ? B.t2 : B.h;
       for (int it = 0; it < K;) {
-        const int steps = tb ? std::min(kTBK, K - it) : 1;
+        const int steps = tb ? std::min(kHfbsMarchSteps, K - it) : 1;
         float* zout = it + steps < K ? G.hist + (size_t)(it + steps) * tv : B.z1;
         const int rec_steps = tb ? std::min(steps, K - 1 - it) : 0;
-        hfbs_launch_steps(B, p, norm, G.hist + (size_t)it * tv, zout, hs, hd, steps,
-                          G.hist + (size_t)(it + 1) * tv, rec_steps, s);
+        if (int st = hfbs_launch_steps(B, p, norm, G.hist + (size_t)it * tv, zout, hs, hd, steps,
+                                       G.hist + (size_t)(it + 1) * tv, rec_steps, s))
+          return st;
         std::swap(hs, hd);
         it += steps;
       }
@@ -1454,62 +959,39 @@ int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s) {
           DTSGB_CUDA(cudaMemcpyAsync(G.ckh + (size_t)(it / S) * tv, hs, gbytes,
                                      cudaMemcpyDeviceToDevice, s));
         }
-        const int steps = tb ? std::min({kTBK, K - it, S - it % S}) : 1;
-        hfbs_launch_steps(B, p, norm, zs, zd, hs, hd, steps, nullptr, 0, s);
+        const int steps = tb ? std::min({kHfbsMarchSteps, K - it, S - it % S}) : 1;
+        if (int st = hfbs_launch_steps(B, p, norm, zs, zd, hs, hd, steps, nullptr, 0, s))
+          return st;
         std::swap(zs, zd);
         std::swap(hs, hd);
         it += steps;
       }
     }
-  } else if (hfbs_uses_tb(B)) {
-    // K heavy-ball steps per pass; h ping-pongs through the free blur
-    // temporary t2 (its final value is not needed).  The shared-memory limit
-    // is a per-device attribute: set on every call (host-side, cheap).
-    DTSGB_CUDA(cudaFuncSetAttribute(k_solve_tb, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kTBSmem));
-    DTSGB_CUDA(cudaFuncSetAttribute(k_solve_tbp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kTBPSmem));
-    // SMs for the persistent form, 0 when it cannot be resident (then the
-    // kernel with one CTA per block runs)
-    static const int sms = [] {
-      int dev = 0, n = 0, per_sm = 0;
-      if (cudaGetDevice(&dev) != cudaSuccess ||
-          cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve_tbp, kTBThreads,
-                                                        kTBPSmem) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return 0;
-      }
-      return per_sm >= 1 ? n : 0;
-    }();
+  } else if (hfbs_uses_march(B)) {
+    // h ping-pongs through the free blur temporary t2 (its final value is not
+    // needed)
     for (const Group& g : groups) {
       zs = B.z0;
       zd = B.z1;
       float* hs = B.h;
       float* hd = B.t2;
-      long long tiles = 1;
-      for (int i = 0; i < g.count; ++i) {
-        const HInst& H = B.h_inst[g.first + i];
-        tiles = std::max(tiles, (long long)((H.gx + kTBT - 1) / kTBT) * ((H.gy + kTBT - 1) / kTBT));
+      const HfbsClusterPlan CP = hfbs_cluster_plan(B, g.first, g.count);
+      if (CP.size > 0 && p.optim_iter_max > 0) {
+        // (every group ends in the buffer its marches would leave it in)
+        if ((p.optim_iter_max + kHfbsMarchSteps - 1) / kHfbsMarchSteps % 2 == 0) zd = B.z0;
+        ProfScope ps(s, DTSGB_K_HFBS_SOLVE);
+        if (int st = hfbs_cluster_solve(B, CP, p, norm, zs, zd, hs, nullptr, p.optim_iter_max,
+                                        nullptr, 0, s))
+          return st;
+        zs = zd;
+        continue;
       }
-      const dim3 gt((unsigned)tiles, g.count);
-      // the persistent form with tensor maps, one CTA per SM; else one CTA
-      // per block
-      const unsigned gp = (unsigned)std::min<long long>(tiles * g.count, sms > 0 ? sms : 1);
-      for (int it = 0; it < p.optim_iter_max; it += kTBK) {
-        const int steps = std::min(kTBK, p.optim_iter_max - it);
-        const TBMaps maps = tb_maps(B, g.first, zs, hs, norm, s);
-        prof_begin(s, DTSGB_K_HFBS_SOLVE);
-        if (maps.b && sms > 0)
-          DTSGB_CUDA(launch_dependent(k_solve_tbp, dim3(gp), dim3(kTBThreads), kTBPSmem, s,
-                                      B.d_inst + g.first, g.count, (int)tiles, zd, hs, hd,
-                                      p.lambda, p.alpha, p.beta, steps, maps));
-        else
-          DTSGB_CUDA(launch_dependent(k_solve_tb, gt, dim3(kTBThreads), kTBSmem, s,
-                                      B.d_inst + g.first, zs, zd, hs, hd, norm, B.b, B.invA,
-                                      p.lambda, p.alpha, p.beta, steps, (float*)nullptr, 0LL,
-                                      0, maps));
-        prof_end(s, DTSGB_K_HFBS_SOLVE);
+      const HfbsMarchPlan P = hfbs_march_plan(B, g.first, g.count);
+      for (int it = 0; it < p.optim_iter_max; it += kHfbsMarchSteps) {
+        const int steps = std::min(kHfbsMarchSteps, p.optim_iter_max - it);
+        ProfScope ps(s, DTSGB_K_HFBS_SOLVE);
+        if (int st = hfbs_march_solve(B, P, p, norm, zs, zd, hs, hd, steps, nullptr, 0, s))
+          return st;
         std::swap(zs, zd);
         std::swap(hs, hd);
       }

@@ -137,12 +137,17 @@ class TmaCache {
   // the same for grids (3D boxes of bx x by x bl voxels)
   const CUtensorMap* get_grid(const TmaGrid* grids, int n, const float* plane, int bx, int by,
                               int bl, cudaStream_t s);
+  // builds the grid tables of several planes with one upload
+  void prepare_grids(const TmaGrid* grids, int n, const std::vector<const float*>& planes, int bx,
+                     int by, int bl, cudaStream_t s);
   void clear();
 
  private:
-  const CUtensorMap* upload(const std::vector<CUtensorMap>& maps,
-                            const std::tuple<const float*, int, int, int>& key);
-  std::map<std::tuple<const float*, int, int, int>, CUtensorMap*> tables_;
+  using Key = std::tuple<const float*, int, int, int>;
+  bool upload(const std::vector<CUtensorMap>& maps, const std::vector<Key>& keys);
+  const CUtensorMap* find(const Key& key) const;
+  std::map<Key, const CUtensorMap*> tables_;
+  std::vector<CUtensorMap*> allocs_;
 };
 
 }  // namespace dtsgb

@@ -3,9 +3,9 @@
 // the per-owner cache of device tables of tensor maps.
 #include <cudaTypedefs.h>
 
-#include <string>
-
+#include <algorithm>
 #include <mutex>
+#include <string>
 
 #include "../../include/dtsgb.h"
 #include "tma.cuh"
@@ -71,24 +71,6 @@ int tma_encode_grid(CUtensorMap* out, const void* base, const TmaGrid& g, int bx
   return DTSGB_OK;
 }
 
-TmaCache::~TmaCache() { clear(); }
-
-const CUtensorMap* TmaCache::upload(const std::vector<CUtensorMap>& maps,
-                                    const std::tuple<const float*, int, int, int>& key) {
-  CUtensorMap* d = nullptr;
-  if (cudaMalloc((void**)&d, sizeof(CUtensorMap) * maps.size()) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return nullptr;
-  }
-  if (upload_table(d, maps.data(), sizeof(CUtensorMap) * maps.size()) != cudaSuccess) {
-    (void)cudaGetLastError();
-    cudaFree(d);
-    return nullptr;
-  }
-  tables_[key] = d;
-  return d;
-}
-
 // No synchronous copies inside a capture: the caller then stages by loads.
 static bool capturing(cudaStream_t s) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -99,37 +81,74 @@ static bool capturing(cudaStream_t s) {
   return cs != cudaStreamCaptureStatusNone;
 }
 
+TmaCache::~TmaCache() { clear(); }
+
+// One device allocation and one copy for the tables of all keys.
+bool TmaCache::upload(const std::vector<CUtensorMap>& maps, const std::vector<Key>& keys) {
+  CUtensorMap* d = nullptr;
+  if (cudaMalloc((void**)&d, sizeof(CUtensorMap) * maps.size()) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  if (upload_table(d, maps.data(), sizeof(CUtensorMap) * maps.size()) != cudaSuccess) {
+    (void)cudaGetLastError();
+    cudaFree(d);
+    return false;
+  }
+  allocs_.push_back(d);
+  const size_t n = maps.size() / keys.size();
+  for (size_t k = 0; k < keys.size(); ++k) tables_[keys[k]] = d + k * n;
+  return true;
+}
+
+const CUtensorMap* TmaCache::find(const Key& key) const {
+  auto it = tables_.find(key);
+  return it == tables_.end() ? nullptr : it->second;
+}
+
+void TmaCache::prepare_grids(const TmaGrid* grids, int n, const std::vector<const float*>& planes,
+                             int bx, int by, int bl, cudaStream_t s) {
+  if (!grids || n <= 0) return;
+  std::vector<Key> keys;
+  std::vector<CUtensorMap> maps;
+  for (const float* p : planes) {
+    const Key key = std::make_tuple(p, bx, by, 1000 + bl);
+    if (!p || find(key) || std::find(keys.begin(), keys.end(), key) != keys.end()) continue;
+    keys.push_back(key);
+    for (int i = 0; i < n; ++i) {
+      maps.emplace_back();
+      if (tma_encode_grid(&maps.back(), p + grids[i].off, grids[i], bx, by, bl)) return;
+    }
+  }
+  if (!keys.empty() && !capturing(s)) (void)upload(maps, keys);
+}
+
 const CUtensorMap* TmaCache::get_grid(const TmaGrid* grids, int n, const float* plane, int bx,
                                       int by, int bl, cudaStream_t s) {
   if (!grids || n <= 0 || !plane) return nullptr;
-  const auto key = std::make_tuple(plane, bx, by, 1000 + bl);
-  auto it = tables_.find(key);
-  if (it != tables_.end()) return it->second;
-  if (capturing(s)) return nullptr;
-  std::vector<CUtensorMap> maps(n);
-  for (int i = 0; i < n; ++i)
-    if (tma_encode_grid(&maps[i], plane + grids[i].off, grids[i], bx, by, bl)) return nullptr;
-  return upload(maps, key);
+  const Key key = std::make_tuple(plane, bx, by, 1000 + bl);
+  if (!find(key)) prepare_grids(grids, n, {plane}, bx, by, bl, s);
+  return find(key);
 }
 
 void TmaCache::clear() {
-  for (auto& kv : tables_) cudaFree(kv.second);
+  for (CUtensorMap* d : allocs_) cudaFree(d);
+  allocs_.clear();
   tables_.clear();
 }
 
 const CUtensorMap* TmaCache::get(const Inst* h_inst, int n, const float* plane, int box_w,
                                  int box_h, cudaStream_t s) {
   if (!h_inst || n <= 0 || !plane) return nullptr;
-  const auto key = std::make_tuple(plane, box_w, box_h, 0);
-  auto it = tables_.find(key);
-  if (it != tables_.end()) return it->second;
+  const Key key = std::make_tuple(plane, box_w, box_h, 0);
+  if (const CUtensorMap* t = find(key)) return t;
   if (capturing(s)) return nullptr;
   std::vector<CUtensorMap> maps(n);
   for (int i = 0; i < n; ++i)
     if (tma_encode_plane(&maps[i], plane + h_inst[i].off, h_inst[i].w, h_inst[i].h,
                          h_inst[i].pitch, box_w, box_h))
       return nullptr;
-  return upload(maps, key);
+  return upload(maps, {key}) ? find(key) : nullptr;
 }
 
 }  // namespace dtsgb

@@ -114,3 +114,47 @@ def test_device_copies_of_any_alignment(gpu_ready, sizes, shift, flags):
         got = o.cpu().numpy()
         assert np.array_equal(got[shift:shift + t.size].reshape(t.shape), want)
         assert (got[:shift] == -1).all() and (got[shift + t.size:] == -1).all()
+
+
+# ---- HFBS: clusters for grids that stay on chip, marches for the others --------
+@pytest.mark.parametrize("gx,gy,sl,steps,bistoch", [
+    (24, 5, 16.0, 5, 7),     # clusters of one row a CTA, of fewer CTAs than 16
+    (25, 1, 16.0, 6, 2),     # one row: one CTA
+    (1, 9, 255.0, 8, 20),    # one column, one level
+    (22, 17, 16.0, 9, 3),    # 16 CTAs, nine of them with rows
+    (49, 12, 15.0, 3, 1),    # 17 levels: five groups, the last with one
+    (128, 64, 16.0, 4, 6),   # the most a cluster holds: 131072 voxels
+    (129, 64, 16.0, 5, 7),   # one column past it: marches, a last pass of one step
+    (240, 33, 17.0, 7, 3),   # ten strips exactly, 15 levels
+    (71, 30, 4.0, 9, 5),     # 64 levels, the most a march takes
+    (30, 7, 3.95, 9, 5),     # 65 levels: one step per launch
+    (73, 150, 8.0, 4, 4),    # 32 levels, several blocks along y
+])
+def test_grid_solvers_match_the_oracle(gpu_ready, oracle_mod, gx, gy, sl, steps, bistoch):
+    """Normalisation and solution of grids at the edges of the clusters' slabs
+    and the marches' strips, levels and passes, against the FP64 oracle at the
+    parity bar (targets small enough that the Huber clamp stays out)."""
+    D, O = gpu_ready, oracle_mod
+    rng = np.random.default_rng(gx * 100 + gy)
+    w, h = 8 * gx - 3 if gx > 1 else 8, 8 * gy - 5
+    luma = rng.integers(0, 256, (h, w)).astype(np.uint8)
+    rgba = np.repeat(luma[..., None], 4, axis=2)
+    t = rng.uniform(-0.5, 0.5, (h, w)).astype(np.float32)
+    c = (rng.random((h, w)) < 0.3).astype(np.float32)
+    gl = int(np.ceil(255.0 / float(np.float32(sl))))
+    params = dict(sigma_x=8.0, sigma_y=8.0, sigma_l=sl, lambda_=8.0, alpha=1.0, beta=0.9,
+                  bistoch_iter_max=bistoch, optim_iter_max=steps, neg_exp_beta=0.9)
+    dims = (gx + 1, gy + 1, gl + 1)
+    s = D.HFBS(D.ImageDim(w, h), *dims)
+    s.SetFilterParams(D.HFBSGridParams(**params))
+    s.InitFrame(D.COLOR_SPACE.RGB, rgba, t, c)
+    s.Optimize()
+    assert s.GridDims() == (gx, gy, gl)
+    ref, o, st = O.hfbs_solve(rgba, t, c, 0, params, max_grid=dims)
+    assert st == 0
+    norm = o.grid("splat_norm")
+    assert np.abs(s.DebugGrid(3) - norm).max() <= 1e-5 * max(1.0, float(np.abs(norm).max()))
+    assert np.abs(s.DebugGrid(7) - o.grid("z_final")).max() <= P.TOL_REL * P.target_range(t)
+    out = s.Download(D.ImageType.OPTIMIZED_QUANTITY)
+    fin = np.isfinite(ref)
+    assert np.abs(out[fin] - ref[fin]).max() <= P.TOL_REL * P.target_range(t)
