@@ -81,6 +81,9 @@ struct dtsgb_batch_s {
   Tile* d_ti_big = nullptr;  // kIterTW x kIterTH tiles
   Tile* d_ti_small = nullptr;  // kIterSmallTW x kIterSmallTH tiles
   int ntb = 0, nti = 0, nti_big = 0, nti_small = 0;
+  // blocks of the DTS passes for halo pass_halo (several instances only)
+  Tile *d_px = nullptr, *d_py = nullptr;
+  int npx = 0, npy = 0, pass_halo = -1;
   bool small = false;
   long long hfbs_group_voxels = 0;  // L2-resident HFBS group budget (0: off)
   int hfbs_solve_steps = 4;         // heavy-ball steps per launch (4 or 1)
@@ -134,9 +137,7 @@ struct dtsgb_batch_s {
   HParams hhp{};
   Graph g_hbwd;
 
-  // tensor maps of the iterate planes (TMA staging of the iteration) and of
-  // the HFBS grid planes (cleared when the grids change)
-  TmaCache tma;
+  // tensor maps of the HFBS grid planes (cleared when the grids change)
   TmaCache htma;
 
   size_t tsize() const { return st == Storage::F32 ? 4 : 2; }
@@ -184,6 +185,8 @@ void batch_free(dtsgb_batch_t b) {
   dfree(b->d_tb);
   dfree(b->d_ti_big);
   dfree(b->d_ti_small);
+  dfree(b->d_px);
+  dfree(b->d_py);
   b->d_ti = nullptr;
   dfree(b->d_hinst);
   for (auto& p : b->hg) dfree(p);
@@ -235,6 +238,36 @@ DtsGrad grad_view(dtsgb_batch_t b, int n_iter) {
 }
 float* grad_plane_t(dtsgb_batch_t b) { return b->gplanes[b->gplanes.size() - 2]; }
 float* grad_plane_c(dtsgb_batch_t b) { return b->gplanes[b->gplanes.size() - 1]; }
+
+// The block tables of the DTS passes for a halo, and a launch that uses them.
+int ensure_pass_blocks(dtsgb_batch_t b, int halo) {
+  if (b->n == 1 || b->pass_halo == halo) return DTSGB_OK;
+  DTSGB_CUDA(cudaStreamSynchronize(b->stream));  // a solve may still read them
+  drop_graph(b, b->g_dts);
+  drop_graph(b, b->g_bwd);
+  dfree(b->d_px);
+  dfree(b->d_py);
+  b->pass_halo = -1;
+  std::vector<Tile> x, y;
+  dts_pass_blocks(b->inst.data(), b->n, halo, &x, &y);
+  if (int st = dalloc(&b->d_px, x.size())) return st;
+  if (int st = dalloc(&b->d_py, y.size())) return st;
+  DTSGB_CUDA(upload_table(b->d_px, x.data(), x.size() * sizeof(Tile)));
+  DTSGB_CUDA(upload_table(b->d_py, y.data(), y.size() * sizeof(Tile)));
+  b->npx = (int)x.size();
+  b->npy = (int)y.size();
+  b->pass_halo = halo;
+  return DTSGB_OK;
+}
+DtsLaunch iter_launch(dtsgb_batch_t b) {
+  DtsLaunch L{b->d_inst, b->d_ti, b->nti, b->n, b->small, b->d_ti_small, b->nti_small,
+              b->inst.data()};
+  L.d_xblocks = b->d_px;
+  L.d_yblocks = b->d_py;
+  L.n_xblocks = (unsigned)b->npx;
+  L.n_yblocks = (unsigned)b->npy;
+  return L;
+}
 
 // Run `enqueue` directly, or through the solve's CUDA graph (captured on the
 // first call with this key, replayed afterwards).
@@ -958,19 +991,9 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
   const bool iterate = p->loss != DTSGB_L1 && p->num_iterations > 0;
   DtsLaunch Lb{b->d_inst, b->d_tb, b->ntb, b->n};
   Lb.bounds_seg = b->bounds_seg;
-  const DtsLaunch Li{b->d_inst, b->d_ti, b->nti, b->n, b->small, b->d_ti_small,
-                     b->nti_small, &b->tma, b->inst.data()};
-  // the iterate planes' tensor maps exist before any capture (a capture
-  // cannot build them: the kernels would stage by loads)
-  {
-    int bw = 0, bh = 0;
-    dts_iter_tma_box(Li, halo, halo, &bw, &bh);
-    if (bw > 0) {
-      for (float* v : b->v) (void)b->tma.get(b->inst.data(), b->n, v, bw, bh, b->stream);
-      if (b->st == Storage::F32)  // the first iteration reads the target
-        (void)b->tma.get(b->inst.data(), b->n, (const float*)b->target, bw, bh, b->stream);
-    }
-  }
+  if (iterate)
+    if (int st = ensure_pass_blocks(b, halo)) return st;
+  const DtsLaunch Li = iter_launch(b);
   const bool over = overwrite > 0.f && overwrite < 1.f;
   const int n_kept = iterate ? p->num_iterations : 0;
   b->grad_n = -1;
@@ -993,7 +1016,6 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
     int st = ensure_grad_planes(b, n_kept, seg);
     if (st) return st;
   }
-  int res = 0;
   const dtsgb_batch_s::BoundsKey bk{b->guide_gen, rx, ry, p->sigma_z, b->ref_y};
   const bool keep_bounds = b->reuse && std::memcmp(&bk, &b->bkey, sizeof bk) == 0;
   auto bounds = [&]() -> int {
@@ -1008,8 +1030,7 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
       if (st) return st;
       return dts_forward_checkpointed(Li, b->st, mode, grad_view(b, n_kept), b->target,
                                       b->conf, b->bounds, p->lambda, p->step_size, halo,
-                                      p->num_iterations, b->v[0], b->v[1], &res,
-                                      b->stream);
+                                      p->num_iterations, b->v[0], b->v[1], b->stream);
     }
     if (!iterate) return launch_init_var(Li, b->st, b->target, b->v[0], b->stream);
     const float* cur = nullptr;
@@ -1018,20 +1039,15 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
     st = bounds();
     if (st) return st;
     const IterMode mode = p->loss == DTSGB_L2 ? IterMode::L2 : IterMode::CHARB;
-    int a = 0;
     for (int it = 0; it < p->num_iterations; ++it) {
-      st = launch_dts_iter(Li, b->st, mode, cur, b->v[1 - a], b->target,
-                           b->conf, b->bounds, p->lambda, p->step_size, overwrite,
-                           it + 1 < p->num_iterations, halo, halo, b->stream);
+      st = launch_dts_iter(Li, b->st, mode, cur, b->v[1], b->v[0], b->target, b->conf, b->bounds,
+                           p->lambda, p->step_size, overwrite, it + 1 < p->num_iterations, halo,
+                           b->stream);
       if (st) return st;
-      a = 1 - a;
-      cur = b->v[a];
+      cur = b->v[0];
     }
     return DTSGB_OK;
   };
-  res = iterate ? (b->grad ? dts_checkpointed_result_index(p->num_iterations, b->grad_seg)
-                           : p->num_iterations % 2)
-                : 0;
   std::vector<char> key;
   key_append(key, *f);
   key_append(key, *p);
@@ -1047,7 +1063,7 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
     return st;
   }
   if (iterate) b->bkey = bk;
-  b->dts_res = res;
+  b->dts_res = 0;
   if (b->grad) {
     b->grad_n = n_kept;
     b->gopt = *p;
@@ -1104,15 +1120,14 @@ static int batch_backward(dtsgb_batch_t b, const float* const* grad_out,
     if (int st = user_plane_copy(b, const_cast<float* const*>(grad_out), G.g[0], true, 0))
       return st;
   }
-  const DtsLaunch Li{b->d_inst, b->d_ti, b->nti, b->n, b->small, b->d_ti_small,
-                     b->nti_small};
+  const DtsLaunch Li = iter_launch(b);
   const dtsgb_optimize_params p = b->gopt;
   const int halo = (int)b->ghalo;
   auto enqueue = [&]() -> int {
     const IterMode mode = p.loss == DTSGB_L2 ? IterMode::L2 : IterMode::CHARB;
     return dts_backward(Li, b->d_inst, b->n, b->total, b->st, mode, G, b->target, b->conf,
-                        b->bounds, p.lambda, p.step_size, halo, n_iter, grad_plane_t(b),
-                        grad_plane_c(b), b->stream);
+                        b->bounds, p.lambda, p.step_size, halo, n_iter, b->v[1],
+                        grad_plane_t(b), grad_plane_c(b), b->stream);
   };
   std::vector<char> key;
   key_append(key, p);

@@ -414,52 +414,28 @@ int dts_checkpoint_segment(int num_iterations) {
   return best;
 }
 
-// Destination of the iterate v_next of an N-iteration forward from v_cur:
-// -1 = checkpoint plane, else ping-pong plane 0 / 1 (never the one read).
-static int forward_dst(int cur, int next, int n, int seg) {
-  if (next < n && next % seg == 0) return -1;
-  return cur == 0 ? 1 : 0;
-}
-
-int dts_checkpointed_result_index(int num_iterations, int seg) {
-  int cur = 0;
-  for (int it = 0; it < num_iterations; ++it) cur = forward_dst(cur, it + 1, num_iterations, seg);
-  return cur;
-}
-
 int dts_forward_checkpointed(const DtsLaunch& L, Storage st, IterMode mode,
                              const DtsGrad& G, const void* target, const void* conf,
                              const uint32_t* bounds, float lambda, float step, int halo,
-                             int num_iterations, float* v0, float* v1, int* result_idx,
-                             cudaStream_t s) {
-  if (num_iterations <= 0) {
-    *result_idx = 0;
-    return launch_init_var(L, st, target, v0, s);
-  }
-  float* buf[2] = {v0, v1};
+                             int num_iterations, float* v0, float* v1, cudaStream_t s) {
+  if (num_iterations <= 0) return launch_init_var(L, st, target, v0, s);
   const float* cur = nullptr;
   int st_ = first_iterate(L, st, target, v0, &cur, s);
   if (st_) return st_;
-  int ci = 0;
-  for (int it = 0; it < num_iterations; ++it) {
-    const int next = it + 1;
-    const int di = forward_dst(ci, next, num_iterations, G.seg);
-    float* dst = di < 0 ? G.cp[next / G.seg - 1] : buf[di];
-    st_ = launch_dts_iter(L, st, mode, cur, dst, target, conf, bounds, lambda, step, -1.f,
-                          0, halo, halo, s);
+  for (int next = 1; next <= num_iterations; ++next) {
+    float* dst = next < num_iterations && next % G.seg == 0 ? G.cp[next / G.seg - 1] : v0;
+    st_ = launch_dts_iter(L, st, mode, cur, v1, dst, target, conf, bounds, lambda, step, -1.f, 0,
+                          halo, s);
     if (st_) return st_;
     cur = dst;
-    ci = di;
   }
-  // the last iteration never writes a checkpoint
-  *result_idx = ci;
   return DTSGB_OK;
 }
 
 int dts_backward(const DtsLaunch& L, const Inst* d_inst, int n_inst, long long plane,
                  Storage st, IterMode mode, const DtsGrad& G, const void* target,
                  const void* conf, const uint32_t* bounds, float lambda, float step,
-                 int halo, int num_iterations, float* grad_t, float* grad_c,
+                 int halo, int num_iterations, float* tmp, float* grad_t, float* grad_c,
                  cudaStream_t s) {
   if (num_iterations <= 0) {  // v = t: dL/dt = dL/dv, dL/dc = 0
     DTSGB_CUDA(cudaMemsetAsync(grad_t, 0, plane * sizeof(float), s));
@@ -485,8 +461,8 @@ int dts_backward(const DtsLaunch& L, const Inst* d_inst, int n_inst, long long p
       return st_;
     }
     for (int k = 1; k < len; ++k) {
-      int st_ = launch_dts_iter(L, st, mode, k == 1 ? x0 : G.segbuf[k - 1], G.segbuf[k],
-                                target, conf, bounds, lambda, step, -1.f, 0, halo, halo, s);
+      int st_ = launch_dts_iter(L, st, mode, k == 1 ? x0 : G.segbuf[k - 1], tmp, G.segbuf[k],
+                                target, conf, bounds, lambda, step, -1.f, 0, halo, s);
       if (st_) return st_;
     }
     for (int k = len - 1; k >= 0; --k) {

@@ -99,22 +99,17 @@ struct dtsgb_dts_s {
   float b_sx = 0.f, b_sy = 0.f;
   int var_idx = -1;
 
-  // tensor maps of the iterate planes (TMA staging of the iteration),
-  // rebuilt when the image dims change
-  mutable TmaCache tma;
-
   size_t tsize() const { return st == Storage::F32 ? 4 : 2; }
   DtsLaunch launch_b() const { return DtsLaunch{d_inst, d_tb, ntb, 1}; }
   bool small = false;
   DtsLaunch launch_i() const {
     return DtsLaunch{d_inst, d_ti, nti, 1, small, small ? nullptr : d_ti_small, nti_small,
-                     &tma, &h_inst};
+                     &h_inst};
   }
 };
 
 static int dts_layout(dtsgb_dts_t h) {
   h->h_inst = Inst{h->w, h->h, h->pitch, 0, 0};
-  h->tma.clear();
   std::vector<Tile> tb = make_tiles(h->w, h->h, kBoundsTW, kBoundsTH);
   const long long t64 = (long long)((h->w + kIterTW - 1) / kIterTW) *
                         ((h->h + kIterTH - 1) / kIterTH);
@@ -464,16 +459,14 @@ DTSGB_API int dtsgb_dts_optimize(dtsgb_dts_t h, const dtsgb_optimize_params* p,
                     sxr * sxr, h->right_ratio};
     sp = &sa;
   }
-  int a = 0, b = 1;
   for (int it = 0; it < p->num_iterations; ++it) {
-    st = launch_dts_iter(h->launch_i(), h->st, mode, cur, h->v[b],
-                         h->target, h->conf, h->bounds, p->lambda, p->step_size,
-                         overwrite, it + 1 < p->num_iterations, halo, halo, h->stream, sp);
+    st = launch_dts_iter(h->launch_i(), h->st, mode, cur, h->v[1], h->v[0], h->target, h->conf,
+                         h->bounds, p->lambda, p->step_size, overwrite,
+                         it + 1 < p->num_iterations, halo, h->stream, sp);
     if (st) return st;
-    std::swap(a, b);
-    cur = h->v[a];
+    cur = h->v[0];
   }
-  h->var_idx = a;
+  h->var_idx = 0;
   return DTSGB_OK;
 }
 
@@ -670,7 +663,7 @@ DTSGB_API int dtsgb_dts_debug_bounds(dtsgb_dts_t h, int axis, float sigma,
 
 DTSGB_API int dtsgb_wait_timeouts(unsigned long long* count) {
   if (!count) return fail(DTSGB_ERR_INVALID_ARGUMENT, "null argument");
-  *count = dts_wait_timeouts() + hfbs_wait_timeouts();
+  *count = hfbs_wait_timeouts();
   return DTSGB_OK;
 }
 

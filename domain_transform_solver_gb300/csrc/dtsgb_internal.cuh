@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <vector>
 
 namespace dtsgb {
 
@@ -185,8 +186,6 @@ struct ProfScope {
 // DTS launchers (dts_kernels.cu).  All take device pointers and a stream and
 // return a DTSGB_* status.
 // ---------------------------------------------------------------------------
-class TmaCache;
-
 struct DtsLaunch {
   const Inst* d_inst;   // device instance table
   const Tile* d_tiles;  // device tile table for the tile shape in use
@@ -197,10 +196,11 @@ struct DtsLaunch {
   // shared memory of the big tiles (null: none)
   const Tile* d_tiles_small = nullptr;
   int n_tiles_small = 0;
-  // tensor maps of the iterate planes for TMA staging, and the host copy of
-  // the instance table they describe (null: the kernels stage by loads)
-  TmaCache* tma = nullptr;
-  const Inst* h_inst = nullptr;
+  const Inst* h_inst = nullptr;  // host copy of the instance table
+  // several instances: the blocks of the iteration's passes for the halo
+  // (dts_pass_blocks)
+  const Tile *d_xblocks = nullptr, *d_yblocks = nullptr;
+  unsigned n_xblocks = 0, n_yblocks = 0;
   // pixels per thread and axis of the window-bound walks (4, 8 or 16)
   int bounds_seg = 8;
   // the same launch on the small tiles
@@ -245,13 +245,18 @@ struct StereoArgs {
   float offset, lam_p, alpha, ratio;
 };
 
-// One iteration from vin to vout.  feeds: another iteration reads vout, so
-// with overwrite in (0, 1) it holds the target where conf > overwrite (the
-// iterate handed in does so already: the first one is the target).
-int launch_dts_iter(const DtsLaunch& L, Storage st, IterMode mode,
-                    const float* vin, float* vout, const void* target,
-                    const void* conf, const uint32_t* bounds, float lambda,
-                    float step, float overwrite, int feeds, int halo_x, int halo_y,
+// The blocks of the X and the Y pass over n instances: (instance, column
+// block, row block).
+void dts_pass_blocks(const Inst* inst, int n, int halo, std::vector<Tile>* x,
+                     std::vector<Tile>* y);
+// One iteration from vin to vout through tmp (the X results): vout may be vin,
+// tmp neither.  L: the instance tables on the device and the host.  feeds:
+// another iteration reads vout, so with overwrite in (0, 1) it holds the
+// target where conf > overwrite (the iterate handed in does so already: the
+// first one is the target).
+int launch_dts_iter(const DtsLaunch& L, Storage st, IterMode mode, const float* vin, float* tmp,
+                    float* vout, const void* target, const void* conf, const uint32_t* bounds,
+                    float lambda, float step, float overwrite, int feeds, int halo,
                     cudaStream_t s, const StereoArgs* stereo = nullptr);
 // v = target (as float), optionally overwritten nowhere: the initial iterate.
 int launch_init_var(const DtsLaunch& L, Storage st, const void* target,
@@ -288,13 +293,6 @@ int launch_row_prefix(const Inst* h_inst, const Inst* d_inst, int n_inst,
                       const float* in, float* out, cudaStream_t s);
 int launch_unpack_bounds(const DtsLaunch& L, const uint32_t* bounds, int axis,
                          int32_t* l, int32_t* u, cudaStream_t s);
-// CTAs of the iteration kernels that gave up waiting for their TMA staging
-// since the library was loaded (0 on a healthy run).
-unsigned long long dts_wait_timeouts();
-// The box (columns x rows) of the iteration kernel's TMA staging for halos
-// hx, hy on L's tile shape; 0 x 0 when it stages by loads.  An owner builds
-// its tensor maps for that box before a graph capture.
-void dts_iter_tma_box(const DtsLaunch& L, int hx, int hy, int* box_w, int* box_h);
 
 // ---------------------------------------------------------------------------
 // Adjoint of the fixed-window solve (dts_adjoint.cu).
@@ -309,22 +307,18 @@ struct DtsGrad {
 // (near sqrt(N)), taking the smallest such length, which recomputes the
 // fewest iterations.
 int dts_checkpoint_segment(int num_iterations);
-// The forward solve (init + num_iterations fused iterations, no overwrite),
-// writing v_seg, v_2seg, ... into G.cp; the result ends in v0 or v1
-// (*result_idx).
+// The forward solve (num_iterations iterations, no overwrite), writing v_seg,
+// v_2seg, ... into G.cp; the result ends in v0 (v1: the X results).
 int dts_forward_checkpointed(const DtsLaunch& L, Storage st, IterMode mode,
                              const DtsGrad& G, const void* target, const void* conf,
                              const uint32_t* bounds, float lambda, float step, int halo,
-                             int num_iterations, float* v0, float* v1, int* result_idx,
-                             cudaStream_t s);
-// Which of v0 / v1 holds the result of dts_forward_checkpointed.
-int dts_checkpointed_result_index(int num_iterations, int seg);
+                             int num_iterations, float* v0, float* v1, cudaStream_t s);
 // dL/dt and dL/dc (planes of the instance layout, overwritten) for the
-// upstream gradient in G.g[0]; G.g[0] and G.g[1] are clobbered.
+// upstream gradient in G.g[0]; G.g[0], G.g[1] and tmp are clobbered.
 int dts_backward(const DtsLaunch& L, const Inst* d_inst, int n_inst, long long plane,
                  Storage st, IterMode mode, const DtsGrad& G, const void* target,
                  const void* conf, const uint32_t* bounds, float lambda, float step,
-                 int halo, int num_iterations, float* grad_t, float* grad_c,
+                 int halo, int num_iterations, float* tmp, float* grad_t, float* grad_c,
                  cudaStream_t s);
 
 }  // namespace dtsgb

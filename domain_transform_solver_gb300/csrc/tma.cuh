@@ -1,12 +1,10 @@
-// Tensor-memory-accelerator (TMA) staging for sm_103a kernels: inline PTX
-// for mbarriers and cp.async.bulk.tensor, bounded waits, and a host-side
-// cache of tensor maps (one per instance of a batch and per source plane).
+// Tensor-memory-accelerator (TMA) loads for sm_103a kernels: inline PTX for
+// mbarriers and cp.async.bulk.tensor, bounded waits, and a host-side cache of
+// tensor maps (one per instance of a batch and per source plane).
 //
-// A tensor map describes one instance's plane as a 2D tensor of W x H
-// 4-byte elements with a row pitch of `pitch` elements (a multiple of 32,
-// so every row starts on a 128-byte boundary).  A tiled load of a box that
-// reaches past the image (negative coordinates, x >= W, y >= H) reads zeros
-// there, which is what the staging kernels need at image borders.  The
+// A tensor map describes one instance's grid as a 3D tensor of 4-byte voxels
+// (rows padded to a multiple of four).  A tiled load of a box that reaches past
+// the grid (negative coordinates, x >= gx, ...) reads zeros there.  The
 // innermost start coordinate times 4 bytes must be a multiple of 16: the
 // kernels start boxes at multiples of 4 columns.
 #pragma once
@@ -62,17 +60,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsig
   return false;
 }
 
-// 2D tiled load of the box at (x, y) of tensor map `tmap` (global memory)
-// into shared memory at dst (128-byte aligned), completing on `bar`.
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tmap, int x, int y,
-                                            unsigned long long* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<unsigned long long>(tmap)), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
-
 // 3D tiled load of the box at (x, y, z) of tensor map `tmap` into shared
 // memory at dst (128-byte aligned), completing on `bar`.
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* tmap, int x, int y,
@@ -102,11 +89,6 @@ constexpr unsigned kTmaWaitPolls = 1u << 22;
 // Host side.
 // ---------------------------------------------------------------------------
 
-// Encodes a tensor map of one 4-byte-element plane (W x H, row pitch in
-// elements) with a box of box_w x box_h elements; a DTSGB_* status.
-int tma_encode_plane(CUtensorMap* out, const void* base, int w, int h, int pitch, int box_w,
-                     int box_h);
-
 // One instance's 3D grid inside a grid plane: gx x gy x gl 4-byte voxels at
 // element offset off, rows of px voxels (px a multiple of 4).
 struct TmaGrid {
@@ -120,7 +102,7 @@ int tma_encode_grid(CUtensorMap* out, const void* base, const TmaGrid& g, int bx
                     int bl);
 
 // Device tables of tensor maps, one entry per instance, for a source plane
-// (the arena base of a per-pixel plane or of a grid plane) and a box shape;
+// (the arena base of a grid plane) and a box shape;
 // built on first use (never while the stream is being captured) and kept
 // until clear() or destruction.  The owner clears the cache when the
 // instances' geometry changes.
@@ -130,11 +112,9 @@ class TmaCache {
   TmaCache(const TmaCache&) = delete;
   TmaCache& operator=(const TmaCache&) = delete;
   ~TmaCache();
-  // the table for `plane` (instances h_inst[0..n)), or nullptr when it is
-  // not built and cannot be built now (capture in progress, failure)
-  const CUtensorMap* get(const Inst* h_inst, int n, const float* plane, int box_w, int box_h,
-                         cudaStream_t s);
-  // the same for grids (3D boxes of bx x by x bl voxels)
+  // the table for grid plane `plane` (boxes of bx x by x bl voxels), or
+  // nullptr when it is not built and cannot be built now (capture in
+  // progress, failure)
   const CUtensorMap* get_grid(const TmaGrid* grids, int n, const float* plane, int bx, int by,
                               int bl, cudaStream_t s);
   // builds the grid tables of several planes with one upload

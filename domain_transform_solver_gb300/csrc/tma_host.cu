@@ -31,26 +31,6 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 }  // namespace
 
-int tma_encode_plane(CUtensorMap* out, const void* base, int w, int h, int pitch, int box_w,
-                     int box_h) {
-  auto fn = encode_fn();
-  if (!fn) return fail(DTSGB_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
-  if (box_w <= 0 || box_w > 256 || box_h <= 0 || box_h > 256 || (box_w * 4) % 16 != 0 ||
-      ((uintptr_t)base & 15) != 0 || (pitch * 4) % 16 != 0)
-    return fail(DTSGB_ERR_UNSUPPORTED, "plane or box outside the TMA limits");
-  const cuuint64_t dims[2] = {(cuuint64_t)w, (cuuint64_t)h};
-  const cuuint64_t strides[1] = {(cuuint64_t)pitch * 4};
-  const cuuint32_t box[2] = {(cuuint32_t)box_w, (cuuint32_t)box_h};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims,
-                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS)
-    return fail(DTSGB_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
-  return DTSGB_OK;
-}
-
 int tma_encode_grid(CUtensorMap* out, const void* base, const TmaGrid& g, int bx, int by,
                     int bl) {
   auto fn = encode_fn();
@@ -135,20 +115,6 @@ void TmaCache::clear() {
   for (CUtensorMap* d : allocs_) cudaFree(d);
   allocs_.clear();
   tables_.clear();
-}
-
-const CUtensorMap* TmaCache::get(const Inst* h_inst, int n, const float* plane, int box_w,
-                                 int box_h, cudaStream_t s) {
-  if (!h_inst || n <= 0 || !plane) return nullptr;
-  const Key key = std::make_tuple(plane, box_w, box_h, 0);
-  if (const CUtensorMap* t = find(key)) return t;
-  if (capturing(s)) return nullptr;
-  std::vector<CUtensorMap> maps(n);
-  for (int i = 0; i < n; ++i)
-    if (tma_encode_plane(&maps[i], plane + h_inst[i].off, h_inst[i].w, h_inst[i].h,
-                         h_inst[i].pitch, box_w, box_h))
-      return nullptr;
-  return upload(maps, {key}) ? find(key) : nullptr;
 }
 
 }  // namespace dtsgb

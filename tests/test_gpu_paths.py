@@ -158,3 +158,39 @@ def test_grid_solvers_match_the_oracle(gpu_ready, oracle_mod, gx, gy, sl, steps,
     out = s.Download(D.ImageType.OPTIMIZED_QUANTITY)
     fin = np.isfinite(ref)
     assert np.abs(out[fin] - ref[fin]).max() <= P.TOL_REL * P.target_range(t)
+
+
+# ---- DTS passes ---------------------------------------------------------------
+@pytest.mark.parametrize("w,h,sz", [
+    (236, 40, 8.0),     # a row of one X segment exactly (two rounds)
+    (237, 33, 8.0),     # one column past it; a second Y tile of one row
+    (365, 200, 16.5),   # three rounds; the widest halo of 8 rows a warp
+    (493, 1100, 17.0),  # four rounds, one column past; 16 rows a warp
+    (900, 600, 56.0), (900, 600, 57.0),     # 16 | 32 rows a warp
+    (780, 720, 61.0),   # halos of more than one round
+    (777, 700, 127.9), (777, 700, 128.0),   # 12 | 16 warps a tile
+    (700, 760, 201.0),  # 20 warps
+    (60, 50, 253.9),    # the widest halo, wider than the image
+    (5000, 3, 30.0), (3, 5000, 30.0),
+])
+def test_passes_match_the_oracle(gpu_ready, oracle_mod, w, h, sz):
+    """Segment, tile and halo edges of both passes, alone and in a batch of two
+    (other launch shapes, the same bits), against the FP64 oracle on the GPU's
+    windows, within the parity bar."""
+    from domain_transform_solver_gb300 import workloads as W
+    from test_gpu_dts import _run_dts
+    D, O = gpu_ready, oracle_mod
+    inst = W.depth_sr_instance(17 + w, w, h, n_poly=7, sample_frac=0.2)
+    other = W.depth_sr_instance(18 + w, 700, 800, n_poly=7, sample_frac=0.2)
+    opt = dict(W.CFG0_OPT, num_iterations=3, sigma_z=sz)
+    v, s = _run_dts(D, inst, 1, W.CFG0_FILTER, opt)
+    szf = float(np.float32(sz))
+    win = {(a, szf): s.DebugBounds(a, szf) for a in (0, 1)}
+    ref, _ = O.dts_solve(inst.rgba, inst.target, inst.confidence, 1, W.CFG0_FILTER, opt,
+                         overrides=win)
+    assert np.abs(v - ref).max() <= P.TOL_REL * P.target_range(inst.target)
+    b = D.Batch([(w, h), (700, 800)])
+    b.upload(D.COLOR_SPACE.YCbCr, [inst.rgba, other.rgba], [inst.target, other.target],
+             [inst.confidence, other.confidence])
+    b.solve_dts(D.DomainFilterParams(**W.CFG0_FILTER), D.DomainOptimizeParams(**opt))
+    assert np.array_equal(b.download(0)[0], v)
