@@ -169,6 +169,9 @@ def _declare(lib: ctypes.CDLL) -> None:
                                      P(OptimizeParams), f, vp, vp], i),
         "dtsgb_soft_create": ([i, P(i), P(i), pvp], i),
         "dtsgb_soft_destroy": ([vp], i),
+        "dtsgb_soft_create_bare": ([i, P(i), P(i), pvp], i),
+        "dtsgb_soft_workspace": ([vp, i, P(ctypes.c_longlong)], i),
+        "dtsgb_soft_lend": ([vp, vp, ctypes.c_longlong], i),
         "dtsgb_soft_set_stream": ([vp, vp], i),
         "dtsgb_soft_edge_weights": ([vp, i, pvp, P(FilterParams), pvp, pvp], i),
         "dtsgb_soft_solve": ([vp, pvp, pvp, pvp, pvp, P(OptimizeParams), f, pvp], i),

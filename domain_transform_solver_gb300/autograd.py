@@ -23,8 +23,9 @@ import threading
 import numpy as np
 import torch
 
+from ._lib import DtsgbError
 from .solvers import (COLOR_SPACE, HFBS, Batch, DomainFilterParams, DomainOptimizeParams,
-                      HFBSGridParams, ImageDim, ImageType, SoftDTS)
+                      HFBSGridParams, ImageDim, ImageType, RobustLoss, SoftDTS)
 
 __all__ = ["DtsSolveFunction", "dts_solve", "HfbsSolveFunction", "hfbs_solve",
            "SoftDtsSolveFunction", "soft_dts_solve", "edge_weights"]
@@ -140,12 +141,15 @@ def _hfbs_max_grid(w, h, p: HFBSGridParams):
 
 
 def _take_hfbs(key):
+    """A handle with a stream of its own (`side`): a batch's solves overlap."""
     with _pool_lock:
         free = _pool.get(key)
         if free:
             return free.pop()
-    _, h, w, gx, gy, gl = key
-    return HFBS(ImageDim(w, h), gx, gy, gl)
+    _, device, h, w, gx, gy, gl = key
+    s = HFBS(ImageDim(w, h), gx, gy, gl)
+    s.side = torch.cuda.Stream(device)
+    return s
 
 
 class HfbsSolveFunction(torch.autograd.Function):
@@ -172,22 +176,23 @@ class HfbsSolveFunction(torch.autograd.Function):
         c = confidence.contiguous()
         g = rgba.contiguous()
         gx, gy, gl = max_grid or _hfbs_max_grid(W, H, grid_params)
-        key = ("hfbs", H, W, gx, gy, gl)
+        key = ("hfbs", t.device, H, W, gx, gy, gl)
         out = torch.empty_like(t)
         cur = torch.cuda.current_stream(t.device)
-        side = _side_stream(t.device)
-        side.wait_stream(cur)
+        ready = cur.record_event()
         solvers = []
         for i in range(B):
             s = _take_hfbs(key)
-            s.SetStream(side.cuda_stream)
+            s.side.wait_event(ready)
+            s.SetStream(s.side.cuda_stream)
             s.EnableGrad(True, int(segment))
             s.InitFrameDevice(color_space, g[i].data_ptr(), t[i].data_ptr(), c[i].data_ptr())
             s.SetFilterParams(grid_params)
             s.Optimize()
             s.DownloadDevice(ImageType.OPTIMIZED_QUANTITY, out[i].data_ptr())
             solvers.append(s)
-        cur.wait_stream(side)
+        for s in solvers:
+            cur.wait_stream(s.side)
         ctx.solvers, ctx.key = solvers, key
         return out
 
@@ -198,13 +203,14 @@ class HfbsSolveFunction(torch.autograd.Function):
         gt = torch.empty_like(go)
         gc = torch.empty_like(go)
         cur = torch.cuda.current_stream(go.device)
-        side = _side_stream(go.device)
-        side.wait_stream(cur)
+        ready = cur.record_event()
         for i, s in enumerate(ctx.solvers):
-            s.SetStream(side.cuda_stream)
+            s.side.wait_event(ready)
+            s.SetStream(s.side.cuda_stream)
             s.BackwardDevice(go[i].data_ptr(), gt[i].data_ptr() if need_t else None,
                              gc[i].data_ptr() if need_c else None)
-        cur.wait_stream(side)
+        for s in ctx.solvers:
+            cur.wait_stream(s.side)
         with _pool_lock:
             _pool.setdefault(ctx.key, []).extend(ctx.solvers)
         ctx.solvers = None
@@ -243,6 +249,30 @@ def edge_weights(rgba: torch.Tensor, filter_params: DomainFilterParams | None = 
     return dh, dv
 
 
+# Free soft handles, the oldest first.  A handle keeps an instance table; its
+# image planes come from PyTorch's allocator for one forward and backward.
+_soft_free: list = []
+_SOFT_FREE_MOST = 32
+
+
+def _take_soft(key):
+    with _pool_lock:
+        for i, (k, s) in enumerate(_soft_free):
+            if k == key:
+                del _soft_free[i]
+                return s
+    _, b, h, w = key
+    return SoftDTS([(w, h)] * b, bare=True)
+
+
+def _give_back_soft(key, s):
+    with _pool_lock:
+        _soft_free.append((key, s))
+        old = _soft_free.pop(0)[1] if len(_soft_free) > _SOFT_FREE_MOST else None
+    if old is not None:
+        old.close()
+
+
 class SoftDtsSolveFunction(torch.autograd.Function):
     """v = soft-window DTS(dH, dV; target, confidence) for a batch of
     equal-size images, differentiable in all four inputs.
@@ -260,14 +290,24 @@ class SoftDtsSolveFunction(torch.autograd.Function):
             raise ValueError("dH, dV, target and confidence must share one [B,H,W] shape")
         B, H, W = target.shape
         dh, dv, t, c = (x.contiguous() for x in ts)
-        s = SoftDTS([(W, H)] * B)
-        cur = torch.cuda.current_stream(t.device)
-        s.set_stream(cur.cuda_stream)
+        key = (t.device, B, H, W)
+        s = _take_soft(key)
+        n = s.workspace(0 if int(optimize_params.loss) == int(RobustLoss.L1)
+                        else optimize_params.num_iterations)
+        try:
+            work = torch.empty(n, dtype=torch.float32, device=t.device)
+        except torch.OutOfMemoryError as e:
+            raise DtsgbError(5, str(e)) from None
         out = torch.empty_like(t)
+        cur = torch.cuda.current_stream(t.device)
+        side = _side_stream(t.device)
+        side.wait_stream(cur)
+        s.set_stream(side.cuda_stream)
+        s.lend(work.data_ptr(), n)
         s.solve(_ptrs(dh), _ptrs(dv), _ptrs(t), _ptrs(c), optimize_params, float(tau),
                 _ptrs(out))
-        ctx.soft = s
-        ctx.keep = (dh, dv, t, c)
+        cur.wait_stream(side)
+        ctx.soft, ctx.key, ctx.work = s, key, work
         return out
 
     @staticmethod
@@ -275,11 +315,16 @@ class SoftDtsSolveFunction(torch.autograd.Function):
         s = ctx.soft
         go = grad_out.contiguous().float()
         grads = [torch.empty_like(go) if need else None for need in ctx.needs_input_grad[:4]]
-        s.set_stream(torch.cuda.current_stream(go.device).cuda_stream)
+        cur = torch.cuda.current_stream(go.device)
+        side = _side_stream(go.device)
+        side.wait_stream(cur)
+        s.set_stream(side.cuda_stream)
         s.backward(_ptrs(go), *[None if g is None else _ptrs(g) for g in grads[2:]],
                    *[None if g is None else _ptrs(g) for g in grads[:2]])
-        s.close()
-        ctx.soft = ctx.keep = None
+        cur.wait_stream(side)
+        s.lend(None)
+        _give_back_soft(ctx.key, s)
+        ctx.soft = ctx.work = None
         return (*grads, None, None)
 
 

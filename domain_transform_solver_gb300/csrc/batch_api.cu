@@ -923,6 +923,7 @@ DTSGB_API int dtsgb_batch_destroy(dtsgb_batch_t b) {
 
 DTSGB_API int dtsgb_batch_set_stream(dtsgb_batch_t b, void* stream) {
   if (!b) return fail(DTSGB_ERR_INVALID_ARGUMENT, "null handle");
+  if (!b->own_stream && same_stream(b->stream, stream)) return DTSGB_OK;
   DTSGB_CUDA(cudaStreamSynchronize(b->stream));
   if (b->own_stream) cudaStreamDestroy(b->stream);
   b->own_stream = false;

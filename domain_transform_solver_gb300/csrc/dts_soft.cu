@@ -1192,6 +1192,7 @@ struct dtsgb_soft_s {
   bool own_stream = false;
   SInst* d_inst = nullptr;
   float* arena = nullptr;
+  bool lent = false;  // the arena is the caller's (dtsgb_soft_lend)
   int planes = 0;
   int n_iter = -1;  // iterations of the last solve (-1: none to differentiate)
   dtsgb_optimize_params opt{};
@@ -1217,6 +1218,7 @@ dim3 soft_grid(const dtsgb_soft_s* s) {
 
 int ensure_planes(dtsgb_soft_t s, int planes) {
   if (planes <= s->planes) return DTSGB_OK;
+  if (s->lent) return fail(DTSGB_ERR_INVALID_ARGUMENT, "the lent workspace is too small");
   DTSGB_CUDA(cudaStreamSynchronize(s->stream));
   dfree(s->arena);
   s->planes = 0;
@@ -1500,10 +1502,8 @@ int copy_planes(dtsgb_soft_t s, const float* const* src, int k, bool in) {
 
 }  // namespace
 
-extern "C" {
-
-DTSGB_API int dtsgb_soft_create(int n, const int* widths, const int* heights,
-                                dtsgb_soft_t* out) {
+static int soft_create(int n, const int* widths, const int* heights, bool arena,
+                       dtsgb_soft_t* out) {
   if (!out || !widths || !heights || n <= 0)
     return fail(DTSGB_ERR_INVALID_ARGUMENT, "bad arguments");
   *out = nullptr;
@@ -1536,7 +1536,7 @@ DTSGB_API int dtsgb_soft_create(int n, const int* widths, const int* heights,
     return st;
   }
   s->own_stream = true;
-  if ((st = ensure_planes(s, P_ITER + 2))) {
+  if (arena && (st = ensure_planes(s, P_ITER + 2))) {
     dtsgb_soft_destroy(s);
     return st;
   }
@@ -1544,10 +1544,43 @@ DTSGB_API int dtsgb_soft_create(int n, const int* widths, const int* heights,
   return DTSGB_OK;
 }
 
+extern "C" {
+
+DTSGB_API int dtsgb_soft_create(int n, const int* widths, const int* heights,
+                                dtsgb_soft_t* out) {
+  return soft_create(n, widths, heights, true, out);
+}
+
+DTSGB_API int dtsgb_soft_create_bare(int n, const int* widths, const int* heights,
+                                     dtsgb_soft_t* out) {
+  return soft_create(n, widths, heights, false, out);
+}
+
+DTSGB_API int dtsgb_soft_workspace(dtsgb_soft_t s, int num_iterations, long long* floats) {
+  if (!s || !floats) return fail(DTSGB_ERR_INVALID_ARGUMENT, "null argument");
+  const long long n = std::max(num_iterations, 0);
+  *floats = std::max<long long>(P_ITER + 6 * n + 1, P_ITER + 2) * s->total;
+  return DTSGB_OK;
+}
+
+DTSGB_API int dtsgb_soft_lend(dtsgb_soft_t s, float* workspace, long long floats) {
+  if (!s || (workspace && floats < 0)) return fail(DTSGB_ERR_INVALID_ARGUMENT, "bad arguments");
+  if ((uintptr_t)workspace % 128) return fail(DTSGB_ERR_INVALID_ARGUMENT, "unaligned workspace");
+  if (!s->lent && s->arena) {
+    DTSGB_CUDA(cudaStreamSynchronize(s->stream));
+    dfree(s->arena);
+  }
+  s->arena = workspace;
+  s->lent = workspace != nullptr;
+  s->planes = workspace ? (int)std::min<long long>(floats / s->total, 1 << 30) : 0;
+  s->n_iter = -1;
+  return DTSGB_OK;
+}
+
 DTSGB_API int dtsgb_soft_destroy(dtsgb_soft_t s) {
   if (!s) return DTSGB_OK;
   if (s->stream) cudaStreamSynchronize(s->stream);
-  dfree(s->arena);
+  if (!s->lent) dfree(s->arena);
   dfree(s->d_inst);
   dfree(s->d_emin);
   dfree(s->d_stat);
@@ -1558,6 +1591,7 @@ DTSGB_API int dtsgb_soft_destroy(dtsgb_soft_t s) {
 
 DTSGB_API int dtsgb_soft_set_stream(dtsgb_soft_t s, void* stream) {
   if (!s) return fail(DTSGB_ERR_INVALID_ARGUMENT, "null handle");
+  if (!s->own_stream && same_stream(s->stream, stream)) return DTSGB_OK;
   DTSGB_CUDA(cudaStreamSynchronize(s->stream));
   if (s->own_stream) cudaStreamDestroy(s->stream);
   s->own_stream = stream == nullptr;

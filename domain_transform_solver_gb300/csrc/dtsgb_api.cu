@@ -217,6 +217,7 @@ DTSGB_API int dtsgb_dts_destroy(dtsgb_dts_t h) {
 
 DTSGB_API int dtsgb_dts_set_stream(dtsgb_dts_t h, void* stream) {
   if (!h) return fail(DTSGB_ERR_INVALID_ARGUMENT, "null handle");
+  if (!h->own_stream && same_stream(h->stream, stream)) return DTSGB_OK;
   DTSGB_CUDA(cudaStreamSynchronize(h->stream));
   if (h->own_stream) cudaStreamDestroy(h->stream);
   h->own_stream = false;
@@ -895,6 +896,7 @@ DTSGB_API int dtsgb_hfbs_destroy(dtsgb_hfbs_t h) {
 
 DTSGB_API int dtsgb_hfbs_set_stream(dtsgb_hfbs_t h, void* stream) {
   if (!h) return fail(DTSGB_ERR_INVALID_ARGUMENT, "null handle");
+  if (!h->own_stream && same_stream(h->stream, stream)) return DTSGB_OK;
   DTSGB_CUDA(cudaStreamSynchronize(h->stream));
   if (h->own_stream) cudaStreamDestroy(h->stream);
   h->own_stream = false;

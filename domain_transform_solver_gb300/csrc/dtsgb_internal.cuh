@@ -147,6 +147,13 @@ int dalloc(T** p, size_t count) {
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemset");
   return 0;
 }
+// A handle told to use the stream that it uses: its work is in order there and
+// waits for nothing.  A stream under capture takes the general way (refused).
+inline bool same_stream(cudaStream_t cur, void* next) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  return next && (void*)cur == next && cudaStreamIsCapturing(cur, &c) == cudaSuccess &&
+         c == cudaStreamCaptureStatusNone;
+}
 // Host table -> device, complete on return: cudaMemcpy from pageable memory
 // may return while the transfer still runs on the legacy default stream,
 // which the handles' non-blocking streams do not wait for, and a kernel on

@@ -816,14 +816,16 @@ class SoftDTS:
     are lists of device pointers (ints), one per instance, as in
     include/dtsgb.h's dtsgb_soft_* calls."""
 
-    def __init__(self, sizes):
+    def __init__(self, sizes, bare=False):
+        """bare: without image planes of its own (lend)."""
         self._lib = _lib.load()
         self.sizes = [(int(w), int(h)) for w, h in sizes]
         n = len(self.sizes)
         ws = (ctypes.c_int * n)(*[w for w, _ in self.sizes])
         hs = (ctypes.c_int * n)(*[h for _, h in self.sizes])
         s = ctypes.c_void_p()
-        check(self._lib.dtsgb_soft_create(n, ws, hs, ctypes.byref(s)))
+        create = self._lib.dtsgb_soft_create_bare if bare else self._lib.dtsgb_soft_create
+        check(create(n, ws, hs, ctypes.byref(s)))
         self._h = s
 
     def close(self) -> None:
@@ -839,6 +841,16 @@ class SoftDTS:
 
     def set_stream(self, stream_handle: int | None) -> None:
         check(self._lib.dtsgb_soft_set_stream(self._h, ctypes.c_void_p(stream_handle or 0)))
+
+    def workspace(self, num_iterations: int) -> int:
+        """Floats that a solve of num_iterations and its adjoint take."""
+        n = ctypes.c_longlong()
+        check(self._lib.dtsgb_soft_workspace(self._h, int(num_iterations), ctypes.byref(n)))
+        return n.value
+
+    def lend(self, ptr: int | None, floats: int = 0) -> None:
+        """Device memory for the handle's planes, the caller's, until the next lend."""
+        check(self._lib.dtsgb_soft_lend(self._h, ctypes.c_void_p(ptr or 0), int(floats)))
 
     def edge_weights(self, color_space, rgba_ptrs, filter_params, dh_ptrs, dv_ptrs) -> None:
         check(self._lib.dtsgb_soft_edge_weights(self._h, int(color_space),

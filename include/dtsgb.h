@@ -321,6 +321,16 @@ typedef struct dtsgb_soft_s* dtsgb_soft_t;
 DTSGB_API int dtsgb_soft_create(int n, const int* widths, const int* heights,
                                 dtsgb_soft_t* out);
 DTSGB_API int dtsgb_soft_destroy(dtsgb_soft_t s);
+/* A handle whose image planes are lent to it: dtsgb_soft_workspace returns the
+ * floats that a solve of num_iterations and its adjoint take, dtsgb_soft_lend
+ * hands that much device memory (128-byte aligned, any content) to the handle
+ * until the next lend; NULL ends the loan.  The memory is the caller's: it has
+ * to outlive the handle's work, and a lend forgets the last solve.  A call
+ * that needs more planes than were lent is refused. */
+DTSGB_API int dtsgb_soft_create_bare(int n, const int* widths, const int* heights,
+                                     dtsgb_soft_t* out);
+DTSGB_API int dtsgb_soft_workspace(dtsgb_soft_t s, int num_iterations, long long* floats);
+DTSGB_API int dtsgb_soft_lend(dtsgb_soft_t s, float* workspace, long long floats);
 DTSGB_API int dtsgb_soft_set_stream(dtsgb_soft_t s, void* cuda_stream);
 /* The guide-derived edge weights dH, dV of ComputeColorSpaceDifferential
  * (filter.cu:92-110; colour conversion as InitFrame) for the filter sigmas,

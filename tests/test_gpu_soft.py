@@ -210,3 +210,60 @@ def test_soft_rejects_bad_arguments(gpu_ready):
     with pytest.raises(D.DtsgbError):
         s.backward(p)  # nothing solved
     s.close()
+
+
+def test_soft_autograd_handles_and_workspaces_are_reused_safely(gpu_ready):
+    """Forwards alive at the same time, adjoints in another order, a forward
+    whose result is dropped, and both current streams: always SoftDTS's bits."""
+    import torch
+    D = gpu_ready
+    from domain_transform_solver_gb300.autograd import soft_dts_solve
+    opt = dict(num_iterations=4, loss=1, lambda_=0.99, sigma_z=8.0, step_size=0.99)
+    data = [_inputs(880 + i, 90, 41) for i in range(4)]
+    dh, dv = _gpu_edges(D, [r for r, _, _, _ in data])
+    ts, cs, gs = ([x[k] for x in data] for k in (1, 2, 3))
+    ref = [_gpu_soft(D, dh[i:i + 1], dv[i:i + 1], ts[i:i + 1], cs[i:i + 1], opt, gs[i:i + 1])
+           for i in range(4)]
+
+    def leaves(i):
+        return [x.clone().requires_grad_()
+                for x in (_dev(ts[i][None]), _dev(cs[i][None]), dh[i:i + 1], dv[i:i + 1])]
+
+    def forward(x):
+        return soft_dts_solve(x[2], x[3], x[0], x[1], D.DomainOptimizeParams(**opt), TAU)
+    for stream in (torch.cuda.default_stream(), torch.cuda.Stream()):
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            for order in ((0, 1, 2, 3), (3, 1, 0, 2)):
+                xs = [leaves(i) for i in range(4)]
+                vs = [forward(x) for x in xs]
+                forward(xs[0])  # dropped
+                for i in order:
+                    (vs[i] * _dev(gs[i][None])).sum().backward()
+                for i in range(4):
+                    assert np.array_equal(vs[i].detach().cpu().numpy(), ref[i][0])
+                    for got, r in zip((x.grad for x in xs[i]), ref[i][1:]):
+                        assert np.array_equal(got.cpu().numpy(), r)
+
+
+def test_soft_lent_workspace(gpu_ready):
+    import torch
+    D = gpu_ready
+    s = D.SoftDTS([(16, 16)], bare=True)
+    x = torch.ones((16, 16), device="cuda")
+    p = [x.data_ptr()]
+    opt = D.DomainOptimizeParams(num_iterations=2, loss=1, sigma_z=4.0)
+    n = s.workspace(2)
+    work = torch.full((n,), float("nan"), device="cuda")
+    with pytest.raises(D.DtsgbError):
+        s.lend(work.data_ptr() + 4, n - 1)
+    s.lend(work.data_ptr(), n - 1)
+    with pytest.raises(D.DtsgbError):
+        s.solve(p, p, p, None, opt, 1.0, p)  # one plane short
+    s.lend(work.data_ptr(), n)
+    s.solve(p, p, p, None, opt, 1.0, p)
+    s.backward(p, p)
+    s.lend(None)
+    with pytest.raises(D.DtsgbError):
+        s.backward(p)  # the solve went with its workspace
+    s.close()
