@@ -185,7 +185,7 @@ __global__ void k_hb_step_adj(const HInst* __restrict__ insts, const float* __re
       if (y + 1 < gy) a += w[i + sy];
       if (zz > 0) a += w[i - sz];
       if (zz + 1 < gl) a += w[i + sz];
-      gzv += gg_in[g] - lambda * nc * a;
+      gzv = hfbs_finish_adj(gzv, gg_in[g], nc, a, lambda);
       gz[g] = gzv;
     }
     if (step) {
@@ -206,16 +206,15 @@ __global__ void k_hb_step_adj(const HInst* __restrict__ insts, const float* __re
         if (zz > 0) a += z[i - sz] * nn[i - sz];
         if (zz + 1 < gl) a += z[i + sz] * nn[i + sz];
       }
-      const float bc = b[g], ic = invA[g];
-      const float q = (bc + lambda * nc * a) * ic;
-      const float grad = z[i] - q;
-      const float u = gh[g] - alpha * gzv;
-      const float m = fabsf(grad) >= 1.345f ? 0.f : u;
-      gh[g] = beta * u;
-      gb[g] -= ic * m;
-      ginv[g] -= (bc + lambda * nc * a) * m;
+      float ghv = gh[g], gbv = gb[g], giv = ginv[g];
+      const float ic = invA[g];
+      float m;
+      hfbs_step_adj(a, z[i], nc, b[g], ic, gzv, lambda, alpha, beta, ghv, gbv, giv, m);
       gg_out[g] = m;
-      gw_out[g] = nc * ic * m;
+      gw_out[g] = hfbs_adj_product(nc, ic, m);
+      gh[g] = ghv;
+      gb[g] = gbv;
+      ginv[g] = giv;
     }
   }
 }
@@ -295,10 +294,15 @@ int hfbs_enqueue_backward(const HfbsBatch& B, const HParams& p, const float* gou
   float* sp = grad_t ? grad_t : grad_c;
   if (!sp) return DTSGB_OK;  // no gradient asked for
   prof_begin(s, DTSGB_K_HFBS_ADJOINT);
+  // the steps in one launch where the grids stay on chip
+  const HfbsClusterPlan CP =
+      S == 1 && K > 0 ? hfbs_cluster_adj_plan(B) : HfbsClusterPlan{};
   DTSGB_CUDA(cudaMemsetAsync(G.gz, 0, gbytes, s));
-  DTSGB_CUDA(cudaMemsetAsync(G.gh, 0, gbytes, s));
-  DTSGB_CUDA(cudaMemsetAsync(G.gb, 0, gbytes, s));
-  DTSGB_CUDA(cudaMemsetAsync(G.ginv, 0, gbytes, s));
+  if (CP.size == 0) {
+    DTSGB_CUDA(cudaMemsetAsync(G.gh, 0, gbytes, s));
+    DTSGB_CUDA(cudaMemsetAsync(G.gb, 0, gbytes, s));
+    DTSGB_CUDA(cudaMemsetAsync(G.ginv, 0, gbytes, s));
+  }
   const dim3 gp(blocks_for_n(B.max_pixels), ni);
   const dim3 gv(blocks_for_n(B.max_voxels), ni);
   const int gflat = blocks_for_n(tv);
@@ -328,7 +332,9 @@ int hfbs_enqueue_backward(const HfbsBatch& B, const HParams& p, const float* gou
     ++launched;
     return DTSGB_OK;
   };
-  if (S == 1) {
+  if (CP.size > 0) {
+    if (int st = hfbs_cluster_adjoint(B, CP, p, norm, G.hist, G.gz, G.gb, G.ginv, K, s)) return st;
+  } else if (S == 1) {
     for (int k = K - 1; k >= 0; --k)
       if (int st = step_adj(G.hist + (size_t)k * tv)) return st;
   } else {

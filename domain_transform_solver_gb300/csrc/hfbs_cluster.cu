@@ -40,6 +40,9 @@ constexpr int kCV = 4;  // levels of an item
 __host__ __device__ constexpr int max_threads(int ipt) {
   return ipt == 1 ? 1024 : ipt == 2 ? 768 : ipt == 3 ? 576 : 512;
 }
+// The same of the adjoint (44 registers an item).
+__host__ __device__ constexpr int adj_threads(int ipt) { return ipt == 1 ? 704 : 640; }
+constexpr int kAdjItems = 2;
 constexpr int kCItems = 4;
 constexpr int kMaxItems = kCItems * max_threads(kCItems);
 constexpr size_t kMaxSmem = 227 * 1024;
@@ -82,15 +85,14 @@ __host__ __device__ inline int slab_rows(int gy, int c) { return (gy + c - 1) / 
 inline long long slab_items(const HInst& H, int c) {
   return (long long)slab_rows(H.gy, c) * H.gx * ((H.gl + kCV - 1) / kCV);
 }
-inline size_t slab_smem(const HInst& H, int c) {
-  return sizeof(float) * 2 * (size_t)((H.gl + kCV - 1) / kCV * kCV) *
+inline size_t slab_smem(const HInst& H, int c) {  // of one buffer
+  return sizeof(float) * (size_t)((H.gl + kCV - 1) / kCV * kCV) *
          (slab_rows(H.gy, c) + 2) * (H.gx + 2);
 }
 
 template <int MODE, bool REC, int IPT>
 __global__ void __launch_bounds__(max_threads(IPT), 1)
     k_hfbs_cluster(const HInst* __restrict__ insts, ClusterArgs A) {
-  pdl_wait_then_release();
   extern __shared__ __align__(16) float smc[];
   const HInst I = insts[blockIdx.y];
   const int gx = I.gx, gy = I.gy, gl = I.gl;
@@ -221,33 +223,181 @@ __global__ void __launch_bounds__(max_threads(IPT), 1)
   }
 }
 
-template <int MODE, bool REC, int IPT>
-cudaError_t launch(const HfbsBatch& B, const HfbsClusterPlan& P, const ClusterArgs& A,
-                   cudaStream_t s, int* clusters) {
-  auto kern = k_hfbs_cluster<MODE, REC, IPT>;
+// ---- the adjoint ---------------------------------------------------------------
+struct ClusterAdjArgs {
+  const float *hist, *n, *b, *a;
+  float *gz, *gb, *ginv;
+  long long stride;  // voxels of an iterate
+  int steps;
+  float lambda, alpha, beta;
+};
+
+// All steps of the heavy-ball adjoint, from the last: the same ownership and
+// exchange as the solve, with two products per step to exchange (z_k * n of the
+// forward iterate, and gw of the step after it, which completes gz) and the
+// next iterate's loads in flight during a step.  64 steps on 80 x 60 x 16:
+// 238 us, 384 by a launch per step; shared memory bounds it (14 words a
+// voxel-step), then the barrier of a step.
+template <int IPT>
+__global__ void __launch_bounds__(adj_threads(IPT), 1)
+    k_hfbs_cluster_adj(const HInst* __restrict__ insts, ClusterAdjArgs A) {
+  extern __shared__ __align__(16) float smc[];
+  const HInst I = insts[blockIdx.y];
+  const int gx = I.gx, gy = I.gy, gl = I.gl;
+  const int rank = (int)cluster_rank(), C = (int)cluster_size();
+  const int R = slab_rows(gy, C), nlc = (gl + kCV - 1) / kCV;
+  const int gxp = gx + 2, PS = (R + 2) * gxp, BUF = nlc * kCV * PS;
+  const int tid = threadIdx.x, T = blockDim.x;
+  for (int i = tid; i < 4 * BUF; i += T) smc[i] = 0.f;
+  const int items = R * gx * nlc, plane = I.px * gy;
+  float z[IPT][kCV], n[IPT][kCV], b[IPT][kCV], a[IPT][kCV];
+  float gz[IPT][kCV], gh[IPT][kCV], gb[IPT][kCV], gi[IPT][kCV], gg[IPT][kCV];
+  int o[IPT], lc[IPT], edge[IPT], g[IPT];
+  const float* zk = A.hist + I.grid_off + (long long)(A.steps - 1) * A.stride;
+  A.n += I.grid_off;
+  A.b += I.grid_off;
+  A.a += I.grid_off;
+  A.gz += I.grid_off;
+  A.gb += I.grid_off;
+  A.ginv += I.grid_off;
+#pragma unroll
+  for (int j = 0; j < IPT; ++j) {
+    const int i = tid + j * T;
+    lc[j] = -1;
+    o[j] = edge[j] = 0;
+    g[j] = 0;
+#pragma unroll
+    for (int v = 0; v < kCV; ++v)
+      z[j][v] = n[j][v] = b[j][v] = a[j][v] = gz[j][v] = gh[j][v] = gb[j][v] = gi[j][v] =
+          gg[j][v] = 0.f;
+    if (i < items) {
+      const int c = i / (R * gx), q = i - c * (R * gx), yy = q / gx, x = q - yy * gx;
+      const int y = rank * R + yy;
+      if (y < gy) {
+        lc[j] = c;
+        o[j] = c * kCV * PS + (yy + 1) * gxp + x + 1;
+        edge[j] = (yy == 0 && rank > 0 ? 1 : 0) | (yy == R - 1 && rank + 1 < C ? 2 : 0);
+        g[j] = c * kCV * plane + y * I.px + x;
+#pragma unroll
+        for (int v = 0; v < kCV; ++v)
+          if (c * kCV + v < gl) {
+            const int gv = g[j] + v * plane;
+            z[j][v] = zk[gv];
+            n[j][v] = A.n[gv];
+            b[j][v] = A.b[gv];
+            a[j][v] = A.a[gv];
+            gz[j][v] = A.gz[gv];
+          }
+      }
+    }
+  }
+  // every CTA of the cluster runs and its buffers are zeroed
+  __syncthreads();
+  cluster_barrier();
+  for (int s = 0; s <= A.steps; ++s) {  // the last pass only completes gz
+    float* P = smc + (s & 1) * BUF;
+    float* G = smc + (2 + (s & 1)) * BUF;
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+      if (lc[j] < 0) continue;
+#pragma unroll
+      for (int v = 0; v < kCV; ++v) {
+        const float p = __fmul_rn(z[j][v], n[j][v]);
+        const float w = hfbs_adj_product(n[j][v], a[j][v], gg[j][v]);
+        float *qp = P + o[j] + v * PS, *qg = G + o[j] + v * PS;
+        *qp = p;
+        *qg = w;
+        if (edge[j] & 1) {
+          store_remote(qp + R * gxp, rank - 1, p);
+          store_remote(qg + R * gxp, rank - 1, w);
+        }
+        if (edge[j] & 2) {
+          store_remote(qp - R * gxp, rank + 1, p);
+          store_remote(qg - R * gxp, rank + 1, w);
+        }
+      }
+    }
+    // the next iterate, in flight over the barrier and this step
+    float zn[IPT][kCV];
+    zk -= A.stride;
+#pragma unroll
+    for (int j = 0; j < IPT; ++j)
+#pragma unroll
+      for (int v = 0; v < kCV; ++v)
+        zn[j][v] = s + 1 < A.steps && lc[j] >= 0 && lc[j] * kCV + v < gl
+                       ? zk[g[j] + v * plane]
+                       : 0.f;
+    cluster_barrier();
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+      if (lc[j] < 0) continue;
+      const bool has_lo = lc[j] > 0, has_hi = lc[j] + 1 < nlc;
+#pragma unroll
+      for (int v = 0; v < kCV; ++v) {
+        const float *qp = P + o[j] + v * PS, *qg = G + o[j] + v * PS;
+        if (s > 0) {
+          float t = __fadd_rn(__fadd_rn(__fadd_rn(qg[-1], qg[1]), qg[-gxp]), qg[gxp]);
+          t = __fadd_rn(t, v > 0 || has_lo ? qg[-PS] : 0.f);
+          t = __fadd_rn(t, v + 1 < kCV || has_hi ? qg[PS] : 0.f);
+          gz[j][v] = hfbs_finish_adj(gz[j][v], gg[j][v], n[j][v], t, A.lambda);
+        }
+        if (s < A.steps) {
+          float t = __fadd_rn(__fadd_rn(__fadd_rn(qp[-1], qp[1]), qp[-gxp]), qp[gxp]);
+          t = __fadd_rn(t, v > 0 || has_lo ? qp[-PS] : 0.f);
+          t = __fadd_rn(t, v + 1 < kCV || has_hi ? qp[PS] : 0.f);
+          hfbs_step_adj(t, z[j][v], n[j][v], b[j][v], a[j][v], gz[j][v], A.lambda, A.alpha,
+                        A.beta, gh[j][v], gb[j][v], gi[j][v], gg[j][v]);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < IPT; ++j)
+#pragma unroll
+      for (int v = 0; v < kCV; ++v) z[j][v] = zn[j][v];
+  }
+#pragma unroll
+  for (int j = 0; j < IPT; ++j) {
+    if (lc[j] < 0) continue;
+#pragma unroll
+    for (int v = 0; v < kCV; ++v)
+      if (lc[j] * kCV + v < gl) {
+        const int gv = g[j] + v * plane;
+        A.gz[gv] = gz[j][v];
+        A.gb[gv] = gb[j][v];
+        A.ginv[gv] = gi[j][v];
+      }
+  }
+}
+
+// Launches a kernel with one cluster of P.size CTAs per instance, or (clusters
+// given) only asks how many such clusters can be resident.
+template <typename F, typename Args>
+cudaError_t launch_cluster(F* kern, const HfbsBatch& B, const HfbsClusterPlan& P, const Args& A,
+                           cudaStream_t s, int* clusters) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)P.smem);
   if (e == cudaSuccess && P.size > 8)
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
-  cudaLaunchAttribute at[2];
+  cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = P.size;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3(P.size, P.count);
   c.blockDim = dim3(P.threads);
   c.dynamicSmemBytes = P.smem;
   c.stream = s;
   c.attrs = at;
-  c.numAttrs = 2;
-  if (clusters) {  // only asked whether a cluster can be resident
-    c.numAttrs = 1;
-    return cudaOccupancyMaxActiveClusters(clusters, kern, &c);
-  }
+  c.numAttrs = 1;
+  if (clusters) return cudaOccupancyMaxActiveClusters(clusters, kern, &c);
   return cudaLaunchKernelEx(&c, kern, B.d_inst + P.first, A);
+}
+
+template <int MODE, bool REC, int IPT>
+cudaError_t launch(const HfbsBatch& B, const HfbsClusterPlan& P, const ClusterArgs& A,
+                   cudaStream_t s, int* clusters) {
+  return launch_cluster(k_hfbs_cluster<MODE, REC, IPT>, B, P, A, s, clusters);
 }
 
 template <int MODE, bool REC>
@@ -261,9 +411,20 @@ cudaError_t launch_items(const HfbsBatch& B, const HfbsClusterPlan& P, const Clu
   return launch<MODE, REC, kCItems>(B, P, A, s, clusters);
 }
 
+cudaError_t launch_adj(const HfbsBatch& B, const HfbsClusterPlan& P, const ClusterAdjArgs& A,
+                       cudaStream_t s, int* clusters = nullptr) {
+  return P.items <= 1 ? launch_cluster(k_hfbs_cluster_adj<1>, B, P, A, s, clusters)
+                      : launch_cluster(k_hfbs_cluster_adj<2>, B, P, A, s, clusters);
+}
+
 }  // namespace
 
-HfbsClusterPlan hfbs_cluster_plan(const HfbsBatch& B, int first, int count) {
+// The cluster of up to 16 CTAs that holds every instance with up to most_items
+// items a thread (threads(items) of them) and `buffers` exchange buffers; size 0
+// where an instance does not fit.
+template <typename T>
+static HfbsClusterPlan plan_cluster(const HfbsBatch& B, int first, int count, int most_items,
+                                    T threads, int buffers) {
   HfbsClusterPlan P;
   if (!hfbs_uses_march(B)) return P;
   int min_gy = 1 << 30;
@@ -274,12 +435,13 @@ HfbsClusterPlan hfbs_cluster_plan(const HfbsBatch& B, int first, int count) {
     size_t smem = 0;
     for (int i = 0; i < count; ++i) {
       items = std::max(items, slab_items(B.h_inst[first + i], c));
-      smem = std::max(smem, slab_smem(B.h_inst[first + i], c));
+      smem = std::max(smem, buffers * slab_smem(B.h_inst[first + i], c));
     }
-    if (items > kMaxItems || smem > kMaxSmem) break;  // smaller clusters hold less
+    if (items > (long long)most_items * threads(most_items) || smem > kMaxSmem)
+      break;  // smaller clusters hold less
     P.size = c;
     P.items = 1;
-    while (items > (long long)P.items * max_threads(P.items)) ++P.items;
+    while (items > (long long)P.items * threads(P.items)) ++P.items;
     P.threads = (int)((items + P.items - 1) / P.items + 31) / 32 * 32;
     P.smem = smem;
     P.first = first;
@@ -287,14 +449,37 @@ HfbsClusterPlan hfbs_cluster_plan(const HfbsBatch& B, int first, int count) {
     // the largest cluster whose instances run side by side
     if ((long long)c * count <= 128) break;
   }
-  if (P.size > 0) {
-    int n = 0;
-    if (launch_items<kHeavyBall, false>(B, P, ClusterArgs{}, nullptr, &n) != cudaSuccess || n < 1) {
-      (void)cudaGetLastError();
-      P.size = 0;
-    }
+  return P;
+}
+
+HfbsClusterPlan hfbs_cluster_plan(const HfbsBatch& B, int first, int count) {
+  HfbsClusterPlan P = plan_cluster(B, first, count, kCItems, max_threads, 2);
+  int n = 0;
+  if (P.size > 0 &&
+      (launch_items<kHeavyBall, false>(B, P, ClusterArgs{}, nullptr, &n) != cudaSuccess || n < 1)) {
+    (void)cudaGetLastError();
+    P.size = 0;
   }
   return P;
+}
+
+HfbsClusterPlan hfbs_cluster_adj_plan(const HfbsBatch& B) {
+  HfbsClusterPlan P = plan_cluster(B, 0, B.n_inst, kAdjItems, adj_threads, 4);
+  int n = 0;
+  if (P.size > 0 && (launch_adj(B, P, ClusterAdjArgs{}, nullptr, &n) != cudaSuccess || n < 1)) {
+    (void)cudaGetLastError();
+    P.size = 0;
+  }
+  return P;
+}
+
+int hfbs_cluster_adjoint(const HfbsBatch& B, const HfbsClusterPlan& P, const HParams& p,
+                         const float* norm, const float* hist, float* gz, float* gb, float* ginv,
+                         int steps, cudaStream_t s) {
+  const ClusterAdjArgs A{hist, norm, B.b, B.invA, gz, gb, ginv, B.total_voxels, steps,
+                         p.lambda, p.alpha, p.beta};
+  DTSGB_CUDA(launch_adj(B, P, A, s));
+  return DTSGB_OK;
 }
 
 int hfbs_cluster_solve(const HfbsBatch& B, const HfbsClusterPlan& P, const HParams& p,

@@ -60,6 +60,31 @@ __device__ __forceinline__ void hfbs_step(float xm, float xp, float ym, float yp
   z = __fmaf_rn(-alpha, h, z);
 }
 
+// The adjoint of a heavy-ball step of one voxel, in two parts that lie one
+// exchange apart.  hfbs_step_adj: from the neighbour sum a of the forward
+// iterate's z * n, z, n, b, invA and gz, the updates of gh, gb and ginv, and
+// gg; the Huber mask is hfbs_step's.  hfbs_finish_adj: gz after the neighbour
+// sum of gw = hfbs_adj_product.
+__device__ __forceinline__ void hfbs_step_adj(float a, float z, float n, float b, float ia,
+                                              float gz, float lambda, float alpha, float beta,
+                                              float& gh, float& gb, float& ginv, float& gg) {
+  const float t = __fmaf_rn(__fmul_rn(lambda, n), a, b);
+  const float grad = __fmaf_rn(-t, ia, z);
+  const float u = __fmaf_rn(-alpha, gz, gh);
+  const float m = fabsf(grad) >= 1.345f ? 0.f : u;
+  gh = __fmul_rn(beta, u);
+  gb = __fmaf_rn(-ia, m, gb);
+  ginv = __fmaf_rn(-t, m, ginv);
+  gg = m;
+}
+__device__ __forceinline__ float hfbs_adj_product(float n, float ia, float gg) {
+  return __fmul_rn(__fmul_rn(n, ia), gg);
+}
+__device__ __forceinline__ float hfbs_finish_adj(float gz, float gg, float n, float a,
+                                                 float lambda) {
+  return __fadd_rn(gz, __fmaf_rn(-__fmul_rn(lambda, n), a, gg));
+}
+
 // Solver parameters shared by a batch (HFBSGridParams minus the grid dims).
 struct HParams {
   float sigma_x, sigma_y, sigma_l, lambda, alpha, beta;
@@ -197,6 +222,13 @@ int hfbs_cluster_solve(const HfbsBatch& B, const HfbsClusterPlan& P, const HPara
 // All `steps` bistochastization iterations, from ones, into dst.
 int hfbs_cluster_bistoch(const HfbsBatch& B, const HfbsClusterPlan& P, float* dst, int steps,
                          cudaStream_t s);
+// The cluster that holds the adjoint of each instance, or size 0 (it keeps
+// twice the registers a voxel), and the adjoint of all `steps` steps from the
+// kept iterates z_k (plane k of hist): gz in place, gb and ginv written.
+HfbsClusterPlan hfbs_cluster_adj_plan(const HfbsBatch& B);
+int hfbs_cluster_adjoint(const HfbsBatch& B, const HfbsClusterPlan& P, const HParams& p,
+                         const float* norm, const float* hist, float* gz, float* gb, float* ginv,
+                         int steps, cudaStream_t s);
 // Builds the tensor maps of grid planes (before a capture).
 void hfbs_march_prepare(const HfbsBatch& B, const std::vector<const float*>& planes,
                         cudaStream_t s);

@@ -194,3 +194,38 @@ def test_passes_match_the_oracle(gpu_ready, oracle_mod, w, h, sz):
              [inst.confidence, other.confidence])
     b.solve_dts(D.DomainFilterParams(**W.CFG0_FILTER), D.DomainOptimizeParams(**opt))
     assert np.array_equal(b.download(0)[0], v)
+
+
+# ---- HFBS adjoint: one cluster per grid where every step's iterate is kept -----
+@pytest.mark.parametrize("w,h,sx,sy,sl,steps", [
+    (200, 8, 8.0, 8.0, 16.0, 9),       # one row: a cluster of one
+    (90, 70, 8.0, 8.0, 29.0, 12),      # nine levels, rows that do not divide
+    (97, 141, 8.0, 8.0, 63.0, 1),      # five levels, one step
+    (640, 480, 8.0, 8.0, 16.0, 6),     # two items a thread, every thread used
+    (512, 512, 8.0, 8.0, 16.0, 5),     # the largest cube of 16 levels
+    (648, 488, 8.0, 8.0, 16.0, 5),     # just above: a launch per step
+])
+def test_adjoint_in_clusters_is_the_adjoint_by_steps(gpu_ready, w, h, sx, sy, sl, steps):
+    """Recomputed segments take a launch per step; both round alike."""
+    D = gpu_ready
+    rng = np.random.default_rng(w * 3 + h)
+    rgba = rng.integers(0, 256, (2, h, w, 4)).astype(np.uint8)
+    t = rng.normal(0, 2, (2, h, w)).astype(np.float32)
+    c = rng.random((2, h, w)).astype(np.float32)
+    gout = rng.standard_normal((2, h, w)).astype(np.float32)
+    f = np.float32
+    dims = (int(np.ceil(f(w) / f(sx))), int(np.ceil(f(h) / f(sy))), int(np.ceil(255.0 / sl)))
+    got = []
+    for segment in (1, 3):
+        s = [D.HFBS(D.ImageDim(w, h), *dims) for _ in range(2)]
+        for i in range(2):
+            s[i].SetFilterParams(D.HFBSGridParams(sigma_x=sx, sigma_y=sy, sigma_l=sl,
+                                                  optim_iter_max=steps))
+            s[i].EnableGrad(True, segment)
+            s[i].InitFrame(D.COLOR_SPACE.RGB, rgba[i], t[i], c[i])
+            s[i].Optimize()
+            got.append(s[i].Backward(gout[i]))
+    for i in range(2):
+        assert np.abs(got[i][0]).max() > 0
+        assert np.array_equal(got[i][0], got[2 + i][0])
+        assert np.array_equal(got[i][1], got[2 + i][1])
