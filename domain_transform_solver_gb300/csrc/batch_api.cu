@@ -76,18 +76,17 @@ struct dtsgb_batch_s {
   bool uptr_valid[3] = {false, false, false};
   unsigned char* stage = nullptr;  // dense x (rgba 4 B, target 4 B, conf 4 B)
   Inst* d_inst = nullptr;
-  Tile* d_tb = nullptr;
   Tile* d_ti = nullptr;     // iteration tiles of the shape in use
   Tile* d_ti_big = nullptr;  // kIterTW x kIterTH tiles
   Tile* d_ti_small = nullptr;  // kIterSmallTW x kIterSmallTH tiles
-  int ntb = 0, nti = 0, nti_big = 0, nti_small = 0;
+  int nti = 0, nti_big = 0, nti_small = 0;
   // blocks of the DTS passes for halo pass_halo (several instances only)
   Tile *d_px = nullptr, *d_py = nullptr;
   int npx = 0, npy = 0, pass_halo = -1;
   bool small = false;
   long long hfbs_group_voxels = 0;  // L2-resident HFBS group budget (0: off)
   int hfbs_solve_steps = 4;         // heavy-ball steps per launch (4 or 1)
-  int bounds_seg = 8;               // pixels per window-bound walk (4, 8, 16)
+  int bounds_seg = 8;               // accepted and returned (DTSGB_TUNE_BOUNDS_SEGMENT)
   // Guide-derived state kept across solves while the guide is unchanged
   // (video frames that change only the target): the DTS window bounds and
   // the HFBS bistochastized normalisation.
@@ -182,7 +181,6 @@ void batch_free(dtsgb_batch_t b) {
   dfree(b->hout);
   dfree(b->scratch);
   dfree(b->d_inst);
-  dfree(b->d_tb);
   dfree(b->d_ti_big);
   dfree(b->d_ti_small);
   dfree(b->d_px);
@@ -843,7 +841,7 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
   b->flags = flags;
   b->st = (flags & DTSGB_FLAG_BF16_STORAGE) ? Storage::BF16 : Storage::F32;
   b->ref_y = (flags & DTSGB_FLAG_FIX_Y_LIMIT) ? 0 : 1;
-  std::vector<Tile> tb, ti, ts;
+  std::vector<Tile> ti, ts;
   long long off = 0, tiles64 = 0;
   for (int i = 0; i < n; ++i)
     tiles64 += (long long)((widths[i] + kIterTW - 1) / kIterTW) *
@@ -857,15 +855,12 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
     off += (long long)I.pitch * I.h;
     b->max_w = std::max(b->max_w, I.w);
     b->max_h = std::max(b->max_h, I.h);
-    for (int y = 0; y < I.h; y += kBoundsTH)
-      for (int x = 0; x < I.w; x += kBoundsTW) tb.push_back(Tile{i, x, y, 0});
     for (int y = 0; y < I.h; y += kIterTH)
       for (int x = 0; x < I.w; x += kIterTW) ti.push_back(Tile{i, x, y, 0});
     for (int y = 0; y < I.h; y += kIterSmallTH)
       for (int x = 0; x < I.w; x += kIterSmallTW) ts.push_back(Tile{i, x, y, 0});
   }
   b->total = off;
-  b->ntb = (int)tb.size();
   b->nti_big = (int)ti.size();
   b->nti_small = (int)ts.size();
   int st = DTSGB_OK;
@@ -885,7 +880,6 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
   if (!st) st = dalloc(&b->hout, T);
   if (!st && b->st == Storage::BF16) st = dalloc(&b->scratch, T);
   if (!st) st = dalloc(&b->d_inst, (size_t)n);
-  if (!st) st = dalloc(&b->d_tb, tb.size());
   if (!st) st = dalloc(&b->d_ti_big, ti.size());
   if (!st) st = dalloc(&b->d_ti_small, ts.size());
   if (!st) st = dalloc(&b->d_hinst, (size_t)n);
@@ -895,8 +889,6 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
     e = upload_table(b->d_inst, b->inst.data(), n * sizeof(Inst));
     if (e == cudaSuccess)
       e = upload_table(b->d_soff, b->soff.data(), n * sizeof(long long));
-    if (e == cudaSuccess)
-      e = upload_table(b->d_tb, tb.data(), tb.size() * sizeof(Tile));
     if (e == cudaSuccess)
       e = upload_table(b->d_ti_big, ti.data(), ti.size() * sizeof(Tile));
     if (e == cudaSuccess)
@@ -990,8 +982,6 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
   const float rx = f->sigma_x / f->sigma_r, ry = f->sigma_y / f->sigma_r;
   const int halo = (int)std::floor(p->sigma_z);
   const bool iterate = p->loss != DTSGB_L1 && p->num_iterations > 0;
-  DtsLaunch Lb{b->d_inst, b->d_tb, b->ntb, b->n};
-  Lb.bounds_seg = b->bounds_seg;
   if (iterate)
     if (int st = ensure_pass_blocks(b, halo)) return st;
   const DtsLaunch Li = iter_launch(b);
@@ -1021,7 +1011,7 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
   const bool keep_bounds = b->reuse && std::memcmp(&bk, &b->bkey, sizeof bk) == 0;
   auto bounds = [&]() -> int {
     if (keep_bounds) return DTSGB_OK;  // same guide and sigmas: windows unchanged
-    return launch_bounds(Lb, b->guide, b->bounds, rx, ry, p->sigma_z, p->sigma_z,
+    return launch_bounds(Li, b->guide, b->bounds, rx, ry, p->sigma_z, p->sigma_z,
                          b->ref_y, b->stream);
   };
   auto enqueue = [&]() -> int {
@@ -1057,7 +1047,6 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
   key_append(key, b->grad_seg);
   key_append(key, b->small);
   key_append(key, keep_bounds);
-  key_append(key, b->bounds_seg);
   int st = run_graph(b, b->g_dts, key, enqueue);
   if (st) {
     b->bkey.gen = ~0ull;
@@ -1469,7 +1458,6 @@ DTSGB_API int dtsgb_batch_autotune(dtsgb_batch_t b, const dtsgb_filter_params* f
     auto dts = [&]() { return dtsgb_batch_solve_dts(b, f, p, overwrite); };
     st = tune_knob(b, DTSGB_TUNE_DTS_TILE, {(long long)kIterTW, (long long)kIterSmallTW}, reps,
                    dts);
-    if (!st) st = tune_knob(b, DTSGB_TUNE_BOUNDS_SEGMENT, {8, 4, 16}, reps, dts);
   }
   if (hp && !st) {
     auto hfbs = [&]() { return dtsgb_batch_solve_hfbs(b, hp); };

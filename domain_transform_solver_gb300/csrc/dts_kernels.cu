@@ -1,6 +1,6 @@
-// DTS kernels for sm_103a: guide ingest, window-bound search, the
-// domain-transform filter pass with the confidence epilogue, and small helpers
-// for downloads.  The iteration is in dts_passes.cu.
+// DTS kernels for sm_103a: guide ingest, the domain-transform filter pass with
+// the confidence epilogue, and small helpers for downloads.  The window bounds
+// are in dts_bounds.cu, the iteration in dts_passes.cu.
 //
 // Key fact used throughout: the edge weights dH, dV are >= 1
 // (sqrt(1 + nonnegative)), so a window of the reference's linear search
@@ -14,7 +14,6 @@
 #include "../../include/dtsgb.h"
 #include "color.cuh"
 #include "dtsgb_internal.cuh"
-#include "fixed_point.cuh"
 #include "raw4.cuh"
 
 namespace dtsgb {
@@ -28,171 +27,6 @@ __global__ void k_color_convert_flat(uchar4* __restrict__ g, long long n,
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     g[i] = convert_pixel(g[i], cs);
-}
-
-// ---------------------------------------------------------------------------
-// Window bounds (a4).  One CTA per TWxTH tile, 256 threads.
-// Lower bound: the largest i < p with sum_{j=i+1..p} w(j) > sigma, else p-1.
-// Upper bound: (the smallest i > p, i < limit, with sum_{j=p+1..i} w(j) >
-// sigma) - 1, else p.  limit is W for X and min(W,H) (reference quirk) or H
-// for Y.  A negative ratio stands for an all-zero domain transform (no
-// differential computed yet): every window is the pixel itself.
-//
-// The weights are clamped to sigma + 1 (a window holding a larger one
-// exceeds sigma either way) and converted to fixed point at 2^F with
-// r * (sigma + 1) * 2^F <= 2^30, so a window sum is the exact difference of
-// two wrapping 32-bit prefixes of the converted weights (each within 2^-F-1
-// of the float weight: decisions differ from float sums only within about
-// r * 2^-F of the threshold).  Shared memory holds the prefix of dH along
-// each tile row over [x0 - r, x0 + TW + r) and of dV along each tile column
-// over [y0 - r, y0 + TH + r).  As p moves forward, both window ends move
-// forward, so a thread walks a segment of 8 pixels with two pointers that
-// only advance: about two prefix reads per end and pixel instead of a search
-// over the whole radius.
-// ---------------------------------------------------------------------------
-// Pixels per thread and axis of the two-pointer walks (a launch knob:
-// DTSGB_TUNE_BOUNDS_SEGMENT selects 4, 8 or 16).
-constexpr int kBoundsSegDefault = 8;
-
-// Lower and upper window ends along one axis for the n pixels starting at
-// prefix index j0 (S[j0 + k] for pixel p0 + k), coordinates p0.., axis length
-// `len` (lower limit 0), upper limit `lim`; stride between prefix entries s.
-// Writes dl | du << 8 to out[k * os].
-__device__ __forceinline__ void bounds_walk(const unsigned* __restrict__ S, int s, int j0,
-                                            int p0, int n, int r, int lim, int T,
-                                            uint16_t* out, int os) {
-  int q = 0, u = 0;
-  for (int k = 0; k < n; ++k) {
-    const int j = j0 + k, p = p0 + k;
-    const unsigned Sj = S[j * s];
-    // lower: the largest q in [j - K, j - 1] with S[j] - S[q] > T (K = min(r, p)),
-    // advanced from the previous pixel's (both only move forward)
-    const int qmin = j - min(r, p);
-    q = k == 0 ? qmin - 1 : max(q, qmin - 1);
-    while (q + 1 <= j - 1 && (int)(Sj - S[(q + 1) * s]) > T) ++q;
-    const int dl = q >= qmin ? j - q : 1;
-    // upper: the smallest u in [j + 1, j + K'] with S[u] - S[j] > T
-    // (K' = min(r, lim - 1 - p)); the first pixel starts from the far end
-    const int umax = j + min(r, lim - 1 - p);
-    if (k == 0) {
-      u = umax + 1;
-      while (u - 1 > j && (int)(S[(u - 1) * s] - Sj) > T) --u;
-    } else {
-      u = max(u, j + 1);
-      while (u <= umax && (int)(S[u * s] - Sj) <= T) ++u;
-    }
-    const int du = u <= umax ? u - j - 1 : 0;
-    out[k * os] = (uint16_t)(dl | (du << 8));
-  }
-}
-
-template <int TW, int TH, int SEG>
-__global__ void __launch_bounds__(kThreads)
-    k_bounds(const Inst* __restrict__ insts, const Tile* __restrict__ tiles,
-             const uchar4* __restrict__ guide, uint32_t* __restrict__ bounds,
-             float ratio_x, float ratio_y, int rx, int ry, int ref_y_limit,
-             float cap_x, float cap_y, float scale_x, float scale_y, int Tx, int Ty) {
-  static_assert(TW == 32 && TH == 32 && kThreads == 256, "bounds tile shape");
-  static_assert(SEG == 4 || SEG == 8 || SEG == 16, "walk segment");
-  constexpr int NW = kThreads / 32;
-  extern __shared__ unsigned smu[];
-  const Tile t = tiles[blockIdx.x];
-  const Inst in = insts[t.inst];
-  const int W = in.w, H = in.h, P = in.pitch;
-  const uchar4* g = guide + in.off;
-  const int DW = TW + 2 * rx, DWp = DW | 1;  // odd row stride: lanes on rows
-  const int DR = TH + 2 * ry;
-  unsigned* SH = smu;             // TH x DWp: prefix of dH, entry 0 = 0 at x0 - rx
-  unsigned* SV = SH + TH * DWp;   // DR x TW: prefix of dV, entry 0 = 0 at y0 - ry
-  uint16_t* BX = reinterpret_cast<uint16_t*>(SV + DR * TW);  // TH x TW
-  uint16_t* BY = BX + TH * TW;                               // TH x TW
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // ---- 1. weights in fixed point.  dH: a warp per row, lanes on columns; a
-  // lane's left neighbour comes from the lane before it (one load per pixel).
-  // dV: eight threads per column, each down a run of rows, the pixel above
-  // carried in a register.  Pixels outside the image read as zero.
-  auto load_g = [&](int x, int y) -> unsigned {
-    return (x >= 0 && x < W && y >= 0 && y < H)
-               ? *reinterpret_cast<const unsigned*>(g + (long long)y * P + x)
-               : 0u;
-  };
-  auto as_px = [](unsigned v) { return *reinterpret_cast<const uchar4*>(&v); };
-  for (int r = warp; r < TH; r += NW) {
-    const int y = t.y0 + r;
-    for (int j0 = 0; j0 < DW; j0 += 32) {
-      const int j = j0 + lane, x = t.x0 - rx + j;
-      const unsigned cur = j < DW ? load_g(x, y) : 0u;
-      unsigned prev = __shfl_up_sync(0xffffffffu, cur, 1);
-      if (lane == 0) prev = load_g(x - 1, y);
-      unsigned q = 0u;
-      if (j > 0 && x >= 0 && x < W && y < H && ratio_x >= 0.f)
-        q = (unsigned)__float2int_rn(
-            fminf(edge_weight(as_px(cur), as_px(prev), ratio_x), cap_x) * scale_x);
-      if (j < DW) SH[r * DWp + j] = q;
-    }
-  }
-  {
-    const int c = tid % TW, sgi = tid / TW, nsg = kThreads / TW;
-    const int seg = (DR + nsg - 1) / nsg;
-    const int j0 = sgi * seg, j1 = min(DR, j0 + seg);
-    const int x = t.x0 + c;
-    unsigned prev = load_g(x, t.y0 - ry + j0 - 1);
-    for (int j = j0; j < j1; ++j) {
-      const int y = t.y0 - ry + j;
-      const unsigned cur = load_g(x, y);
-      unsigned q = 0u;
-      if (j > 0 && x < W && y >= 0 && y < H && ratio_y >= 0.f)
-        q = (unsigned)__float2int_rn(
-            fminf(edge_weight(as_px(cur), as_px(prev), ratio_y), cap_y) * scale_y);
-      SV[j * TW + c] = q;
-      prev = cur;
-    }
-  }
-  __syncthreads();
-  // ---- 2. inclusive prefixes: a thread per row of SH, a thread per column of SV
-  // (a segmented scan over all warps was slower: its extra pass costs more
-  // issue slots than the serial chains, which the other resident blocks hide)
-  if (tid < TH) {
-    unsigned* row = SH + tid * DWp;
-    unsigned acc = 0u;
-    for (int j = 0; j < DW; ++j) row[j] = acc += row[j];
-  } else if (tid >= 32 && tid < 32 + TW) {
-    unsigned* col = SV + (tid - 32);
-    unsigned acc = 0u;
-    for (int j = 0; j < DR; ++j) col[j * TW] = acc += col[j * TW];
-  }
-  __syncthreads();
-  // ---- 3. two-pointer walks: warps 0-3 rows (X), warps 4-7 columns (Y), each
-  // taking the SEG-pixel segments sg = warp, warp + 4, ... of its lines
-  const int ylim = ref_y_limit ? min(W, H) : H;
-  constexpr int NSEG = TW / SEG;
-  if (tid < 4 * 32) {
-    const int r = lane, y = t.y0 + r;  // lanes on rows
-    for (int sg = warp; sg < NSEG; sg += 4) {
-      const int xs = t.x0 + sg * SEG;
-      const int n = min(SEG, W - xs);
-      if (y < H && n > 0)
-        bounds_walk(SH + r * DWp, 1, xs - t.x0 + rx, xs, n, rx, W, Tx,
-                    BX + r * TW + sg * SEG, 1);
-    }
-  } else {
-    const int c = lane, x = t.x0 + c;  // lanes on columns
-    for (int sg = warp - 4; sg < NSEG; sg += 4) {
-      const int ys = t.y0 + sg * SEG;
-      const int n = min(SEG, H - ys);
-      if (x < W && n > 0)
-        bounds_walk(SV + c, TW, ys - t.y0 + ry, ys, n, ry, ylim, Ty, BY + sg * SEG * TW + c,
-                    TW);
-    }
-  }
-  __syncthreads();
-  // ---- 4. packed bounds, rows written coalesced
-  uint32_t* bo = bounds + in.off;
-  for (int i = tid; i < TH * TW; i += kThreads) {
-    const int r = i / TW, c = i % TW;
-    const int x = t.x0 + c, y = t.y0 + r;
-    if (x < W && y < H) bo[y * P + x] = (uint32_t)BX[i] | ((uint32_t)BY[i] << 16);
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -416,43 +250,6 @@ int launch_color_convert_flat(uchar4* guide, long long n, int color_space,
   k_color_convert_flat<<<grid_for(n), kThreads, 0, s>>>(guide, n, color_space);
   DTSGB_CUDA(cudaGetLastError());
   return DTSGB_OK;
-}
-
-int launch_bounds(const DtsLaunch& L, const uchar4* guide, uint32_t* bounds,
-                  float ratio_x, float ratio_y, float sigma_x, float sigma_y,
-                  int ref_y_limit, cudaStream_t s) {
-  const int rx = (int)floorf(sigma_x) + 1, ry = (int)floorf(sigma_y) + 1;
-  if (rx > 255 || ry > 255)
-    return fail(DTSGB_ERR_UNSUPPORTED, "sigma >= 255 is not supported");
-  const int TW = kBoundsTW, TH = kBoundsTH;
-  const size_t smem = sizeof(unsigned) * ((size_t)TH * ((TW + 2 * rx) | 1) +
-                                          (size_t)(TH + 2 * ry) * TW) +
-                      2 * sizeof(uint16_t) * TH * TW;
-  if (smem > kMaxSmem) return fail(DTSGB_ERR_UNSUPPORTED, "sigma too large");
-  // fixed point per axis: r * (sigma + 1) * 2^F <= 2^30; threshold floor(sigma 2^F)
-  auto fx = [](int r, float sigma, float* cap, float* scale, int* T) {
-    *cap = sigma + 1.f;
-    const int F = 30 - (int)std::ceil(std::log2((double)r * (double)*cap));
-    *scale = std::ldexp(1.f, F);
-    *T = (int)std::floor((double)sigma * std::ldexp(1.0, F));
-  };
-  float cap_x, cap_y, scale_x, scale_y;
-  int Tx, Ty;
-  fx(rx, sigma_x, &cap_x, &scale_x, &Tx);
-  fx(ry, sigma_y, &cap_y, &scale_y, &Ty);
-  auto go = [&](auto kern) -> int {
-    int st = set_smem(kern, smem);
-    if (st) return st;
-    ProfScope ps(s, DTSGB_K_BOUNDS);
-    kern<<<L.n_tiles, kThreads, smem, s>>>(L.d_inst, L.d_tiles, guide, bounds, ratio_x,
-                                           ratio_y, rx, ry, ref_y_limit, cap_x, cap_y,
-                                           scale_x, scale_y, Tx, Ty);
-    DTSGB_CUDA(cudaGetLastError());
-    return DTSGB_OK;
-  };
-  if (L.bounds_seg == 4) return go(k_bounds<kBoundsTW, kBoundsTH, 4>);
-  if (L.bounds_seg == 16) return go(k_bounds<kBoundsTW, kBoundsTH, 16>);
-  return go(k_bounds<kBoundsTW, kBoundsTH, kBoundsSegDefault>);
 }
 
 int launch_target_to_float(const DtsLaunch& L, Storage st, const void* src,

@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "../../include/dtsgb.h"
+#include "dts_geom.cuh"
 #include "dtsgb_internal.cuh"
 #include "fixed_point.cuh"
 #include "raw4.cuh"
@@ -36,50 +37,7 @@
 namespace dtsgb {
 namespace {
 
-constexpr int kXWarps = 4;  // row segments of a block, each a warp's own
 constexpr int kNaNBits = 0x7fc00000;
-
-// ---- geometry --------------------------------------------------------------
-// How an instance's lines are cut, from its own size and the halo alone: the
-// fixed-point scale of a window sum comes from the largest magnitude in its
-// segment, so an image has the same bits alone and in a batch.
-//
-// (Without divisions: a thread has a dozen pixels to do.)
-//
-// X: a warp takes a segment of tw pixels of a row and its halo, in rounds of
-// 128 columns that it holds in registers: long segments repeat less halo,
-// short ones spread an image that is too small for the SMs.
-constexpr int kRoundsX = 4, kRoundsWide = 8;  // Wide: halos that need more
-struct XGeom {
-  int tw, ha, halo;  // segment, left halo, both halos
-};
-__host__ __device__ inline int x_rounds(int w, int h, int halo) {
-  const long long px = (long long)w * h;
-  const int need = (halo + 127) / 128 + 1;  // rounds of a segment of 128 pixels
-  const int want = px < (1 << 16) ? 2 : px < (1 << 19) ? 3 : kRoundsX;
-  return need <= 2 ? want : need == 3 ? kRoundsX : kRoundsWide;
-}
-__host__ __device__ inline XGeom x_geom(int w, int h, int hx) {
-  XGeom g;
-  g.ha = (hx + 4) & ~3;
-  g.halo = g.ha + ((hx + 3) & ~3);
-  g.tw = 128 * x_rounds(w, h, g.halo) - g.halo;
-  return g;
-}
-// Y: tiles of 32 columns x th rows, th + 2hy a multiple of the rows that a warp
-// of the launch holds in registers (8, 16 or 32: the tile, and so the result,
-// does not depend on which).
-__host__ __device__ inline int y_lg(int hy) { return hy <= 56 ? 4 : 5; }
-__host__ __device__ inline int y_th(int w, int h, int hy) {
-  const long long px = (long long)w * h;
-  const int lg = y_lg(hy);
-  // up to 16 warps of 16 rows; more where the halo would be most of the tile
-  const int full = hy <= 16 ? 8 : hy <= 56 ? 16 : hy <= 127 ? 12 : hy <= 200 ? 16 : 20;
-  const int want = px < (1 << 16) ? 32 : 64;  // rows of a tile of a small image
-  int warps = (want + 2 * hy + (1 << lg) - 1) >> lg;
-  if (px >= (1 << 19) || warps > full) warps = full;
-  return (warps << lg) - 2 * hy;
-}
 
 // Prefix entry t of a row segment: entry t & 3 of quad t >> 2, one plane of
 // quads per entry of a quad, so that the lanes of a warp (a quad each) read
@@ -488,21 +446,10 @@ template <typename TS, int MODE, bool STEREO, bool OVER>
 int launch_iter(const DtsLaunch& L, const float* vin, float* tmp, float* vout, const void* target,
                 const void* conf, const uint32_t* bounds, float lambda, float step,
                 float overwrite, int feeds, int halo, const StereoArgs& sa, cudaStream_t s) {
-  int rounds = 1, rows = 1;
-  long long px = 0;
-  for (int i = 0; i < L.n_inst; ++i) {
-    const Inst& I = L.h_inst[i];
-    rounds = std::max(rounds, x_rounds(I.w, I.h, x_geom(I.w, I.h, halo).halo));
-    rows = std::max(rows, y_th(I.w, I.h, halo) + 2 * halo);
-    px += (long long)I.w * I.h;
-  }
-  dim3 gx(L.n_xblocks), gy(L.n_yblocks);
-  if (L.n_inst == 1) {
-    const Inst& I = L.h_inst[0];
-    const int tw = x_geom(I.w, I.h, halo).tw, th = y_th(I.w, I.h, halo);
-    gx = dim3((I.h + kXWarps - 1) / kXWarps, (I.w + tw - 1) / tw);
-    gy = dim3((I.w + 31) / 32, (I.h + th - 1) / th);
-  }
+  const PassGrid G = pass_grid(L, halo, halo);
+  const dim3 gx = G.x, gy = G.y;
+  const int rounds = G.rounds, rows = G.rows;
+  const long long px = G.px;
   ProfScope ps(s, DTSGB_K_DTS_ITER);
   int st;
 #define X_ROUNDS(NR)                                                                           \
@@ -542,6 +489,25 @@ int launch_iter_t(const DtsLaunch& L, const float* vin, float* tmp, float* vout,
 }
 
 }  // namespace
+
+PassGrid pass_grid(const DtsLaunch& L, int hx, int hy) {
+  PassGrid G;
+  for (int i = 0; i < L.n_inst; ++i) {
+    const Inst& I = L.h_inst[i];
+    G.rounds = std::max(G.rounds, x_rounds(I.w, I.h, x_geom(I.w, I.h, hx).halo));
+    G.rows = std::max(G.rows, y_th(I.w, I.h, hy) + 2 * hy);
+    G.px += (long long)I.w * I.h;
+  }
+  G.x = dim3(L.n_xblocks);
+  G.y = dim3(L.n_yblocks);
+  if (L.n_inst == 1) {
+    const Inst& I = L.h_inst[0];
+    const int tw = x_geom(I.w, I.h, hx).tw, th = y_th(I.w, I.h, hy);
+    G.x = dim3((I.h + kXWarps - 1) / kXWarps, (I.w + tw - 1) / tw);
+    G.y = dim3((I.w + 31) / 32, (I.h + th - 1) / th);
+  }
+  return G;
+}
 
 void dts_pass_blocks(const Inst* inst, int n, int halo, std::vector<Tile>* x,
                      std::vector<Tile>* y) {

@@ -80,10 +80,9 @@ struct dtsgb_dts_s {
 
   Inst h_inst{};
   Inst* d_inst = nullptr;
-  Tile* d_tb = nullptr;  // bounds tiles
   Tile* d_ti = nullptr;  // iteration tiles
   Tile* d_ti_small = nullptr;  // small iteration tiles when d_ti holds big ones
-  int ntb = 0, nti = 0, nti_small = 0;
+  int nti = 0, nti_small = 0;
 
   bool diff_valid = false;
   float ratio_x = 0.f, ratio_y = 0.f;
@@ -100,7 +99,6 @@ struct dtsgb_dts_s {
   int var_idx = -1;
 
   size_t tsize() const { return st == Storage::F32 ? 4 : 2; }
-  DtsLaunch launch_b() const { return DtsLaunch{d_inst, d_tb, ntb, 1}; }
   bool small = false;
   DtsLaunch launch_i() const {
     return DtsLaunch{d_inst, d_ti, nti, 1, small, small ? nullptr : d_ti_small, nti_small,
@@ -110,14 +108,12 @@ struct dtsgb_dts_s {
 
 static int dts_layout(dtsgb_dts_t h) {
   h->h_inst = Inst{h->w, h->h, h->pitch, 0, 0};
-  std::vector<Tile> tb = make_tiles(h->w, h->h, kBoundsTW, kBoundsTH);
   const long long t64 = (long long)((h->w + kIterTW - 1) / kIterTW) *
                         ((h->h + kIterTH - 1) / kIterTH);
   h->small = use_small_iter_tiles(t64);
   std::vector<Tile> ti =
       h->small ? make_tiles(h->w, h->h, kIterSmallTW, kIterSmallTH)
                : make_tiles(h->w, h->h, kIterTW, kIterTH);
-  h->ntb = (int)tb.size();
   h->nti = (int)ti.size();
   if (!h->small) {
     // small tiles too, for halos that do not fit the big tiles' shared memory
@@ -128,8 +124,6 @@ static int dts_layout(dtsgb_dts_t h) {
     DTSGB_CUDA(cudaStreamSynchronize(h->stream));
   }
   DTSGB_CUDA(cudaMemcpyAsync(h->d_inst, &h->h_inst, sizeof(Inst),
-                             cudaMemcpyHostToDevice, h->stream));
-  DTSGB_CUDA(cudaMemcpyAsync(h->d_tb, tb.data(), tb.size() * sizeof(Tile),
                              cudaMemcpyHostToDevice, h->stream));
   DTSGB_CUDA(cudaMemcpyAsync(h->d_ti, ti.data(), ti.size() * sizeof(Tile),
                              cudaMemcpyHostToDevice, h->stream));
@@ -147,7 +141,6 @@ static void dts_free(dtsgb_dts_t h) {
   for (auto& p : h->v) dfree(p);
   for (auto& p : h->scr) dfree(p);
   dfree(h->d_inst);
-  dfree(h->d_tb);
   dfree(h->d_ti);
   dfree(h->d_ti_small);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
@@ -180,8 +173,6 @@ DTSGB_API int dtsgb_dts_create(int max_w, int max_h, unsigned flags,
     return cuda_fail(e, "cudaStreamCreate");
   }
   h->own_stream = true;
-  const size_t ntiles_b = (size_t)((max_w + kBoundsTW - 1) / kBoundsTW) *
-                          ((max_h + kBoundsTH - 1) / kBoundsTH);
   const size_t ntiles_i = (size_t)((max_w + kIterSmallTW - 1) / kIterSmallTW) *
                           ((max_h + kIterSmallTH - 1) / kIterSmallTH);
   if (!st) st = dalloc(&h->guide, h->plane);
@@ -192,7 +183,6 @@ DTSGB_API int dtsgb_dts_create(int max_w, int max_h, unsigned flags,
   for (int i = 0; i < 4 && !st; ++i) st = dalloc(&h->v[i], h->plane);
   for (int i = 0; i < 2 && !st; ++i) st = dalloc(&h->scr[i], h->plane);
   if (!st) st = dalloc(&h->d_inst, 1);
-  if (!st) st = dalloc(&h->d_tb, ntiles_b);
   if (!st) st = dalloc(&h->d_ti, ntiles_i);
   if (!st) st = dalloc(&h->d_ti_small, ntiles_i);
   if (!st) st = dts_layout(h);
@@ -408,7 +398,7 @@ static int dts_bounds(dtsgb_dts_t h, float sx, float sy, bool use_cache) {
     return DTSGB_OK;
   if (!finite_pos(sx) || !finite_pos(sy))
     return fail(DTSGB_ERR_INVALID_ARGUMENT, "sigma must be finite and positive");
-  int st = launch_bounds(h->launch_b(), h->guide, h->bounds,
+  int st = launch_bounds(h->launch_i(), h->guide, h->bounds,
                          h->diff_valid ? h->ratio_x : -1.f,
                          h->diff_valid ? h->ratio_y : -1.f, sx, sy, h->ref_y,
                          h->stream);

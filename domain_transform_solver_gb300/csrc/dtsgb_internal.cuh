@@ -204,12 +204,10 @@ struct DtsLaunch {
   const Tile* d_tiles_small = nullptr;
   int n_tiles_small = 0;
   const Inst* h_inst = nullptr;  // host copy of the instance table
-  // several instances: the blocks of the iteration's passes for the halo
+  // several instances: the blocks of the passes (bounds, iteration) for the halo
   // (dts_pass_blocks)
   const Tile *d_xblocks = nullptr, *d_yblocks = nullptr;
   unsigned n_xblocks = 0, n_yblocks = 0;
-  // pixels per thread and axis of the window-bound walks (4, 8 or 16)
-  int bounds_seg = 8;
   // the same launch on the small tiles
   DtsLaunch as_small() const {
     DtsLaunch s = *this;
@@ -221,7 +219,6 @@ struct DtsLaunch {
 };
 
 // Tile shapes (compile-time in the kernels).
-constexpr int kBoundsTW = 32, kBoundsTH = 32;
 constexpr int kIterTW = 64, kIterTH = 128;
 // Work too small to give every SM a few 64x64-pixel blocks (under about
 // 2.5 Mpx in all) uses 32x32 tiles.  tiles_big counts kIterTW x kIterTH tiles.

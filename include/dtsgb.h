@@ -492,10 +492,8 @@ DTSGB_API int dtsgb_batch_debug_plane(dtsgb_batch_t b, int i, int which, void* d
  * L2).  The two add a voxel's six neighbour products in different roundings:
  * results agree to FP32 rounding, and each is differentiated exactly. */
 #define DTSGB_TUNE_HFBS_SOLVE_STEPS 3
-/* DTSGB_TUNE_BOUNDS_SEGMENT: pixels each thread of the window-bound search
- * walks per axis with its two pointers (4, 8 or 16; default 8).  Longer
- * segments restart the walk less often, shorter ones spread a tile's lines
- * over more threads; the windows are identical. */
+/* DTSGB_TUNE_BOUNDS_SEGMENT: 4, 8 or 16 (default 8), kept and returned, without
+ * effect: the window-bound search has no segments to choose. */
 #define DTSGB_TUNE_BOUNDS_SEGMENT 4
 DTSGB_API int dtsgb_batch_set_tuning(dtsgb_batch_t b, int knob, long long value);
 DTSGB_API int dtsgb_batch_get_tuning(dtsgb_batch_t b, int knob, long long* value);

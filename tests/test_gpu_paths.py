@@ -229,3 +229,50 @@ def test_adjoint_in_clusters_is_the_adjoint_by_steps(gpu_ready, w, h, sx, sy, sl
         assert np.abs(got[i][0]).max() > 0
         assert np.array_equal(got[i][0], got[2 + i][0])
         assert np.array_equal(got[i][1], got[2 + i][1])
+
+
+# ---- window bounds: a pass along rows and a pass down columns ------------------
+@pytest.mark.parametrize("w,h,sigma", [
+    (1, 1, 8.0), (3, 200, 8.0), (200, 3, 8.0), (40, 300, 71.0),  # lines shorter than a window
+    (130, 70, 8.0), (333, 257, 0.5), (109, 110, 15.9),           # one tile more or less
+    (493, 450, 8.0), (1030, 520, 8.0),                           # segments of 3 and 4 rounds
+    (700, 90, 64.0), (90, 700, 130.0), (1200, 460, 253.0),       # wide halos, 32 rows a warp
+])
+@pytest.mark.parametrize("fix_y", [0, 1])
+def test_window_bounds_are_the_searches_of_the_fixed_point_weights(gpu_ready, w, h, sigma, fix_y):
+    """The linear search over the fixed-point weights, bit for bit."""
+    D = gpu_ready
+    rng = np.random.default_rng(w + 7 * h)
+    y, x = np.mgrid[0:h, 0:w]
+    rgba = (rng.integers(0, 40, (h, w, 4)) + ((x // 9 + y // 5) % 3 * 60)[..., None]).astype(np.uint8)
+    rgba[..., 3] = 255
+    s = D.DomainTransformSolver(D.ImageDim(w, h), D.FLAG_FIX_Y_LIMIT if fix_y else 0)
+    s.InitFrame(D.COLOR_SPACE.RGB, rgba, np.zeros((h, w), np.float32), None)
+    fp = D.DomainFilterParams(sigma_x=8.0, sigma_y=6.0, sigma_r=0.3)
+    s.ComputeColorSpaceDifferential(fp)
+    f = np.float32
+    r = int(np.floor(f(sigma))) + 1
+    F = 30 - int(np.ceil(np.log2(r * float(f(sigma) + f(1)))))
+    T = int(np.floor(float(f(sigma)) * 2.0 ** F))
+    for axis, sig in ((0, fp.sigma_x), (1, fp.sigma_y)):
+        g = rgba.astype(np.int64) if axis == 0 else rgba.astype(np.int64).transpose(1, 0, 2)
+        n, lines = g.shape[1], g.shape[0]
+        ratio = f(sig) / f(fp.sigma_r)
+        d = ((g[:, 1:] - g[:, :-1]) ** 2).sum(-1).astype(f)
+        t = (d * f(0.0000153787)) * ratio
+        wt = np.sqrt((t.astype(np.float64) * float(ratio) + 1.0).astype(f))
+        q = np.rint(np.minimum(wt, f(sigma) + f(1)) * f(2.0 ** F)).astype(np.int64)
+        S = np.concatenate([np.zeros((lines, 1), np.int64), np.cumsum(q, axis=1)], axis=1)
+        lim = n if axis == 0 else (n if fix_y else min(w, h))
+        pos = np.arange(n)[None, :]
+        lower = np.broadcast_to(pos - 1, (lines, n)).copy()
+        upper = np.broadcast_to(pos, (lines, n)).copy()
+        for k in range(min(r, n - 1), 0, -1):  # the nearest pixel beyond sigma wins
+            far = S[:, k:] - S[:, :-k] > T
+            lower[:, k:][far] = np.broadcast_to(pos[:, k:] - k, far.shape)[far]
+            stop = far & (pos[:, k:] < lim)
+            upper[:, :-k][stop] = np.broadcast_to(pos[:, :-k] + k - 1, far.shape)[stop]
+        got = s.DebugBounds(axis, sigma)
+        want = (lower, upper) if axis == 0 else (lower.T, upper.T)
+        assert np.array_equal(got[0], want[0]), axis
+        assert np.array_equal(got[1], want[1]), axis
