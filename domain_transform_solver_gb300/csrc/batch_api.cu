@@ -71,9 +71,6 @@ struct dtsgb_batch_s {
   // device copies of caller pointer arrays (3 x n), for the _device calls,
   // and the host copy of what each slot holds (a slot is re-sent only when
   // the caller's pointers change)
-  float** d_uptr = nullptr;
-  std::vector<const void*> uptr_host;
-  bool uptr_valid[3] = {false, false, false};
   unsigned char* stage = nullptr;  // dense x (rgba 4 B, target 4 B, conf 4 B)
   Inst* d_inst = nullptr;
   Tile* d_ti = nullptr;     // iteration tiles of the shape in use
@@ -191,7 +188,6 @@ void batch_free(dtsgb_batch_t b) {
   dfree(b->ovf);
   dfree(b->sgrid);
   dfree(b->d_soff);
-  dfree(b->d_uptr);
   dfree(b->stage);
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
   b->stream = nullptr;
@@ -527,86 +523,80 @@ int host_upload_plane(dtsgb_batch_t b, const float* const* src, float* dst, int 
   return DTSGB_OK;
 }
 
+// Caller pointers of up to kPtrs instances, handed to a kernel by value: a
+// table in device memory would cost a copy from pageable host memory, which
+// also waits for the stream, before each launch.
+constexpr int kPtrs = 128;
+struct PtrTable {
+  void* p[kPtrs];
+};
+PtrTable ptr_table(const void* const* ptrs, int first, int n) {
+  PtrTable t = {};
+  for (int i = 0; ptrs && i < n; ++i) t.p[i] = const_cast<void*>(ptrs[first + i]);
+  return t;
+}
+
 // Caller device images (dense W x H, one pointer each; null: skipped) <->
 // pitched arena plane: one kernel instead of a row-by-row copy per image.
 template <bool TO_ARENA>
 __global__ void __launch_bounds__(256)
-    k_user_copy(const Inst* __restrict__ insts, float* const* __restrict__ user, float* arena,
-                int cols) {
-  float* u = user[blockIdx.y];
+    k_user_copy(const Inst* __restrict__ insts, const __grid_constant__ PtrTable user,
+                float* arena, int cols) {
+  float* u = static_cast<float*>(user.p[blockIdx.y]);
   if (u) copy_tile_f32<TO_ARENA>(insts[blockIdx.y], u, arena, cols);
 }
 
-// Copies between n caller device images and an arena plane (slot 0..2 of the
-// pointer table, so that up to three such copies can be in flight in order).
-// Send n caller pointers to device slot `slot` unless it already holds them.
-// The copy comes from pageable host memory, so the call may wait for the
-// stream's earlier work; repeated calls with the same buffers skip it.
-int upload_slot(dtsgb_batch_t b, int slot, const void* const* ptrs) {
-  const size_t n = (size_t)b->n;
-  if (b->uptr_host.size() != 3 * n) b->uptr_host.assign(3 * n, nullptr);
-  const void** h = b->uptr_host.data() + slot * n;
-  if (b->uptr_valid[slot] && std::memcmp(h, ptrs, sizeof(void*) * n) == 0) return DTSGB_OK;
-  DTSGB_CUDA(cudaMemcpyAsync(b->d_uptr + slot * n, ptrs, sizeof(void*) * n,
-                             cudaMemcpyHostToDevice, b->stream));
-  std::memcpy(h, ptrs, sizeof(void*) * n);
-  b->uptr_valid[slot] = true;
-  return DTSGB_OK;
-}
-
-int user_plane_copy(dtsgb_batch_t b, float* const* user, float* arena, bool to_arena,
-                    int slot) {
-  float** d = b->d_uptr + (size_t)slot * b->n;
-  if (int st = upload_slot(b, slot, reinterpret_cast<const void* const*>(user))) return st;
+// Copies between n caller device images and an arena plane.
+int user_plane_copy(dtsgb_batch_t b, float* const* user, float* arena, bool to_arena) {
   int cols = 0;
-  const dim3 grid = copy_grid(b, &cols);
-  if (to_arena)
-    k_user_copy<true><<<grid, 256, 0, b->stream>>>(b->d_inst, d, arena, cols);
-  else
-    k_user_copy<false><<<grid, 256, 0, b->stream>>>(b->d_inst, d, arena, cols);
+  dim3 grid = copy_grid(b, &cols);
+  for (int first = 0; first < b->n; first += kPtrs) {
+    grid.y = (unsigned)std::min(kPtrs, b->n - first);
+    const PtrTable t = ptr_table(reinterpret_cast<const void* const*>(user), first, (int)grid.y);
+    if (to_arena)
+      k_user_copy<true><<<grid, 256, 0, b->stream>>>(b->d_inst + first, t, arena, cols);
+    else
+      k_user_copy<false><<<grid, 256, 0, b->stream>>>(b->d_inst + first, t, arena, cols);
+  }
   DTSGB_CUDA(cudaGetLastError());
   return DTSGB_OK;
 }
 
 // Caller device images -> pitched planes (the _device uploads): the guide
-// (color-converted; not written when rgba is null), target and confidence in
+// (color-converted; not written when guide is null), target and confidence in
 // the storage type; a null confidence image stands for ones.
 template <typename TS>
 __global__ void __launch_bounds__(256)
-    k_ingest_ptr(const Inst* __restrict__ insts, uchar4* const* __restrict__ rgba,
-                 float* const* __restrict__ tgt, float* const* __restrict__ cnf,
+    k_ingest_ptr(const Inst* __restrict__ insts, const __grid_constant__ PtrTable rgba,
+                 const __grid_constant__ PtrTable tgt, const __grid_constant__ PtrTable cnf,
                  uchar4* __restrict__ guide, TS* __restrict__ target, TS* __restrict__ conf,
                  int cs, int cols) {
-  ingest_tile<TS>(insts[blockIdx.y], rgba ? rgba[blockIdx.y] : nullptr, tgt[blockIdx.y],
-                  cnf ? cnf[blockIdx.y] : nullptr, guide, target, conf, cs, cols);
+  const int i = blockIdx.y;
+  ingest_tile<TS>(insts[i], static_cast<const uchar4*>(rgba.p[i]),
+                  static_cast<const float*>(tgt.p[i]), static_cast<const float*>(cnf.p[i]), guide,
+                  target, conf, cs, cols);
 }
 
 int device_ingest(dtsgb_batch_t b, int cs, const void* const* rgba,
                   const float* const* target, const float* const* conf) {
-  const size_t n = (size_t)b->n;
-  float** slots = b->d_uptr;  // [rgba | target | confidence]
-  std::vector<const void*> cf(n, nullptr);
-  if (conf)
-    for (size_t i = 0; i < n; ++i) cf[i] = conf[i];
-  int st = DTSGB_OK;
-  if (rgba) st = upload_slot(b, 0, rgba);
-  if (!st) st = upload_slot(b, 1, reinterpret_cast<const void* const*>(target));
-  if (!st) st = upload_slot(b, 2, cf.data());
-  if (st) return st;
-  // the pointer copies come from pageable host memory: the calls return
-  // once the arrays are copied out, so cf may go out of scope
   int cols = 0;
-  const dim3 grid = copy_grid(b, &cols);
-  uchar4* const* rp = rgba ? reinterpret_cast<uchar4* const*>(slots) : nullptr;
+  dim3 grid = copy_grid(b, &cols);
   uchar4* g = rgba ? b->guide : nullptr;
-  if (b->st == Storage::F32)
-    k_ingest_ptr<float><<<grid, 256, 0, b->stream>>>(b->d_inst, rp, slots + n, slots + 2 * n,
-                                                     g, (float*)b->target, (float*)b->conf,
-                                                     cs, cols);
-  else
-    k_ingest_ptr<__nv_bfloat16><<<grid, 256, 0, b->stream>>>(
-        b->d_inst, rp, slots + n, slots + 2 * n, g, (__nv_bfloat16*)b->target,
-        (__nv_bfloat16*)b->conf, cs, cols);
+  for (int first = 0; first < b->n; first += kPtrs) {
+    const int m = std::min(kPtrs, b->n - first);
+    grid.y = (unsigned)m;
+    const PtrTable tr = ptr_table(rgba, first, m);
+    const PtrTable tt = ptr_table(reinterpret_cast<const void* const*>(target), first, m);
+    const PtrTable tc = ptr_table(reinterpret_cast<const void* const*>(conf), first, m);
+    if (b->st == Storage::F32)
+      k_ingest_ptr<float><<<grid, 256, 0, b->stream>>>(b->d_inst + first, tr, tt, tc, g,
+                                                       (float*)b->target, (float*)b->conf, cs,
+                                                       cols);
+    else
+      k_ingest_ptr<__nv_bfloat16><<<grid, 256, 0, b->stream>>>(
+          b->d_inst + first, tr, tt, tc, g, (__nv_bfloat16*)b->target, (__nv_bfloat16*)b->conf,
+          cs, cols);
+  }
   DTSGB_CUDA(cudaGetLastError());
   if (rgba) ++b->guide_gen;
   b->dts_res = -1;
@@ -884,7 +874,6 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
   if (!st) st = dalloc(&b->d_ti_small, ts.size());
   if (!st) st = dalloc(&b->d_hinst, (size_t)n);
   if (!st) st = dalloc(&b->d_soff, (size_t)n);
-  if (!st) st = dalloc(&b->d_uptr, (size_t)3 * n);
   if (!st) {
     e = upload_table(b->d_inst, b->inst.data(), n * sizeof(Inst));
     if (e == cudaSuccess)
@@ -1107,7 +1096,7 @@ static int batch_backward(dtsgb_batch_t b, const float* const* grad_out,
   if (up == cudaMemcpyHostToDevice) {
     if (int st = host_upload_plane(b, grad_out, G.g[0], 0)) return st;
   } else {
-    if (int st = user_plane_copy(b, const_cast<float* const*>(grad_out), G.g[0], true, 0))
+    if (int st = user_plane_copy(b, const_cast<float* const*>(grad_out), G.g[0], true))
       return st;
   }
   const DtsLaunch Li = iter_launch(b);
@@ -1131,7 +1120,7 @@ static int batch_backward(dtsgb_batch_t b, const float* const* grad_out,
     const float* src = k == 0 ? grad_plane_t(b) : grad_plane_c(b);
     if (!dst) continue;
     if (down == cudaMemcpyDeviceToDevice) {
-      if (int st = user_plane_copy(b, dst, const_cast<float*>(src), false, 1 + k)) return st;
+      if (int st = user_plane_copy(b, dst, const_cast<float*>(src), false)) return st;
       continue;
     }
     for (int i = 0; i < b->n; ++i) {
@@ -1300,7 +1289,7 @@ static int batch_hfbs_backward(dtsgb_batch_t b, const float* const* grad_out,
   if (up == cudaMemcpyHostToDevice) {
     if (int st = host_upload_plane(b, grad_out, gout, 0)) return st;
   } else {
-    if (int st = user_plane_copy(b, const_cast<float* const*>(grad_out), gout, true, 0))
+    if (int st = user_plane_copy(b, const_cast<float* const*>(grad_out), gout, true))
       return st;
   }
   std::vector<char> key;
@@ -1316,7 +1305,7 @@ static int batch_hfbs_backward(dtsgb_batch_t b, const float* const* grad_out,
     const float* src = k == 0 ? gt : gc;
     if (!dst) continue;
     if (down == cudaMemcpyDeviceToDevice) {
-      if (int st = user_plane_copy(b, dst, const_cast<float*>(src), false, 1 + k)) return st;
+      if (int st = user_plane_copy(b, dst, const_cast<float*>(src), false)) return st;
       continue;
     }
     for (int i = 0; i < b->n; ++i) {
@@ -1589,7 +1578,7 @@ static int batch_download(dtsgb_batch_t b, int which, float* const* dst,
   for (int i = 0; i < b->n; ++i)
     if (!dst[i]) return fail(DTSGB_ERR_INVALID_ARGUMENT, "null output pointer");
   if (kind == cudaMemcpyDeviceToDevice)
-    return user_plane_copy(b, dst, const_cast<float*>(src), false, 0);
+    return user_plane_copy(b, dst, const_cast<float*>(src), false);
   for (int i = 0; i < b->n; ++i) {
     const Inst& I = b->inst[i];
     const size_t wb = (size_t)I.w * 4;

@@ -276,3 +276,29 @@ def test_window_bounds_are_the_searches_of_the_fixed_point_weights(gpu_ready, w,
         want = (lower, upper) if axis == 0 else (lower.T, upper.T)
         assert np.array_equal(got[0], want[0]), axis
         assert np.array_equal(got[1], want[1]), axis
+
+
+# ---- caller pointers by value: 128 instances a launch --------------------------
+@pytest.mark.parametrize("n", [128, 129, 300])
+def test_more_images_than_a_launch_has_pointers_for(gpu_ready, n):
+    import torch
+    D = gpu_ready
+    rng = np.random.default_rng(n)
+    sizes = [(int(w), int(h)) for w, h in rng.integers(1, 24, (n, 2))]
+    g = [rng.integers(0, 256, (h, w, 4)).astype(np.uint8) for w, h in sizes]
+    t = [rng.normal(0, 1, (h, w)).astype(np.float32) for w, h in sizes]
+    c = [rng.random((h, w)).astype(np.float32) for w, h in sizes]
+    host, dev = D.Batch(sizes), D.Batch(sizes)
+    dev.set_stream(torch.cuda.Stream().cuda_stream)
+    to = [[torch.from_numpy(a).cuda() for a in x] for x in (g, t, c)]
+    out = [torch.full((h, w), -1.0, device="cuda") for w, h in sizes]
+    torch.cuda.synchronize()
+    fp, op = D.DomainFilterParams(), D.DomainOptimizeParams(num_iterations=2, loss=1, sigma_z=4.0)
+    host.upload(D.COLOR_SPACE.YCbCr, g, t, c)
+    host.solve_dts(fp, op)
+    dev.upload_device(D.COLOR_SPACE.YCbCr, *[[a.data_ptr() for a in x] for x in to])
+    dev.solve_dts(fp, op)
+    dev.download_device(0, [o.data_ptr() for o in out])
+    torch.cuda.synchronize()
+    for a, o in zip(host.download(0), out):
+        assert np.array_equal(a, o.cpu().numpy())
