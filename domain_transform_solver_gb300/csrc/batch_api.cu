@@ -68,19 +68,12 @@ struct dtsgb_batch_s {
   std::vector<long long> soff;
   long long dense = 0;
   long long* d_soff = nullptr;
-  // device copies of caller pointer arrays (3 x n), for the _device calls,
-  // and the host copy of what each slot holds (a slot is re-sent only when
-  // the caller's pointers change)
   unsigned char* stage = nullptr;  // dense x (rgba 4 B, target 4 B, conf 4 B)
   Inst* d_inst = nullptr;
-  Tile* d_ti = nullptr;     // iteration tiles of the shape in use
-  Tile* d_ti_big = nullptr;  // kIterTW x kIterTH tiles
-  Tile* d_ti_small = nullptr;  // kIterSmallTW x kIterSmallTH tiles
-  int nti = 0, nti_big = 0, nti_small = 0;
   // blocks of the DTS passes for halo pass_halo (several instances only)
   Tile *d_px = nullptr, *d_py = nullptr;
   int npx = 0, npy = 0, pass_halo = -1;
-  bool small = false;
+  bool small = false;               // accepted and returned (DTSGB_TUNE_DTS_TILE)
   long long hfbs_group_voxels = 0;  // L2-resident HFBS group budget (0: off)
   int hfbs_solve_steps = 4;         // heavy-ball steps per launch (4 or 1)
   int bounds_seg = 8;               // accepted and returned (DTSGB_TUNE_BOUNDS_SEGMENT)
@@ -155,12 +148,6 @@ void free_grad_planes(dtsgb_batch_t b) {
   b->gplanes.clear();
 }
 
-void select_tiles(dtsgb_batch_t b, bool small) {
-  b->small = small;
-  b->d_ti = small ? b->d_ti_small : b->d_ti_big;
-  b->nti = small ? b->nti_small : b->nti_big;
-}
-
 void batch_free(dtsgb_batch_t b) {
   drop_graph(b, b->g_dts);
   drop_graph(b, b->g_hfbs);
@@ -178,11 +165,8 @@ void batch_free(dtsgb_batch_t b) {
   dfree(b->hout);
   dfree(b->scratch);
   dfree(b->d_inst);
-  dfree(b->d_ti_big);
-  dfree(b->d_ti_small);
   dfree(b->d_px);
   dfree(b->d_py);
-  b->d_ti = nullptr;
   dfree(b->d_hinst);
   for (auto& p : b->hg) dfree(p);
   dfree(b->ovf);
@@ -254,8 +238,7 @@ int ensure_pass_blocks(dtsgb_batch_t b, int halo) {
   return DTSGB_OK;
 }
 DtsLaunch iter_launch(dtsgb_batch_t b) {
-  DtsLaunch L{b->d_inst, b->d_ti, b->nti, b->n, b->small, b->d_ti_small, b->nti_small,
-              b->inst.data()};
+  DtsLaunch L{b->d_inst, nullptr, 0, b->n, false, nullptr, 0, b->inst.data()};
   L.d_xblocks = b->d_px;
   L.d_yblocks = b->d_py;
   L.n_xblocks = (unsigned)b->npx;
@@ -831,7 +814,6 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
   b->flags = flags;
   b->st = (flags & DTSGB_FLAG_BF16_STORAGE) ? Storage::BF16 : Storage::F32;
   b->ref_y = (flags & DTSGB_FLAG_FIX_Y_LIMIT) ? 0 : 1;
-  std::vector<Tile> ti, ts;
   long long off = 0, tiles64 = 0;
   for (int i = 0; i < n; ++i)
     tiles64 += (long long)((widths[i] + kIterTW - 1) / kIterTW) *
@@ -845,14 +827,8 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
     off += (long long)I.pitch * I.h;
     b->max_w = std::max(b->max_w, I.w);
     b->max_h = std::max(b->max_h, I.h);
-    for (int y = 0; y < I.h; y += kIterTH)
-      for (int x = 0; x < I.w; x += kIterTW) ti.push_back(Tile{i, x, y, 0});
-    for (int y = 0; y < I.h; y += kIterSmallTH)
-      for (int x = 0; x < I.w; x += kIterSmallTW) ts.push_back(Tile{i, x, y, 0});
   }
   b->total = off;
-  b->nti_big = (int)ti.size();
-  b->nti_small = (int)ts.size();
   int st = DTSGB_OK;
   cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
@@ -870,21 +846,14 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
   if (!st) st = dalloc(&b->hout, T);
   if (!st && b->st == Storage::BF16) st = dalloc(&b->scratch, T);
   if (!st) st = dalloc(&b->d_inst, (size_t)n);
-  if (!st) st = dalloc(&b->d_ti_big, ti.size());
-  if (!st) st = dalloc(&b->d_ti_small, ts.size());
   if (!st) st = dalloc(&b->d_hinst, (size_t)n);
   if (!st) st = dalloc(&b->d_soff, (size_t)n);
   if (!st) {
     e = upload_table(b->d_inst, b->inst.data(), n * sizeof(Inst));
     if (e == cudaSuccess)
       e = upload_table(b->d_soff, b->soff.data(), n * sizeof(long long));
-    if (e == cudaSuccess)
-      e = upload_table(b->d_ti_big, ti.data(), ti.size() * sizeof(Tile));
-    if (e == cudaSuccess)
-      e = upload_table(b->d_ti_small, ts.data(), ts.size() * sizeof(Tile));
     if (e != cudaSuccess) st = cuda_fail(e, "batch tables");
   }
-  select_tiles(b, b->small);
   if (st) {
     batch_free(b);
     delete b;
@@ -1034,7 +1003,6 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
   key_append(key, overwrite);
   key_append(key, b->grad);
   key_append(key, b->grad_seg);
-  key_append(key, b->small);
   key_append(key, keep_bounds);
   int st = run_graph(b, b->g_dts, key, enqueue);
   if (st) {
@@ -1112,7 +1080,6 @@ static int batch_backward(dtsgb_batch_t b, const float* const* grad_out,
   key_append(key, p);
   key_append(key, n_iter);
   key_append(key, b->grad_seg);
-  key_append(key, b->small);
   int st = run_graph(b, b->g_bwd, key, enqueue);
   if (st) return st;
   for (int k = 0; k < 2; ++k) {
@@ -1348,8 +1315,8 @@ DTSGB_API int dtsgb_batch_set_tuning(dtsgb_batch_t b, int knob, long long value)
       return fail(DTSGB_ERR_INVALID_ARGUMENT, "DTS tile must be 64 or 32");
     const bool small = value == kIterSmallTW;
     if (small != b->small) {
-      select_tiles(b, small);
-      b->grad_n = -1;  // checkpoints were computed with the other tile shape
+      b->small = small;
+      b->grad_n = -1;  // a solve before the change is not differentiated
     }
     return DTSGB_OK;
   }
@@ -1406,30 +1373,6 @@ DTSGB_API int dtsgb_batch_get_tuning(dtsgb_batch_t b, int knob, long long* value
 
 }  // extern "C"
 
-// The knob value of `choices` that gives the shortest run, each run timed
-// reps times after one untimed run; choices the kernels cannot take
-// (DTSGB_ERR_UNSUPPORTED) are skipped.  Leaves the knob at the best value.
-template <typename F>
-static int tune_knob(dtsgb_batch_t b, int knob, std::initializer_list<long long> choices,
-                     int reps, F run) {
-  float best = 3.4e38f;
-  long long best_v = -1;
-  for (long long v : choices) {
-    int st = dtsgb_batch_set_tuning(b, knob, v);
-    if (st) return st;
-    float ms = 0.f;
-    st = time_runs(b, reps, run, &ms);
-    if (st == DTSGB_ERR_UNSUPPORTED) continue;  // e.g. a halo too large for this shape
-    if (st) return st;
-    if (ms < best) {
-      best = ms;
-      best_v = v;
-    }
-  }
-  if (best_v < 0) return fail(DTSGB_ERR_UNSUPPORTED, "no tuning choice runs");
-  return dtsgb_batch_set_tuning(b, knob, best_v);
-}
-
 extern "C" {
 
 DTSGB_API int dtsgb_batch_autotune(dtsgb_batch_t b, const dtsgb_filter_params* f,
@@ -1443,12 +1386,8 @@ DTSGB_API int dtsgb_batch_autotune(dtsgb_batch_t b, const dtsgb_filter_params* f
   const bool reuse = b->reuse;
   b->reuse = false;
   int st = DTSGB_OK;
-  if (f) {
-    auto dts = [&]() { return dtsgb_batch_solve_dts(b, f, p, overwrite); };
-    st = tune_knob(b, DTSGB_TUNE_DTS_TILE, {(long long)kIterTW, (long long)kIterSmallTW}, reps,
-                   dts);
-  }
-  if (hp && !st) {
+  // (no knob changes how a DTS solve runs)
+  if (hp) {
     auto hfbs = [&]() { return dtsgb_batch_solve_hfbs(b, hp); };
     float best = 3.4e38f;
     long long best_s = kHfbsMarchSteps, best_g = 0;

@@ -14,8 +14,11 @@
 // (fixed_point.cuh) added with wrapping 32-bit arithmetic, so the
 // shared-memory atomics that build the difference array are exact and their
 // order does not matter: the result is deterministic.
-// One kernel does Y^T for the tile rows over the tile columns plus the X
-// halo, then X^T for the tile, mirroring the forward kernel's X-then-Y tile.
+// Y^T and X^T are a pass each, cut like the forward's (dts_geom.cuh).  In one
+// kernel, 64 x 128 tiles with their halos in shared memory, an iteration took
+// 216 us for 16 images of 1024x768 (456 instructions a pixel, two blocks an SM);
+// the two passes take 142 (52 and 90), bound by the latency of their loads and by
+// HBM3e (12 and 40 B/px).
 //
 // The forward iterates the adjoint needs (the X-step inputs v_k) are
 // recomputed segment by segment from checkpoints v_0 = t, v_K, v_2K, ...
@@ -23,314 +26,262 @@
 #include <algorithm>
 
 #include "../../include/dtsgb.h"
+#include "dts_geom.cuh"
 #include "dtsgb_internal.cuh"
 #include "fixed_point.cuh"
+#include "raw4.cuh"
 
 namespace dtsgb {
 namespace {
 
 constexpr int kT = 256;
 constexpr int kAdjFirst = 1, kAdjLast = 2;
+// Halos above this are refused.
+constexpr int kAdjMaxHalo = 76;
 
-
-// Shared-memory layout (byte offsets, 16-byte aligned regions).
-template <int TW, int TH, int NT>
-struct AdjSmem {
-  size_t s2, by, d, seg, rt, mx, total;
-  AdjSmem(int hx, int hy) {
-    const size_t SR = TH + 2 * hy, SWc = TW + 2 * hx;
-    const size_t nseg = std::max<size_t>(1, NT / SWc);
-    auto up = [](size_t v) { return (v + 15) / 16 * 16; };
-    // The Y bounds (By), the Y segment totals and the X buffers are alive in
-    // turn (By until the scatter, the totals in the column prefix, the X
-    // buffers in X^T) and share one region; this keeps the 64 x 128 tile of
-    // sigma_z = 8 within two CTAs per SM.
-    s2 = 0;                                                    // SR x SWc f32
-    by = up(s2 + SR * SWc * 4);                                // By | totals | X buffers
-    seg = by;                                                  // nseg x SWc u32
-    d = up(by + std::max({SR * SWc * 2, (size_t)(NT / 32) * (TW + 1) * 4,
-                          nseg * SWc * 4}));
-    rt = up(d + (size_t)(TH + 1) * SWc * 4);                   // (TH+1) x SWc u32 at d
-    mx = up(rt + (size_t)(2 * std::max(hx, hy) + 2) * 4);
-    total = mx + 16;
-  }
-};
-
-template <typename TS, int MODE, int TW, int TH, int NT>
-__global__ void __launch_bounds__(NT, 1024 / NT)
-    k_dts_adjoint(const Inst* __restrict__ insts, const Tile* __restrict__ tiles,
-                  const float* __restrict__ gin, float* __restrict__ gout,
-                  const float* __restrict__ vk, const TS* __restrict__ tgt,
-                  const TS* __restrict__ cnf, const uint32_t* __restrict__ bnd,
-                  float* __restrict__ grad_t, float* __restrict__ grad_c,
-                  float lambda, float step, int hx, int hy, int flags,
-                  AdjSmem<TW, TH, NT> L) {
-  // flags: kAdjFirst, the first adjoint of a backward (dL/dt and dL/dc start
-  // at zero: not read); kAdjLast, the last (its dL/dv_0 goes into dL/dt, as
-  // v_0 = t, instead of to gout)
-  const bool first = flags & kAdjFirst, last = flags & kAdjLast;
-  constexpr int NW = NT / 32;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const Tile t = tiles[blockIdx.x];
+// Y^T: gout = (1 - slam) gin + slam * By^T gin.  A block per 32 columns x th
+// rows, lanes on columns; a warp holds RM staged rows (gradient and bounds) in
+// registers, scatters the ends of their windows into the block's difference
+// array (lanes on 32 banks) and completes the rows of the tile among them.
+template <int RM>
+__global__ void __launch_bounds__(RM == 32 ? 768 : 512, RM == 8 ? 3 : RM == 16 ? 2 : 1)
+    k_adj_y(const Inst* __restrict__ insts, const float* __restrict__ gin,
+            float* __restrict__ gout, const uint32_t* __restrict__ bnd, float slam, int hy,
+            const Tile* __restrict__ blocks) {
+  extern __shared__ unsigned smy[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x;
+  const Tile t = blocks ? blocks[blockIdx.x] : Tile{0, (int)blockIdx.x, (int)blockIdx.y, 0};
   const Inst in = insts[t.inst];
   const int W = in.w, H = in.h, P = in.pitch;
-  const int SR = TH + 2 * hy, SWc = TW + 2 * hx;
-  const int NSEG = max(1, NT / SWc);
-  float* S2 = reinterpret_cast<float*>(smraw + L.s2);  // a2 = g2/n_y, then g1
-  uint16_t* By = reinterpret_cast<uint16_t*>(smraw + L.by);
-  unsigned* Xb = reinterpret_cast<unsigned*>(smraw + L.by);  // X phase, per warp
-  unsigned* D = reinterpret_cast<unsigned*>(smraw + L.d);
-  unsigned* segtot = reinterpret_cast<unsigned*>(smraw + L.seg);
-  float* rtab = reinterpret_cast<float*>(smraw + L.rt);
-  unsigned* smax = reinterpret_cast<unsigned*>(smraw + L.mx);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // per-instance bases: every offset below is a 32-bit pixel index
-  const float* gin_i = gin + in.off;
-  float* gout_i = gout + in.off;
-  const float* vk_i = vk + in.off;
-  const TS* tgt_i = tgt + in.off;
-  const TS* cnf_i = cnf + in.off;
-  const uint32_t* bnd_i = bnd + in.off;
-  float* gt_i = grad_t + in.off;
-  float* gc_i = grad_c + in.off;
-  const int nrt = 2 * max(hx, hy) + 2;
-  for (int i = tid; i < nrt; i += NT) rtab[i] = i ? __frcp_rn((float)i) : 0.f;
-  for (int i = tid; i < (TH + 1) * SWc; i += NT) D[i] = 0u;
+  const int th = y_th(W, H, hy), rows = th + 2 * hy, warps = rows / RM;
+  const int nrt = 2 * hy + 2;
+  unsigned* smax = smy;
+  float* rtab = reinterpret_cast<float*>(smy + 1);  // 1/n
+  unsigned* tot = smy + 1 + nrt;                    // warps x 32
+  unsigned* D = tot + warps * 32;                   // (rows + 1) x 32
+  for (int i = tid; i < nrt; i += nt) rtab[i] = i ? __frcp_rn((float)i) : 0.f;
+  for (int i = tid; i < (rows + 1) * 32; i += nt) D[i] = 0u;
   if (tid == 0) *smax = 0u;
   __syncthreads();
-  const int gx0 = t.x0 - hx, gy0 = t.y0 - hy;
-  const float slam = step * lambda;
-  const int lgx = ceil_log2(2 * hx + 1), lgy = ceil_log2(2 * hy + 1);
-  // ---- Y^T: a2 = g2 / n_y over the tile + halo --------------------------------
-  float m = 0.f;
-  // one warp per row, lanes along the row (no index divisions), two rows of
-  // loads in flight
-  constexpr int NWp = NT / 32;
-  for (int r0 = warp; r0 < SR; r0 += 2 * NWp) {
-    for (int c0 = lane; c0 < SWc; c0 += 32) {
-      uint32_t bb[2];
-      float gg[2];
+  pdl_wait_then_release();
+  if (warp >= warps) return;  // (whole warps; see the barriers)
+  const int live = 32 * warps;
+  const int x = t.x0 * 32 + lane, y0 = t.y0 * th;
+  const bool inx = x < W;
+  const int s0 = warp * RM;      // the warp's first staged row
+  const int ys = y0 - hy + s0;   // its image row
+  const long long first = in.off + (long long)ys * P + x;
+  const float* gc = gin + first;
+  const uint32_t* bc = bnd + first;
+  float v[RM];
+  uint32_t b[RM];
+  if (t.x0 * 32 + 32 <= W && ys >= 0 && ys + RM <= H) {  // the whole warp inside
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int r = r0 + u * NWp, x = gx0 + c0, y = gy0 + r;
-        const bool ok = r < SR && (unsigned)x < (unsigned)W && (unsigned)y < (unsigned)H;
-        const int p = y * P + x;
-        bb[u] = ok ? __ldg(bnd_i + p) : 0u;
-        gg[u] = ok ? __ldg(gin_i + p) : 0.f;
-      }
+    for (int k = 0; k < RM; ++k) v[k] = __ldg(gc + (long long)k * P);
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int r = r0 + u * NWp;
-        if (r >= SR) break;
-        const uint16_t b16 = (uint16_t)(bb[u] >> 16);
-        const int n = min((int)(b16 & 0xff), hy + 1) + min((int)(b16 >> 8), hy);
-        const float a = b16 ? gg[u] * rtab[n] : 0.f;
-        S2[r * SWc + c0] = a;
-        By[r * SWc + c0] = b16;
-        m = fmaxf(m, fabsf(a));
-      }
+    for (int k = 0; k < RM; ++k) b[k] = __ldg(bc + (long long)k * P) >> 16;
+  } else {
+#pragma unroll
+    for (int k = 0; k < RM; ++k) {
+      const bool ok = inx && (unsigned)(ys + k) < (unsigned)H;
+      v[k] = ok ? __ldg(gc + (long long)k * P) : 0.f;
+      b[k] = ok ? __ldg(bc + (long long)k * P) >> 16 : 0u;
     }
   }
+  float m = 0.f;
+#pragma unroll
+  for (int k = 0; k < RM; ++k) m = fmaxf(m, fabsf(v[k] * rtab[(b[k] & 0xff) + (b[k] >> 8)]));
   m = warp_max_nonneg(m);
   if (lane == 0) atomicMax(smax, __float_as_uint(m));
-  __syncthreads();
-  {
-    const int F = fx_shift(__uint_as_float(*smax), lgy);
-    const float sF = pow2f(F);
-    for (int r = warp; r < SR; r += NWp) {
-      for (int c = lane; c < SWc; c += 32) {
-        const int i = r * SWc + c;
-        const uint16_t b16 = By[i];
-        if (!b16) continue;  // outside the image (a window always holds its pixel)
-        const int dl = min((int)(b16 & 0xff), hy + 1), du = min((int)(b16 >> 8), hy);
-        const int lo = max(r - hy - dl + 1, 0), hi = min(r - hy + du, TH - 1);
-        if (lo > hi) continue;
-        const unsigned A = fx_from(S2[i], sF);
-        atomicAdd(D + lo * SWc + c, A);
-        atomicAdd(D + (hi + 1) * SWc + c, 0u - A);
-      }
-    }
-    __syncthreads();
-    // column prefix over the tile rows, in segments
-    const int seg = (TH + NSEG - 1) / NSEG;
-    for (int i = tid; i < SWc * NSEG; i += NT) {
-      const int c = i % SWc, sg = i / SWc;
-      const int k0 = min(sg * seg, TH), k1 = min(k0 + seg, TH);
-      unsigned acc = 0;
-      for (int k = k0; k < k1; ++k) {
-        acc += D[k * SWc + c];
-        D[k * SWc + c] = acc;
-      }
-      segtot[sg * SWc + c] = acc;
-    }
-    __syncthreads();
-    const float isF = pow2f(-F);
-    for (int i = tid; i < SWc * NSEG; i += NT) {
-      const int c = i % SWc, sg = i / SWc;
-      const int k0 = min(sg * seg, TH), k1 = min(k0 + seg, TH);
-      unsigned off = 0;
-      for (int s2 = 0; s2 < sg; ++s2) off += segtot[s2 * SWc + c];
-      const int x = gx0 + c;
-      const bool xok = (unsigned)x < (unsigned)W;
-      for (int k = k0; k < k1; k += 4) {
-        float gv[4];
+  asm volatile("bar.sync 1, %0;" ::"r"(live) : "memory");
+  const int F = fx_shift(__uint_as_float(*smax), ceil_log2(2 * hy + 1));
+  const float sF = pow2f(F), isF = pow2f(-F);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int y = t.y0 + k + j;
-          gv[j] = (k + j < k1 && xok && y < H) ? __ldg(gin_i + y * P + x) : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (k + j >= k1) break;
-          const int y = t.y0 + k + j;
-          float g1 = 0.f;
-          if (xok && y < H) {
-            const float bt = fx_window(D[(k + j) * SWc + c] + off, 0u, isF);
-            g1 = __fmaf_rn(1.f - slam, gv[j], slam * bt);
-          }
-          S2[(k + j) * SWc + c] = g1;  // g1, rows of the tile only
-        }
-      }
+  for (int k = 0; k < RM; ++k) {
+    if (b[k]) {  // (a window holds its pixel: 0 is outside the image)
+      const int dl = (int)(b[k] & 0xff), du = (int)(b[k] >> 8);
+      const unsigned A = fx_from(v[k] * rtab[dl + du], sF);
+      atomicAdd(D + max(s0 + k - dl + 1, 0) * 32 + lane, A);
+      atomicAdd(D + min(s0 + k + du + 1, rows) * 32 + lane, 0u - A);
     }
   }
+  asm volatile("bar.sync 1, %0;" ::"r"(live) : "memory");
+  const unsigned* Dw = D + s0 * 32 + lane;
+  unsigned acc = 0u;
+#pragma unroll
+  for (int k = 0; k < RM; ++k) acc += Dw[k * 32];
+  tot[warp * 32 + lane] = acc;
+  asm volatile("bar.sync 1, %0;" ::"r"(live) : "memory");
+  if (!inx) return;
+  acc = 0u;
+  for (int w = 0; w < warp; ++w) acc += tot[w * 32 + lane];
+  const int k0 = max(hy - s0, 0), k1 = min(min(th, H - y0) + hy - s0, RM);  // tile rows
+  float* oc = gout + first;
+#pragma unroll
+  for (int k = 0; k < RM; ++k) {
+    acc += Dw[k * 32];
+    if (k >= k0 && k < k1)
+      oc[(long long)k * P] = __fmaf_rn(1.f - slam, v[k], slam * fx_window(acc, 0u, isF));
+  }
+}
+
+// X^T and the parameter gradients, from g1 = Y^T's result: a warp per row
+// segment, four adjacent pixels a lane and round in registers, the difference
+// array and its prefix in the warp's shared memory.  flags: kAdjFirst, the
+// first adjoint of a backward (dL/dt and dL/dc start at zero: not read);
+// kAdjLast, the last (its dL/dv_0 goes into dL/dt, as v_0 = t, instead of to
+// gout).  The five planes of a round are loaded when the round is due: loads a
+// round ahead held 124 registers, four blocks an SM (115 us against 90).
+template <typename TS, int MODE, int NR>
+__global__ void __launch_bounds__(32 * kXWarps, NR <= 4 ? 7 : 4)
+    k_adj_x(const Inst* __restrict__ insts, const float* __restrict__ g1p,
+            float* __restrict__ gout, const float* __restrict__ vk, const TS* __restrict__ tgt,
+            const TS* __restrict__ cnf, const uint32_t* __restrict__ bnd,
+            float* __restrict__ grad_t, float* __restrict__ grad_c, float lambda, float step,
+            int hx, int flags, const Tile* __restrict__ blocks) {
+  using PX = XPrefix<NR>;
+  extern __shared__ unsigned smx[];
+  const bool read = !(flags & kAdjFirst), last = flags & kAdjLast;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned* S = smx + warp * (4 * PX::QS);
+  char* Sb = reinterpret_cast<char*>(S);
+  float* rtab = reinterpret_cast<float*>(smx + kXWarps * 4 * PX::QS);  // 1/n
+  const Tile t = blocks ? blocks[blockIdx.x] : Tile{0, (int)blockIdx.y, (int)blockIdx.x, 0};
+  const Inst in = insts[t.inst];
+  const int W = in.w;
+  const XGeom g = x_geom(W, in.h, hx);
+  const int row = t.y0 * kXWarps + warp, x0 = t.x0 * g.tw;
+  const int nrt = 2 * hx + 2;
+  for (int i = tid; i < nrt; i += 32 * kXWarps) rtab[i] = i ? __frcp_rn((float)i) : 0.f;
+#pragma unroll
+  for (int r = 0; r < NR; ++r)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) S[k * PX::QS + lane + 32 * r] = 0u;
   __syncthreads();
-  // ---- X^T and the parameter gradients: one warp per tile row ----------------
-  // A warp's global loads for its next row are issued before it works on the
-  // current one.  Each lane owns CPL adjacent tile columns (vector loads and
-  // stores; one warp scan per row).
-  constexpr int CPL = TW / 32;  // tile columns per lane, adjacent
-  constexpr int BPL = 4;        // prefetched window columns per lane
-  static_assert(CPL == 1 || CPL == 2, "tile width 32 or 64");
-  struct RowAdj {
-    uint32_t bh[BPL];  // packed bounds of window columns lane + 32j
-    float v[CPL], tv[CPL], cv[CPL], gt[CPL], gc[CPL];  // tile columns CPL*lane + k
-  };
-  const int xl = t.x0 + CPL * lane;  // first tile column of this lane
-  auto fetch = [&](int rr, RowAdj& R) {
-    const int row = (t.y0 + rr) * P;
+  pdl_wait_then_release();
+  if (row >= in.h) return;
+  const int xe = min(x0 + g.tw, W);
+  const int rounds = (xe - x0 + g.halo + 127) >> 7;
+  const int xl = x0 - g.ha + 4 * lane;  // the lane's first pixel of round 0
+  const long long base = in.off + (long long)row * in.pitch;
+  float4 v[NR];
+  uint4 b[NR];
 #pragma unroll
-    for (int j = 0; j < BPL; ++j) {
-      const int c = lane + 32 * j, x = gx0 + c;
-      R.bh[j] = (c < SWc && (unsigned)x < (unsigned)W) ? __ldg(bnd_i + row + x) : 0u;
+  for (int r = 0; r < NR; ++r) {
+    const int x = xl + 128 * r;
+    v[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+    b[r] = make_uint4(0u, 0u, 0u, 0u);
+    if (x >= 0 && x < W && r < rounds) {
+      v[r] = __ldg(reinterpret_cast<const float4*>(g1p + base + x));
+      b[r] = __ldg(reinterpret_cast<const uint4*>(bnd + base + x));
+      // columns past the width: the pitch's padding
+      if (x + 1 >= W) b[r].y = 0u;
+      if (x + 2 >= W) b[r].z = 0u;
+      if (x + 3 >= W) b[r].w = 0u;
     }
-    const int p = row + xl;
-    if (CPL == 2 && xl + 1 < W) {  // both columns inside: 8-byte aligned pairs
-      const float2 v = __ldg(reinterpret_cast<const float2*>(vk_i + p));
-      const float2 g0 =
-          first ? make_float2(0.f, 0.f) : *reinterpret_cast<const float2*>(gt_i + p);
-      const float2 g1 =
-          first ? make_float2(0.f, 0.f) : *reinterpret_cast<const float2*>(gc_i + p);
-      R.v[0] = v.x;
-      R.v[CPL - 1] = v.y;
-      R.gt[0] = g0.x;
-      R.gt[CPL - 1] = g0.y;
-      R.gc[0] = g1.x;
-      R.gc[CPL - 1] = g1.y;
-#pragma unroll
-      for (int k = 0; k < CPL; ++k) {
-        R.tv[k] = load_f(tgt_i + p + k);
-        R.cv[k] = load_f(cnf_i + p + k);
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < CPL; ++k) {
-        const bool ok = xl + k < W;
-        R.v[k] = ok ? __ldg(vk_i + p + k) : 0.f;
-        R.tv[k] = ok ? load_f(tgt_i + p + k) : 0.f;
-        R.cv[k] = ok ? load_f(cnf_i + p + k) : 0.f;
-        R.gt[k] = ok && !first ? gt_i[p + k] : 0.f;
-        R.gc[k] = ok && !first ? gc_i[p + k] : 0.f;
+  }
+  struct Quad {
+    float4 v, gt, gc;
+    Raw4<TS> tv, cv;
+  };
+  auto mine = [&](int r) { return xl + 128 * r >= x0 && xl + 128 * r < xe; };
+  auto fetch = [&](int r, Quad& Q) {
+    if (r < rounds && mine(r)) {
+      const long long p = base + xl + 128 * r;
+      Q.v = __ldg(reinterpret_cast<const float4*>(vk + p));
+      Q.tv.load(tgt + p);
+      Q.cv.load(cnf + p);
+      if (read) {
+        Q.gt = *reinterpret_cast<const float4*>(grad_t + p);
+        Q.gc = *reinterpret_cast<const float4*>(grad_c + p);
       }
     }
   };
-  const int rows = min(TH, H - t.y0);
-  unsigned* xb = Xb + warp * (TW + 1);
-  RowAdj cur, nxt;
-  if (warp < rows) fetch(warp, cur);
-  for (int rr = warp; rr < rows; rr += NW) {
-    if (rr + NW < rows) fetch(rr + NW, nxt);
-    const int row = (t.y0 + rr) * P;
-    const float* g1r = S2 + rr * SWc;
-    // visit(b, c) for the window columns c of this lane: the first BPL from
-    // the prefetched registers, any further ones (halos above 32) reloaded
-    auto for_columns = [&](auto&& visit) {
+  Quad Q;
+  Q.v = Q.gt = Q.gc = make_float4(0.f, 0.f, 0.f, 0.f);
+  Q.tv.zero();
+  Q.cv.zero();
+  // n of a pixel of its packed bounds (0 outside the image: 1/n = 0)
+  auto count = [](uint32_t w) { return (w & 0xff) + ((w >> 8) & 0xff); };
+  float m = 0.f;
 #pragma unroll
-      for (int j = 0; j < BPL; ++j) {
-        const int c = lane + 32 * j;
-        if (c < SWc && cur.bh[j]) visit(cur.bh[j], c);
-      }
-      for (int c = lane + 32 * BPL; c < SWc; c += 32) {
-        const int x = gx0 + c;
-        if ((unsigned)x < (unsigned)W) visit(__ldg(bnd_i + row + x), c);
-      }
-    };
-    for (int k = lane; k <= TW; k += 32) xb[k] = 0u;
-    float mx = 0.f;
-    for_columns([&](uint32_t b, int c) {
-      const int n = min((int)(b & 0xff), hx + 1) + min((int)((b >> 8) & 0xff), hx);
-      mx = fmaxf(mx, fabsf(g1r[c] * rtab[n]));
-    });
-    mx = warp_max_nonneg(mx);
-    const int F = fx_shift(mx, lgx);
-    const float sF = pow2f(F), isF = pow2f(-F);
-    __syncwarp();
-    for_columns([&](uint32_t b, int c) {
-      const int dl = min((int)(b & 0xff), hx + 1), du = min((int)((b >> 8) & 0xff), hx);
-      const int lo = max(c - hx - dl + 1, 0), hi = min(c - hx + du, TW - 1);
-      if (lo > hi) return;
-      const unsigned A = fx_from(g1r[c] * rtab[dl + du], sF);
-      atomicAdd(xb + lo, A);
-      atomicAdd(xb + hi + 1, 0u - A);
-    });
-    __syncwarp();
-    // inclusive prefix of the difference array over this lane's columns
-    unsigned incl[CPL];
-    incl[0] = xb[CPL * lane];
+  for (int r = 0; r < NR; ++r)
 #pragma unroll
-    for (int k = 1; k < CPL; ++k) incl[k] = incl[k - 1] + xb[CPL * lane + k];
-    const unsigned off = warp_incl_scan(incl[CPL - 1], lane) - incl[CPL - 1];
-    float go[CPL], gtn[CPL], gcn[CPL];
+    for (int k = 0; k < 4; ++k)
+      if (r < rounds && u4_get(b[r], k))
+        m = fmaxf(m, fabsf(f4_get(v[r], k) * rtab[count(u4_get(b[r], k))]));
+  m = warp_max_nonneg(m);
+  const int F = fx_shift(m, ceil_log2(2 * hx + 1));
+  const float sF = pow2f(F), isF = pow2f(-F);
+  const int end = 128 * rounds;
 #pragma unroll
-    for (int k = 0; k < CPL; ++k) {
-      const int x = xl + k;
-      go[k] = gtn[k] = gcn[k] = 0.f;
-      if (x >= W) continue;
-      const float bt = fx_window(incl[k] + off, 0u, isF);
-      const float g1 = g1r[hx + CPL * lane + k];
-      const uint32_t b = __ldg(bnd_i + row + x);
-      const float rn = rtab[min((int)(b & 0xff), hx + 1) + min((int)((b >> 8) & 0xff), hx)];
-      const float v = cur.v[k], tv = cur.tv[k], cv = cur.cv[k];
-      const float d = v - tv;
-      float dh_dv, dh_dc;
-      if (MODE == 0) {
-        dh_dv = cv * rn;
-        dh_dc = d * rn;
-      } else {
-        const float rt = __fsqrt_rn(__fmaf_rn(d, d, 1e-6f));
-        dh_dv = __fdiv_rn(0.5f * (cv * rn) * 1e-6f, rt * rt * rt);
-        dh_dc = __fdiv_rn(0.5f * d * rn, rt);
-      }
-      go[k] = __fmaf_rn(1.f - slam - step * dh_dv, g1, slam * bt);
-      gtn[k] = cur.gt[k] + step * dh_dv * g1;
-      gcn[k] = cur.gc[k] - step * dh_dc * g1;
-      if (last) gtn[k] += go[k];
-    }
-    const int p = row + xl;
-    if (CPL == 2 && xl + 1 < W) {
-      if (!last) *reinterpret_cast<float2*>(gout_i + p) = make_float2(go[0], go[CPL - 1]);
-      *reinterpret_cast<float2*>(gt_i + p) = make_float2(gtn[0], gtn[CPL - 1]);
-      *reinterpret_cast<float2*>(gc_i + p) = make_float2(gcn[0], gcn[CPL - 1]);
-    } else {
+  for (int r = 0; r < NR; ++r)
+    if (r < rounds)
 #pragma unroll
-      for (int k = 0; k < CPL; ++k)
-        if (xl + k < W) {
-          if (!last) gout_i[p + k] = go[k];
-          gt_i[p + k] = gtn[k];
-          gc_i[p + k] = gcn[k];
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t w = u4_get(b[r], k);
+        if (w) {
+          const int dl = (int)(w & 0xff), du = (int)((w >> 8) & 0xff);
+          const int i = 4 * lane + 128 * r + k;
+          const unsigned A = fx_from(f4_get(v[r], k) * rtab[dl + du], sF);
+          atomicAdd(PX::entry(Sb, max(i - dl + 1, 0)), A);
+          atomicAdd(PX::entry(Sb, min(i + du + 1, end)), 0u - A);
         }
+      }
+  __syncwarp();
+  const float slam = step * lambda;
+  unsigned carry = 0u;
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    if (r < rounds) {
+      unsigned a[4];
+      fetch(r, Q);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) a[k] = S[k * PX::QS + lane + 32 * r];
+#pragma unroll
+      for (int k = 1; k < 4; ++k) a[k] += a[k - 1];
+      const unsigned incl = warp_incl_scan(a[3], lane);
+      const unsigned off = carry + incl - a[3];
+      carry += __shfl_sync(0xffffffffu, incl, 31);
+      const Quad& q = Q;
+      if (!mine(r)) continue;
+      float go[4], gt[4], gc[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float bt = fx_window(off + a[k], 0u, isF);
+        const float g1 = f4_get(v[r], k), rn = rtab[count(u4_get(b[r], k))];
+        const float vv = f4_get(q.v, k), tv = q.tv[k], cv = q.cv[k];
+        const float d = vv - tv;
+        float dh_dv, dh_dc;
+        if (MODE == 0) {
+          dh_dv = cv * rn;
+          dh_dc = d * rn;
+        } else {
+          const float rt = __fsqrt_rn(__fmaf_rn(d, d, 1e-6f));
+          dh_dv = __fdiv_rn(0.5f * (cv * rn) * 1e-6f, rt * rt * rt);
+          dh_dc = __fdiv_rn(0.5f * d * rn, rt);
+        }
+        go[k] = __fmaf_rn(1.f - slam - step * dh_dv, g1, slam * bt);
+        gt[k] = f4_get(q.gt, k) + step * dh_dv * g1;
+        gc[k] = f4_get(q.gc, k) - step * dh_dc * g1;
+        if (last) gt[k] += go[k];
+      }
+      const int x = xl + 128 * r;
+      const long long p = base + x;
+      if (x + 4 <= W) {
+        if (!last) *reinterpret_cast<float4*>(gout + p) = make_float4(go[0], go[1], go[2], go[3]);
+        *reinterpret_cast<float4*>(grad_t + p) = make_float4(gt[0], gt[1], gt[2], gt[3]);
+        *reinterpret_cast<float4*>(grad_c + p) = make_float4(gc[0], gc[1], gc[2], gc[3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (x + k < W) {
+            if (!last) gout[p + k] = go[k];
+            grad_t[p + k] = gt[k];
+            grad_c[p + k] = gc[k];
+          }
+      }
     }
-    __syncwarp();  // the warp's buffer is cleared for its next row
-    cur = nxt;
   }
 }
 
@@ -343,57 +294,56 @@ __global__ void k_axpy_planes(const Inst* __restrict__ insts, const float* __res
     y[in.off + i] += a[in.off + i];
 }
 
-template <typename TS, int MODE, int TW, int TH>
-int launch_adj_shape(const DtsLaunch& L, const float* gin, float* gout, const float* vk,
-                     const void* t, const void* c, const uint32_t* bounds, float* gt,
-                     float* gc, float lambda, float step, int hx, int hy, int flags,
-                     cudaStream_t s) {
-  constexpr int NT = TW >= 64 ? 512 : 256;
-  const AdjSmem<TW, TH, NT> lay(hx, hy);
-  if (lay.total > 227 * 1024)
-    return fail(DTSGB_ERR_UNSUPPORTED, "sigma_z too large for the adjoint");
-  if (lay.total > 48 * 1024)
-    DTSGB_CUDA(cudaFuncSetAttribute(k_dts_adjoint<TS, MODE, TW, TH, NT>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)lay.total));
-  k_dts_adjoint<TS, MODE, TW, TH, NT><<<L.n_tiles, NT, lay.total, s>>>(
-      L.d_inst, L.d_tiles, gin, gout, vk, (const TS*)t, (const TS*)c, bounds, gt, gc,
-      lambda, step, hx, hy, flags, lay);
-  DTSGB_CUDA(cudaGetLastError());
+template <int RM>
+int launch_y(const DtsLaunch& L, const PassGrid& G, const float* gin, float* gout,
+             const uint32_t* bounds, float slam, int hy, cudaStream_t s) {
+  auto kern = k_adj_y<RM>;
+  const int warps = G.rows / RM;
+  const size_t smem = sizeof(unsigned) *
+                      ((size_t)(2 * hy + 3) + warps * 32 + ((size_t)G.rows + 1) * 32);
+  if (smem > 48 * 1024)
+    DTSGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DTSGB_CUDA(launch_dependent(kern, G.y, dim3(32 * warps), smem, s, L.d_inst, gin, gout, bounds,
+                              slam, hy, L.n_inst > 1 ? L.d_yblocks : (const Tile*)nullptr));
   return DTSGB_OK;
 }
 
 template <typename TS, int MODE>
-int launch_adj_t(const DtsLaunch& L, const float* gin, float* gout, const float* vk,
-                 const void* t, const void* c, const uint32_t* bounds, float* gt, float* gc,
-                 float lambda, float step, int hx, int hy, int flags, cudaStream_t s) {
-  if (L.small)
-    return launch_adj_shape<TS, MODE, kIterSmallTW, kIterSmallTH>(
-        L, gin, gout, vk, t, c, bounds, gt, gc, lambda, step, hx, hy, flags, s);
-  if (L.d_tiles_small && AdjSmem<kIterTW, kIterTH, 512>(hx, hy).total > 227 * 1024)
-    return launch_adj_shape<TS, MODE, kIterSmallTW, kIterSmallTH>(
-        L.as_small(), gin, gout, vk, t, c, bounds, gt, gc, lambda, step, hx, hy, flags, s);
-  return launch_adj_shape<TS, MODE, kIterTW, kIterTH>(L, gin, gout, vk, t, c, bounds, gt,
-                                                      gc, lambda, step, hx, hy, flags, s);
+int launch_adj_t(const DtsLaunch& L, float* g, float* g1, const float* vk, const void* t,
+                 const void* c, const uint32_t* bounds, float* gt, float* gc, float lambda,
+                 float step, int halo, int flags, cudaStream_t s) {
+  const PassGrid G = pass_grid(L, halo, halo);
+  const float slam = step * lambda;
+  int st;
+  // the rows a warp holds: as the forward's Y pass
+  if (G.rows <= 128 && G.px < (4 << 20)) st = launch_y<8>(L, G, g, g1, bounds, slam, halo, s);
+  else if (G.rows <= 256) st = launch_y<16>(L, G, g, g1, bounds, slam, halo, s);
+  else st = launch_y<32>(L, G, g, g1, bounds, slam, halo, s);
+  if (st) return st;
+  auto x = [&](auto kern, int qs) -> int {
+    const size_t smem = sizeof(unsigned) * ((size_t)kXWarps * 4 * qs + 2 * halo + 2);
+    DTSGB_CUDA(launch_dependent(kern, G.x, dim3(32 * kXWarps), smem, s, L.d_inst, g1, g, vk,
+                                (const TS*)t, (const TS*)c, bounds, gt, gc, lambda, step, halo,
+                                flags, L.n_inst > 1 ? L.d_xblocks : (const Tile*)nullptr));
+    return DTSGB_OK;
+  };
+  if (G.rounds <= 2) return x(k_adj_x<TS, MODE, 2>, XPrefix<2>::QS);
+  if (G.rounds <= 3) return x(k_adj_x<TS, MODE, 3>, XPrefix<3>::QS);
+  if (G.rounds <= kRoundsX) return x(k_adj_x<TS, MODE, kRoundsX>, XPrefix<kRoundsX>::QS);
+  return x(k_adj_x<TS, MODE, kRoundsWide>, XPrefix<kRoundsWide>::QS);
 }
 
-int launch_adjoint(const DtsLaunch& L, Storage st, IterMode mode, const float* gin,
-                   float* gout, const float* vk, const void* t, const void* c,
-                   const uint32_t* bounds, float* gt, float* gc, float lambda,
-                   float step, int hx, int hy, int flags, cudaStream_t s) {
+// One iteration's adjoint of g, in place (g1: scratch).
+int launch_adjoint(const DtsLaunch& L, Storage st, IterMode mode, float* g, float* g1,
+                   const float* vk, const void* t, const void* c, const uint32_t* bounds,
+                   float* gt, float* gc, float lambda, float step, int halo, int flags,
+                   cudaStream_t s) {
   ProfScope ps(s, DTSGB_K_DTS_ADJOINT);
-  if (st == Storage::F32) {
-    if (mode == IterMode::L2)
-      return launch_adj_t<float, 0>(L, gin, gout, vk, t, c, bounds, gt, gc, lambda, step,
-                                    hx, hy, flags, s);
-    return launch_adj_t<float, 1>(L, gin, gout, vk, t, c, bounds, gt, gc, lambda, step, hx,
-                                  hy, flags, s);
-  }
-  if (mode == IterMode::L2)
-    return launch_adj_t<__nv_bfloat16, 0>(L, gin, gout, vk, t, c, bounds, gt, gc, lambda,
-                                          step, hx, hy, flags, s);
-  return launch_adj_t<__nv_bfloat16, 1>(L, gin, gout, vk, t, c, bounds, gt, gc, lambda,
-                                        step, hx, hy, flags, s);
+#define ADJ_T(TS, M) \
+  launch_adj_t<TS, M>(L, g, g1, vk, t, c, bounds, gt, gc, lambda, step, halo, flags, s)
+  if (st == Storage::F32) return mode == IterMode::L2 ? ADJ_T(float, 0) : ADJ_T(float, 1);
+  return mode == IterMode::L2 ? ADJ_T(__nv_bfloat16, 0) : ADJ_T(__nv_bfloat16, 1);
+#undef ADJ_T
 }
 
 }  // namespace
@@ -446,8 +396,8 @@ int dts_backward(const DtsLaunch& L, const Inst* d_inst, int n_inst, long long p
   }
   // the first adjoint writes dL/dt and dL/dc (no zeroing pass), the last
   // adds dL/dv_0 to dL/dt (no final pass)
-  float* g = G.g[0];  // holds dL/dv_N on entry
-  float* gn = G.g[1];
+  if (halo > kAdjMaxHalo)
+    return fail(DTSGB_ERR_UNSUPPORTED, "sigma_z too large for the adjoint");
   const int nseg = (num_iterations + G.seg - 1) / G.seg;
   for (int j = nseg - 1; j >= 0; --j) {
     const int start = j * G.seg;
@@ -468,10 +418,10 @@ int dts_backward(const DtsLaunch& L, const Inst* d_inst, int n_inst, long long p
     for (int k = len - 1; k >= 0; --k) {
       const int flags = (j == nseg - 1 && k == len - 1 ? kAdjFirst : 0) |
                         (j == 0 && k == 0 ? kAdjLast : 0);
-      int st_ = launch_adjoint(L, st, mode, g, gn, k == 0 ? x0 : G.segbuf[k], target, conf,
-                               bounds, grad_t, grad_c, lambda, step, halo, halo, flags, s);
+      // (G.g[0] holds dL/dv_N on entry)
+      int st_ = launch_adjoint(L, st, mode, G.g[0], G.g[1], k == 0 ? x0 : G.segbuf[k], target,
+                               conf, bounds, grad_t, grad_c, lambda, step, halo, flags, s);
       if (st_) return st_;
-      std::swap(g, gn);
     }
   }
   return DTSGB_OK;

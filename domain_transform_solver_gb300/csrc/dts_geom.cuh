@@ -46,6 +46,21 @@ __host__ __device__ inline int y_th(int w, int h, int hy) {
   return (warps << lg) - 2 * hy;
 }
 
+// Entry t of a row segment: entry t & 3 of quad t >> 2, one plane of quads per
+// entry of a quad, so that the lanes of a warp (a quad each) read and write 32
+// banks.  Byte offset t + (t & 3) * (4 QS - 1), QS words a plane (and room for
+// 32 entries past the rounds).
+template <int NR>
+struct XPrefix {
+  static constexpr int QS = NR * 32 + 8;
+  static __device__ __forceinline__ unsigned* entry(char* S, int t) {
+    return reinterpret_cast<unsigned*>(S + t + (t & 3) * (4 * QS - 1));
+  }
+  static __device__ __forceinline__ unsigned at(const char* S, int t) {
+    return *reinterpret_cast<const unsigned*>(S + t + (t & 3) * (4 * QS - 1));
+  }
+};
+
 // The passes' grids over a launch's instances (one instance: from its size;
 // several: the block tables of dts_pass_blocks for this halo), and the rounds
 // and staged rows of the largest.

@@ -39,17 +39,6 @@ namespace {
 
 constexpr int kNaNBits = 0x7fc00000;
 
-// Prefix entry t of a row segment: entry t & 3 of quad t >> 2, one plane of
-// quads per entry of a quad, so that the lanes of a warp (a quad each) read
-// and write 32 banks.  Byte offset t + (t & 3) * (4 QS - 1), QS words a plane.
-template <int NR>
-struct XPrefix {
-  static constexpr int QS = NR * 32 + 8;
-  static __device__ __forceinline__ unsigned at(const char* S, int t) {
-    return *reinterpret_cast<const unsigned*>(S + t + (t & 3) * (4 * QS - 1));
-  }
-};
-
 // X half-step update of one pixel (src/domain_transform_solver.cuh:37-86);
 // rn = 1/n correctly rounded.
 template <int MODE, bool STEREO>
@@ -97,8 +86,10 @@ __device__ __forceinline__ bool finite_bits(float v) { return mag_bits(v) < kNon
 // segment and its halo as float4 (four adjacent pixels, 128 a round, kept in
 // registers), the largest magnitude sets the scale, a shuffle scan per round
 // leaves the prefix in the warp's shared memory, and each lane updates the
-// pixels it already holds, the next round's bounds, target and confidence in
-// flight.  Warps are independent.
+// pixels it already holds.  AHEAD: the next round's bounds, target and
+// confidence are in flight meanwhile (64 registers); without, 48, and ten
+// blocks an SM take turns, which is better where there are that many (see
+// launch_iter).  Warps are independent.
 //
 // The window ends come from k_bounds for the same sigma (dl <= hx + 1, du <=
 // hx), so a prefix index never leaves the staged columns.
@@ -107,8 +98,8 @@ __device__ __forceinline__ bool finite_bits(float v) { return mag_bits(v) < kNon
 // adds its windows in float, pixel by pixel, and every result that is not
 // finite is NaN (never finite garbage).
 // ---------------------------------------------------------------------------
-template <typename TS, int MODE, bool STEREO, bool OVER, int NR>
-__global__ void __launch_bounds__(32 * kXWarps)
+template <typename TS, int MODE, bool STEREO, bool OVER, int NR, bool AHEAD>
+__global__ void __launch_bounds__(32 * kXWarps, AHEAD ? 1 : 10)
     k_dts_x(const Inst* __restrict__ insts, const float* __restrict__ vin,
             float* __restrict__ vout, const TS* __restrict__ tgt, const TS* __restrict__ cnf,
             const uint32_t* __restrict__ bnd, float lambda, float step, float overwrite, int hx,
@@ -156,7 +147,8 @@ __global__ void __launch_bounds__(32 * kXWarps)
       }
     }
   };
-  Quad Q[2];
+  constexpr int NQ = AHEAD ? 2 : 1;
+  Quad Q[NQ];
   float4 v[NR];
   if (x0 - g.ha >= 0 && x0 - g.ha + 128 * rounds <= W) {  // the whole warp inside
 #pragma unroll
@@ -177,12 +169,13 @@ __global__ void __launch_bounds__(32 * kXWarps)
       }
     }
   }
-  Q[0].b = Q[1].b = make_uint4(0u, 0u, 0u, 0u);
-  Q[0].tv.zero();
-  Q[0].cv.zero();
-  Q[1].tv.zero();
-  Q[1].cv.zero();
-  fetch(0, Q[0]);
+#pragma unroll
+  for (int i = 0; i < NQ; ++i) {
+    Q[i].b = make_uint4(0u, 0u, 0u, 0u);
+    Q[i].tv.zero();
+    Q[i].cv.zero();
+  }
+  if (AHEAD) fetch(0, Q[0]);
   unsigned mb = 0u;
 #pragma unroll
   for (int r = 0; r < NR; ++r)
@@ -245,8 +238,9 @@ __global__ void __launch_bounds__(32 * kXWarps)
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
     if (r < rounds) {
-      if (r + 1 < NR) fetch(r + 1, Q[(r + 1) & 1]);
-      const Quad& q = Q[r & 1];
+      if (!AHEAD) fetch(r, Q[0]);
+      if (AHEAD && r + 1 < NR) fetch(r + 1, Q[(r + 1) % NQ]);
+      const Quad& q = Q[r % NQ];
       const int t0 = 4 * lane + 128 * r;
       if (mine(r)) {
         float o[4];
@@ -414,11 +408,11 @@ int set_smem(K* f, size_t bytes) {
   return DTSGB_OK;
 }
 
-template <typename TS, int MODE, bool STEREO, bool OVER, int NR>
+template <typename TS, int MODE, bool STEREO, bool OVER, int NR, bool AHEAD = true>
 int launch_x(const DtsLaunch& L, const float* vin, float* vout, const void* target,
              const void* conf, const uint32_t* bounds, float lambda, float step,
              float overwrite, int hx, dim3 grid, const StereoArgs& sa, cudaStream_t s) {
-  auto kern = k_dts_x<TS, MODE, STEREO, OVER, NR>;
+  auto kern = k_dts_x<TS, MODE, STEREO, OVER, NR, AHEAD>;
   const size_t smem = sizeof(unsigned) * (kXWarps * 4 * XPrefix<NR>::QS + 2 * hx + 2);
   DTSGB_CUDA(launch_dependent(kern, grid, dim3(32 * kXWarps), smem, s, L.d_inst, vin, vout,
                               (const TS*)target, (const TS*)conf, bounds, lambda, step,
@@ -452,11 +446,16 @@ int launch_iter(const DtsLaunch& L, const float* vin, float* tmp, float* vout, c
   const long long px = G.px;
   ProfScope ps(s, DTSGB_K_DTS_ITER);
   int st;
-#define X_ROUNDS(NR)                                                                           \
-  launch_x<TS, MODE, STEREO, OVER, NR>(L, vin, tmp, target, conf, bounds, lambda, step,        \
+  // enough blocks to fill the SMs without the loads ahead: 3264x2448 950 -> 898
+  // us a solve, 16 x 1024x768 2427 -> 2386 a training step; 1376x1088, five
+  // blocks an SM, 147 with them and 167 without (seven at sigma_z 71: 240, 235)
+  const bool many = (long long)gx.x * gx.y > 6 * 152;
+#define X_ROUNDS(...)                                                                          \
+  launch_x<TS, MODE, STEREO, OVER, __VA_ARGS__>(L, vin, tmp, target, conf, bounds, lambda, step,        \
                                        overwrite, halo, gx, sa, s)
   if (!STEREO && rounds <= 2) st = X_ROUNDS(STEREO ? kRoundsX : 2);
   else if (!STEREO && rounds <= 3) st = X_ROUNDS(STEREO ? kRoundsX : 3);
+  else if (!STEREO && rounds <= kRoundsX && many) st = X_ROUNDS(kRoundsX, STEREO);
   else if (rounds <= kRoundsX) st = X_ROUNDS(kRoundsX);
   else st = X_ROUNDS(kRoundsWide);
 #undef X_ROUNDS

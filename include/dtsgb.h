@@ -468,15 +468,14 @@ DTSGB_API int dtsgb_batch_download_device(dtsgb_batch_t b, int which,
 DTSGB_API int dtsgb_batch_debug_plane(dtsgb_batch_t b, int i, int which, void* dst,
                                       long long dst_bytes);
 
-/* ---- Tuning (new).  DTSGB_TUNE_DTS_TILE: tile width of the fused DTS
- * iteration and its adjoint, 64 (64 x 128 tiles) or 32 (32 x 32 tiles;
- * the default when the batch holds under 4 x 152 x 64 x 64 pixels).
+/* ---- Tuning (new).  DTSGB_TUNE_DTS_TILE: 64 or 32 (32 by default when the
+ * batch holds under 4 x 152 x 64 x 64 pixels), kept and returned, without
+ * effect on a solve: its passes are cut by each image's size.
  * DTSGB_TUNE_HFBS_GROUP_VOXELS:
  * the HFBS iterations run over groups of consecutive instances holding at
  * most this many grid voxels, all iterations of one group before the next,
  * so that a group's grids can stay in L2 (0, the default: all instances at
- * once).  Neither changes results beyond the last bits of the DTS iterate
- * (HFBS: bitwise identical). */
+ * once); results are bitwise the same. */
 #define DTSGB_TUNE_DTS_TILE 0
 #define DTSGB_TUNE_HFBS_GROUP_VOXELS 1
 /* DTSGB_TUNE_REUSE_GUIDE_STATE (default 1): while the guide is unchanged
@@ -485,12 +484,13 @@ DTSGB_API int dtsgb_batch_debug_plane(dtsgb_batch_t b, int i, int which, void* d
  * and an HFBS solve with the same grid keeps the bistochastized
  * normalisation instead of recomputing them; results are identical. */
 #define DTSGB_TUNE_REUSE_GUIDE_STATE 2
-/* DTSGB_TUNE_HFBS_SOLVE_STEPS: heavy-ball steps per launch, 4 (default:
- * a temporally blocked kernel, each launch four steps on 24 x 24-column
- * blocks staged in shared memory, for grids of at most 16 levels) or 1
- * (one step per launch, any grid; with a group budget its grids can stay in
- * L2).  The two add a voxel's six neighbour products in different roundings:
- * results agree to FP32 rounding, and each is differentiated exactly. */
+/* DTSGB_TUNE_HFBS_SOLVE_STEPS: heavy-ball steps per launch, 4 (default: for
+ * grids of at most 64 levels, clusters that keep a small grid on chip for all
+ * steps, and marches through the planes of larger ones, four steps a launch)
+ * or 1 (one step per launch, any grid; with a group budget its grids can stay
+ * in L2).  The two add a voxel's six neighbour products in different
+ * roundings: results agree to FP32 rounding, and each is differentiated
+ * exactly. */
 #define DTSGB_TUNE_HFBS_SOLVE_STEPS 3
 /* DTSGB_TUNE_BOUNDS_SEGMENT: 4, 8 or 16 (default 8), kept and returned, without
  * effect: the window-bound search has no segments to choose. */

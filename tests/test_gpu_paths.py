@@ -302,3 +302,51 @@ def test_more_images_than_a_launch_has_pointers_for(gpu_ready, n):
     torch.cuda.synchronize()
     for a, o in zip(host.download(0), out):
         assert np.array_equal(a, o.cpu().numpy())
+
+
+# ---- DTS adjoint: a Y^T pass and an X^T pass -----------------------------------
+@pytest.mark.parametrize("w,h,sz", [
+    (1, 1, 8.0), (3, 130, 8.0), (129, 33, 0.5), (365, 200, 8.0),  # segments of 2 and 3 rounds
+    (1030, 520, 8.0),                                             # of 4, 128 staged rows
+    (300, 120, 40.0), (700, 300, 76.9),                           # wide halos, 32 rows a warp
+])
+@pytest.mark.parametrize("bf16", [0, 1])
+def test_adjoint_passes_match_the_oracle(gpu_ready, oracle_mod, w, h, sz, bf16):
+    """The bar of the adjoint's tests (1e-4 of the largest gradient), alone and
+    in a batch with the same bits."""
+    import test_gpu_adjoint as A
+    D = gpu_ready
+    rng = np.random.default_rng(w + h)
+    flags = D.FLAG_BF16_STORAGE if bf16 else 0
+    data = []
+    for ww, hh in ((w, h), (37, 21)):
+        y, x = np.mgrid[0:hh, 0:ww]
+        rgba = (rng.integers(0, 9, (hh, ww, 4)) + ((x // 23 + y // 17) % 3 * 70)[..., None])
+        t, c, g = (rng.standard_normal((hh, ww)).astype(np.float32),
+                   rng.random((hh, ww)).astype(np.float32),
+                   rng.standard_normal((hh, ww)).astype(np.float32))
+        if bf16:
+            t, c = P.bf16_round(t), P.bf16_round(c)
+        data.append((rgba.astype(np.uint8), t, c, g))
+    opt = dict(num_iterations=3, loss=1, lambda_=0.9, sigma_z=sz, step_size=0.8)
+    got = []
+    for d in (data[:1], data):
+        b = A._batch(D, d, opt, flags=flags)
+        gt, gc = b.backward([g for _, _, _, g in d])
+        got.append((gt[0], gc[0]))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+    rgba, t, c, g = data[0]
+    o = A._oracle(oracle_mod, rgba, t, c, A._gpu_windows(D, rgba, t, c, sz, flags))
+    rt, rc = o.backward(3, 1, 0.9, sz, 0.8, g)
+    A._check_grad(got[0][0], rt, 1)
+    if rc.any():  # windows of one pixel leave v at t: dL/dc is zero, its float form rounding
+        A._check_grad(got[0][1], rc, 1)
+
+
+def test_adjoint_of_wider_windows_is_refused(gpu_ready):
+    import test_gpu_adjoint as A
+    D = gpu_ready
+    data = [(np.zeros((9, 9, 4), np.uint8), *(np.ones((9, 9), np.float32) for _ in range(3)))]
+    opt = dict(num_iterations=2, loss=1, lambda_=0.9, sigma_z=77.0, step_size=0.8)
+    with pytest.raises(D.DtsgbError):
+        A._batch(D, data, opt).backward([data[0][3]])
