@@ -182,6 +182,8 @@ __global__ void __launch_bounds__(512, 1)
   const bool has_lo = w > 0, has_hi = w + 1 < nw;
   int slot = 0, is = 0;       // j % SL, j % NB
   unsigned parity = 0;        // of input slot `is`: flips when it wraps
+  // (by two: half of the moves between planes are renamings; 3% of a solve)
+#pragma unroll (REC ? 1 : 2)
   for (int j = 0; j < N; ++j) {
     const bool got = !use_tma || mbar_wait_bounded(&bar[is], parity, kTmaWaitPolls);
     const float* zi = inp + is * NI * PL + own;
