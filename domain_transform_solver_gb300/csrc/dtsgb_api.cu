@@ -691,7 +691,8 @@ struct dtsgb_hfbs_s {
   size_t plane = 0, gsize = 0;
   uchar4* guide = nullptr;
   float *target = nullptr, *conf = nullptr, *out = nullptr;
-  float* g[16] = {};
+  float* g[13] = {};  // by the enum below
+  const float *norm = nullptr, *z_final = nullptr;  // of the last solve, among g
   // tensor maps of the grid planes and the grid they describe
   TmaCache tma;
   HInst tma_inst{};
@@ -728,8 +729,9 @@ struct dtsgb_hfbs_s {
 
 enum {
   G_COUNT = 0, G_CSUM, G_B, G_N0, G_N1, G_INVA, G_Z0, G_Z1, G_H, G_T0, G_T1,
-  G_T2, G_DBG_NORM, G_DBG_BLUR_C, G_DBG_Z_INIT, G_DBG_Z_FINAL, G_NUM
+  G_T2, G_DBG_Z_INIT, G_NUM
 };
+static_assert(sizeof(dtsgb_hfbs_s::g) == G_NUM * sizeof(float*), "grids of a handle");
 
 static void hfbs_free(dtsgb_hfbs_t h) {
   dfree(h->guide);
@@ -782,11 +784,7 @@ static void hfbs_fill_batch(dtsgb_hfbs_t h, const HInst* hi, HfbsBatch& B) {
   B.sgrid = h->sgrid;
   B.ovf = h->ovf;
   B.keep_debug = true;
-  B.grid_bytes = (size_t)I.px * I.gy * I.gl * 4;  // pitched
-  B.dbg_norm = h->g[G_DBG_NORM];
-  B.dbg_blur_c = h->g[G_DBG_BLUR_C];
   B.dbg_z_init = h->g[G_DBG_Z_INIT];
-  B.dbg_z_final = h->g[G_DBG_Z_FINAL];
 }
 
 // Carve the gradient arena for K heavy-ball steps over tv voxels: the kept
@@ -1001,7 +999,8 @@ DTSGB_API int dtsgb_hfbs_clear_all(dtsgb_hfbs_t h) {
   DTSGB_CUDA(cudaMemsetAsync(h->target, 0, h->plane * 4, h->stream));
   DTSGB_CUDA(cudaMemsetAsync(h->conf, 0, h->plane * 4, h->stream));
   DTSGB_CUDA(cudaMemsetAsync(h->out, 0, h->plane * 4, h->stream));
-  for (auto* p : h->g) DTSGB_CUDA(cudaMemsetAsync(p, 0, h->gsize * 4, h->stream));
+  for (int i = 0; i < G_NUM; ++i)
+    DTSGB_CUDA(cudaMemsetAsync(h->g[i], 0, h->gsize * 4, h->stream));
   DTSGB_CUDA(cudaMemsetAsync(h->ovf, 0, (size_t)h->max_gx * h->max_gy * 4,
                              h->stream));
   h->solved = false;
@@ -1080,12 +1079,15 @@ DTSGB_API int dtsgb_hfbs_optimize(dtsgb_hfbs_t h) {
   nk.sigma_l = p.sigma_l;
   nk.bistoch_iter_max = p.bistoch_iter_max;
   B.reuse_norm = had_norm && std::memcmp(&nk, &h->nkey, sizeof nk) == 0;
-  int st = hfbs_enqueue_solve(B, hp, h->stream);
+  const float* z_final = nullptr;
+  int st = hfbs_enqueue_solve(B, hp, h->stream, &z_final);
   if (st) return st;
   h->nkey = nk;
   h->nkey_valid = true;
   h->inst = I;
   h->solved = true;
+  h->norm = h->g[p.bistoch_iter_max % 2 ? G_N1 : G_N0];
+  h->z_final = z_final;
   h->grad_ready = h->grad;
   return DTSGB_OK;
 }
@@ -1125,13 +1127,13 @@ DTSGB_API int dtsgb_hfbs_grid_dims(dtsgb_hfbs_t h, int* gx, int* gy, int* gl) {
 
 DTSGB_API int dtsgb_hfbs_debug_grid(dtsgb_hfbs_t h, int which, float* dst) {
   if (!h || !dst) return fail(DTSGB_ERR_INVALID_ARGUMENT, "null argument");
-  static const int map[8] = {G_COUNT,      G_CSUM,       G_B,
-                             G_DBG_NORM,   G_INVA,       G_DBG_BLUR_C,
-                             G_DBG_Z_INIT, G_DBG_Z_FINAL};
+  // the solve's own grids, which stay until the next one
+  const float* grids[8] = {h->g[G_COUNT], h->g[G_CSUM], h->g[G_B],           h->norm,
+                           h->g[G_INVA],  h->g[G_T0],   h->g[G_DBG_Z_INIT], h->z_final};
   if (which < 0 || which >= 8) return fail(DTSGB_ERR_INVALID_ARGUMENT, "which");
   if (!h->solved) return fail(DTSGB_ERR_INVALID_ARGUMENT, "no solve yet");
   // rows of round_up(gx, 4) voxels on the device, of gx in dst
-  DTSGB_CUDA(cudaMemcpy2DAsync(dst, (size_t)h->gx * 4, h->g[map[which]],
+  DTSGB_CUDA(cudaMemcpy2DAsync(dst, (size_t)h->gx * 4, grids[which],
                                (size_t)round_up(h->gx, 4) * 4, (size_t)h->gx * 4,
                                (size_t)h->gy * h->gl, cudaMemcpyDeviceToHost, h->stream));
   DTSGB_CUDA(cudaStreamSynchronize(h->stream));

@@ -178,8 +178,7 @@ struct HfbsBatch {
   float2* sgrid;  // the instances' slice grids (HInst::slice_off)
   // optional debug copies (single-instance class API)
   bool keep_debug;
-  size_t grid_bytes;
-  float *dbg_norm, *dbg_blur_c, *dbg_z_init, *dbg_z_final;
+  float* dbg_z_init;  // a copy of the first iterate (keep_debug)
   // non-null: record the forward iterates for hfbs_enqueue_backward (the
   // one-step heavy-ball kernel, all instances as one group)
   const HfbsGradState* grad = nullptr;
@@ -234,7 +233,8 @@ void hfbs_march_prepare(const HfbsBatch& B, const std::vector<const float*>& pla
                         cudaStream_t s);
 
 // Enqueue the whole HFBS::Optimize sequence (splat .. slice) on a stream.
-int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s);
+int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s,
+                       const float** z_final = nullptr);
 
 // Builds the grid tensor maps the solve of B will stage from (grid planes
 // b, invA, both z and h buffers, both normalisation buffers, the counts),

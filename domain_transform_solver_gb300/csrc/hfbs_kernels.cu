@@ -523,11 +523,15 @@ __device__ __forceinline__ float div_by_c_plus_eps(float b, float c) {
 // InitZ<true> (src/hfbs.cu:337-353): z = blur(b) / (blur(c) + 1e-7), the
 // division in double as the reference's double literal makes it; h = 0.
 __global__ void k_init_z(const float* __restrict__ blur_b, const float* __restrict__ blur_c,
-                         float* __restrict__ z, float* __restrict__ h, long long n) {
+                         float* __restrict__ z, float* __restrict__ h, long long n,
+                         float* __restrict__ copy0, float* __restrict__ copy1) {
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < n;
        g += (long long)gridDim.x * blockDim.x) {
-    z[g] = div_by_c_plus_eps(blur_b[g], blur_c[g]);
+    const float v = div_by_c_plus_eps(blur_b[g], blur_c[g]);
+    z[g] = v;
     h[g] = 0.f;
+    if (copy0) copy0[g] = v;
+    if (copy1) copy1[g] = v;
   }
 }
 
@@ -764,7 +768,8 @@ void hfbs_launch_blur_pair(const HfbsBatch& B, const HParams& p, const float* s0
   k_laplace<<<gl_lines, kT, 0, s>>>(B.d_inst, 2, y0, x0, y1, x1, p.neg_exp_beta);
 }
 
-int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s) {
+int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s,
+                       const float** z_final) {
   const int ni = B.n_inst;
   // row kernels: one warp per grid row, 8 warps per block
   const dim3 gr((unsigned)std::min<long long>((B.max_rows + 7) / 8, 4096), ni);
@@ -904,16 +909,11 @@ int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s) {
   k_laplace<<<gl_lines, kT, 0, s>>>(B.d_inst, 2, B.t2, B.t0, spare, B.t1,
                                     p.neg_exp_beta);
   // blur_c = t0, blur_b = t1
-  k_init_z<<<gflat, kT, 0, s>>>(B.t1, B.t0, B.z0, B.h, B.total_voxels);
+  // z_0 is overwritten: kept for inspection, and as the adjoint's first iterate
+  float* z_kept = B.grad && B.grad->segment == 1 && p.optim_iter_max > 0 ? B.grad->hist : nullptr;
+  k_init_z<<<gflat, kT, 0, s>>>(B.t1, B.t0, B.z0, B.h, B.total_voxels,
+                                B.keep_debug ? B.dbg_z_init : nullptr, z_kept);
   prof_end(s, DTSGB_K_HFBS_OTHER);
-  if (B.keep_debug) {
-    DTSGB_CUDA(cudaMemcpyAsync(B.dbg_blur_c, B.t0, B.grid_bytes,
-                               cudaMemcpyDeviceToDevice, s));
-    DTSGB_CUDA(cudaMemcpyAsync(B.dbg_z_init, B.z0, B.grid_bytes,
-                               cudaMemcpyDeviceToDevice, s));
-    DTSGB_CUDA(cudaMemcpyAsync(B.dbg_norm, norm, B.grid_bytes,
-                               cudaMemcpyDeviceToDevice, s));
-  }
   float* zs = B.z0;
   float* zd = B.z1;
   if (B.grad) {
@@ -925,7 +925,6 @@ int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s) {
     const size_t gbytes = (size_t)tv * sizeof(float);
     const HfbsClusterPlan CP = hfbs_cluster_plan(B, 0, ni);
     if (S == 1 && CP.size > 0 && K > 0) {
-      DTSGB_CUDA(cudaMemcpyAsync(G.hist, B.z0, gbytes, cudaMemcpyDeviceToDevice, s));
       ProfScope ps(s, DTSGB_K_HFBS_SOLVE);
       if (int st = hfbs_cluster_solve(B, CP, p, norm, B.z0, B.z1, B.h, nullptr, K, G.hist + tv,
                                       K - 1, s))
@@ -933,8 +932,6 @@ int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s) {
       zs = B.z1;
     } else if (S == 1) {
       // z_k in hist plane k; h ping-pongs through the free blur temporary t2
-      if (K > 0)
-        DTSGB_CUDA(cudaMemcpyAsync(G.hist, B.z0, gbytes, cudaMemcpyDeviceToDevice, s));
       float* hs = B.h;
       float* hd = tb ? B.t2 : B.h;
       for (int it = 0; it < K;) {
@@ -1014,9 +1011,7 @@ int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s) {
       std::swap(zs, zd);
     }
   }
-  if (B.keep_debug)
-    DTSGB_CUDA(cudaMemcpyAsync(B.dbg_z_final, zs, B.grid_bytes,
-                               cudaMemcpyDeviceToDevice, s));
+  if (z_final) *z_final = zs;
   prof_begin(s, DTSGB_K_HFBS_SLICE);
   long long prows = 1;  // rows of the largest padded slice grid
   for (int i = 0; B.h_inst && i < ni; ++i)
