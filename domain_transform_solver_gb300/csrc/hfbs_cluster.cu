@@ -6,16 +6,18 @@
 // Each CTA of the cluster owns a slab of grid rows y; a thread owns items of
 // four levels of one (x, y) column and keeps their z, h, n, b and invA in
 // registers for the whole solve.  Per step the products z * n go to shared
-// memory (two buffers in turn), those of a slab's first and last row also to
+// memory (two buffers in turn, the four levels of an item side by side: one
+// 16-byte access), those of a slab's first and last row also to
 // the neighbouring CTA's halo row through distributed shared memory; one
 // cluster barrier later every neighbour is a local read.  Memory is touched
 // before the first and after the last step only.
 //
-// Bound by latency: a step is one exchange (18 shared-memory reads per four
-// voxels, about 25 instructions a voxel) and one cluster barrier.  Measured:
-// 140 steps on a 22 x 17 x 16 grid in 90 us, 64 on 80 x 60 x 16 in 105; a
-// launch per four steps, the form this replaces, took 12 to 16 us on such grids
-// whatever their size (a launch, a round of loads and four block barriers).
+// Bound by latency: a step is one exchange (6 shared-memory reads per four
+// voxels) and one cluster barrier.  Measured: 140 steps on a 22 x 17 x 16 grid
+// in 71 us, 64 on 80 x 60 x 16 in 109 with every iterate recorded (89 and 117
+// with planes of levels, 18 reads per four voxels); a launch per four steps, the
+// form this replaces, took 12 to 16 us on such grids whatever their size (a
+// launch, a round of loads and four block barriers).
 //
 // Taken where every instance of the launch fits: per CTA 2048 items (8192
 // voxels; registers) and 227 KB of the two buffers, so 131072 voxels for 16
@@ -44,7 +46,6 @@ __host__ __device__ constexpr int max_threads(int ipt) {
 __host__ __device__ constexpr int adj_threads(int ipt) { return ipt == 1 ? 704 : 640; }
 constexpr int kAdjItems = 2;
 constexpr int kCItems = 4;
-constexpr int kMaxItems = kCItems * max_threads(kCItems);
 constexpr size_t kMaxSmem = 227 * 1024;
 
 struct ClusterArgs {
@@ -73,10 +74,16 @@ __device__ __forceinline__ void cluster_barrier() {
                ::: "memory");
 }
 // Stores v at the address that `local` has in the shared memory of CTA `rank`.
-__device__ __forceinline__ void store_remote(const float* local, unsigned rank, float v) {
+__device__ __forceinline__ void store_remote(const float4* local, unsigned rank, float4 v) {
   unsigned a = (unsigned)__cvta_generic_to_shared(local), r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(r), "f"(v) : "memory");
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(r), "f"(v.x), "f"(v.y),
+               "f"(v.z), "f"(v.w)
+               : "memory");
+}
+// Level v of an item's four.
+__device__ __forceinline__ float lev(const float4& q, int v) {
+  return v == 0 ? q.x : v == 1 ? q.y : v == 2 ? q.z : q.w;
 }
 
 // Rows of a CTA's slab, items of a CTA and its shared memory for a cluster of
@@ -93,33 +100,36 @@ inline size_t slab_smem(const HInst& H, int c) {  // of one buffer
 template <int MODE, bool REC, int IPT>
 __global__ void __launch_bounds__(max_threads(IPT), 1)
     k_hfbs_cluster(const HInst* __restrict__ insts, ClusterArgs A) {
-  extern __shared__ __align__(16) float smc[];
+  extern __shared__ float4 smc[];  // [buffer][group of levels][R + 2][gx + 2]
   const HInst I = insts[blockIdx.y];
   const int gx = I.gx, gy = I.gy, gl = I.gl;
   const int rank = (int)cluster_rank(), C = (int)cluster_size();
   const int R = slab_rows(gy, C), nlc = (gl + kCV - 1) / kCV;
-  const int gxp = gx + 2, PS = (R + 2) * gxp, BUF = nlc * kCV * PS;
+  const int gxp = gx + 2, PS = (R + 2) * gxp, BUF = nlc * PS;
   const int tid = threadIdx.x, T = blockDim.x;
-  for (int i = tid; i < 2 * BUF; i += T) smc[i] = 0.f;
+  for (int i = tid; i < 2 * BUF; i += T) smc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   __syncthreads();
   if (MODE == kBistoch) {
     // the covered pad faces read 1 on even iterations (the first buffer), 0 on
     // odd ones
     const int rows = min(R, gy - rank * R);  // may be <= 0
+    auto at = [&](int l, int r, int x) -> float& {
+      return reinterpret_cast<float*>(smc + (l / kCV) * PS + r * gxp + x)[l % kCV];
+    };
     if (I.cov_x)
       for (int i = tid; i < gl * max(rows, 0); i += T) {
         const int l = i / rows, yy = i - l * rows;
-        smc[l * PS + (yy + 1) * gxp + gx + 1] = 1.f;
+        at(l, yy + 1, gx + 1) = 1.f;
       }
     if (I.cov_y && rows > 0 && rank * R + rows == gy)
       for (int i = tid; i < gl * gx; i += T) {
         const int l = i / gx, x = i - l * gx;
-        smc[l * PS + (rows + 1) * gxp + x + 1] = 1.f;
+        at(l, rows + 1, x + 1) = 1.f;
       }
   }
   const int items = R * gx * nlc, plane = I.px * gy;
   float z[IPT][kCV], h[IPT][kCV], n[IPT][kCV], b[IPT][kCV], a[IPT][kCV];
-  int o[IPT];        // index of level 0 of the item in a buffer
+  int o[IPT];        // index of the item in a buffer
   int lc[IPT];       // its group of levels (-1: no item)
   int edge[IPT];     // bit 0: first row of the slab, bit 1: last
   long long g[IPT];  // element of level 0 in a grid plane
@@ -136,7 +146,7 @@ __global__ void __launch_bounds__(max_threads(IPT), 1)
       const int y = rank * R + yy;
       if (y < gy) {
         lc[j] = c;
-        o[j] = c * kCV * PS + (yy + 1) * gxp + x + 1;
+        o[j] = c * PS + (yy + 1) * gxp + x + 1;
         edge[j] = (yy == 0 && rank > 0 ? 1 : 0) | (yy == R - 1 && rank + 1 < C ? 2 : 0);
         g[j] = I.grid_off + (long long)c * kCV * plane + (long long)y * I.px + x;
 #pragma unroll
@@ -159,43 +169,43 @@ __global__ void __launch_bounds__(max_threads(IPT), 1)
   // every CTA of the cluster runs and its buffers are zeroed
   cluster_barrier();
   for (int s = 0; s < A.steps; ++s) {
-    float* P = smc + (s & 1) * BUF;
+    float4* P = smc + (s & 1) * BUF;
     float p[IPT][kCV];
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
 #pragma unroll
-      for (int v = 0; v < kCV; ++v) {
+      for (int v = 0; v < kCV; ++v)
         p[j][v] = MODE == kHeavyBall ? __fmul_rn(z[j][v], n[j][v]) : z[j][v];
-        if (lc[j] >= 0) {
-          float* q = P + o[j] + v * PS;
-          *q = p[j][v];
-          if (edge[j] & 1) store_remote(q + R * gxp, rank - 1, p[j][v]);
-          if (edge[j] & 2) store_remote(q - R * gxp, rank + 1, p[j][v]);
-        }
+      if (lc[j] >= 0) {
+        float4* q = P + o[j];
+        const float4 p4 = make_float4(p[j][0], p[j][1], p[j][2], p[j][3]);
+        *q = p4;
+        if (edge[j] & 1) store_remote(q + R * gxp, rank - 1, p4);
+        if (edge[j] & 2) store_remote(q - R * gxp, rank + 1, p4);
       }
     }
     cluster_barrier();
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
       if (lc[j] < 0) continue;
-      const float* q = P + o[j];
-      const float lo = lc[j] > 0 ? q[-PS] : 0.f;
-      const float hi = lc[j] + 1 < nlc ? q[kCV * PS] : 0.f;
+      const float4* q = P + o[j];
+      const float lo = lc[j] > 0 ? q[-PS].w : 0.f;
+      const float hi = lc[j] + 1 < nlc ? q[PS].x : 0.f;
+      const float4 xm = q[-1], xp = q[1], ym = q[-gxp], yp = q[gxp];
       const float pz = MODE == kBistoch && I.cov_l && !(s & 1) ? 1.f : 0.f;
 #pragma unroll
       for (int v = 0; v < kCV; ++v) {
         const float below = v > 0 ? p[j][v > 0 ? v - 1 : 0] : lo;
         float above = v + 1 < kCV ? p[j][v + 1 < kCV ? v + 1 : v] : hi;
-        const float* qv = q + v * PS;
         if (MODE == kHeavyBall) {
-          hfbs_step(qv[-1], qv[1], qv[-gxp], qv[gxp], below, above, n[j][v], b[j][v], a[j][v],
-                    A.lambda, A.alpha, A.beta, z[j][v], h[j][v]);
+          hfbs_step(lev(xm, v), lev(xp, v), lev(ym, v), lev(yp, v), below, above, n[j][v],
+                    b[j][v], a[j][v], A.lambda, A.alpha, A.beta, z[j][v], h[j][v]);
         } else if (lc[j] * kCV + v < gl) {
           if (lc[j] * kCV + v + 1 == gl) above = pz;
-          float t = qv[-1];
-          t += qv[1];
-          t += qv[-gxp];
-          t += qv[gxp];
+          float t = lev(xm, v);
+          t += lev(xp, v);
+          t += lev(ym, v);
+          t += lev(yp, v);
           t += below;
           t += above;
           const float blurred = 2.f * p[j][v] + t;
@@ -236,19 +246,19 @@ struct ClusterAdjArgs {
 // exchange as the solve, with two products per step to exchange (z_k * n of the
 // forward iterate, and gw of the step after it, which completes gz) and the
 // next iterate's loads in flight during a step.  64 steps on 80 x 60 x 16:
-// 238 us, 384 by a launch per step; shared memory bounds it (14 words a
-// voxel-step), then the barrier of a step.
+// 192 us (238 with planes of levels), 384 by a launch per step; bound by the
+// shared memory's bandwidth (13 words a voxel-step) and the barrier of a step.
 template <int IPT>
 __global__ void __launch_bounds__(adj_threads(IPT), 1)
     k_hfbs_cluster_adj(const HInst* __restrict__ insts, ClusterAdjArgs A) {
-  extern __shared__ __align__(16) float smc[];
+  extern __shared__ float4 smc[];  // [buffer][group of levels][R + 2][gx + 2]
   const HInst I = insts[blockIdx.y];
   const int gx = I.gx, gy = I.gy, gl = I.gl;
   const int rank = (int)cluster_rank(), C = (int)cluster_size();
   const int R = slab_rows(gy, C), nlc = (gl + kCV - 1) / kCV;
-  const int gxp = gx + 2, PS = (R + 2) * gxp, BUF = nlc * kCV * PS;
+  const int gxp = gx + 2, PS = (R + 2) * gxp, BUF = nlc * PS;
   const int tid = threadIdx.x, T = blockDim.x;
-  for (int i = tid; i < 4 * BUF; i += T) smc[i] = 0.f;
+  for (int i = tid; i < 4 * BUF; i += T) smc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   const int items = R * gx * nlc, plane = I.px * gy;
   float z[IPT][kCV], n[IPT][kCV], b[IPT][kCV], a[IPT][kCV];
   float gz[IPT][kCV], gh[IPT][kCV], gb[IPT][kCV], gi[IPT][kCV], gg[IPT][kCV];
@@ -275,7 +285,7 @@ __global__ void __launch_bounds__(adj_threads(IPT), 1)
       const int y = rank * R + yy;
       if (y < gy) {
         lc[j] = c;
-        o[j] = c * kCV * PS + (yy + 1) * gxp + x + 1;
+        o[j] = c * PS + (yy + 1) * gxp + x + 1;
         edge[j] = (yy == 0 && rank > 0 ? 1 : 0) | (yy == R - 1 && rank + 1 < C ? 2 : 0);
         g[j] = c * kCV * plane + y * I.px + x;
 #pragma unroll
@@ -295,26 +305,29 @@ __global__ void __launch_bounds__(adj_threads(IPT), 1)
   __syncthreads();
   cluster_barrier();
   for (int s = 0; s <= A.steps; ++s) {  // the last pass only completes gz
-    float* P = smc + (s & 1) * BUF;
-    float* G = smc + (2 + (s & 1)) * BUF;
+    float4* P = smc + (s & 1) * BUF;
+    float4* G = smc + (2 + (s & 1)) * BUF;
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
       if (lc[j] < 0) continue;
+      float p[kCV], w[kCV];
 #pragma unroll
       for (int v = 0; v < kCV; ++v) {
-        const float p = __fmul_rn(z[j][v], n[j][v]);
-        const float w = hfbs_adj_product(n[j][v], a[j][v], gg[j][v]);
-        float *qp = P + o[j] + v * PS, *qg = G + o[j] + v * PS;
-        *qp = p;
-        *qg = w;
-        if (edge[j] & 1) {
-          store_remote(qp + R * gxp, rank - 1, p);
-          store_remote(qg + R * gxp, rank - 1, w);
-        }
-        if (edge[j] & 2) {
-          store_remote(qp - R * gxp, rank + 1, p);
-          store_remote(qg - R * gxp, rank + 1, w);
-        }
+        p[v] = __fmul_rn(z[j][v], n[j][v]);
+        w[v] = hfbs_adj_product(n[j][v], a[j][v], gg[j][v]);
+      }
+      const float4 p4 = make_float4(p[0], p[1], p[2], p[3]);
+      const float4 w4 = make_float4(w[0], w[1], w[2], w[3]);
+      float4 *qp = P + o[j], *qg = G + o[j];
+      *qp = p4;
+      *qg = w4;
+      if (edge[j] & 1) {
+        store_remote(qp + R * gxp, rank - 1, p4);
+        store_remote(qg + R * gxp, rank - 1, w4);
+      }
+      if (edge[j] & 2) {
+        store_remote(qp - R * gxp, rank + 1, p4);
+        store_remote(qg - R * gxp, rank + 1, w4);
       }
     }
     // the next iterate, in flight over the barrier and this step
@@ -331,23 +344,31 @@ __global__ void __launch_bounds__(adj_threads(IPT), 1)
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
       if (lc[j] < 0) continue;
-      const bool has_lo = lc[j] > 0, has_hi = lc[j] + 1 < nlc;
+      // the neighbour sums of four levels, in the order x, y, l
+      auto sums = [&](const float4* q, float (&t)[kCV]) {
+        const float4 xm = q[-1], xp = q[1], ym = q[-gxp], yp = q[gxp], c = q[0];
+        const float lo = lc[j] > 0 ? q[-PS].w : 0.f;
+        const float hi = lc[j] + 1 < nlc ? q[PS].x : 0.f;
 #pragma unroll
-      for (int v = 0; v < kCV; ++v) {
-        const float *qp = P + o[j] + v * PS, *qg = G + o[j] + v * PS;
-        if (s > 0) {
-          float t = __fadd_rn(__fadd_rn(__fadd_rn(qg[-1], qg[1]), qg[-gxp]), qg[gxp]);
-          t = __fadd_rn(t, v > 0 || has_lo ? qg[-PS] : 0.f);
-          t = __fadd_rn(t, v + 1 < kCV || has_hi ? qg[PS] : 0.f);
-          gz[j][v] = hfbs_finish_adj(gz[j][v], gg[j][v], n[j][v], t, A.lambda);
+        for (int v = 0; v < kCV; ++v) {
+          t[v] = __fadd_rn(__fadd_rn(__fadd_rn(lev(xm, v), lev(xp, v)), lev(ym, v)), lev(yp, v));
+          t[v] = __fadd_rn(t[v], v > 0 ? lev(c, v > 0 ? v - 1 : 0) : lo);
+          t[v] = __fadd_rn(t[v], v + 1 < kCV ? lev(c, v + 1 < kCV ? v + 1 : v) : hi);
         }
-        if (s < A.steps) {
-          float t = __fadd_rn(__fadd_rn(__fadd_rn(qp[-1], qp[1]), qp[-gxp]), qp[gxp]);
-          t = __fadd_rn(t, v > 0 || has_lo ? qp[-PS] : 0.f);
-          t = __fadd_rn(t, v + 1 < kCV || has_hi ? qp[PS] : 0.f);
-          hfbs_step_adj(t, z[j][v], n[j][v], b[j][v], a[j][v], gz[j][v], A.lambda, A.alpha,
+      };
+      float t[kCV];
+      if (s > 0) {
+        sums(G + o[j], t);
+#pragma unroll
+        for (int v = 0; v < kCV; ++v)
+          gz[j][v] = hfbs_finish_adj(gz[j][v], gg[j][v], n[j][v], t[v], A.lambda);
+      }
+      if (s < A.steps) {
+        sums(P + o[j], t);
+#pragma unroll
+        for (int v = 0; v < kCV; ++v)
+          hfbs_step_adj(t[v], z[j][v], n[j][v], b[j][v], a[j][v], gz[j][v], A.lambda, A.alpha,
                         A.beta, gh[j][v], gb[j][v], gi[j][v], gg[j][v]);
-        }
       }
     }
 #pragma unroll
