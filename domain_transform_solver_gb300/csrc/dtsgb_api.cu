@@ -46,6 +46,36 @@ float filter_sigma_multiplier(int it, int n) {
 
 namespace {
 
+// Zeroes a handle's buffers in one launch (ClearAll): a memset each was 8 or 18
+// of them, 1.5 us on the device and 3.4 on the host.  Buffers start on 256
+// bytes and hold a multiple of four.
+constexpr int kZeroes = 24;
+struct ZeroList {
+  void* p[kZeroes];
+  long long words[kZeroes];
+  int n = 0;
+  void add(void* q, size_t bytes) {
+    p[n] = q;
+    words[n++] = (long long)(bytes / 4);
+  }
+};
+__global__ void __launch_bounds__(256) k_zero(const __grid_constant__ ZeroList L) {
+  const long long n = L.words[blockIdx.y], step = (long long)gridDim.x * blockDim.x;
+  const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  uint4* q = static_cast<uint4*>(L.p[blockIdx.y]);
+  for (long long i = i0; i < n / 4; i += step) q[i] = make_uint4(0u, 0u, 0u, 0u);
+  unsigned* w = static_cast<unsigned*>(L.p[blockIdx.y]);
+  for (long long i = (n & ~3LL) + i0; i < n; i += step) w[i] = 0u;
+}
+int launch_zero(const ZeroList& L, cudaStream_t s) {
+  long long most = 1;
+  for (int i = 0; i < L.n; ++i) most = std::max(most, L.words[i]);
+  const int blocks = (int)std::min<long long>((most + 4095) / 4096, 152);
+  k_zero<<<dim3(blocks, L.n), 256, 0, s>>>(L);
+  DTSGB_CUDA(cudaGetLastError());
+  return DTSGB_OK;
+}
+
 std::vector<Tile> make_tiles(int w, int h, int tw, int th) {
   std::vector<Tile> t;
   for (int y = 0; y < h; y += th)
@@ -231,6 +261,10 @@ DTSGB_API int dtsgb_dts_set_image_dim(dtsgb_dts_t h, int w, int hh) {
     return fail(DTSGB_ERR_INVALID_DIMS,
                 "Invalid image dims WxH:" + std::to_string(w) + " x " +
                     std::to_string(hh));
+  if (w == h->w && hh == h->h) {  // the tables on the device are these dims'
+    h->bounds_valid = false;
+    return DTSGB_OK;
+  }
   h->w = w;
   h->h = hh;
   return dts_layout(h);
@@ -621,11 +655,13 @@ DTSGB_API int dtsgb_dts_download_device(dtsgb_dts_t h, int type, void* image) {
 
 DTSGB_API int dtsgb_dts_clear_all(dtsgb_dts_t h) {
   if (!h) return fail(DTSGB_ERR_INVALID_ARGUMENT, "null handle");
-  DTSGB_CUDA(cudaMemsetAsync(h->guide, 0, h->plane * 4, h->stream));
-  DTSGB_CUDA(cudaMemsetAsync(h->target, 0, h->plane * h->tsize(), h->stream));
-  DTSGB_CUDA(cudaMemsetAsync(h->conf, 0, h->plane * h->tsize(), h->stream));
-  DTSGB_CUDA(cudaMemsetAsync(h->bounds, 0, h->plane * 4, h->stream));
-  for (auto* p : h->v) DTSGB_CUDA(cudaMemsetAsync(p, 0, h->plane * 4, h->stream));
+  ZeroList L;
+  L.add(h->guide, h->plane * 4);
+  L.add(h->target, h->plane * h->tsize());
+  L.add(h->conf, h->plane * h->tsize());
+  L.add(h->bounds, h->plane * 4);
+  for (auto* p : h->v) L.add(p, h->plane * 4);
+  if (int st = launch_zero(L, h->stream)) return st;
   h->diff_valid = false;
   h->bounds_valid = false;
   h->var_idx = -1;
@@ -995,14 +1031,14 @@ DTSGB_API int dtsgb_hfbs_set_filter_params(dtsgb_hfbs_t h,
 
 DTSGB_API int dtsgb_hfbs_clear_all(dtsgb_hfbs_t h) {
   if (!h) return fail(DTSGB_ERR_INVALID_ARGUMENT, "null handle");
-  DTSGB_CUDA(cudaMemsetAsync(h->guide, 0, h->plane * 4, h->stream));
-  DTSGB_CUDA(cudaMemsetAsync(h->target, 0, h->plane * 4, h->stream));
-  DTSGB_CUDA(cudaMemsetAsync(h->conf, 0, h->plane * 4, h->stream));
-  DTSGB_CUDA(cudaMemsetAsync(h->out, 0, h->plane * 4, h->stream));
-  for (int i = 0; i < G_NUM; ++i)
-    DTSGB_CUDA(cudaMemsetAsync(h->g[i], 0, h->gsize * 4, h->stream));
-  DTSGB_CUDA(cudaMemsetAsync(h->ovf, 0, (size_t)h->max_gx * h->max_gy * 4,
-                             h->stream));
+  ZeroList L;
+  L.add(h->guide, h->plane * 4);
+  L.add(h->target, h->plane * 4);
+  L.add(h->conf, h->plane * 4);
+  L.add(h->out, h->plane * 4);
+  for (int i = 0; i < G_NUM; ++i) L.add(h->g[i], h->gsize * 4);
+  L.add(h->ovf, (size_t)h->max_gx * h->max_gy * 4);
+  if (int st = launch_zero(L, h->stream)) return st;
   h->solved = false;
   h->grad_ready = false;
   ++h->guide_gen;
