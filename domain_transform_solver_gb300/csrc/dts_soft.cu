@@ -847,9 +847,8 @@ __global__ void __launch_bounds__(256)
 }
 
 // sum_q w_pq V(q) over pixel i's planned window, in the walks' order.  Eight
-// pixels at a time under a predicate each: a loop with a turn a pixel made the
-// kernels issue-bound (255 instructions a pixel in the X half-step, 28 us for
-// 3.1 Mpx; XXX and YYY so).
+// pixels at a time under a predicate each: with a turn a pixel the X adjoint of
+// 3.1 Mpx took 51 us, 45 so; n comes from the plan.
 template <class LN>
 __device__ __forceinline__ float plan_sum(const LN& ln, int i, unsigned cnt, float2 w2,
                                           float wc) {

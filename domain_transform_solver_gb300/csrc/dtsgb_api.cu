@@ -427,12 +427,14 @@ DTSGB_API int dtsgb_dts_integrate(dtsgb_dts_t h) {
 // Window bounds for (sx, sy) on the current domain transform.  Without a
 // differential (after ClearAll) the reference's dH / ct buffers are zero and
 // every window collapses to the pixel itself.
-static int dts_bounds(dtsgb_dts_t h, float sx, float sy, bool use_cache) {
+// plane: where they go (null: the handle's).
+static int dts_bounds(dtsgb_dts_t h, float sx, float sy, bool use_cache,
+                      uint32_t* plane = nullptr) {
   if (use_cache && h->bounds_valid && h->b_sx == sx && h->b_sy == sy)
     return DTSGB_OK;
   if (!finite_pos(sx) || !finite_pos(sy))
     return fail(DTSGB_ERR_INVALID_ARGUMENT, "sigma must be finite and positive");
-  int st = launch_bounds(h->launch_i(), h->guide, h->bounds,
+  int st = launch_bounds(h->launch_i(), h->guide, plane ? plane : h->bounds,
                          h->diff_valid ? h->ratio_x : -1.f,
                          h->diff_valid ? h->ratio_y : -1.f, sx, sy, h->ref_y,
                          h->stream);
@@ -495,26 +497,17 @@ DTSGB_API int dtsgb_dts_optimize(dtsgb_dts_t h, const dtsgb_optimize_params* p,
   return DTSGB_OK;
 }
 
-// num_iter X/Y box passes of the current v[src] with the sigma schedule of
-// DomainTransformFilter::Filter; returns the index of the result buffer.
-static int dts_filter_device(dtsgb_dts_t h, float sx, float sy, int num_iter,
-                             int* result_idx) {
-  int a = 0, b = 1;
-  for (int it = 0; it < num_iter; ++it) {
-    const float m = filter_sigma_multiplier(it, num_iter);
-    const float six = sx * m, siy = sy * m;
-    if (six >= 254.f || siy >= 254.f)
-      return fail(DTSGB_ERR_UNSUPPORTED, "filter sigma must be below 254");
-    int st = dts_bounds(h, six, siy, false);
-    if (st) return st;
-    st = launch_filter_pass(h->launch_i(), 1, h->v[a], nullptr, h->v[b], nullptr,
-                            h->bounds, (int)std::floor(six), (int)std::floor(siy),
-                            h->st, nullptr, 0.f, 0, h->stream);
-    if (st) return st;
-    std::swap(a, b);
-  }
-  *result_idx = a;
-  return DTSGB_OK;
+// Window bounds of box pass `it` of num_iter (the sigma schedule of
+// DomainTransformFilter::Filter), into the plane that pass reads.
+static uint32_t* filter_bounds_plane(dtsgb_dts_t h, int it) {
+  return it == 1 || it == 2 ? (uint32_t*)h->scr[it - 1] : h->bounds;
+}
+static int dts_filter_bounds(dtsgb_dts_t h, float sx, float sy, int it, int num_iter) {
+  const float m = filter_sigma_multiplier(it, num_iter);
+  const float six = sx * m, siy = sy * m;
+  if (six >= 254.f || siy >= 254.f)
+    return fail(DTSGB_ERR_UNSUPPORTED, "filter sigma must be below 254");
+  return dts_bounds(h, six, siy, false, filter_bounds_plane(h, it));
 }
 
 DTSGB_API int dtsgb_dts_filter(dtsgb_dts_t h, const dtsgb_filter_params* p,
@@ -525,19 +518,29 @@ DTSGB_API int dtsgb_dts_filter(dtsgb_dts_t h, const dtsgb_filter_params* p,
   int st = check_filter_params(p->sigma_x, p->sigma_y, p->sigma_r);
   if (st) return st;
   const size_t wb = (size_t)h->w * 4;
-  DTSGB_CUDA(cudaMemcpy2DAsync(h->v[0], (size_t)h->pitch * 4, input, wb, wb,
-                               h->h, cudaMemcpyHostToDevice, h->stream));
   // Filter recomputes the DT with its own sigmas (filter.cu:128-129).
   h->ratio_x = p->sigma_x / p->sigma_r;
   h->ratio_y = p->sigma_y / p->sigma_r;
   h->diff_valid = true;
   h->bounds_valid = false;
-  int res = 0;
-  st = dts_filter_device(h, p->sigma_x, p->sigma_y, num_iter, &res);
-  if (st) return st;
-  if (res != 0)
-    DTSGB_CUDA(cudaMemcpyAsync(h->v[0], h->v[res], h->plane * 4,
-                               cudaMemcpyDeviceToDevice, h->stream));
+  // The bounds of the first three passes come from the guide alone: they run
+  // while the host still copies the input (18 us each for 1280x720).
+  constexpr int kAhead = 3;
+  for (int it = 0; it < std::min(num_iter, kAhead); ++it)
+    if ((st = dts_filter_bounds(h, p->sigma_x, p->sigma_y, it, num_iter))) return st;
+  int a = num_iter & 1;  // the result lands in v[0]
+  DTSGB_CUDA(cudaMemcpy2DAsync(h->v[a], (size_t)h->pitch * 4, input, wb, wb,
+                               h->h, cudaMemcpyHostToDevice, h->stream));
+  for (int it = 0; it < num_iter; ++it) {
+    if (it >= kAhead)
+      if ((st = dts_filter_bounds(h, p->sigma_x, p->sigma_y, it, num_iter))) return st;
+    const float m = filter_sigma_multiplier(it, num_iter);
+    st = launch_filter_pass(h->launch_i(), 1, h->v[a], nullptr, h->v[a ^ 1], nullptr,
+                            filter_bounds_plane(h, it), (int)std::floor(p->sigma_x * m),
+                            (int)std::floor(p->sigma_y * m), h->st, nullptr, 0.f, 0, h->stream);
+    if (st) return st;
+    a ^= 1;
+  }
   h->var_idx = 0;
   DTSGB_CUDA(cudaMemcpy2DAsync(output, wb, h->v[0], (size_t)h->pitch * 4, wb,
                                h->h, cudaMemcpyDeviceToHost, h->stream));
