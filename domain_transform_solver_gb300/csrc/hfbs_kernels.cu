@@ -381,7 +381,7 @@ __global__ void k_laplace_x(const HInst* __restrict__ insts,
   for (int line = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; line < nlines;
        line += nwarps) {
     const long long base = I.grid_off + (long long)line * I.px;
-    for (int f = 0; f < 2; ++f) {
+    for (int f = blockIdx.z; f < 2; f += gridDim.z) {  // the field
       const float* s = (f ? s1 : s0) + base;
       float* d = (f ? d1 : d0) + base;
       // forward: F
@@ -433,6 +433,7 @@ __global__ void k_laplace(const HInst* __restrict__ insts, int axis,
                           const float* __restrict__ s0, float* __restrict__ d0,
                           const float* __restrict__ s1, float* __restrict__ d1,
                           float beta) {
+  const int f = blockIdx.z;  // the field: a line of each is a thread's work
   constexpr int U = kLapChunk;
   const HInst I = insts[blockIdx.y];
   const int gx = I.gx, gy = I.gy, gl = I.gl;
@@ -454,7 +455,7 @@ __global__ void k_laplace(const HInst* __restrict__ insts, int axis,
     else if (axis == 1) base = (long long)bb * px * gy + a;
     else base = (long long)bb * px + a;
     base += I.grid_off;
-    for (int f = 0; f < 2; ++f) {
+    {
       const float* s = (f ? s1 : s0) + base;
       float* d = (f ? d1 : d0) + base;
       // forward: d(0) = s(0), d(i) = beta * d(i-1) + s(i)
@@ -494,6 +495,39 @@ __global__ void k_laplace(const HInst* __restrict__ insts, int axis,
         }
       }
     }
+  }
+}
+
+// The same along l for grids of up to NL levels: a line stays in registers, so
+// each element is read and written once (the general form reads it twice more
+// and writes it once more; at 64 levels it is the faster one, 73 against 102 us
+// on 408 x 306).
+template <int NL>
+__global__ void __launch_bounds__(128)
+    k_laplace_l(const HInst* __restrict__ insts, const float* __restrict__ s0,
+                float* __restrict__ d0, const float* __restrict__ s1, float* __restrict__ d1,
+                float beta) {
+  const HInst I = insts[blockIdx.y];
+  const int px = I.px, gl = I.gl;
+  const float* sf = (blockIdx.z ? s1 : s0) + I.grid_off;
+  float* df = (blockIdx.z ? d1 : d0) + I.grid_off;
+  const int plane = px * I.gy;  // (the padding columns too: they are never read)
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < plane; c += gridDim.x * blockDim.x) {
+    float v[NL], w[NL];
+#pragma unroll
+    for (int l = 0; l < NL; ++l) v[l] = l < gl ? sf[(long long)l * plane + c] : 0.f;
+    float r = 0.f;
+#pragma unroll
+    for (int l = 0; l < NL; ++l) w[l] = r = l == 0 ? v[0] : __fmaf_rn(beta, r, v[l]);
+    r = 0.f;
+#pragma unroll
+    for (int l = NL - 1; l >= 0; --l) {
+      if (l + 1 < gl) w[l] = __fmaf_rn(beta, r, w[l]);
+      if (l < gl) r = l + 1 < gl ? __fmaf_rn(beta, r, v[l]) : v[l];
+    }
+#pragma unroll
+    for (int l = 0; l < NL; ++l)
+      if (l < gl) df[(long long)l * plane + c] = w[l];
   }
 }
 
@@ -758,14 +792,28 @@ int hfbs_launch_steps(const HfbsBatch& B, const HParams& p, const float* norm,
   return DTSGB_OK;
 }
 
+// The Laplace blur X -> Y -> Z of the pair (s0, s1) by way of (x0, x1) and (y0,
+// y1) into (x0, x1); a field of the pair on each z of the grids (both in one
+// thread took 10 us a sweep of 80 x 60 x 16, which waits on its loads; 8.6 along y
+// and 2.8 along l so).
 void hfbs_launch_blur_pair(const HfbsBatch& B, const HParams& p, const float* s0,
                            const float* s1, float* x0, float* x1, float* y0, float* y1,
                            cudaStream_t s) {
-  const dim3 gr((unsigned)std::min<long long>((B.max_rows + 7) / 8, 4096), B.n_inst);
-  const dim3 gl_lines(blocks_for(B.max_lines), B.n_inst);
+  const int ni = B.n_inst;
+  // (rows: both fields in one warp where there are rows enough, whose warps
+  // share their powers of beta: 64 ragged grids 125 us, 151 split)
+  const dim3 gr((unsigned)std::min<long long>((B.max_rows + 7) / 8, 4096), ni,
+                B.max_rows * ni > 152 * 64 ? 1 : 2);
+  const dim3 gl_lines(blocks_for(B.max_lines), ni, 2);
   k_laplace_x<<<gr, kT, 0, s>>>(B.d_inst, s0, x0, s1, x1, p.neg_exp_beta);
   k_laplace<<<gl_lines, kT, 0, s>>>(B.d_inst, 1, x0, y0, x1, y1, p.neg_exp_beta);
-  k_laplace<<<gl_lines, kT, 0, s>>>(B.d_inst, 2, y0, x0, y1, x1, p.neg_exp_beta);
+  const dim3 gz((unsigned)std::min<long long>((B.max_cells + 127) / 128 + 1, 4096), ni, 2);
+  if (B.max_gl <= 16)
+    k_laplace_l<16><<<gz, 128, 0, s>>>(B.d_inst, y0, x0, y1, x1, p.neg_exp_beta);
+  else if (B.max_gl <= 32)
+    k_laplace_l<32><<<gz, 128, 0, s>>>(B.d_inst, y0, x0, y1, x1, p.neg_exp_beta);
+  else
+    k_laplace<<<gl_lines, kT, 0, s>>>(B.d_inst, 2, y0, x0, y1, x1, p.neg_exp_beta);
 }
 
 int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s,
@@ -901,13 +949,8 @@ int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s,
   prof_begin(s, DTSGB_K_HFBS_OTHER);
   k_inv_diag<<<gflat, kT, 0, s>>>(B.count, B.csum, norm, B.invA, p.lambda,
                                   B.total_voxels);
-  // Laplace blur of (c, b): X -> Y -> Z.
-  const dim3 gl_lines(blocks_for(B.max_lines), ni);
-  k_laplace_x<<<gr, kT, 0, s>>>(B.d_inst, B.csum, B.t0, B.b, B.t1, p.neg_exp_beta);
-  k_laplace<<<gl_lines, kT, 0, s>>>(B.d_inst, 1, B.t0, B.t2, B.t1, spare,
-                                    p.neg_exp_beta);
-  k_laplace<<<gl_lines, kT, 0, s>>>(B.d_inst, 2, B.t2, B.t0, spare, B.t1,
-                                    p.neg_exp_beta);
+  // Laplace blur of (c, b)
+  hfbs_launch_blur_pair(B, p, B.csum, B.b, B.t0, B.t1, B.t2, spare, s);
   // blur_c = t0, blur_b = t1
   // z_0 is overwritten: kept for inspection, and as the adjoint's first iterate
   float* z_kept = B.grad && B.grad->segment == 1 && p.optim_iter_max > 0 ? B.grad->hist : nullptr;

@@ -91,7 +91,7 @@ constexpr size_t smem_bytes(int nw) {
 
 // D: planes requested ahead of the one in use.
 template <int MODE, bool REC, int K, int D>
-__global__ void __launch_bounds__(512, 1)
+__global__ void __launch_bounds__(MODE == kBistoch ? 640 : 512, 1)
     k_hfbs_march(const HInst* __restrict__ insts, MarchArgs A, MarchMaps m) {
   pdl_wait_then_release();  // launched as a dependent of the previous pass
   constexpr int NR = MODE == kHeavyBall ? 3 : 1;  // arrays in the ring
@@ -182,8 +182,9 @@ __global__ void __launch_bounds__(512, 1)
   const bool has_lo = w > 0, has_hi = w + 1 < nw;
   int slot = 0, is = 0;       // j % SL, j % NB
   unsigned parity = 0;        // of input slot `is`: flips when it wraps
-  // (by two: half of the moves between planes are renamings; 3% of a solve)
-#pragma unroll (REC ? 1 : 2)
+  // (by two: half of the moves between planes are renamings; 3% of a solve.  The
+  // normalisation does without and fits five blocks of four warps an SM.)
+#pragma unroll (REC || MODE == kBistoch ? 1 : 2)
   for (int j = 0; j < N; ++j) {
     const bool got = !use_tma || mbar_wait_bounded(&bar[is], parity, kTmaWaitPolls);
     const float* zi = inp + is * NI * PL + own;
