@@ -48,14 +48,15 @@ sys.path.insert(0, str(ROOT / "oracle"))
 METRIC = "DTS/HFBS solve Mpix/s at fixed iters, fwd+bwd Mpix/s, %HBM peak; RMSE vs FP64"
 FALLBACK_HBM_GBS = 6800.0
 L2_FLUSH_BYTES = 256 << 20
-KERNEL_NAMES = {0: "k_bounds", 1: "k_dts_iter", 2: "k_filter", 3: "k_splat",
-                4: "k_bistoch", 5: "k_solve (HFBS heavy-ball)", 6: "hfbs setup kernels",
-                7: "k_slice", 8: "k_to_float", 9: "k_dts_adjoint",
+KERNEL_NAMES = {0: "k_bounds_x + k_bounds_y", 1: "k_dts_x + k_dts_y", 2: "k_filter",
+                3: "k_splat", 4: "HFBS bistochastization", 5: "HFBS heavy-ball",
+                6: "hfbs setup kernels", 7: "k_slice", 8: "k_to_float",
+                9: "k_adj_y + k_adj_x",
                 10: "hfbs adjoint (whole backward)",
                 11: "soft-window plans, line scans and other",
                 12: "k_soft_half_plan X", 13: "k_soft_adjoint_fused X",
                 14: "k_soft_adjoint_fused Y", 15: "k_soft_half_plan Y"}
-HFBS_TB_STEPS = 4  # heavy-ball steps per launch of the temporally blocked kernel
+HFBS_TB_STEPS = 4  # heavy-ball steps per pass of the march over a grid
 
 
 def peaks():
@@ -209,10 +210,12 @@ def _stratified(sizes, k: int) -> list[int]:
 #     bistochastization step 12 B/vx, invA 16 + blur 48 + init 12 B/vx, per
 #     heavy-ball step 28 B/vx, slice 8 B/px.  Kernels it does not describe
 #     (the iterate initialisation, the adjoints) use the fused contract.
-#   fused_bytes: what the fused kernels here must move at minimum (the DTS
-#     iteration reads v, t, c and the packed bounds once and writes v; the
-#     temporally blocked heavy-ball launch reads z, n, b, invA, h once and
-#     writes h, z for four steps).
+#   fused_bytes: what an iteration fused over its two passes would have to
+#     move at minimum (the DTS iteration reads v, t, c and the packed bounds
+#     once and writes v; four heavy-ball steps read z, n, b, invA, h once and
+#     write h, z).  The passes here move 12 B/px more per iteration (the X
+#     result written and read, the bounds read twice), a cluster that keeps a
+#     grid on chip less.
 class Batched:
     """Shared parts of the many-instance workloads."""
 
