@@ -373,6 +373,9 @@ __global__ void k_soft_half(const SInst* __restrict__ insts, const float* __rest
 // Y tiles kTYC columns x kTYR rows; the tile and its halo are staged once
 // (coalesced rows) and every walk reads shared memory.  Same arithmetic in
 // the same order as the global form, so the results are identical.
+// Largest tile halo of the shared-memory kernels (the Y adjoint tile then
+// holds 5 x 32 x (64 + 80) floats, 92 KB).
+constexpr int kMaxHalo = 40;
 constexpr int kTX = 256, kTYC = 32, kTYR = 64, kTYT = 8;  // Y: kTYC x kTYT threads
 
 template <int AXIS>
@@ -846,104 +849,123 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// sum_q w_pq V(q) over pixel i's planned window, in the walks' order.  Eight
-// pixels at a time under a predicate each: with a turn a pixel the X adjoint of
-// 3.1 Mpx took 51 us, 45 so; n comes from the plan.
-template <class LN>
+// sum_q w_pq V(q) over pixel i's planned window, in the walks' order, eight
+// pixels at a time under a predicate each (with a turn a pixel the X adjoint of
+// 3.1 Mpx took 51 us, 45 so).  AHEAD: the eight are loaded before they are added,
+// whether the window holds them or not, which takes kPlanPad entries past the
+// widest window on each side of a tile: better in the X half-step (22.9 us
+// against 25), whose row stands alone, worse in the adjoints (54 against 45).
+constexpr int kPlanPad = 8;
+template <bool AHEAD = false, class LN>
 __device__ __forceinline__ float plan_sum(const LN& ln, int i, unsigned cnt, float2 w2,
                                           float wc) {
   const int dl = cnt & 255, du = (cnt >> 8) & 255, nrl = (cnt >> 16) & 255, nru = cnt >> 24;
-  constexpr int U = 8;
+  constexpr int U = kPlanPad;
   float S = wc * ln.V(i);
-  for (int b = 0; b < du; b += U) {
+  auto side = [&](int m, auto&& at) {
+    for (int b = 0; b < m; b += U) {
+      float v[U];
+      if (AHEAD) {
 #pragma unroll
-    for (int k = 0; k < U; ++k)
-      if (b + k < du) S += ln.V(i + 1 + b + k);
-  }
+        for (int k = 0; k < U; ++k) v[k] = at(b + k + 1);
+      }
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        if (b + k < m) S += AHEAD ? v[k] : at(b + k + 1);
+    }
+  };
+  side(du, [&](int k) { return ln.V(i + k); });
   if (nru) S = __fmaf_rn(w2.y, ln.V(i + du + 1), S);
-  for (int b = 0; b < dl; b += U) {
-#pragma unroll
-    for (int k = 0; k < U; ++k)
-      if (b + k < dl) S += ln.V(i - 1 - b - k);
-  }
+  side(dl, [&](int k) { return ln.V(i - k); });
   if (nrl) S = __fmaf_rn(w2.x, ln.V(i - dl - 1), S);
   return S;
 }
 
-// X tiles of PX x 256 pixels (a thread takes pixels t, t + 256, ...): more
-// loads in flight per thread on wide images.
-template <int AXIS, int PX = 1>
+// The planned half-steps.  X: a warp takes kSXP x 32 pixels of a row and its
+// halo, on its own; the iterate goes to shared memory and a lane's own operands
+// to registers first (all of its loads in flight together), at fixed offsets
+// from one address a plane: 28 to 22.9 us for 3.1 Mpx against row tiles of a
+// block.  Y: a block takes 32 columns x 64 rows, eight rows a thread (31 us; the
+// X form, with its operands in registers first, 35).
+constexpr int kSXP = 4;
+
+__global__ void __launch_bounds__(128)
+    k_soft_half_x(const SInst* __restrict__ insts, const float* __restrict__ vin,
+                  float* __restrict__ vout, const unsigned* __restrict__ counts,
+                  const float2* __restrict__ wts, const float* __restrict__ nplan,
+                  const float* __restrict__ t, const float* __restrict__ c,
+                  float* __restrict__ Bout, int mode, float wc, float lambda, float step,
+                  int halo) {
+  extern __shared__ float smf[];
+  const SInst I = insts[blockIdx.z];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int x0 = blockIdx.x * (32 * kSXP);
+  if (x0 >= I.w) return;
+  const int TL = 32 * kSXP + 2 * halo;
+  float* s = smf + warp * (TL + 2 * kPlanPad) + kPlanPad;
+  for (int y = blockIdx.y * 4 + warp; y < I.h; y += gridDim.y * 4) {
+    const long long row = I.off + (long long)y * I.w, p0 = row + x0 + lane;
+    unsigned cn[kSXP];
+    float2 w2[kSXP];
+    float nv[kSXP], tv[kSXP], cv[kSXP];
+    const int left = I.w - x0 - lane;  // own pixel k is in the row if 32 k < left
+#pragma unroll
+    for (int k = 0; k < kSXP; ++k) {
+      const bool in = 32 * k < left;
+      cn[k] = in ? counts[p0 + 32 * k] : 0u;
+      w2[k] = in ? wts[p0 + 32 * k] : make_float2(0.f, 0.f);
+      nv[k] = in ? nplan[p0 + 32 * k] : 1.f;
+      tv[k] = in ? t[p0 + 32 * k] : 0.f;
+      cv[k] = in ? c[p0 + 32 * k] : 0.f;
+    }
+    constexpr int NS = kSXP + (2 * kMaxHalo + 31) / 32;
+    float v[NS];
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+      const int x = x0 - halo + lane + 32 * k;
+      v[k] = x >= 0 && x < I.w && lane + 32 * k < TL ? vin[row + x] : 0.f;
+    }
+    __syncwarp();  // the row before is read
+#pragma unroll
+    for (int k = 0; k < NS; ++k)
+      if (lane + 32 * k < TL) s[lane + 32 * k] = v[k];
+    __syncwarp();
+    const TileLine ln{nullptr, s, nullptr, nullptr, nullptr, 0, 1, 0, 0};
+#pragma unroll
+    for (int k = 0; k < kSXP; ++k) {
+      if (32 * k >= left) break;
+      const int i = halo + lane + 32 * k;
+      const float S = plan_sum<true>(ln, i, cn[k], w2[k], wc);
+      half_update_v(p0 + 32 * k, s[i], nv[k], S, tv[k], cv[k], vout, nullptr, Bout, 1, mode,
+                    lambda, step);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(256)
-    k_soft_half_plan(const SInst* __restrict__ insts, const float* __restrict__ vin,
-                     float* __restrict__ vout, const unsigned* __restrict__ counts,
-                     const float2* __restrict__ wts, const float* __restrict__ nplan,
-                     const float* __restrict__ t, const float* __restrict__ c,
-                     float* __restrict__ Bout, int data, int mode, float wc, float lambda,
-                     float step, int halo) {
+    k_soft_half_y(const SInst* __restrict__ insts, const float* __restrict__ vin,
+                  float* __restrict__ vout, const unsigned* __restrict__ counts,
+                  const float2* __restrict__ wts, const float* __restrict__ nplan,
+                  float* __restrict__ Bout, float wc, float lambda, float step, int halo) {
   extern __shared__ float smf[];
   const SInst I = insts[blockIdx.y];
-  const int len = AXIS == 0 ? kTX * PX : kTYR;
-  const TileGeom<AXIS> G(I, len);
+  const TileGeom<1> G(I);
   const float* srcs[1] = {vin};
   float* dsts[1] = {smf};
-  constexpr int OWN = AXIS == 0 ? PX : kTYR / kTYT;  // pixels per thread
   for (int tile = blockIdx.x; tile < G.n0 * G.n1; tile += gridDim.x) {
     const int t1 = tile / G.n0, t0 = tile - t1 * G.n0;
-    const int l0 = t0 * len, cross = AXIS == 0 ? t1 : t1 * kTYC;
-    // own pixel k: line index and global index (< 0: outside the image)
-    auto own_i = [&](int k) -> int {
-      return AXIS == 0 ? l0 + (int)threadIdx.x + kTX * k : l0 + (int)threadIdx.y + kTYT * k;
-    };
-    auto own_p = [&](int k) -> long long {
-      if (AXIS == 0) {
-        const int x = l0 + threadIdx.x + kTX * k;
-        return x < I.w ? I.off + (long long)cross * I.w + x : -1;
-      }
-      const int x = cross + threadIdx.x, y = l0 + threadIdx.y + kTYT * k;
-      return (x < I.w && y < I.h) ? I.off + (long long)y * I.w + x : -1;
-    };
-    // X: the own pixels' plan, t and c, loaded before the tile is staged, so
-    // that these loads are in flight with the staging's (Y's eight pixels a
-    // thread load after the staging)
-    constexpr int OP = AXIS == 0 ? OWN : 1;
-    unsigned cn[OP];
-    float2 w2[OP];
-    float tv[OP], cv[OP], nv[OP];
-    if (AXIS == 0) {
-#pragma unroll
-      for (int k = 0; k < OP; ++k) {
-        const long long p = own_p(k);
-        cn[k] = p >= 0 ? counts[p] : 0u;
-        w2[k] = p >= 0 ? wts[p] : make_float2(0.f, 0.f);
-        nv[k] = p >= 0 ? nplan[p] : 1.f;
-        tv[k] = p >= 0 && data ? t[p] : 0.f;
-        cv[k] = p >= 0 && data ? c[p] : 0.f;
-      }
-    }
+    const int l0 = t0 * kTYR, cross = t1 * kTYC;
     __syncthreads();
-    stage_tile<AXIS, 1>(I, l0, cross, srcs, dsts, halo, len);
+    stage_tile<1, 1>(I, l0, cross, srcs, dsts, halo, kTYR);
     __syncthreads();
-    const TileLine ln{nullptr, smf, nullptr, nullptr, nullptr, l0 - halo,
-                      AXIS == 0 ? 1 : kTYC, AXIS == 0 ? 0 : (int)threadIdx.x,
-                      AXIS == 0 ? I.w : I.h};
-    if (AXIS == 0) {
-#pragma unroll
-      for (int k = 0; k < OP; ++k) {
-        const long long p = own_p(k);
-        if (p < 0) continue;
-        const int i = own_i(k);
-        const float S = plan_sum(ln, i, cn[k], w2[k], wc);
-        half_update_v(p, ln.V(i), nv[k], S, tv[k], cv[k], vout, nullptr, Bout, data, mode, lambda,
-                      step);
-      }
-    } else {
-      const int x = cross + threadIdx.x;
-      for (int y = l0 + threadIdx.y; y < min(l0 + kTYR, I.h); y += kTYT) {
-        if (x >= I.w) break;
-        const long long p = I.off + (long long)y * I.w + x;
-        const float S = plan_sum(ln, y, counts[p], wts[p], wc);
-        half_update(p, ln.V(y), nplan[p], S, t, c, vout, nullptr, Bout, data, mode, lambda, step);
-      }
+    const TileLine ln{nullptr, smf, nullptr, nullptr, nullptr, l0 - halo, kTYC,
+                      (int)threadIdx.x, I.h};
+    const int x = cross + threadIdx.x;
+    for (int y = l0 + threadIdx.y; y < min(l0 + kTYR, I.h); y += kTYT) {
+      if (x >= I.w) break;
+      const long long p = I.off + (long long)y * I.w + x;
+      const float S = plan_sum(ln, y, counts[p], wts[p], wc);
+      half_update_v(p, ln.V(y), nplan[p], S, 0.f, 0.f, vout, nullptr, Bout, 0, 0, lambda, step);
     }
   }
 }
@@ -1253,10 +1275,6 @@ int ensure_planes(dtsgb_soft_t s, int planes) {
   return DTSGB_OK;
 }
 
-// Largest tile halo of the shared-memory kernels (the Y adjoint tile then
-// holds 5 x 32 x (64 + 80) floats, 92 KB).
-constexpr int kMaxHalo = 40;
-
 long long max_tiles(const dtsgb_soft_s* s, int axis, int px = 1) {
   long long m = 1;
   const int lx = kTX * px;
@@ -1392,19 +1410,22 @@ int launch_half(dtsgb_soft_t s, const float* vin, float* vout, const float* e, c
     const int PH = s->plan_halo, base = axis == 0 ? P_PNX : P_PNY;
     const unsigned* cnt = reinterpret_cast<const unsigned*>(s->plane(base + 1));
     const float2* wts = reinterpret_cast<const float2*>(s->plane(base + 2));
-    const int px = axis == 0 ? plan_px(s) : 1;
-    const dim3 g((unsigned)std::min<long long>(max_tiles(s, axis, px), 152 * 16), s->n);
-    if (axis == 0 && px == 4)
-      k_soft_half_plan<0, 4><<<g, kTX, sizeof(float) * (4 * kTX + 2 * PH), s->stream>>>(
-          s->d_inst, vin, vout, cnt, wts, s->plane(base), t, c, Bout, data, mode, R.wc, lambda, step, PH);
-    else if (axis == 0)
-      k_soft_half_plan<0><<<g, kTX, sizeof(float) * (kTX + 2 * PH), s->stream>>>(
-          s->d_inst, vin, vout, cnt, wts, s->plane(base), t, c, Bout, data, mode, R.wc, lambda, step, PH);
-    else
-      k_soft_half_plan<1><<<g, dim3(kTYC, kTYT), sizeof(float) * (kTYR + 2 * PH) * kTYC,
-                            s->stream>>>(s->d_inst, vin, vout, cnt, wts, s->plane(base), t, c, Bout,
-                                         data, mode,
-                                         R.wc, lambda, step, PH);
+    int max_w = 1, max_h = 1;
+    for (const SInst& I : s->inst) {
+      max_w = std::max(max_w, I.w);
+      max_h = std::max(max_h, I.h);
+    }
+    if (axis == 0) {
+      const dim3 g((unsigned)((max_w + 32 * kSXP - 1) / (32 * kSXP)),
+                   (unsigned)std::min((max_h + 3) / 4, 32768), s->n);
+      k_soft_half_x<<<g, 128, sizeof(float) * 4 * (32 * kSXP + 2 * (PH + kPlanPad)), s->stream>>>(
+          s->d_inst, vin, vout, cnt, wts, s->plane(base), t, c, Bout, mode, R.wc, lambda, step,
+          PH);
+    } else {
+      const dim3 g((unsigned)std::min<long long>(max_tiles(s, axis), 152 * 16), s->n);
+      k_soft_half_y<<<g, dim3(kTYC, kTYT), sizeof(float) * (kTYR + 2 * PH) * kTYC, s->stream>>>(
+          s->d_inst, vin, vout, cnt, wts, s->plane(base), Bout, R.wc, lambda, step, PH);
+    }
   } else if (H > kMaxHalo) {
     k_soft_half<<<soft_grid(s), kST, 0, s->stream>>>(s->d_inst, vin, vout, e, t, c, nout, Bout,
                                                      axis, data, mode, R, lambda, step);

@@ -267,3 +267,15 @@ def test_soft_lent_workspace(gpu_ready):
     with pytest.raises(D.DtsgbError):
         s.backward(p)  # the solve went with its workspace
     s.close()
+
+
+@pytest.mark.parametrize("w,h", [(1, 5), (31, 4), (127, 3), (128, 9), (129, 65), (385, 1)])
+def test_soft_half_steps_at_the_edges_of_their_segments(gpu_ready, oracle_mod, w, h):
+    """Rows around the 128 pixels of a warp, columns around the 64 rows of a
+    tile; held to the oracle's bars."""
+    D = gpu_ready
+    data = [_inputs(910 + w, w, h)]
+    opt = dict(num_iterations=3, loss=1, lambda_=0.99, sigma_z=8.0, step_size=0.99)
+    dh, dv = _gpu_edges(D, [data[0][0]])
+    res = _gpu_soft(D, dh, dv, [data[0][1]], [data[0][2]], opt, [data[0][3]])
+    _check_against_oracle(oracle_mod, data, dh.cpu().numpy(), dv.cpu().numpy(), opt, res)
