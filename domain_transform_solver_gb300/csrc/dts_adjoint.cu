@@ -303,6 +303,7 @@ int launch_y(const DtsLaunch& L, const PassGrid& G, const float* gin, float* gou
                       ((size_t)(2 * hy + 3) + warps * 32 + ((size_t)G.rows + 1) * 32);
   if (smem > 48 * 1024)
     DTSGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  ProfScope ps(s, DTSGB_K_DTS_ADJOINT);
   DTSGB_CUDA(launch_dependent(kern, G.y, dim3(32 * warps), smem, s, L.d_inst, gin, gout, bounds,
                               slam, hy, L.n_inst > 1 ? L.d_yblocks : (const Tile*)nullptr));
   return DTSGB_OK;
@@ -322,6 +323,7 @@ int launch_adj_t(const DtsLaunch& L, float* g, float* g1, const float* vk, const
   if (st) return st;
   auto x = [&](auto kern, int qs) -> int {
     const size_t smem = sizeof(unsigned) * ((size_t)kXWarps * 4 * qs + 2 * halo + 2);
+    ProfScope ps(s, DTSGB_K_DTS_ADJOINT);
     DTSGB_CUDA(launch_dependent(kern, G.x, dim3(32 * kXWarps), smem, s, L.d_inst, g1, g, vk,
                                 (const TS*)t, (const TS*)c, bounds, gt, gc, lambda, step, halo,
                                 flags, L.n_inst > 1 ? L.d_xblocks : (const Tile*)nullptr));
@@ -338,7 +340,6 @@ int launch_adjoint(const DtsLaunch& L, Storage st, IterMode mode, float* g, floa
                    const float* vk, const void* t, const void* c, const uint32_t* bounds,
                    float* gt, float* gc, float lambda, float step, int halo, int flags,
                    cudaStream_t s) {
-  ProfScope ps(s, DTSGB_K_DTS_ADJOINT);
 #define ADJ_T(TS, M) \
   launch_adj_t<TS, M>(L, g, g1, vk, t, c, bounds, gt, gc, lambda, step, halo, flags, s)
   if (st == Storage::F32) return mode == IterMode::L2 ? ADJ_T(float, 0) : ADJ_T(float, 1);

@@ -414,6 +414,7 @@ int launch_x(const DtsLaunch& L, const float* vin, float* vout, const void* targ
              float overwrite, int hx, dim3 grid, const StereoArgs& sa, cudaStream_t s) {
   auto kern = k_dts_x<TS, MODE, STEREO, OVER, NR, AHEAD>;
   const size_t smem = sizeof(unsigned) * (kXWarps * 4 * XPrefix<NR>::QS + 2 * hx + 2);
+  ProfScope ps(s, DTSGB_K_DTS_ITER);
   DTSGB_CUDA(launch_dependent(kern, grid, dim3(32 * kXWarps), smem, s, L.d_inst, vin, vout,
                               (const TS*)target, (const TS*)conf, bounds, lambda, step,
                               overwrite, hx, sa,
@@ -430,6 +431,7 @@ int launch_y(const DtsLaunch& L, const float* u, float* vout, const void* conf,
   const size_t smem = sizeof(unsigned) *
                       ((size_t)(2 * hy + 3) + warps * 32 + ((size_t)rows + 1) * 32);
   if (int st = set_smem(kern, smem)) return st;
+  ProfScope ps(s, DTSGB_K_DTS_ITER);
   DTSGB_CUDA(launch_dependent(kern, grid, dim3(32 * warps), smem, s, L.d_inst, u, vout,
                               (const TS*)conf, bounds, slam, overwrite, feeds, hy,
                               L.n_inst > 1 ? L.d_yblocks : (const Tile*)nullptr));
@@ -444,7 +446,6 @@ int launch_iter(const DtsLaunch& L, const float* vin, float* tmp, float* vout, c
   const dim3 gx = G.x, gy = G.y;
   const int rounds = G.rounds, rows = G.rows;
   const long long px = G.px;
-  ProfScope ps(s, DTSGB_K_DTS_ITER);
   int st;
   // enough blocks to fill the SMs without the loads ahead: 3264x2448 950 -> 898
   // us a solve, 16 x 1024x768 2427 -> 2386 a training step; 1376x1088, five
