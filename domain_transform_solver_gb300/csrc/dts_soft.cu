@@ -1685,6 +1685,7 @@ DTSGB_API int dtsgb_soft_edge_weights(dtsgb_soft_t s, int color_space,
     return fail(DTSGB_ERR_INVALID_ARGUMENT, "invalid color space");
   if (!finite_pos(f->sigma_x) || !finite_pos(f->sigma_y) || !finite_pos(f->sigma_r))
     return fail(DTSGB_ERR_INVALID_ARGUMENT, "filter sigmas must be finite, positive");
+  if (int st = ensure_planes(s, P_U + 1)) return st;  // (a bare handle's)
   // the guide goes through plane P_U (4 bytes per pixel), converted in place
   uchar4* g = reinterpret_cast<uchar4*>(s->plane(P_U));
   for (int i = 0; i < s->n; ++i) {

@@ -350,3 +350,52 @@ def test_adjoint_of_wider_windows_is_refused(gpu_ready):
     opt = dict(num_iterations=2, loss=1, lambda_=0.9, sigma_z=77.0, step_size=0.8)
     with pytest.raises(D.DtsgbError):
         A._batch(D, data, opt).backward([data[0][3]])
+
+
+# ---- HFBS blur: lines of up to 32 levels in registers --------------------------
+@pytest.mark.parametrize("sl", [255.0, 17.0, 16.0, 15.0, 8.0, 7.9])  # 1, 15, 16, 17, 32, 33 levels
+@pytest.mark.parametrize("w,h", [(40, 90), (700, 600)])  # both fields in a warp or one
+def test_blur_is_the_recursion_along_each_axis(gpu_ready, sl, w, h):
+    """Sums of positive terms, two roundings a step and direction: relative
+    error at most 4 * 2^-24 a step of the three sweeps."""
+    D = gpu_ready
+    rng = np.random.default_rng(int(sl) + w)
+    rgba = rng.integers(0, 256, (h, w, 4)).astype(np.uint8)
+    c = rng.random((h, w)).astype(np.float32)
+    f = np.float32
+    dims = (int(np.ceil(f(w) / f(4))), int(np.ceil(f(h) / f(4))), int(np.ceil(255.0 / sl)))
+    s = D.HFBS(D.ImageDim(w, h), *dims)
+    s.SetFilterParams(D.HFBSGridParams(sigma_x=4.0, sigma_y=4.0, sigma_l=sl, bistoch_iter_max=1,
+                                       optim_iter_max=1, neg_exp_beta=0.9))
+    s.InitFrame(D.COLOR_SPACE.RGB, rgba, np.ones((h, w), np.float32), c)
+    s.Optimize()
+    ref = s.DebugGrid(1).astype(np.float64)
+    beta = float(f(0.9))
+    for axis in (2, 1, 0):
+        a = np.moveaxis(ref, axis, 0)
+        fwd, bwd = a.copy(), np.zeros_like(a)
+        for i in range(1, len(a)):
+            fwd[i] += beta * fwd[i - 1]
+        for i in range(len(a) - 2, -1, -1):
+            bwd[i] = beta * (bwd[i + 1] + a[i + 1])
+        ref = np.moveaxis(fwd + bwd, 0, axis)
+    got = s.DebugGrid(5)
+    assert (np.abs(got - ref) <= sum(dims) * 2.0 ** -22 * ref).all()
+
+
+# ---- host images whose rows do not fill the pitch ------------------------------
+@pytest.mark.parametrize("w,h", [(1001, 300), (1002, 262), (720, 540), (999, 262), (1024, 256)])
+@pytest.mark.parametrize("bf16", [0, 1])
+def test_host_images_of_a_megabyte_arrive_whole(gpu_ready, w, h, bf16):
+    D = gpu_ready
+    rng = np.random.default_rng(w + h)
+    rgba = rng.integers(0, 256, (h, w, 4)).astype(np.uint8)
+    t, c = rng.random((2, h, w)).astype(np.float32)
+    s = D.DomainTransformSolver(D.ImageDim(w + 7, h + 3), D.FLAG_BF16_STORAGE if bf16 else 0)
+    s.SetImageDim(D.ImageDim(w, h))
+    s.ClearAll()
+    s.InitFrame(D.COLOR_SPACE.RGB, rgba, t, c)
+    r = P.bf16_round if bf16 else lambda a: a
+    assert np.array_equal(s.Download(D.ImageType.TARGET), r(t))
+    assert np.array_equal(s.Download(D.ImageType.CONFIDENCE), r(c))
+    assert np.array_equal(s.Download(D.ImageType.COLOR_IMAGE), rgba)

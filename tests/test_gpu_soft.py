@@ -269,6 +269,22 @@ def test_soft_lent_workspace(gpu_ready):
     s.close()
 
 
+def test_bare_handle_without_a_loan_has_planes_of_its_own(gpu_ready):
+    import torch
+    D = gpu_ready
+    rgba = torch.randint(0, 256, (20, 33, 4), dtype=torch.uint8, device="cuda")
+    outs = []
+    for bare in (False, True):
+        s = D.SoftDTS([(33, 20)], bare=bare)
+        dh, dv = (torch.empty((20, 33), device="cuda") for _ in range(2))
+        torch.cuda.synchronize()
+        s.edge_weights(D.COLOR_SPACE.YCbCr, [rgba.data_ptr()], D.DomainFilterParams(**FILT),
+                       [dh.data_ptr()], [dv.data_ptr()])
+        s.close()
+        outs.append((dh, dv))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
 @pytest.mark.parametrize("w,h", [(1, 5), (31, 4), (127, 3), (128, 9), (129, 65), (385, 1)])
 def test_soft_half_steps_at_the_edges_of_their_segments(gpu_ready, oracle_mod, w, h):
     """Rows around the 128 pixels of a warp, columns around the 64 rows of a
