@@ -91,7 +91,7 @@ __device__ __forceinline__ bool finite_bits(float v) { return mag_bits(v) < kNon
 // blocks an SM take turns, which is better where there are that many (see
 // launch_iter).  Warps are independent.
 //
-// The window ends come from k_bounds for the same sigma (dl <= hx + 1, du <=
+// The window ends come from dts_bounds.cu for the same sigma (dl <= hx + 1, du <=
 // hx), so a prefix index never leaves the staged columns.
 //
 // A non-finite value in the segment has no fixed-point form: the warp then

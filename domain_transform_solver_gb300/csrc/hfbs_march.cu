@@ -23,10 +23,11 @@
 // barrier per plane: the ends of the four levels (z * n of the next plane's
 // centre) cross it through a double-buffered exchange.
 //
-// Bound by issue slots (74% of them busy): about 34 instructions per voxel and
-// step, 13 of them floating point, 2 shuffles, 4 shared-memory reads and 10
-// moves and selects; memory traffic is 28 B a voxel and pass, a quarter of the
-// DRAM's rate.
+// Bound by dependent instructions at 16 warps an SM, which take every register
+// (issue slots 74% busy at 64 levels, 46% at 16): about 34 instructions per
+// voxel and step, 13 of them floating point, 2 shuffles, 4 shared-memory reads
+// and 10 moves and selects; memory traffic is 28 B a voxel and pass, a quarter
+// of the DRAM's rate.
 //
 // Outside the grid and above level gl everything is zero (the TMA fill), so
 // z * n adds zero to a neighbour sum there; those voxels are never updated.
