@@ -220,6 +220,9 @@ float* grad_plane_c(dtsgb_batch_t b) { return b->gplanes[b->gplanes.size() - 1];
 // The block tables of the DTS passes for a halo, and a launch that uses them.
 int ensure_pass_blocks(dtsgb_batch_t b, int halo) {
   if (b->n == 1 || b->pass_halo == halo) return DTSGB_OK;
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  DTSGB_CUDA(cudaStreamIsCapturing(b->stream, &c));
+  if (c != cudaStreamCaptureStatusNone) return DTSGB_OK;  // a launch per instance then
   DTSGB_CUDA(cudaStreamSynchronize(b->stream));  // a solve may still read them
   drop_graph(b, b->g_dts);
   drop_graph(b, b->g_bwd);
@@ -237,8 +240,9 @@ int ensure_pass_blocks(dtsgb_batch_t b, int halo) {
   b->pass_halo = halo;
   return DTSGB_OK;
 }
-DtsLaunch iter_launch(dtsgb_batch_t b) {
+DtsLaunch iter_launch(dtsgb_batch_t b, int halo) {
   DtsLaunch L{b->d_inst, nullptr, 0, b->n, false, nullptr, 0, b->inst.data()};
+  if (b->pass_halo != halo) return L;
   L.d_xblocks = b->d_px;
   L.d_yblocks = b->d_py;
   L.n_xblocks = (unsigned)b->npx;
@@ -942,7 +946,7 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
   const bool iterate = p->loss != DTSGB_L1 && p->num_iterations > 0;
   if (iterate)
     if (int st = ensure_pass_blocks(b, halo)) return st;
-  const DtsLaunch Li = iter_launch(b);
+  const DtsLaunch Li = iter_launch(b, halo);
   const bool over = overwrite > 0.f && overwrite < 1.f;
   const int n_kept = iterate ? p->num_iterations : 0;
   b->grad_n = -1;
@@ -1067,9 +1071,9 @@ static int batch_backward(dtsgb_batch_t b, const float* const* grad_out,
     if (int st = user_plane_copy(b, const_cast<float* const*>(grad_out), G.g[0], true))
       return st;
   }
-  const DtsLaunch Li = iter_launch(b);
   const dtsgb_optimize_params p = b->gopt;
   const int halo = (int)b->ghalo;
+  const DtsLaunch Li = iter_launch(b, halo);
   auto enqueue = [&]() -> int {
     const IterMode mode = p.loss == DTSGB_L2 ? IterMode::L2 : IterMode::CHARB;
     return dts_backward(Li, b->d_inst, b->n, b->total, b->st, mode, G, b->target, b->conf,

@@ -340,6 +340,13 @@ int launch_adjoint(const DtsLaunch& L, Storage st, IterMode mode, float* g, floa
                    const float* vk, const void* t, const void* c, const uint32_t* bounds,
                    float* gt, float* gc, float lambda, float step, int halo, int flags,
                    cudaStream_t s) {
+  if (L.one_by_one()) {
+    for (int i = 0; i < L.n_inst; ++i)
+      if (int e = launch_adjoint(L.one(i), st, mode, g, g1, vk, t, c, bounds, gt, gc, lambda, step,
+                                 halo, flags, s))
+        return e;
+    return DTSGB_OK;
+  }
 #define ADJ_T(TS, M) \
   launch_adj_t<TS, M>(L, g, g1, vk, t, c, bounds, gt, gc, lambda, step, halo, flags, s)
   if (st == Storage::F32) return mode == IterMode::L2 ? ADJ_T(float, 0) : ADJ_T(float, 1);

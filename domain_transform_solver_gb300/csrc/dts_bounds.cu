@@ -257,6 +257,13 @@ int launch_bounds(const DtsLaunch& L, const uchar4* guide, uint32_t* bounds,
   const int rx = (int)floorf(sigma_x) + 1, ry = (int)floorf(sigma_y) + 1;
   if (rx > 255 || ry > 255)
     return fail(DTSGB_ERR_UNSUPPORTED, "sigma >= 255 is not supported");
+  if (L.one_by_one()) {
+    for (int i = 0; i < L.n_inst; ++i)
+      if (int e = launch_bounds(L.one(i), guide, bounds, ratio_x, ratio_y, sigma_x, sigma_y,
+                                ref_y_limit, s))
+        return e;
+    return DTSGB_OK;
+  }
   // fixed point per axis: r * (sigma + 1) * 2^F <= 2^30; threshold floor(sigma 2^F)
   auto fx = [](int r, float sigma, float ratio) {
     Weight w;

@@ -526,6 +526,13 @@ int launch_dts_iter(const DtsLaunch& L, Storage st, IterMode mode, const float* 
                     float* vout, const void* target, const void* conf, const uint32_t* bounds,
                     float lambda, float step, float overwrite, int feeds, int halo,
                     cudaStream_t s, const StereoArgs* stereo) {
+  if (L.one_by_one()) {
+    for (int i = 0; i < L.n_inst; ++i)
+      if (int e = launch_dts_iter(L.one(i), st, mode, vin, tmp, vout, target, conf, bounds, lambda,
+                                  step, overwrite, feeds, halo, s, stereo))
+        return e;
+    return DTSGB_OK;
+  }
 #define ITER_T(TS, M)                                                                    \
   launch_iter_t<TS, M>(L, vin, tmp, vout, target, conf, bounds, lambda, step, overwrite, \
                        feeds, halo, stereo, s)

@@ -208,6 +208,15 @@ struct DtsLaunch {
   // (dts_pass_blocks)
   const Tile *d_xblocks = nullptr, *d_yblocks = nullptr;
   unsigned n_xblocks = 0, n_yblocks = 0;
+  // no block tables (first solve under a capture): one instance after the other
+  bool one_by_one() const { return n_inst > 1 && !d_xblocks; }
+  DtsLaunch one(int i) const {
+    DtsLaunch s = *this;
+    s.d_inst += i;
+    s.h_inst += i;
+    s.n_inst = 1;
+    return s;
+  }
   // the same launch on the small tiles
   DtsLaunch as_small() const {
     DtsLaunch s = *this;

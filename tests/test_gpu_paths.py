@@ -399,3 +399,35 @@ def test_host_images_of_a_megabyte_arrive_whole(gpu_ready, w, h, bf16):
     assert np.array_equal(s.Download(D.ImageType.TARGET), r(t))
     assert np.array_equal(s.Download(D.ImageType.CONFIDENCE), r(c))
     assert np.array_equal(s.Download(D.ImageType.COLOR_IMAGE), rgba)
+
+
+# ---- a first solve under a capture: no block tables, an instance a launch -------
+def test_first_solve_of_a_batch_under_a_capture(gpu_ready):
+    import torch
+    D = gpu_ready
+    rng = np.random.default_rng(5)
+    sizes = [(90, 60), (33, 140), (401, 77)]
+    g = [rng.integers(0, 256, (h, w, 4)).astype(np.uint8) for w, h in sizes]
+    t = [rng.normal(0, 1, (h, w)).astype(np.float32) for w, h in sizes]
+    c = [rng.random((h, w)).astype(np.float32) for w, h in sizes]
+    fp, op = D.DomainFilterParams(), D.DomainOptimizeParams(num_iterations=3, loss=1, sigma_z=8.0)
+    ref = D.Batch(sizes)
+    ref.upload(D.COLOR_SPACE.YCbCr, g, t, c)
+    ref.solve_dts(fp, op)
+    want = ref.download(0)
+    b = D.Batch(sizes, use_graphs=False)
+    stream = torch.cuda.Stream()
+    b.set_stream(stream.cuda_stream)
+    keep = [[torch.from_numpy(a).cuda() for a in x] for x in (g, t, c)]
+    out = [torch.full((h, w), -1.0, device="cuda") for w, h in sizes]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+        b.upload_device(D.COLOR_SPACE.YCbCr, *[[a.data_ptr() for a in x] for x in keep])
+        b.solve_dts(fp, op)
+        b.download_device(0, [o.data_ptr() for o in out])
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    for a, o in zip(want, out):
+        assert np.array_equal(a, o.cpu().numpy())
