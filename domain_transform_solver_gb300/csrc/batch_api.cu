@@ -15,6 +15,7 @@
 #include <cstring>
 #include <fstream>
 #include <initializer_list>
+#include <map>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -70,9 +71,15 @@ struct dtsgb_batch_s {
   long long* d_soff = nullptr;
   unsigned char* stage = nullptr;  // dense x (rgba 4 B, target 4 B, conf 4 B)
   Inst* d_inst = nullptr;
-  // blocks of the DTS passes for halo pass_halo (several instances only)
-  Tile *d_px = nullptr, *d_py = nullptr;
-  int npx = 0, npy = 0, pass_halo = -1;
+  // blocks of the DTS passes per halo (several instances only), carved from
+  // pass_mem; kept until the batch is destroyed (ensure_pass_blocks)
+  struct PassTables {
+    Tile *x = nullptr, *y = nullptr;
+    unsigned nx = 0, ny = 0;
+  };
+  std::map<int, PassTables> pass;
+  std::vector<Tile*> pass_mem;
+  size_t pass_room = 0, pass_left = 0;  // blocks of an allocation, left in the last one
   bool small = false;               // accepted and returned (DTSGB_TUNE_DTS_TILE)
   long long hfbs_group_voxels = 0;  // L2-resident HFBS group budget (0: off)
   int hfbs_solve_steps = 4;         // heavy-ball steps per launch (4 or 1)
@@ -165,8 +172,7 @@ void batch_free(dtsgb_batch_t b) {
   dfree(b->hout);
   dfree(b->scratch);
   dfree(b->d_inst);
-  dfree(b->d_px);
-  dfree(b->d_py);
+  for (Tile*& p : b->pass_mem) dfree(p);
   dfree(b->d_hinst);
   for (auto& p : b->hg) dfree(p);
   dfree(b->ovf);
@@ -217,36 +223,63 @@ DtsGrad grad_view(dtsgb_batch_t b, int n_iter) {
 float* grad_plane_t(dtsgb_batch_t b) { return b->gplanes[b->gplanes.size() - 2]; }
 float* grad_plane_c(dtsgb_batch_t b) { return b->gplanes[b->gplanes.size() - 1]; }
 
-// The block tables of the DTS passes for a halo, and a launch that uses them.
-int ensure_pass_blocks(dtsgb_batch_t b, int halo) {
-  if (b->n == 1 || b->pass_halo == halo) return DTSGB_OK;
+// Blocks of the passes over the whole batch for a halo.
+dim3 pass_block_totals(dtsgb_batch_t b, int halo) {
+  dim3 t(0, 0);
+  for (const Inst& I : b->inst) {
+    const dim3 c = dts_pass_block_counts(I, halo);
+    t.x += c.x;
+    t.y += c.y;
+  }
+  return t;
+}
+
+// The block tables of the DTS passes for a halo.  A graph that the caller has
+// captured may hold their addresses, so they stay, and are not changed, until
+// the batch is destroyed.  They are written by a kernel on the batch's stream
+// into memory set aside at creation (a few halos' worth, more is allocated
+// then): a solve with a halo of its own waits for nothing.  *fresh: written now.
+int ensure_pass_blocks(dtsgb_batch_t b, int halo, bool* fresh) {
+  *fresh = false;
+  if (b->n == 1 || b->pass.count(halo)) return DTSGB_OK;
   cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
   DTSGB_CUDA(cudaStreamIsCapturing(b->stream, &c));
   if (c != cudaStreamCaptureStatusNone) return DTSGB_OK;  // a launch per instance then
-  DTSGB_CUDA(cudaStreamSynchronize(b->stream));  // a solve may still read them
-  drop_graph(b, b->g_dts);
-  drop_graph(b, b->g_bwd);
-  dfree(b->d_px);
-  dfree(b->d_py);
-  b->pass_halo = -1;
-  std::vector<Tile> x, y;
-  dts_pass_blocks(b->inst.data(), b->n, halo, &x, &y);
-  if (int st = dalloc(&b->d_px, x.size())) return st;
-  if (int st = dalloc(&b->d_py, y.size())) return st;
-  DTSGB_CUDA(upload_table(b->d_px, x.data(), x.size() * sizeof(Tile)));
-  DTSGB_CUDA(upload_table(b->d_py, y.data(), y.size() * sizeof(Tile)));
-  b->npx = (int)x.size();
-  b->npy = (int)y.size();
-  b->pass_halo = halo;
+  const dim3 n = pass_block_totals(b, halo);
+  const size_t need = (size_t)n.x + n.y;
+  if (need > b->pass_left) {
+    const size_t room = std::max(need, b->pass_room);
+    Tile* p = nullptr;
+    const cudaError_t e = cudaMalloc((void**)&p, room * sizeof(Tile));
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      return e == cudaErrorMemoryAllocation
+                 ? fail(DTSGB_ERR_OUT_OF_MEMORY, "cudaMalloc: out of memory")
+                 : cuda_fail(e, "cudaMalloc");
+    }
+    b->pass_mem.push_back(p);
+    b->pass_room = b->pass_left = room;
+  }
+  dtsgb_batch_s::PassTables t;
+  t.x = b->pass_mem.back() + (b->pass_room - b->pass_left);
+  t.y = t.x + n.x;
+  t.nx = n.x;
+  t.ny = n.y;
+  if (int st = launch_pass_blocks(b->d_inst, b->inst.data(), b->n, halo, t.x, t.y, b->stream))
+    return st;
+  b->pass_left -= need;
+  b->pass[halo] = t;
+  *fresh = true;
   return DTSGB_OK;
 }
 DtsLaunch iter_launch(dtsgb_batch_t b, int halo) {
   DtsLaunch L{b->d_inst, nullptr, 0, b->n, false, nullptr, 0, b->inst.data()};
-  if (b->pass_halo != halo) return L;
-  L.d_xblocks = b->d_px;
-  L.d_yblocks = b->d_py;
-  L.n_xblocks = (unsigned)b->npx;
-  L.n_yblocks = (unsigned)b->npy;
+  const auto t = b->pass.find(halo);
+  if (t == b->pass.end()) return L;
+  L.d_xblocks = t->second.x;
+  L.d_yblocks = t->second.y;
+  L.n_xblocks = t->second.nx;
+  L.n_yblocks = t->second.ny;
   return L;
 }
 
@@ -852,6 +885,16 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
   if (!st) st = dalloc(&b->d_inst, (size_t)n);
   if (!st) st = dalloc(&b->d_hinst, (size_t)n);
   if (!st) st = dalloc(&b->d_soff, (size_t)n);
+  if (!st && n > 1) {
+    // room for four halos' block tables (16 bytes a block of some 1000 pixels)
+    for (int halo : {8, 30, 64, 253}) {
+      const dim3 t = pass_block_totals(b, halo);
+      b->pass_room = std::max(b->pass_room, 4 * ((size_t)t.x + t.y));
+    }
+    b->pass_mem.push_back(nullptr);
+    st = dalloc(&b->pass_mem.back(), b->pass_room);
+    b->pass_left = b->pass_room;
+  }
   if (!st) {
     e = upload_table(b->d_inst, b->inst.data(), n * sizeof(Inst));
     if (e == cudaSuccess)
@@ -944,8 +987,9 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
   const float rx = f->sigma_x / f->sigma_r, ry = f->sigma_y / f->sigma_r;
   const int halo = (int)std::floor(p->sigma_z);
   const bool iterate = p->loss != DTSGB_L1 && p->num_iterations > 0;
+  bool fresh = false;
   if (iterate)
-    if (int st = ensure_pass_blocks(b, halo)) return st;
+    if (int st = ensure_pass_blocks(b, halo, &fresh)) return st;
   const DtsLaunch Li = iter_launch(b, halo);
   const bool over = overwrite > 0.f && overwrite < 1.f;
   const int n_kept = iterate ? p->num_iterations : 0;
@@ -970,7 +1014,9 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
     if (st) return st;
   }
   const dtsgb_batch_s::BoundsKey bk{b->guide_gen, rx, ry, p->sigma_z, b->ref_y};
-  const bool keep_bounds = b->reuse && std::memcmp(&bk, &b->bkey, sizeof bk) == 0;
+  // (the passes are dependent launches that read their block before they wait:
+  // with new tables the bounds pass, a plain launch, comes in between)
+  const bool keep_bounds = b->reuse && !fresh && std::memcmp(&bk, &b->bkey, sizeof bk) == 0;
   auto bounds = [&]() -> int {
     if (keep_bounds) return DTSGB_OK;  // same guide and sigmas: windows unchanged
     return launch_bounds(Li, b->guide, b->bounds, rx, ry, p->sigma_z, p->sigma_z,

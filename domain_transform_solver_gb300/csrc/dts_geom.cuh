@@ -62,7 +62,7 @@ struct XPrefix {
 };
 
 // The passes' grids over a launch's instances (one instance: from its size;
-// several: the block tables of dts_pass_blocks for this halo), and the rounds
+// several: the block tables of launch_pass_blocks for this halo), and the rounds
 // and staged rows of the largest.
 struct PassGrid {
   dim3 x, y;

@@ -26,7 +26,6 @@
 // the gap only in part.
 #include <algorithm>
 #include <cmath>
-#include <vector>
 
 #include "../../include/dtsgb.h"
 #include "dts_geom.cuh"
@@ -401,6 +400,24 @@ __global__ void __launch_bounds__(RM == 32 ? 768 : 512, RM == 8 ? 3 : RM == 16 ?
   }
 }
 
+// The block tables of several instances: instance blockIdx.y's blocks in rows,
+// from the starts that the host has added up.
+constexpr int kBlockStarts = 128;
+struct BlockStarts {
+  int x[kBlockStarts + 1], y[kBlockStarts + 1];
+};
+__global__ void __launch_bounds__(256)
+    k_pass_blocks(const Inst* __restrict__ insts, int first,
+                  const __grid_constant__ BlockStarts S, int halo, Tile* __restrict__ x,
+                  Tile* __restrict__ y) {
+  const int i = blockIdx.y, e = blockIdx.x * 256 + threadIdx.x;
+  const Inst in = insts[first + i];
+  const int tw = x_geom(in.w, in.h, halo).tw;
+  const int xc = (in.w + tw - 1) / tw, yc = (in.w + 31) / 32;
+  if (e < S.x[i + 1] - S.x[i]) x[S.x[i] + e] = Tile{first + i, e % xc, e / xc, 0};
+  if (e < S.y[i + 1] - S.y[i]) y[S.y[i] + e] = Tile{first + i, e % yc, e / yc, 0};
+}
+
 template <typename K>
 int set_smem(K* f, size_t bytes) {
   if (bytes > 48 * 1024)
@@ -509,17 +526,34 @@ PassGrid pass_grid(const DtsLaunch& L, int hx, int hy) {
   return G;
 }
 
-void dts_pass_blocks(const Inst* inst, int n, int halo, std::vector<Tile>* x,
-                     std::vector<Tile>* y) {
-  x->clear();
-  y->clear();
-  for (int i = 0; i < n; ++i) {
-    const int w = inst[i].w, h = inst[i].h, tw = x_geom(w, h, halo).tw, th = y_th(w, h, halo);
-    for (int r = 0; r * kXWarps < h; ++r)
-      for (int c = 0; c * tw < w; ++c) x->push_back(Tile{i, c, r, 0});
-    for (int r = 0; r * th < h; ++r)
-      for (int c = 0; c * 32 < w; ++c) y->push_back(Tile{i, c, r, 0});
+dim3 dts_pass_block_counts(const Inst& I, int halo) {
+  const int tw = x_geom(I.w, I.h, halo).tw, th = y_th(I.w, I.h, halo);
+  const unsigned xr = (I.h + kXWarps - 1) / kXWarps, xc = (I.w + tw - 1) / tw;
+  const unsigned yr = (I.h + th - 1) / th, yc = (I.w + 31) / 32;
+  return dim3(xr * xc, yr * yc);
+}
+
+int launch_pass_blocks(const Inst* d_inst, const Inst* h_inst, int n, int halo, Tile* x, Tile* y,
+                       cudaStream_t s) {
+  int nx = 0, ny = 0;
+  for (int first = 0; first < n; first += kBlockStarts) {
+    const int m = std::min(kBlockStarts, n - first);
+    BlockStarts S = {};
+    unsigned most = 1;
+    for (int i = 0; i < m; ++i) {
+      const dim3 c = dts_pass_block_counts(h_inst[first + i], halo);
+      S.x[i] = nx;
+      S.y[i] = ny;
+      nx += c.x;
+      ny += c.y;
+      most = std::max(most, std::max(c.x, c.y));
+    }
+    S.x[m] = nx;
+    S.y[m] = ny;
+    k_pass_blocks<<<dim3((most + 255) / 256, m), 256, 0, s>>>(d_inst, first, S, halo, x, y);
+    DTSGB_CUDA(cudaGetLastError());
   }
+  return DTSGB_OK;
 }
 
 int launch_dts_iter(const DtsLaunch& L, Storage st, IterMode mode, const float* vin, float* tmp,

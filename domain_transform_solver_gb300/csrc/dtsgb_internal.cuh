@@ -7,7 +7,6 @@
 #include <stdint.h>
 
 #include <string>
-#include <vector>
 
 namespace dtsgb {
 
@@ -205,7 +204,7 @@ struct DtsLaunch {
   int n_tiles_small = 0;
   const Inst* h_inst = nullptr;  // host copy of the instance table
   // several instances: the blocks of the passes (bounds, iteration) for the halo
-  // (dts_pass_blocks)
+  // (launch_pass_blocks)
   const Tile *d_xblocks = nullptr, *d_yblocks = nullptr;
   unsigned n_xblocks = 0, n_yblocks = 0;
   // no block tables (first solve under a capture): one instance after the other
@@ -258,10 +257,11 @@ struct StereoArgs {
   float offset, lam_p, alpha, ratio;
 };
 
-// The blocks of the X and the Y pass over n instances: (instance, column
-// block, row block).
-void dts_pass_blocks(const Inst* inst, int n, int halo, std::vector<Tile>* x,
-                     std::vector<Tile>* y);
+// Blocks of the X (.x) and the Y pass (.y) over an instance, and the tables of
+// those over n instances, (instance, column block, row block), written on s.
+dim3 dts_pass_block_counts(const Inst& I, int halo);
+int launch_pass_blocks(const Inst* d_inst, const Inst* h_inst, int n, int halo, Tile* x, Tile* y,
+                       cudaStream_t s);
 // One iteration from vin to vout through tmp (the X results): vout may be vin,
 // tmp neither.  L: the instance tables on the device and the host.  feeds:
 // another iteration reads vout, so with overwrite in (0, 1) it holds the

@@ -431,3 +431,82 @@ def test_first_solve_of_a_batch_under_a_capture(gpu_ready):
     torch.cuda.synchronize()
     for a, o in zip(want, out):
         assert np.array_equal(a, o.cpu().numpy())
+
+
+# ---- block tables of a batch: per halo, for the batch's life --------------------
+def _batch_on_a_stream(D, sizes, seed=5):
+    """A batch without graphs of its own on a stream, its inputs on host and device."""
+    import torch
+    rng = np.random.default_rng(seed)
+    host = ([rng.integers(0, 256, (h, w, 4)).astype(np.uint8) for w, h in sizes],
+            [rng.normal(0, 1, (h, w)).astype(np.float32) for w, h in sizes],
+            [rng.random((h, w)).astype(np.float32) for w, h in sizes])
+    b = D.Batch(sizes, use_graphs=False)
+    stream = torch.cuda.Stream()
+    b.set_stream(stream.cuda_stream)
+    dev = [[torch.from_numpy(a).cuda() for a in x] for x in host]
+    torch.cuda.synchronize()
+    return b, stream, host, dev
+
+
+def _dts_op(D, sigma_z, n=3):
+    return D.DomainOptimizeParams(num_iterations=n, loss=1, sigma_z=sigma_z)
+
+
+@pytest.mark.parametrize("grad", [0, 1])
+def test_a_callers_graph_outlives_solves_at_other_sigmas(gpu_ready, grad):
+    """Captured after a solve at its own sigma, replayed after solves at more
+    sigmas than the batch sets memory aside for: the same bits."""
+    import torch
+    D = gpu_ready
+    sizes = [(90, 60), (33, 140), (401, 77)]
+    b, stream, host, dev = _batch_on_a_stream(D, sizes)
+    fp = D.DomainFilterParams(sigma_x=8.0, sigma_y=8.0, sigma_r=4.0)
+    ptrs = [[a.data_ptr() for a in x] for x in dev]
+    out = [[torch.full((h, w), -1.0, device="cuda") for w, h in sizes] for _ in range(3)]
+    optr = [[o.data_ptr() for o in x] for x in out]
+    b.enable_grad(bool(grad), 2)
+
+    def work(sigma):
+        b.upload_device(D.COLOR_SPACE.YCbCr, *ptrs)
+        b.solve_dts(fp, _dts_op(D, sigma))
+        b.download_device(0, optr[0])
+        if grad:
+            b.backward_device(ptrs[2], optr[1], optr[2])
+    work(8.0)
+    torch.cuda.synchronize()
+    want = [o.cpu().numpy() for x in out for o in x]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+        work(8.0)
+    for sigma in (30.0, *np.linspace(1.5, 75.5, 38)):
+        work(float(sigma))
+    torch.cuda.synchronize()
+    other = [o.cpu().numpy() for x in out for o in x]
+    assert not np.array_equal(other[0], want[0])
+    torch.cuda.empty_cache()
+    graph.replay()
+    torch.cuda.synchronize()
+    for a, o in zip(want, (o for x in out for o in x)):
+        assert np.array_equal(a, o.cpu().numpy())
+
+
+def test_a_solve_at_a_new_sigma_waits_for_nothing(gpu_ready):
+    """The first solve of a batch, and one at another sigma, behind work that
+    takes a while on the batch's stream."""
+    import torch
+    D = gpu_ready
+    sizes = [(90, 60), (33, 140), (401, 77)]
+    fp = D.DomainFilterParams()
+    for warm in (1, 0):  # (a kernel's first launch in the process may wait)
+        b, stream, host, dev = _batch_on_a_stream(D, sizes)
+        b.upload(D.COLOR_SPACE.YCbCr, *host)
+        for sigma in (8.0, 30.0, 64.0, 8.0):
+            if not warm:
+                with torch.cuda.stream(stream):
+                    torch.cuda._sleep(200_000_000)  # 0.1 s
+                    done = stream.record_event()
+            b.solve_dts(fp, _dts_op(D, sigma))
+            if not warm:
+                assert not done.query(), sigma
+            torch.cuda.synchronize()
