@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(RM == 32 ? 768 : 512, RM == 8 ? 3 : RM == 16 ?
   }
   float m = 0.f;
 #pragma unroll
-  for (int k = 0; k < RM; ++k) m = fmaxf(m, fabsf(v[k] * rtab[(b[k] & 0xff) + (b[k] >> 8)]));
+  for (int k = 0; k < RM; ++k) m = fmaxf(m, fabsf(v[k] * rtab[window_count(b[k], hy)]));
   m = warp_max_nonneg(m);
   if (lane == 0) atomicMax(smax, __float_as_uint(m));
   asm volatile("bar.sync 1, %0;" ::"r"(live) : "memory");
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(RM == 32 ? 768 : 512, RM == 8 ? 3 : RM == 16 ?
   for (int k = 0; k < RM; ++k) {
     if (b[k]) {  // (a window holds its pixel: 0 is outside the image)
       const int dl = (int)(b[k] & 0xff), du = (int)(b[k] >> 8);
-      const unsigned A = fx_from(v[k] * rtab[dl + du], sF);
+      const unsigned A = fx_from(v[k] * rtab[window_count(b[k], hy)], sF);
       atomicAdd(D + max(s0 + k - dl + 1, 0) * 32 + lane, A);
       atomicAdd(D + min(s0 + k + du + 1, rows) * 32 + lane, 0u - A);
     }
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(32 * kXWarps, NR <= 4 ? 7 : 4)
   Q.tv.zero();
   Q.cv.zero();
   // n of a pixel of its packed bounds (0 outside the image: 1/n = 0)
-  auto count = [](uint32_t w) { return (w & 0xff) + ((w >> 8) & 0xff); };
+  auto count = [hx](uint32_t w) { return window_count(w, hx); };
   float m = 0.f;
 #pragma unroll
   for (int r = 0; r < NR; ++r)
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(32 * kXWarps, NR <= 4 ? 7 : 4)
         if (w) {
           const int dl = (int)(w & 0xff), du = (int)((w >> 8) & 0xff);
           const int i = 4 * lane + 128 * r + k;
-          const unsigned A = fx_from(f4_get(v[r], k) * rtab[dl + du], sF);
+          const unsigned A = fx_from(f4_get(v[r], k) * rtab[count(w)], sF);
           atomicAdd(PX::entry(Sb, max(i - dl + 1, 0)), A);
           atomicAdd(PX::entry(Sb, min(i + du + 1, end)), 0u - A);
         }

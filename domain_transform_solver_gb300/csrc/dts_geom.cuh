@@ -61,6 +61,19 @@ struct XPrefix {
   }
 };
 
+// A window's radii from the low byte of a packed word, held to the staged halo:
+// whatever the plane holds, no window reads outside its tile.
+__device__ __forceinline__ int radius_l(unsigned b, int halo) {
+  return min((int)(b & 0xff), halo + 1);
+}
+__device__ __forceinline__ int radius_u(unsigned b, int halo) {
+  return min((int)(b & 0xff), halo);
+}
+// Its pixels, dl + du from the low two bytes, for the table of 1/n alone.
+__device__ __forceinline__ int window_count(unsigned b, int halo) {
+  return min((int)((b & 0xff) + ((b >> 8) & 0xff)), 2 * halo + 1);
+}
+
 // The passes' grids over a launch's instances (one instance: from its size;
 // several: the block tables of launch_pass_blocks for this halo), and the rounds
 // and staged rows of the largest.

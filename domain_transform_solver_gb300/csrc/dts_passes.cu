@@ -91,7 +91,8 @@ __device__ __forceinline__ bool finite_bits(float v) { return mag_bits(v) < kNon
 // launch_iter).  Warps are independent.
 //
 // The window ends come from dts_bounds.cu for the same sigma (dl <= hx + 1, du <=
-// hx), so a prefix index never leaves the staged columns.
+// hx).  The caller's graphs may leave another sigma's in the plane: radius_l and
+// radius_u keep a prefix index within the staged columns then too.
 //
 // A non-finite value in the segment has no fixed-point form: the warp then
 // adds its windows in float, pixel by pixel, and every result that is not
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(32 * kXWarps, AHEAD ? 1 : 10)
     __syncwarp();
     for (int x = x0 + lane; x < xe; x += 32) {
       const uint32_t b = __ldg(bnd + base + x);
-      const int dl = (int)(b & 0xff), du = (int)((b >> 8) & 0xff), t = x - x0 + g.ha;
+      const int dl = radius_l(b, hx), du = radius_u(b >> 8, hx), t = x - x0 + g.ha;
       float B = 0.f;
       for (int j = t - dl + 1; j <= t + du; ++j) B += __uint_as_float(PX::at(Sb, j));
       const float rn = rtab[dl + du], vv = __uint_as_float(PX::at(Sb, t));
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(32 * kXWarps, AHEAD ? 1 : 10)
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const uint32_t b = u4_get(q.b, k);
-          const int dl = (int)(b & 0xff), du = (int)((b >> 8) & 0xff);
+          const int dl = radius_l(b, hx), du = radius_u(b >> 8, hx);
           const float rn = rtab[dl + du];
           const float vv = f4_get(v[r], k), tv = q.tv[k], cv = q.cv[k];
           const float B =
@@ -353,7 +354,7 @@ __global__ void __launch_bounds__(RM == 32 ? 768 : 512, RM == 8 ? 3 : RM == 16 ?
       if (!inx || (unsigned)j >= (unsigned)jm) continue;
       const long long p = first + (long long)k * P;
       const uint32_t bb = __ldg(bnd + p) >> 16;
-      const int dl = (int)(bb & 0xff), du = (int)(bb >> 8);
+      const int dl = radius_l(bb, hy), du = radius_u(bb >> 8, hy);
       float B = 0.f;
       for (int q = k - dl + 1; q <= k + du; ++q) B += __uint_as_float(Sw[q * 32]);
       const float vv = __uint_as_float(Sw[k * 32]);
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(RM == 32 ? 768 : 512, RM == 8 ? 3 : RM == 16 ?
   for (int k = 0; k < RM; ++k) {
     if (k >= k0 && k < k1) {
       const uint32_t bk = kEarly ? b[kEarly ? k : 0] : __ldg(bc + (long long)k * P);
-      const int dl = (int)((bk >> 16) & 0xff), du = (int)(bk >> 24);
+      const int dl = radius_l(bk >> 16, hy), du = radius_u(bk >> 24, hy);
       const unsigned hi = *reinterpret_cast<const unsigned*>(Sc + du * 128 + k * 128);
       const unsigned lo = *reinterpret_cast<const unsigned*>(Sc - dl * 128 + k * 128);
       const float rn = *reinterpret_cast<const float*>(rt + (dl + du) * 4);

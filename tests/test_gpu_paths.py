@@ -510,3 +510,55 @@ def test_a_solve_at_a_new_sigma_waits_for_nothing(gpu_ready):
             if not warm:
                 assert not done.query(), sigma
             torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("sizes", [[(400, 300)], [(90, 60), (333, 140)], [(700, 900)]])
+def test_windows_wider_than_a_pass_stages_are_held_to_it(gpu_ready, oracle_mod, sizes):
+    """A caller's graph that has kept its bounds finds another sigma's in the
+    plane: the passes use those windows as far as their own sigma reaches (the
+    FP64 oracle with the windows cut there, parity bar), and the adjoint stays
+    in its tiles."""
+    import torch
+    D, O = gpu_ready, oracle_mod
+    b, stream, host, dev = _batch_on_a_stream(D, sizes)
+    rng = np.random.default_rng(3)
+    for g, d in zip(host[0], dev[0]):  # flat blocks: windows as wide as sigma allows
+        g[:] = np.kron(rng.integers(0, 256, (g.shape[0] // 50 + 1, g.shape[1] // 70 + 1, 1)),
+                       np.ones((50, 70, 1)))[:g.shape[0], :g.shape[1]].astype(np.uint8)
+        d.copy_(torch.from_numpy(g))
+    torch.cuda.synchronize()
+    fp = D.DomainFilterParams(sigma_x=8.0, sigma_y=8.0, sigma_r=4.0)
+    ptrs = [[a.data_ptr() for a in x] for x in dev]
+    out = [torch.full((h, w), -1.0, device="cuda") for w, h in sizes]
+    gt, gc = ([torch.full((h, w), -1.0, device="cuda") for w, h in sizes] for _ in range(2))
+    b.enable_grad(True, 2)
+    b.upload_device(D.COLOR_SPACE.RGB, *ptrs)
+
+    def solve(sigma):
+        b.solve_dts(fp, _dts_op(D, sigma))
+        b.download_device(0, [o.data_ptr() for o in out])
+        b.backward_device(ptrs[2], [o.data_ptr() for o in gt], [o.data_ptr() for o in gc])
+    solve(8.0)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+        solve(8.0)  # (the guide is unchanged: no bounds pass in it)
+    solve(40.0)
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    for (w, h), g, t, c, o in zip(sizes, *host, out):
+        s = D.DomainTransformSolver(D.ImageDim(w, h))
+        s.InitFrame(D.COLOR_SPACE.RGB, g, t, c)
+        s.ComputeColorSpaceDifferential(fp)
+        win = {}
+        for axis in (0, 1):
+            lo, hi = s.DebugBounds(axis, 40.0)
+            pos = np.arange(w)[None, :] if axis == 0 else np.arange(h)[:, None]
+            assert (hi - pos).max() > 8 and (pos - lo).max() > 9
+            win[(axis, 8.0)] = np.maximum(lo, pos - 9), np.minimum(hi, pos + 8)
+        ref, _ = O.dts_solve(g, t, c, 0, dict(sigma_x=8.0, sigma_y=8.0, sigma_r=4.0),
+                             dict(num_iterations=3, loss=1, lambda_=1.0, sigma_z=8.0,
+                                  step_size=0.99), overrides=win)
+        assert np.abs(o.cpu().numpy() - ref).max() <= P.TOL_REL * P.target_range(t)
+    assert all(torch.isfinite(x).all() for x in gt + gc)
