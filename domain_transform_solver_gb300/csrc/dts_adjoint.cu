@@ -301,8 +301,7 @@ int launch_y(const DtsLaunch& L, const PassGrid& G, const float* gin, float* gou
   const int warps = G.rows / RM;
   const size_t smem = sizeof(unsigned) *
                       ((size_t)(2 * hy + 3) + warps * 32 + ((size_t)G.rows + 1) * 32);
-  if (smem > 48 * 1024)
-    DTSGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DTSGB_CUDA(allow_smem(kern, smem));
   ProfScope ps(s, DTSGB_K_DTS_ADJOINT);
   DTSGB_CUDA(launch_dependent(kern, G.y, dim3(32 * warps), smem, s, L.d_inst, gin, gout, bounds,
                               slam, hy, L.n_inst > 1 ? L.d_yblocks : (const Tile*)nullptr));

@@ -242,8 +242,7 @@ int launch_y(const DtsLaunch& L, const PassGrid& G, const uchar4* guide, uint32_
   auto kern = k_bounds_y<RM>;
   const int warps = G.rows / RM;
   const size_t smem = sizeof(unsigned) * 32 * (size_t)(warps + G.rows);
-  if (smem > 48 * 1024)
-    DTSGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DTSGB_CUDA(allow_smem(kern, smem));
   DTSGB_CUDA(launch_dependent(kern, G.y, dim3(32 * warps), smem, s, L.d_inst, guide, bounds, wt,
                               hy, ref_y_limit, L.n_inst > 1 ? L.d_yblocks : (const Tile*)nullptr));
   return DTSGB_OK;

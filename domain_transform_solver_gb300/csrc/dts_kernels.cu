@@ -231,17 +231,6 @@ int grid_for(long long n, int threads = kThreads) {
   return (int)b;
 }
 
-template <typename F>
-int set_smem(F* f, size_t bytes) {
-  if (bytes > 48 * 1024) {
-    DTSGB_CUDA(cudaFuncSetAttribute(
-        f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  }
-  return DTSGB_OK;
-}
-
-constexpr size_t kMaxSmem = 227 * 1024;
-
 }  // namespace
 
 int launch_color_convert_flat(uchar4* guide, long long n, int color_space,
@@ -317,8 +306,7 @@ static int launch_filter_shape(const DtsLaunch& L, const float* in0,
   const size_t smem = NCH * sizeof(float) *
                       ((size_t)(TH + 2 * hy) * (TW + 2 * hx) + (size_t)(TH + 2 * hy) * TW);
   if (smem > kMaxSmem) return fail(DTSGB_ERR_UNSUPPORTED, "filter sigma too large");
-  int st = set_smem(k_filter<NCH, CONF, TS, TW, TH>, smem);
-  if (st) return st;
+  DTSGB_CUDA((allow_smem(k_filter<NCH, CONF, TS, TW, TH>, smem)));
   ProfScope ps(s, DTSGB_K_FILTER);
   k_filter<NCH, CONF, TS, TW, TH><<<L.n_tiles, kThreads, smem, s>>>(
       L.d_inst, L.d_tiles, in0, in1, out0, out1, bounds, hx, hy, (TS*)conf_out,

@@ -419,13 +419,6 @@ __global__ void __launch_bounds__(256)
   if (e < S.y[i + 1] - S.y[i]) y[S.y[i] + e] = Tile{first + i, e % yc, e / yc, 0};
 }
 
-template <typename K>
-int set_smem(K* f, size_t bytes) {
-  if (bytes > 48 * 1024)
-    DTSGB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return DTSGB_OK;
-}
-
 template <typename TS, int MODE, bool STEREO, bool OVER, int NR, bool AHEAD = true>
 int launch_x(const DtsLaunch& L, const float* vin, float* vout, const void* target,
              const void* conf, const uint32_t* bounds, float lambda, float step,
@@ -448,7 +441,7 @@ int launch_y(const DtsLaunch& L, const float* u, float* vout, const void* conf,
   const int warps = rows / RM;
   const size_t smem = sizeof(unsigned) *
                       ((size_t)(2 * hy + 3) + warps * 32 + ((size_t)rows + 1) * 32);
-  if (int st = set_smem(kern, smem)) return st;
+  DTSGB_CUDA(allow_smem(kern, smem));
   ProfScope ps(s, DTSGB_K_DTS_ITER);
   DTSGB_CUDA(launch_dependent(kern, grid, dim3(32 * warps), smem, s, L.d_inst, u, vout,
                               (const TS*)conf, bounds, slam, overwrite, feeds, hy,

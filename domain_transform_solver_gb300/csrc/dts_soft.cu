@@ -1465,8 +1465,7 @@ int launch_adjoint(dtsgb_soft_t s, const float* adiag, const float* coef, const 
                                                         val, e, aout, diff, R, lambda, H);
     } else {
       const size_t sm = sizeof(float) * 5 * (kTYR + 2 * H) * kTYC;
-      DTSGB_CUDA(cudaFuncSetAttribute(k_soft_adjoint_tile<1>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+      DTSGB_CUDA(allow_smem(k_soft_adjoint_tile<1>, sm));
       k_soft_adjoint_tile<1><<<g, dim3(kTYC, kTYT), sm, s->stream>>>(
           s->d_inst, adiag, coef, alpha, beta, val, e, aout, diff, R, lambda, H);
     }
@@ -1500,8 +1499,7 @@ int launch_adjoint_fused(dtsgb_soft_t s, const float* a, const float* Bk, const 
         step, wc, PH, flags);
   } else {
     const size_t sm = sizeof(float) * nf * (kTYR + 2 * PH) * kTYC;
-    DTSGB_CUDA(cudaFuncSetAttribute(k_soft_adjoint_fused<1>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DTSGB_CUDA(allow_smem(k_soft_adjoint_fused<1>, sm));
     k_soft_adjoint_fused<1><<<g, dim3(kTYC, kTYT), sm, s->stream>>>(
         s->d_inst, a, nplan, Bk, val, t, c, cnt, wts, aout, diff, gt, gc, data, mode, lambda,
         step, wc, PH, flags);

@@ -104,6 +104,18 @@ __device__ __forceinline__ void pdl_wait_then_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Lets a kernel be launched with `bytes` of dynamic shared memory beside
+// `statics` of its own.  What a kernel may use is state of the whole process:
+// it is always set to the most that an SM gives a block, so that a thread that
+// launches the kernel with less never takes from one that needs more.
+constexpr size_t kMaxSmem = 227 * 1024;
+template <typename K>
+inline cudaError_t allow_smem(K* kernel, size_t bytes, size_t statics = 0) {
+  if (bytes + statics <= 48 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(kMaxSmem - statics));
+}
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block,
                                     size_t smem, cudaStream_t s, Args... args) {

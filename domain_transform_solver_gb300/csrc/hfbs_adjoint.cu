@@ -310,9 +310,7 @@ int hfbs_enqueue_backward(const HfbsBatch& B, const HParams& p, const float* gou
   // overwrites it)
   k_hb_slice_scale<<<gp, kA, 0, s>>>(B.d_inst, B.guide, B.count, B.ovf, gout, sp, p);
   const size_t hsmem = sizeof(float) * (size_t)(B.max_gl + 2) * kGatherThreads;
-  if (hsmem > 48 * 1024)
-    DTSGB_CUDA(cudaFuncSetAttribute(k_hb_slice_gather,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem));
+  DTSGB_CUDA(allow_smem(k_hb_slice_gather, hsmem));
   const dim3 gcol((unsigned)((B.max_cells + kGatherCols - 1) / kGatherCols), ni);
   k_hb_slice_gather<<<gcol, kGatherThreads, hsmem, s>>>(B.d_inst, B.guide, sp, B.count, G.gz,
                                                         p);

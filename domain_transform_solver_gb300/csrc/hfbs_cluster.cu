@@ -46,7 +46,6 @@ __host__ __device__ constexpr int max_threads(int ipt) {
 __host__ __device__ constexpr int adj_threads(int ipt) { return ipt == 1 ? 704 : 640; }
 constexpr int kAdjItems = 2;
 constexpr int kCItems = 4;
-constexpr size_t kMaxSmem = 227 * 1024;
 
 struct ClusterArgs {
   const float *z, *h, *n, *b, *a;  // normalisation: n the counts
@@ -395,8 +394,7 @@ __global__ void __launch_bounds__(adj_threads(IPT), 1)
 template <typename F, typename Args>
 cudaError_t launch_cluster(F* kern, const HfbsBatch& B, const HfbsClusterPlan& P, const Args& A,
                            cudaStream_t s, int* clusters) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)P.smem);
+  cudaError_t e = allow_smem(kern, P.smem);
   if (e == cudaSuccess && P.size > 8)
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;

@@ -828,6 +828,7 @@ int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s,
   const dim3 gp((unsigned)std::min<long long>((max_h + 7) / 8, 4096), ni);
   const dim3 gc((B.max_cells + 63) / 64, ni);
   const size_t splat_smem = sizeof(float) * 3 * (size_t)B.max_gl * 64;
+  const size_t lbin_smem = sizeof(int) * 256;  // k_splat's luma table
   // a CTA per cell for large ones (k_splat_cell holds a bin per thread)
   const bool by_cell = (double)p.sigma_x * (double)p.sigma_y >= kSplatCellPx &&
                        B.max_gl < kSplatCellT;
@@ -842,18 +843,12 @@ int hfbs_enqueue_solve(const HfbsBatch& B, const HParams& p, cudaStream_t s,
         B.d_inst, B.guide, (const __nv_bfloat16*)B.target, (const __nv_bfloat16*)B.conf,
         B.count, B.csum, B.b, B.ovf, p);
   } else if (B.st == Storage::F32) {
-    if (splat_smem + sizeof(int) * 256 > 48 * 1024)  // plus the static luma table
-      DTSGB_CUDA(cudaFuncSetAttribute(k_splat<float>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)splat_smem));
+    DTSGB_CUDA(allow_smem(k_splat<float>, splat_smem, lbin_smem));
     k_splat<float><<<gc, 64, splat_smem, s>>>(
         B.d_inst, B.guide, (const float*)B.target, (const float*)B.conf, B.count,
         B.csum, B.b, B.ovf, p);
   } else {
-    if (splat_smem + sizeof(int) * 256 > 48 * 1024)  // plus the static luma table
-      DTSGB_CUDA(cudaFuncSetAttribute(k_splat<__nv_bfloat16>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)splat_smem));
+    DTSGB_CUDA(allow_smem(k_splat<__nv_bfloat16>, splat_smem, lbin_smem));
     k_splat<__nv_bfloat16><<<gc, 64, splat_smem, s>>>(
         B.d_inst, B.guide, (const __nv_bfloat16*)B.target,
         (const __nv_bfloat16*)B.conf, B.count, B.csum, B.b, B.ovf, p);

@@ -313,7 +313,7 @@ int launch(const HfbsBatch& B, const HfbsMarchPlan& P, const MarchArgs& A, const
            cudaStream_t s) {
   const size_t smem = smem_bytes<MODE, K, D>(P.warps);
   auto kern = k_hfbs_march<MODE, REC, K, D>;
-  DTSGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DTSGB_CUDA(allow_smem(kern, smem));
   DTSGB_CUDA(launch_dependent(kern, dim3(P.blocks, P.count), dim3(P.warps * 32), smem, s,
                               B.d_inst + P.first, A, m));
   return DTSGB_OK;
@@ -378,7 +378,7 @@ HfbsMarchPlan hfbs_march_plan(const HfbsBatch& B, int first, int count) {
   int max_gy = 1;
   for (int i = 0; i < count; ++i) max_gy = std::max(max_gy, B.h_inst[first + i].gy);
   // SMs and blocks an SM holds (128 registers a thread; shared memory)
-  constexpr int sms = 152, sm_smem = 228 * 1024, most_smem = 227 * 1024;
+  constexpr int sms = 152, sm_smem = 228 * 1024;
   const int smem = (int)smem_bytes<kHeavyBall, K, 1>(P.warps) + 1024;
   const int per_sm = std::max(1, std::min(16 / P.warps, sm_smem / smem));
   const double latency = 600.0, issue = 30.0 * K * P.warps;
@@ -409,7 +409,7 @@ HfbsMarchPlan hfbs_march_plan(const HfbsBatch& B, int first, int count) {
       blocks = total;
     }
   }
-  P.ahead = blocks <= 2 * sms && smem_bytes<kHeavyBall, K, kAhead>(P.warps) <= most_smem ? kAhead : 1;
+  P.ahead = blocks <= 2 * sms && smem_bytes<kHeavyBall, K, kAhead>(P.warps) <= kMaxSmem ? kAhead : 1;
   return P;
 }
 

@@ -257,11 +257,9 @@ extern "C" DTSGB_API int dtsgb_dts_solve_noalloc(
   const size_t smem_b = sizeof(float) * 2 * (size_t)kNaTile * (kNaTile + 2 * r - 1);
   const size_t smem_i = sizeof(float) * ((size_t)(kNaTile + 2 * hx) * (kNaTile + 2 * hx) +
                                          (size_t)(kNaTile + 2 * hx) * kNaTile);
-  if (smem_b > 227 * 1024 || smem_i > 227 * 1024)
+  if (smem_b > kMaxSmem || smem_i > kMaxSmem)
     return fail(DTSGB_ERR_UNSUPPORTED, "sigma_z too large for the no-alloc kernels");
-  if (smem_b > 48 * 1024)
-    DTSGB_CUDA(cudaFuncSetAttribute(k_na_bounds, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem_b));
+  DTSGB_CUDA(allow_smem(k_na_bounds, smem_b));
   const float rx = filter->sigma_x / filter->sigma_r, ry = filter->sigma_y / filter->sigma_r;
   k_na_bounds<<<tiles, kNaThreads, smem_b, s>>>((const uchar4*)rgba, width, height,
                                                 color_space, rx, ry, sz, r, 1, bounds);
@@ -273,18 +271,12 @@ extern "C" DTSGB_API int dtsgb_dts_solve_noalloc(
   for (int k = 0; k < N; ++k) {
     float* dst = ((N - 1 - k) % 2 == 0) ? output : iterate;
     if (optimize->loss == DTSGB_L2) {
-      if (smem_i > 48 * 1024)
-        DTSGB_CUDA(cudaFuncSetAttribute(k_na_iter<0>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem_i));
+      DTSGB_CUDA(allow_smem(k_na_iter<0>, smem_i));
       k_na_iter<0><<<tiles, kNaThreads, smem_i, s>>>(src, dst, target, confidence, bounds,
                                                      width, height, optimize->lambda,
                                                      optimize->step_size, overwrite, hx);
     } else {
-      if (smem_i > 48 * 1024)
-        DTSGB_CUDA(cudaFuncSetAttribute(k_na_iter<1>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem_i));
+      DTSGB_CUDA(allow_smem(k_na_iter<1>, smem_i));
       k_na_iter<1><<<tiles, kNaThreads, smem_i, s>>>(src, dst, target, confidence, bounds,
                                                      width, height, optimize->lambda,
                                                      optimize->step_size, overwrite, hx);

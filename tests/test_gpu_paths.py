@@ -562,3 +562,52 @@ def test_windows_wider_than_a_pass_stages_are_held_to_it(gpu_ready, oracle_mod, 
                                   step_size=0.99), overrides=win)
         assert np.abs(o.cpu().numpy() - ref).max() <= P.TOL_REL * P.target_range(t)
     assert all(torch.isfinite(x).all() for x in gt + gc)
+
+
+# ---- shared memory beyond 48 KB: threads whose launches of a kernel differ -------
+@pytest.mark.parametrize("kind,sizes", [
+    ("hfbs", [(512, 512, 16.0), (100, 80, 16.0), (60, 50, 16.0)]),      # clusters
+    ("hfbs", [(1200, 1000, 4.0), (1200, 1000, 17.0), (1200, 1000, 8.0)]),  # marches
+    ("hfbs", [(512, 512, 2.0), (60, 50, 1.0), (512, 512, 3.0)]),        # splats of many levels
+    ("dts", [(900, 700, 60.0), (900, 700, 100.0), (900, 700, 253.0)]),  # Y passes
+])
+def test_threads_with_launches_of_other_sizes(gpu_ready, kind, sizes):
+    """A solver in each thread; every result is the one it has alone."""
+    import threading
+    D = gpu_ready
+    solvers, runs = [], []
+    for w, h, s in sizes:
+        rng = np.random.default_rng(w)
+        frame = (rng.integers(0, 256, (h, w, 4)).astype(np.uint8),
+                 rng.normal(0, 1, (h, w)).astype(np.float32), rng.random((h, w)).astype(np.float32))
+        if kind == "hfbs":
+            v = D.HFBS(D.ImageDim(w, h), -(-w // 8), -(-h // 8), int(np.ceil(255 / s)))
+            v.SetFilterParams(D.HFBSGridParams(sigma_x=8.0, sigma_y=8.0, sigma_l=s,
+                                               bistoch_iter_max=2, optim_iter_max=2))
+            v.InitFrame(D.COLOR_SPACE.RGB, *frame)
+            runs.append(v.Optimize)
+        else:
+            v = D.DomainTransformSolver(D.ImageDim(w, h))
+            v.InitFrame(D.COLOR_SPACE.RGB, *frame)
+            v.ComputeColorSpaceDifferential(D.DomainFilterParams())
+            runs.append(lambda v=v, s=s: v.Optimize(_dts_op(D, s, 10)))
+        solvers.append(v)
+    want, errors = [], []
+    for v, run in zip(solvers, runs):
+        run()
+        want.append(v.Download(D.ImageType.OPTIMIZED_QUANTITY))
+
+    def loop(run):
+        try:
+            for _ in range(300):
+                run()
+        except D.DtsgbError as e:
+            errors.append(e)
+    threads = [threading.Thread(target=loop, args=(r,)) for r in runs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for v, a in zip(solvers, want):
+        assert np.array_equal(v.Download(D.ImageType.OPTIMIZED_QUANTITY), a, equal_nan=True)
