@@ -55,11 +55,11 @@ template <int STRIDE, int N, typename AT>
 __device__ __forceinline__ void window_ends(int h, int T, AT&& at, const int (&p)[N], int lim,
                                             unsigned (&ends)[N]) {
   const char *c[N], *lo[N], *hi[N];
-  int s[N];
+  unsigned s[N];  // (the prefixes wrap: only their differences are signed)
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     c[k] = lo[k] = hi[k] = at(k);
-    s[k] = *reinterpret_cast<const int*>(c[k]);
+    s[k] = *reinterpret_cast<const unsigned*>(c[k]);
   }
   // the farthest entries within T, h >= 0 pixels away at most
   for (int n = h; n > 0; n >>= 1) {
@@ -67,8 +67,8 @@ __device__ __forceinline__ void window_ends(int h, int T, AT&& at, const int (&p
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       const char *l = lo[k] - step, *u = hi[k] + step;
-      if (s[k] - *reinterpret_cast<const int*>(l) <= T) lo[k] = l;
-      if (*reinterpret_cast<const int*>(u) - s[k] <= T) hi[k] = u;
+      if ((int)(s[k] - *reinterpret_cast<const unsigned*>(l)) <= T) lo[k] = l;
+      if ((int)(*reinterpret_cast<const unsigned*>(u) - s[k]) <= T) hi[k] = u;
     }
   }
 #pragma unroll
