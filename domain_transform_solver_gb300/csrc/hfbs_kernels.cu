@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(64)
         for (int k = 0; k < U; ++k) {
           if (x0 + k >= xe) break;
           const int bl = lbin[lum[k]];
-          const float ct = cv[k] * tv[k];
+          const float ct = __fmul_rn(cv[k], tv[k]);  // (not fused: as k_splat_cell)
           if (bl != run) {
             flush();
             run = bl;
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(64)
             r_c = cv[k];
             r_n = 1.f;
           } else {
-            r_ct += ct;
+            r_ct = __fadd_rn(r_ct, ct);
             r_c += cv[k];
             r_n += 1.f;
           }

@@ -611,3 +611,36 @@ def test_threads_with_launches_of_other_sizes(gpu_ready, kind, sizes):
     assert not errors
     for v, a in zip(solvers, want):
         assert np.array_equal(v.Download(D.ImageType.OPTIMIZED_QUANTITY), a, equal_nan=True)
+
+
+# ---- splat: both forms add the same products in the same order ------------------
+@pytest.mark.parametrize("w,h,sx,sy", [(102, 60, 51.0, 5.0),    # 255 pixels: a thread per cell
+                                       (96, 48, 16.0, 16.0)])   # 256: a CTA per cell
+@pytest.mark.parametrize("bf16", [0, 1])
+def test_splat_sums_bit_for_bit(gpu_ready, w, h, sx, sy, bf16):
+    """Rounded products added in row-major order of a cell's runs, each run
+    first: in float32 on the host."""
+    D = gpu_ready
+    rng = np.random.default_rng(w + bf16)
+    luma = np.repeat(rng.integers(0, 256, (h, (w + 3) // 4)), 4, axis=1)[:, :w].astype(np.uint8)
+    t = rng.normal(0, 10, (h, w)).astype(np.float32)
+    c = rng.random((h, w)).astype(np.float32)
+    b = D.Batch([(w, h)], flags=D.FLAG_BF16_STORAGE if bf16 else 0)
+    b.upload(D.COLOR_SPACE.RGB, [np.repeat(luma[..., None], 4, axis=2)], [t], [c])
+    b.solve_hfbs(D.HFBSGridParams(sigma_x=sx, sigma_y=sy, sigma_l=64.0, bistoch_iter_max=1,
+                                  optim_iter_max=1))
+    if bf16:
+        t, c = P.bf16_round(t), P.bf16_round(c)
+    ct = c * t
+    gx, gy, gl = round(w / sx), round(h / sy), 4
+    want = np.zeros((2, gl, gy, gx), np.float32)
+    for y in range(gy):
+        for x in range(gx):
+            at = np.s_[int(y * sy):int((y + 1) * sy), int(x * sx):int((x + 1) * sx)]
+            bins = (luma[at] // 64).ravel()
+            starts = np.flatnonzero(np.r_[True, bins[1:] != bins[:-1]])
+            for a, e in zip(starts, np.r_[starts[1:], bins.size]):
+                for k, v in enumerate((c[at].ravel(), ct[at].ravel())):
+                    want[k, bins[a], y, x] += np.add.accumulate(v[a:e])[-1]
+    for k in (0, 1):
+        assert np.array_equal(b.debug_grid(0, 2 + k, (gx, gy, gl)), want[k])
