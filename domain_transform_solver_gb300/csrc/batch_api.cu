@@ -1363,11 +1363,7 @@ DTSGB_API int dtsgb_batch_set_tuning(dtsgb_batch_t b, int knob, long long value)
   if (knob == DTSGB_TUNE_DTS_TILE) {
     if (value != kIterTW && value != kIterSmallTW)
       return fail(DTSGB_ERR_INVALID_ARGUMENT, "DTS tile must be 64 or 32");
-    const bool small = value == kIterSmallTW;
-    if (small != b->small) {
-      b->small = small;
-      b->grad_n = -1;  // a solve before the change is not differentiated
-    }
+    b->small = value == kIterSmallTW;  // (no solve depends on it)
     return DTSGB_OK;
   }
   if (knob == DTSGB_TUNE_HFBS_GROUP_VOXELS) {

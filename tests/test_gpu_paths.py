@@ -644,3 +644,19 @@ def test_splat_sums_bit_for_bit(gpu_ready, w, h, sx, sy, bf16):
                     want[k, bins[a], y, x] += np.add.accumulate(v[a:e])[-1]
     for k in (0, 1):
         assert np.array_equal(b.debug_grid(0, 2 + k, (gx, gy, gl)), want[k])
+
+
+# ---- knobs that no solve depends on --------------------------------------------
+def test_a_solve_stays_differentiable_when_the_dts_knobs_change(gpu_ready):
+    import test_gpu_adjoint as A
+    D = gpu_ready
+    rng = np.random.default_rng(8)
+    data = [(rng.integers(0, 256, (40, 60, 4)).astype(np.uint8),
+             *(rng.standard_normal((40, 60)).astype(np.float32) for _ in range(3)))]
+    b = A._batch(D, data, dict(num_iterations=3, loss=1, lambda_=0.9, sigma_z=8.0, step_size=0.8))
+    want = b.backward([data[0][3]])
+    for knob, values in ((D.TUNE_DTS_TILE, (64, 32)), (D.TUNE_BOUNDS_SEGMENT, (4, 16))):
+        for v in values:
+            b.set_tuning(knob, v)
+            got = b.backward([data[0][3]])
+            assert all(np.array_equal(x[0], y[0]) for x, y in zip(got, want))
