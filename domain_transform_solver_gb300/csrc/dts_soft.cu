@@ -1554,6 +1554,11 @@ struct CopyPlanes {
     for (int i = 0; i < s->n; ++i) {
       float *a = s->plane(k) + s->inst[i].off, *u = const_cast<float*>(user[i]);
       const long long px = (long long)s->inst[i].w * s->inst[i].h;
+      if ((uintptr_t)u % sizeof(float)) {  // bytes at any address: not for a kernel
+        DTSGB_CUDA(cudaMemcpyAsync(in ? a : u, in ? u : a, (size_t)px * sizeof(float),
+                                   cudaMemcpyDeviceToDevice, s->stream));
+        continue;
+      }
       list.src[n] = in ? u : a;
       list.dst[n] = in ? a : u;
       list.n[n] = px;

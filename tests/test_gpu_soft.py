@@ -295,3 +295,30 @@ def test_soft_half_steps_at_the_edges_of_their_segments(gpu_ready, oracle_mod, w
     dh, dv = _gpu_edges(D, [data[0][0]])
     res = _gpu_soft(D, dh, dv, [data[0][1]], [data[0][2]], opt, [data[0][3]])
     _check_against_oracle(oracle_mod, data, dh.cpu().numpy(), dv.cpu().numpy(), opt, res)
+
+
+def test_soft_images_at_any_address(gpu_ready):
+    """Device images that start between two floats are copied all the same."""
+    import torch
+    D = gpu_ready
+    w, h, n = 37, 23, 37 * 23 * 4
+    rgba, t, c, gout = _inputs(77, w, h)
+    dh, dv = _gpu_edges(D, [rgba])
+    opt = D.DomainOptimizeParams(num_iterations=2, loss=1, sigma_z=4.0)
+    data = [dh[0].cpu().numpy(), dv[0].cpu().numpy(), t, c, gout]
+    got = []
+    for shift in (0, 1, 2, 3):
+        bufs = [torch.zeros(n + 16, dtype=torch.uint8, device="cuda") for _ in range(10)]
+        for b, a in zip(bufs, data):
+            b[shift:shift + n] = torch.from_numpy(np.ascontiguousarray(a, np.float32)
+                                                  .view(np.uint8).reshape(-1)).cuda()
+        torch.cuda.synchronize()
+        p = [[b.data_ptr() + shift] for b in bufs]
+        s = D.SoftDTS([(w, h)])
+        s.solve(p[0], p[1], p[2], p[3], opt, 1.0, p[5])
+        s.backward(p[4], p[6], p[7], p[8], p[9])
+        s.close()
+        got.append([b[shift:shift + n].cpu().numpy() for b in bufs[5:]])
+        assert all(x.any() for x in got[-1])
+    for g in got[1:]:
+        assert all(np.array_equal(x, y) for x, y in zip(g, got[0]))
