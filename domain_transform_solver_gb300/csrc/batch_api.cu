@@ -223,6 +223,14 @@ DtsGrad grad_view(dtsgb_batch_t b, int n_iter) {
 float* grad_plane_t(dtsgb_batch_t b) { return b->gplanes[b->gplanes.size() - 2]; }
 float* grad_plane_c(dtsgb_batch_t b) { return b->gplanes[b->gplanes.size() - 1]; }
 
+// Whether the caller is capturing the batch's stream (without graphs of the
+// batch's own, which a capture refuses): what is enqueued runs at a replay.
+bool callers_capture(dtsgb_batch_t b) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  return !b->use_graphs && cudaStreamIsCapturing(b->stream, &c) == cudaSuccess &&
+         c != cudaStreamCaptureStatusNone;
+}
+
 // Blocks of the passes over the whole batch for a halo.
 dim3 pass_block_totals(dtsgb_batch_t b, int halo) {
   dim3 t(0, 0);
@@ -1060,6 +1068,7 @@ DTSGB_API int dtsgb_batch_solve_dts(dtsgb_batch_t b, const dtsgb_filter_params* 
     return st;
   }
   if (iterate) b->bkey = bk;
+  if (iterate && !keep_bounds && callers_capture(b)) b->bkey.gen = ~0ull;  // not run yet
   b->dts_res = 0;
   if (b->grad) {
     b->grad_n = n_kept;
@@ -1279,6 +1288,7 @@ DTSGB_API int dtsgb_batch_solve_hfbs(dtsgb_batch_t b, const dtsgb_hfbs_params* p
     return st;
   }
   b->nkey = nk;
+  if (!B.reuse_norm && callers_capture(b)) b->nkey.gen = ~0ull;  // not run yet
   b->hfbs_done = true;
   if (b->grad) {
     b->hB = B;

@@ -420,7 +420,14 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
 DTSGB_API int dtsgb_batch_destroy(dtsgb_batch_t b);
 DTSGB_API int dtsgb_batch_set_stream(dtsgb_batch_t b, void* cuda_stream);
 /* Capture each solve as a CUDA graph on first use and replay it while the
- * parameters stay the same (default on). */
+ * parameters stay the same (default on).  Off, device uploads, solves,
+ * backwards and device downloads may be captured into a graph of the caller's
+ * (which goes before the batch).  Its DTS calls stay valid whatever is solved
+ * in between, its backwards while the gradient planes stay (num_iterations and
+ * segment), its HFBS calls until the batch solves another grid.  State kept
+ * from the guide (DTSGB_TUNE_REUSE_GUIDE_STATE) is not computed by a replay:
+ * capture the guide's upload with the solve where solves with other parameters
+ * come in between. */
 DTSGB_API int dtsgb_batch_use_graphs(dtsgb_batch_t b, int enable);
 /* Host arrays of n pointers: rgba (W*H*4 bytes each), target and confidence
  * (W*H floats each).  confidence may be NULL, or hold NULL entries: ones. */

@@ -660,3 +660,36 @@ def test_a_solve_stays_differentiable_when_the_dts_knobs_change(gpu_ready):
             b.set_tuning(knob, v)
             got = b.backward([data[0][3]])
             assert all(np.array_equal(x[0], y[0]) for x, y in zip(got, want))
+
+
+# ---- guide state that only a replay computes ------------------------------------
+@pytest.mark.parametrize("solver", ["dts", "hfbs"])
+def test_a_captured_solve_leaves_no_guide_state_behind(gpu_ready, solver):
+    """Solved at one set of parameters, captured at another and not replayed,
+    then solved at the captured one: that solve computes its own windows or
+    normalisation."""
+    import torch
+    D = gpu_ready
+    sizes = [(90, 60), (333, 140)]
+    b, stream, host, dev = _batch_on_a_stream(D, sizes)
+    ref = D.Batch(sizes)
+
+    def solve(batch, k):
+        if solver == "dts":
+            batch.solve_dts(D.DomainFilterParams(sigma_x=8.0, sigma_y=8.0, sigma_r=4.0),
+                            _dts_op(D, (30.0, 8.0)[k]))
+        else:
+            batch.solve_hfbs(D.HFBSGridParams(sigma_x=8.0, sigma_y=8.0, sigma_l=16.0,
+                                              bistoch_iter_max=(2, 20)[k], optim_iter_max=4))
+    for batch in (b, ref):
+        batch.upload(D.COLOR_SPACE.YCbCr, *host)
+    solve(b, 0)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+        solve(b, 1)
+    solve(b, 1)
+    solve(ref, 1)
+    which = 0 if solver == "dts" else 1
+    for x, y in zip(b.download(which), ref.download(which)):
+        assert np.array_equal(x, y, equal_nan=True)
