@@ -693,3 +693,32 @@ def test_a_captured_solve_leaves_no_guide_state_behind(gpu_ready, solver):
     which = 0 if solver == "dts" else 1
     for x, y in zip(b.download(which), ref.download(which)):
         assert np.array_equal(x, y, equal_nan=True)
+
+
+# ---- DTS adjoint: large gradients among small ones in a row ---------------------
+@pytest.mark.parametrize("sz", [8.0, 30.5, 70.0])
+def test_small_gradients_beside_large_ones_keep_their_bits(gpu_ready, oracle_mod, sz):
+    """A gradient of 1e7 in each row, out of reach of the columns compared: the
+    adjoint's bar there, relative to the largest of them (1e-4; a sum's
+    conversions are within (2h + 1)^2 / 2 * 2^-30 of its largest term)."""
+    import test_gpu_adjoint as A
+    D = gpu_ready
+    h, w, n = 60, 900, 2
+    rng = np.random.default_rng(int(sz))
+    y, x = np.mgrid[0:h, 0:w]
+    rgba = (rng.integers(0, 9, (h, w, 4)) + ((x // 23 + y // 17) % 3 * 70)[..., None]).astype(np.uint8)
+    t, c, g = (rng.standard_normal((h, w)).astype(np.float32),
+               rng.random((h, w)).astype(np.float32),
+               rng.standard_normal((h, w)).astype(np.float32))
+    reach = n * (int(sz) + 1) + int(sz) + 64
+    clear = slice(20 + reach, w)
+    g[:, 20] = 1e7
+    opt = dict(num_iterations=n, loss=1, lambda_=0.9, sigma_z=sz, step_size=0.8)
+    b = A._batch(D, [(rgba, t, c, g)], opt)
+    gt, gc = b.backward([g])
+    o = A._oracle(oracle_mod, rgba, t, c, A._gpu_windows(D, rgba, t, c, sz, 0))
+    rt, rc = o.backward(n, 1, 0.9, sz, 0.8, g)
+    for got, ref in ((gt[0], rt), (gc[0], rc)):
+        got, ref = got[:, clear], ref[:, clear]
+        assert 0.1 < np.abs(ref).max() < 100
+        assert np.abs(got - ref).max() <= 1e-4 * np.abs(ref).max()
