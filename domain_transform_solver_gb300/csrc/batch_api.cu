@@ -53,7 +53,6 @@ struct dtsgb_batch_s {
   int ref_y = 1;
   std::vector<Inst> inst;
   long long total = 0;
-  int max_w = 0, max_h = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   uchar4* guide = nullptr;
@@ -62,7 +61,6 @@ struct dtsgb_batch_s {
   uint32_t* bounds = nullptr;
   float* v[2] = {nullptr, nullptr};
   float* hout = nullptr;
-  float* scratch = nullptr;
   // host uploads: every image is copied whole (one contiguous copy per
   // plane) into a dense staging area, then one kernel writes the pitched
   // planes; soff[i] = pixels of the instances before i
@@ -170,7 +168,6 @@ void batch_free(dtsgb_batch_t b) {
   dfree(b->v[0]);
   dfree(b->v[1]);
   dfree(b->hout);
-  dfree(b->scratch);
   dfree(b->d_inst);
   for (Tile*& p : b->pass_mem) dfree(p);
   dfree(b->d_hinst);
@@ -327,20 +324,6 @@ int run_graph(dtsgb_batch_t b, Graph& g, std::vector<char> key, F enqueue) {
   }
   g.key = key;
   DTSGB_CUDA(cudaGraphLaunch(g.exec, b->stream));
-  return DTSGB_OK;
-}
-
-int upload_plane(dtsgb_batch_t b, int i, const float* src, void* dst,
-                 cudaMemcpyKind kind) {
-  const Inst& I = b->inst[i];
-  const size_t wb = (size_t)I.w * 4;
-  if (b->st == Storage::F32) {
-    DTSGB_CUDA(cudaMemcpy2DAsync((float*)dst + I.off, (size_t)I.pitch * 4, src, wb,
-                                 wb, I.h, kind, b->stream));
-  } else {
-    DTSGB_CUDA(cudaMemcpy2DAsync(b->scratch + I.off, (size_t)I.pitch * 4, src, wb,
-                                 wb, I.h, kind, b->stream));
-  }
   return DTSGB_OK;
 }
 
@@ -687,40 +670,7 @@ int batch_upload_targets(dtsgb_batch_t b, const float* const* target,
                          bool sync_host = true) {
   if (kind == cudaMemcpyHostToDevice)
     return host_ingest(b, DTSGB_RGB, nullptr, target, conf, sync_host);
-  if (kind == cudaMemcpyDeviceToDevice) return device_ingest(b, DTSGB_RGB, nullptr, target, conf);
-  int st;
-  for (int i = 0; i < b->n; ++i)
-    if ((st = upload_plane(b, i, target[i], b->target, kind))) return st;
-  if (b->st == Storage::BF16 &&
-      (st = launch_storage_from_float(nullptr, 0, b->st, b->scratch, b->target,
-                                      b->total, b->stream)))
-    return st;
-  // confidence (missing -> ones)
-  for (int i = 0; i < b->n; ++i) {
-    const Inst& I = b->inst[i];
-    if (conf && conf[i]) {
-      if ((st = upload_plane(b, i, conf[i], b->conf, kind))) return st;
-    } else if (b->st == Storage::F32) {
-      if ((st = launch_fill_storage(Storage::F32, (float*)b->conf + I.off,
-                                    (long long)I.pitch * I.h, 1.f, b->stream)))
-        return st;
-    } else {
-      if ((st = launch_fill_storage(Storage::F32, b->scratch + I.off,
-                                    (long long)I.pitch * I.h, 1.f, b->stream)))
-        return st;
-    }
-  }
-  if (b->st == Storage::BF16 &&
-      (st = launch_storage_from_float(nullptr, 0, b->st, b->scratch, b->conf,
-                                      b->total, b->stream)))
-    return st;
-  b->dts_res = -1;
-  b->grad_n = -1;
-  b->hfbs_done = false;
-  b->hgrad_ready = false;
-  if (kind == cudaMemcpyHostToDevice && sync_host)
-    DTSGB_CUDA(cudaStreamSynchronize(b->stream));
-  return DTSGB_OK;
+  return device_ingest(b, DTSGB_RGB, nullptr, target, conf);
 }
 
 int batch_upload(dtsgb_batch_t b, int cs, const void* const* rgba,
@@ -734,17 +684,7 @@ int batch_upload(dtsgb_batch_t b, int cs, const void* const* rgba,
       return fail(DTSGB_ERR_INVALID_ARGUMENT, "null image pointer");
   if (kind == cudaMemcpyHostToDevice)
     return host_ingest(b, cs, rgba, target, conf, sync_host);
-  if (kind == cudaMemcpyDeviceToDevice) return device_ingest(b, cs, rgba, target, conf);
-  for (int i = 0; i < b->n; ++i) {
-    const Inst& I = b->inst[i];
-    const size_t wb = (size_t)I.w * 4;
-    DTSGB_CUDA(cudaMemcpy2DAsync(b->guide + I.off, (size_t)I.pitch * 4, rgba[i], wb,
-                                 wb, I.h, kind, b->stream));
-  }
-  int st = launch_color_convert_flat(b->guide, b->total, cs, b->stream);
-  if (st) return st;
-  ++b->guide_gen;
-  return batch_upload_targets(b, target, conf, kind, sync_host);
+  return device_ingest(b, cs, rgba, target, conf);
 }
 
 // The HFBS gradient arena for K heavy-ball steps over tv voxels (the choice
@@ -870,8 +810,6 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
     b->soff.push_back(b->dense);
     b->dense += (long long)widths[i] * heights[i];
     off += (long long)I.pitch * I.h;
-    b->max_w = std::max(b->max_w, I.w);
-    b->max_h = std::max(b->max_h, I.h);
   }
   b->total = off;
   int st = DTSGB_OK;
@@ -889,7 +827,6 @@ DTSGB_API int dtsgb_batch_create(int n, const int* widths, const int* heights,
   if (!st) st = dalloc(&b->v[0], T);
   if (!st) st = dalloc(&b->v[1], T);
   if (!st) st = dalloc(&b->hout, T);
-  if (!st && b->st == Storage::BF16) st = dalloc(&b->scratch, T);
   if (!st) st = dalloc(&b->d_inst, (size_t)n);
   if (!st) st = dalloc(&b->d_hinst, (size_t)n);
   if (!st) st = dalloc(&b->d_soff, (size_t)n);
@@ -1425,11 +1362,6 @@ DTSGB_API int dtsgb_batch_get_tuning(dtsgb_batch_t b, int knob, long long* value
   }
   return fail(DTSGB_ERR_INVALID_ARGUMENT, "unknown tuning knob");
 }
-
-
-}  // extern "C"
-
-extern "C" {
 
 DTSGB_API int dtsgb_batch_autotune(dtsgb_batch_t b, const dtsgb_filter_params* f,
                                    const dtsgb_optimize_params* p, float overwrite,

@@ -36,7 +36,9 @@ namespace {
 
 constexpr int kT = 256;
 constexpr int kAdjFirst = 1, kAdjLast = 2;
-// Halos above this are refused.
+// Halos above this are refused: the form before had to keep a tile and its
+// halos in shared memory, and what it refused stays so (X^T is instantiated for
+// up to kRoundsX rounds, which halos up to 127 need at most).
 constexpr int kAdjMaxHalo = 76;
 
 // Y^T: gout = (1 - slam) gin + slam * By^T gin.  A block per 32 columns x th
@@ -141,7 +143,7 @@ __global__ void __launch_bounds__(RM == 32 ? 768 : 512, RM == 8 ? 3 : RM == 16 ?
 // gout).  The five planes of a round are loaded when the round is due: loads a
 // round ahead held 124 registers, four blocks an SM (115 us against 90).
 template <typename TS, int MODE, int NR>
-__global__ void __launch_bounds__(32 * kXWarps, NR <= 4 ? 7 : 4)
+__global__ void __launch_bounds__(32 * kXWarps, 7)
     k_adj_x(const Inst* __restrict__ insts, const float* __restrict__ g1p,
             float* __restrict__ gout, const float* __restrict__ vk, const TS* __restrict__ tgt,
             const TS* __restrict__ cnf, const uint32_t* __restrict__ bnd,
@@ -415,8 +417,7 @@ int launch_adj_t(const DtsLaunch& L, float* g, float* g1, const float* vk, const
   };
   if (G.rounds <= 2) return x(k_adj_x<TS, MODE, 2>, 2, XPrefix<2>::QS);
   if (G.rounds <= 3) return x(k_adj_x<TS, MODE, 3>, 3, XPrefix<3>::QS);
-  if (G.rounds <= kRoundsX) return x(k_adj_x<TS, MODE, kRoundsX>, kRoundsX, XPrefix<kRoundsX>::QS);
-  return x(k_adj_x<TS, MODE, kRoundsWide>, kRoundsWide, XPrefix<kRoundsWide>::QS);
+  return x(k_adj_x<TS, MODE, kRoundsX>, kRoundsX, XPrefix<kRoundsX>::QS);
 }
 
 // One iteration's adjoint of g, in place (g1: scratch).

@@ -999,7 +999,6 @@ __global__ void __launch_bounds__(256)
   const int len = AXIS == 0 ? kTX * PX : kTYR;
   const TileGeom<AXIS> G(I, len);
   const int TL = len + 2 * halo, TS = AXIS == 0 ? TL : TL * kTYC;
-  const int nf = data ? 6 : 4;
   float* F[6] = {smf, smf + TS, smf + 2 * TS, smf + 3 * TS, smf + 4 * TS, smf + 5 * TS};
   const float* srcs[6] = {a, nplan, Bk, val, t, c};
   for (int tile = blockIdx.x; tile < G.n0 * G.n1; tile += gridDim.x) {

@@ -247,8 +247,6 @@ inline bool use_small_iter_tiles(long long tiles_big) {
   return tiles_big * kIterTW * kIterTH < 4LL * 152 * 64 * 64;
 }
 
-int launch_color_convert(const Inst* h_inst, const Inst* d_inst, int n_inst,
-                         uchar4* guide, int color_space, cudaStream_t s);
 // in-place conversion over a flat run of n pixels (ignores pitch padding)
 int launch_color_convert_flat(uchar4* guide, long long n, int color_space,
                               cudaStream_t s);

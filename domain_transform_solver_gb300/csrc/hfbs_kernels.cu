@@ -440,9 +440,7 @@ __global__ void k_laplace(const HInst* __restrict__ insts, int axis,
   int len, na, nlines;
   long long stride;
   const int px = I.px;
-  if (axis == 0) {
-    len = gx; stride = 1; na = gy; nlines = gy * gl;
-  } else if (axis == 1) {
+  if (axis == 1) {
     len = gy; stride = px; na = gx; nlines = gx * gl;
   } else {
     len = gl; stride = (long long)px * gy; na = gx; nlines = gx * gy;
@@ -451,8 +449,7 @@ __global__ void k_laplace(const HInst* __restrict__ insts, int axis,
        line += gridDim.x * blockDim.x) {
     const int a = line % na, bb = line / na;
     long long base;
-    if (axis == 0) base = ((long long)bb * gy + a) * px;
-    else if (axis == 1) base = (long long)bb * px * gy + a;
+    if (axis == 1) base = (long long)bb * px * gy + a;
     else base = (long long)bb * px + a;
     base += I.grid_off;
     {
