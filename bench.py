@@ -54,8 +54,8 @@ KERNEL_NAMES = {0: "k_bounds_x + k_bounds_y", 1: "k_dts_x + k_dts_y", 2: "k_filt
                 9: "k_adj_y + k_adj_x",
                 10: "hfbs adjoint (whole backward)",
                 11: "soft-window plans, line scans and other",
-                12: "k_soft_half_plan X", 13: "k_soft_adjoint_fused X",
-                14: "k_soft_adjoint_fused Y", 15: "k_soft_half_plan Y"}
+                12: "k_soft_half_x", 13: "k_soft_adjoint_fused X",
+                14: "k_soft_adjoint_fused Y", 15: "k_soft_half_y"}
 HFBS_TB_STEPS = 4  # heavy-ball steps per pass of the march over a grid
 
 

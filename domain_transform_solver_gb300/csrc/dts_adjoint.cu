@@ -17,8 +17,8 @@
 // Y^T and X^T are a pass each, cut like the forward's (dts_geom.cuh).  In one
 // kernel, 64 x 128 tiles with their halos in shared memory, an iteration took
 // 216 us for 16 images of 1024x768 (456 instructions a pixel, two blocks an SM);
-// the two passes take 142 (52 and 90), bound by the latency of their loads and by
-// HBM3e (12 and 40 B/px).
+// the two passes take 146 (52 and 94), bound by issue slots and the latency of their
+// loads (12 and 40 B/px).
 //
 // The forward iterates the adjoint needs (the X-step inputs v_k) are
 // recomputed segment by segment from checkpoints v_0 = t, v_K, v_2K, ...

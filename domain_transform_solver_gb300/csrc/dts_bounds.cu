@@ -20,8 +20,8 @@
 // found by a binary search over the radius in the prefix, four pixels at a
 // time: the steps are the same for every lane, where two pointers that advance
 // along a segment made a warp wait for its longest advance at every pixel.
-// Bound by issue slots (540 instructions a pixel in tiles with two pointers,
-// about 190 here at radius 9).
+// Bound by issue slots (540 instructions a pixel in tiles with two pointers;
+// here 160 and 162 at radius 9, 86% and 81% of the slots busy).
 #include <algorithm>
 #include <cmath>
 

@@ -6,8 +6,9 @@
 // (sqrt(1 + nonnegative)), so a window of the reference's linear search
 // (src/domain_transform_filter.cuh:7-28) never reaches further than
 // floor(sigma)+1 pixels from its centre.  Every pass is therefore a
-// bounded-radius stencil over a tile plus halo held in shared memory: no
-// global prefix sums, no transposes, no long-row cancellation.
+// bounded-radius stencil (here over tiles plus halo in shared memory, in
+// dts_passes.cu over segments of a row or strips of columns): no global prefix
+// sums, no transposes, no long-row cancellation.
 #include <algorithm>
 #include <cmath>
 

@@ -20,8 +20,8 @@
 // 15.5; 3264x2448 with 30 and overwrite: 147 -> 86; 64 ragged BF16 images (47
 // Mpx) with 8: 366 -> 316; 160x120: 6.7 -> 5.8.
 //
-// Bound by issue slots and latency, half and half (X: 78 instructions a pixel,
-// 56% of the slots busy, 4.8 TB/s; Y: 66, 50%, 2.7 TB/s at 12.6 Mpx): loads come
+// Bound by issue slots and latency, half and half (X: 73 instructions a pixel,
+// 58% of the slots busy, 45 us; Y: 66, 60%, 39 us at 12.6 Mpx): loads come
 // first in a warp and the arithmetic after, and the other warps of an SM fill
 // the gap only in part.
 #include <algorithm>

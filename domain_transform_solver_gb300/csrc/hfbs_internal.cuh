@@ -179,8 +179,8 @@ struct HfbsBatch {
   // optional debug copies (single-instance class API)
   bool keep_debug;
   float* dbg_z_init;  // a copy of the first iterate (keep_debug)
-  // non-null: record the forward iterates for hfbs_enqueue_backward (the
-  // one-step heavy-ball kernel, all instances as one group)
+  // non-null: record the forward iterates for hfbs_enqueue_backward (all
+  // instances as one group)
   const HfbsGradState* grad = nullptr;
 };
 
