@@ -504,7 +504,7 @@ def test_a_solve_at_a_new_sigma_waits_for_nothing(gpu_ready):
         for sigma in (8.0, 30.0, 64.0, 8.0):
             if not warm:
                 with torch.cuda.stream(stream):
-                    torch.cuda._sleep(200_000_000)  # 0.1 s
+                    torch.cuda._sleep(500_000_000)  # a quarter of a second
                     done = stream.record_event()
             b.solve_dts(fp, _dts_op(D, sigma))
             if not warm:
