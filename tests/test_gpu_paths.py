@@ -696,14 +696,15 @@ def test_a_captured_solve_leaves_no_guide_state_behind(gpu_ready, solver):
 
 
 # ---- DTS adjoint: large gradients among small ones in a row ---------------------
-@pytest.mark.parametrize("sz", [8.0, 30.5, 70.0])
-def test_small_gradients_beside_large_ones_keep_their_bits(gpu_ready, oracle_mod, sz):
+@pytest.mark.parametrize("h,sz", [(60, 8.0), (60, 30.5), (60, 70.0),  # 2 and 4 rounds a segment
+                                  (200, 8.0), (600, 8.0)])            # 3 and 4
+def test_small_gradients_beside_large_ones_keep_their_bits(gpu_ready, oracle_mod, h, sz):
     """A gradient of 1e7 in each row, out of reach of the columns compared: the
     adjoint's bar there, relative to the largest of them (1e-4; a sum's
     conversions are within (2h + 1)^2 / 2 * 2^-30 of its largest term)."""
     import test_gpu_adjoint as A
     D = gpu_ready
-    h, w, n = 60, 900, 2
+    w, n = 900, 2
     rng = np.random.default_rng(int(sz))
     y, x = np.mgrid[0:h, 0:w]
     rgba = (rng.integers(0, 9, (h, w, 4)) + ((x // 23 + y // 17) % 3 * 70)[..., None]).astype(np.uint8)
